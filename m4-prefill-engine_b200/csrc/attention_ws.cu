@@ -1,0 +1,632 @@
+// Causal attention on tensor memory, head dim 64 and 128, any group size up to 128, the key range split where that fills
+// the GPU.
+//
+//   Q [Hq][M][D] fp16, K and V [Hkv][Mkv][D] fp16 (a Q8_0 cache is expanded once per call by dequant_q8_0_kernel; value =
+//   fp16(q * d), the rounding of the reference's dequantize_q8_0), O [M][Hq*D] or [Hq][M][D] fp16.  Query row i sits at
+//   position pos0 + i and attends keys 0 .. pos0 + i (brick4_attn_kernels.metal:573-911, unified_8b_kernels.metal:857-998).
+//
+// One CTA = one kv head x two query tiles of 128 rows; a tile packs BP = 128 / G neighbouring positions of the G query
+// heads that share the kv head (row r = head r / BP, position r % BP), so that one decode token still fills G rows and no
+// K or V tile is fetched twice for the same positions.
+//
+//   warps 0-3, 4-7   softmax of tile 0 / tile 1: thread = query row = tensor-memory lane.  Scores come out of tensor
+//                    memory, P = 2^(s - m) goes back as fp16 over the front half of the same columns, from where
+//                    tcgen05.mma takes it as its A operand: P never passes through shared memory, a row's maximum and sum
+//                    need no shuffle, no exchange and no CTA barrier.
+//   warp 8           issues every MMA: O0 += P0.V(kt), S0 = Q0.K(kt+1)^T, O1 += P1.V(kt), S1 = Q1.K(kt+1)^T.  While one
+//                    tile's MMAs run the other tile's softmax has the exponential unit to itself.
+//   warp 9           TMA: the Q tiles, then K(kt), V(kt), K(kt+1), ... through one ring of slots.
+//
+//   tensor memory    S0 / P0 columns 0..127, S1 / P1 128..255, O0 and O1 behind them (2 D columns).  S(kt+1) may overwrite
+//                    P(kt) because MMAs of one thread run in the order they are issued; the completion of S(kt+1) that a
+//                    softmax warp waits for therefore also covers PV(kt), so O is stable whenever that warp rescales it.
+//
+// Every mbarrier wait is bounded; on expiry the CTA records a code, stops issuing work, lets its copies land and leaves.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <cstring>
+
+#include "attention_ws.cuh"
+#include "bridge_state.cuh"
+#include "ptx.cuh"
+
+namespace attn {
+namespace ws {
+
+constexpr int ROWS = 128, BK = 128;                      // query rows of a tile, keys of a step
+constexpr int SOFTMAX_THREADS = 256, THREADS = SOFTMAX_THREADS + 64;
+constexpr int ATOM = 128 * 128;                          // bytes of [128 rows][64 fp16] in the 128-byte-swizzled layout
+constexpr int MAX_SPLITS = 32;
+
+template <int D> struct Cfg {
+    static constexpr int ATOMS = D / 64;
+    static constexpr int TILE = ATOMS * ATOM;
+    static constexpr int SLOTS = D == 128 ? 5 : 6;       // K and V tiles in flight
+    static constexpr size_t USED = 1024 + (size_t)(2 + SLOTS) * TILE + 256;
+    // At least 160 KB: the CTA holds all 512 tensor-memory columns, so no CTA of a neighbouring kernel that also holds some
+    // (the projection kernels, 80 KB and more) may share its SM.
+    static constexpr size_t SMEM = USED < 160 * 1024 ? 160 * 1024 : USED;
+};
+
+struct Params {
+    __half* O;
+    float* part_o;               // [split][Hq * M][D], unnormalised (split launches)
+    float2* part_ml;             // [split][Hq * M]: reference maximum (log2 domain), sum
+    uint32_t Hq, M, Mkv, pos0, G, BP, tiles_per_split;
+    float scale_log2e;
+    int out_tokens_major, split;
+    int* err;
+};
+
+// key tiles that the rows at positions [p, p + BP) of this call attend
+__device__ __forceinline__ uint32_t key_tiles(uint32_t p, uint32_t BP, uint32_t M, uint32_t Mkv, uint32_t pos0) {
+    if (p >= M) return 0u;
+    return min(pos0 + min(p + BP, M) - 1u, Mkv - 1u) / (uint32_t)BK + 1u;
+}
+
+__device__ __forceinline__ float ex2(float x) {           // 2^x, one instruction on the special-function unit; ex2(-inf) = 0
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// two fp32 values per instruction
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// 2^x of two values without the special-function unit: x = n + f with n the nearest integer (in the low mantissa bits of
+// x + 1.5 * 2^23) and |f| <= 1/2, 2^f as the degree-5 Taylor polynomial (relative error 3e-6, far below the fp16 rounding of
+// the probabilities), n added to the exponent field.  Inputs below -120 (masked scores are -inf) give 2^-120; a NaN stays
+// non-finite (the maximum propagates it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float y;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
+}
+__device__ __forceinline__ void ex2_poly2(float x0, float x1, float& e0, float& e1) {
+    const uint64_t x = pack2(max_nan(x0, -120.0f), max_nan(x1, -120.0f));
+    const uint64_t r = add2(x, pack2(12582912.0f, 12582912.0f));
+    const uint64_t n = add2(r, pack2(-12582912.0f, -12582912.0f));
+    const uint64_t f = fma2(n, pack2(-1.0f, -1.0f), x);
+    uint64_t p = pack2(1.3333558146e-3f, 1.3333558146e-3f);
+    p = fma2(p, f, pack2(9.6181291076e-3f, 9.6181291076e-3f));
+    p = fma2(p, f, pack2(5.5504108665e-2f, 5.5504108665e-2f));
+    p = fma2(p, f, pack2(2.4022650696e-1f, 2.4022650696e-1f));
+    p = fma2(p, f, pack2(6.9314718056e-1f, 6.9314718056e-1f));
+    p = fma2(p, f, pack2(1.0f, 1.0f));
+    float p0, p1, r0, r1;
+    unpack2(p, p0, p1);
+    unpack2(r, r0, r1);
+    e0 = __int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23));
+    e1 = __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23));
+}
+#ifndef ATTN_POLY
+#define ATTN_POLY ((1 << 1) | (1 << 4) | (1 << 6))
+#endif
+__device__ constexpr bool poly_pair(int j) { return (ATTN_POLY >> (j & 7)) & 1; }
+
+__device__ __forceinline__ void tmem_ld_x32(uint32_t taddr, float* r) {
+    uint32_t v[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; i++) r[i] = __uint_as_float(v[i]);
+}
+__device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+          "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+          "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem desc]: fp16 operands, fp32 accumulate, A rows = lanes, two consecutive k per column
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+template <int D>
+__global__ void __launch_bounds__(THREADS, 1)
+attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+               const Params p) {
+    using C = Cfg<D>;
+    extern __shared__ uint8_t smem_raw_[];
+    uint8_t* sQ = smem_raw_ + ((1024u - (ptx::smem_u32(smem_raw_) & 1023u)) & 1023u);    // [2 tiles]
+    uint8_t* sKV = sQ + 2 * C::TILE;                                                      // [SLOTS]
+    uint64_t* q_full = reinterpret_cast<uint64_t*>(sKV + C::SLOTS * C::TILE);             // [2] query tile landed
+    uint64_t* s_full = q_full + 2;                        // [2] scores of the step complete (and with them the PV before it)
+    uint64_t* p_full = s_full + 2;                        // [2] probabilities written, O rescaled: one arrival per softmax warp
+    uint64_t* o_full = p_full + 2;                        // [2] last PV of the tile complete
+    uint64_t* kv_full = o_full + 2;                       // [SLOTS]
+    uint64_t* kv_empty = kv_full + C::SLOTS;              // [SLOTS]
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(kv_empty + C::SLOTS);
+    volatile uint32_t* abort_flag = tmem_holder + 1;
+
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // kv heads along x, position blocks along y, latest (longest) block first; splits of the key range along z
+    const uint32_t hk = blockIdx.x;
+    const uint32_t p0 = (gridDim.y - 1u - blockIdx.y) * 2u * p.BP;
+    const uint32_t t0 = blockIdx.z * p.tiles_per_split;
+    // steps of tile g inside this split
+    auto steps_of = [&](uint32_t g) {
+        const uint32_t n = key_tiles(p0 + g * p.BP, p.BP, p.M, p.Mkv, p.pos0);
+        return n > t0 ? min(n - t0, p.tiles_per_split) : 0u;
+    };
+    const uint32_t cnt0 = steps_of(0u), cnt1 = steps_of(1u);
+    const uint32_t n_steps = max(cnt0, cnt1);
+    if (n_steps == 0u) return;                            // this split lies behind the block's last key tile
+
+    if (tid == SOFTMAX_THREADS + 32) {
+        for (int i = 0; i < 2; i++) { ptx::mbar_init(&q_full[i], 1); ptx::mbar_init(&s_full[i], 1); ptx::mbar_init(&p_full[i], 4); ptx::mbar_init(&o_full[i], 1); }
+        for (int i = 0; i < C::SLOTS; i++) { ptx::mbar_init(&kv_full[i], 1); ptx::mbar_init(&kv_empty[i], 1); }
+        *abort_flag = 0u;
+        ptx::fence_barrier_init();
+        ptx::prefetch_tensormap(&tmQ); ptx::prefetch_tensormap(&tmK); ptx::prefetch_tensormap(&tmV);
+    }
+    __syncwarp();
+    if (warp == 8) { ptx::tmem_alloc(tmem_holder, 512); ptx::tmem_relinquish(); }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    ptx::tc_fence_after_sync();
+    const uint32_t tmem = *tmem_holder;
+    const uint32_t tO = tmem + 256u;
+    // everything above touched only this CTA's shared and tensor memory; global memory is first touched below
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+
+    if (warp == 9) {
+        // ---------------- copies ----------------
+        if (lane == 0) {
+            const uint32_t q_bytes = p.BP * p.G * 128u * (uint32_t)C::ATOMS;     // rows BP * G .. 127 of a tile stay unwritten: no output reads them
+            for (uint32_t g = 0; g < 2u; g++) {
+                if ((g ? cnt1 : cnt0) == 0u) continue;
+                ptx::mbar_arrive_expect_tx(&q_full[g], q_bytes);
+                for (int a = 0; a < C::ATOMS; a++)
+                    ptx::tma_load_3d(sQ + g * C::TILE + a * ATOM, &tmQ, &q_full[g], a * 64, (int)(p0 + g * p.BP), (int)(hk * p.G));
+            }
+        }
+        __syncwarp();
+        uint32_t slot = 0, ph = 0;
+        bool ok = true;
+        for (uint32_t i = 0; ok && i < 2u * n_steps; i++) {
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&kv_empty[slot], ph ^ 1u, abort_flag, p.err, 220));
+            if (!ok) break;
+            if (lane == 0) {
+                const CUtensorMap* map = (i & 1u) ? &tmV : &tmK;
+                ptx::mbar_arrive_expect_tx(&kv_full[slot], C::TILE);
+                for (int a = 0; a < C::ATOMS; a++)
+                    ptx::tma_load_3d(sKV + slot * C::TILE + a * ATOM, map, &kv_full[slot], a * 64, (int)((t0 + (i >> 1)) * BK), (int)hk);
+            }
+            __syncwarp();
+            if (++slot == (uint32_t)C::SLOTS) { slot = 0; ph ^= 1u; }
+        }
+    } else if (warp == 8) {
+        // ---------------- MMAs ----------------
+        const uint32_t idesc_s = ptx::umma_idesc_f16(128, 128);
+        const uint32_t idesc_pv = ptx::umma_idesc_f16(128, D) | (1u << 16);       // B (= V) MN-major
+        const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
+        // V [key][d]: the 64 d of an atom row are the contiguous run, the second atom lies ATOM bytes further (leading byte
+        // offset), groups of eight keys are 1024 bytes apart (stride byte offset); 16 keys further = 2048 bytes
+        const uint64_t vdesc_hi = ((uint64_t)(ATOM >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+        const uint32_t q_lo = (ptx::smem_u32(sQ) & 0x3FFFFu) >> 4, kv_lo = (ptx::smem_u32(sKV) & 0x3FFFFu) >> 4;
+        auto issue_s = [&](uint32_t g, uint32_t slot) {
+            const uint64_t qd = desc_hi | (uint64_t)(q_lo + g * (C::TILE >> 4)), kd = desc_hi | (uint64_t)(kv_lo + slot * (C::TILE >> 4));
+#pragma unroll
+            for (int a = 0; a < C::ATOMS; a++)
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++)
+                    ptx::umma_f16_ss(tmem + g * 128u, qd + a * (ATOM >> 4) + 2 * kk, kd + a * (ATOM >> 4) + 2 * kk, idesc_s, (uint32_t)(a | kk) != 0u);
+            ptx::umma_commit(&s_full[g]);
+        };
+        auto issue_pv = [&](uint32_t g, uint32_t slot, bool first) {
+            const uint64_t vd = vdesc_hi | (uint64_t)(kv_lo + slot * (C::TILE >> 4));
+#pragma unroll
+            for (int s = 0; s < BK / 16; s++)
+                umma_f16_ts(tO + g * (uint32_t)D, tmem + g * 128u + s * 8u, vd + s * (2048 >> 4), idesc_pv, (first ? 0u : 1u) | (uint32_t)(s != 0));
+        };
+        uint32_t slot = 0, ph = 0;                        // next slot of the ring to be consumed, and its parity
+        auto next_slot = [&]() { if (++slot == (uint32_t)C::SLOTS) { slot = 0; ph ^= 1u; } };
+        auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+            const bool r = __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag, p.err, code));
+            ptx::tc_fence_after_sync();
+            return r;
+        };
+        bool ok = wait(&kv_full[0], 0u, 221);
+        for (uint32_t g = 0; g < 2u && ok; g++) {
+            if ((g ? cnt1 : cnt0) == 0u) continue;
+            ok = wait(&q_full[g], 0u, 222);
+            if (ok && ptx::elect_one()) issue_s(g, 0u);
+            __syncwarp();
+        }
+        if (ok && ptx::elect_one()) ptx::umma_commit(&kv_empty[0]);
+        __syncwarp();
+        next_slot();
+        for (uint32_t it = 0; ok && it < n_steps; it++) {
+            const uint32_t v_slot = slot, v_ph = ph;
+            next_slot();
+            const uint32_t k_slot = slot, k_ph = ph;      // K of the next step
+            const bool more = it + 1u < n_steps;
+            if (more) next_slot();
+            ok = wait(&kv_full[v_slot], v_ph, 223);
+#pragma unroll
+            for (uint32_t g = 0; g < 2u; g++) {
+                const uint32_t cnt = g ? cnt1 : cnt0;
+                if (ok && it < cnt) {
+                    ok = wait(&p_full[g], it & 1u, 224);
+                    if (ok && ptx::elect_one()) {
+                        issue_pv(g, v_slot, it == 0u);
+                        if (it + 1u == cnt) ptx::umma_commit(&o_full[g]);
+                    }
+                    __syncwarp();
+                }
+                if (g == 1u && ok && ptx::elect_one()) ptx::umma_commit(&kv_empty[v_slot]);
+                __syncwarp();
+                if (ok && it + 1u < cnt) {
+                    ok = wait(&kv_full[k_slot], k_ph, 225);
+                    if (ok && ptx::elect_one()) issue_s(g, k_slot);
+                    __syncwarp();
+                }
+            }
+            if (more && ok && ptx::elect_one()) ptx::umma_commit(&kv_empty[k_slot]);
+            __syncwarp();
+        }
+    } else {
+        // ---------------- softmax ----------------
+        const uint32_t g = warp >> 2;
+        const uint32_t cnt = g ? cnt1 : cnt0;
+        const uint32_t row = tid & 127u, hl = row / p.BP, pl = row - hl * p.BP;
+        const uint32_t pos_first = p0 + g * p.BP, pos = pos_first + pl;
+        const uint32_t last_key = min(p.pos0 + pos, p.Mkv - 1u);
+        const uint32_t lane_addr = ((warp & 3u) * 32u) << 16;
+        const uint32_t tS = tmem + lane_addr + g * 128u, tOg = tO + lane_addr + g * (uint32_t)D;
+        // tiles whose keys all lie at or below every row's position (and inside the cache) need no mask
+        const uint32_t free_keys = min(p.pos0 + pos_first + 1u, p.Mkv);
+        float m_run = -1e30f, l_run = 0.0f;
+        bool ok = true;
+        for (uint32_t it = 0; it < cnt; it++) {
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&s_full[g], it & 1u, abort_flag, p.err, 226));
+            if (!ok) break;
+            ptx::tc_fence_after_sync();
+            const uint32_t k0 = (t0 + it) * BK;
+            float sc[BK];
+#pragma unroll
+            for (int c = 0; c < BK; c += 32) tmem_ld_x32(tS + c, sc + c);
+            ptx::tmem_ld_wait();
+            if (k0 + BK > free_keys) {
+#pragma unroll
+                for (int j = 0; j < BK; j++) if (k0 + j > last_key) sc[j] = -INFINITY;
+            }
+            float mx = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < BK; j += 4) {
+                mx = fmaxf(fmaxf(mx, sc[j]), sc[j + 1]);
+                mx1 = fmaxf(fmaxf(mx1, sc[j + 2]), sc[j + 3]);
+            }
+            mx = fmaxf(mx, mx1) * p.scale_log2e;          // the scale is positive: max and scaling commute
+            // The reference maximum moves only for jumps above 2^8: probabilities are then at most 256 instead of 1, which fp16
+            // and the fp32 sums hold just as well, the division by the row sum removes the common factor, and O is rescaled
+            // hardly ever after the first step.
+            float corr = 1.0f;
+            if (mx > m_run + 8.0f) { corr = ex2(m_run - mx); m_run = mx; }
+            if (it > 0u && __any_sync(0xffffffffu, corr != 1.0f)) {
+#pragma unroll
+                for (int c = 0; c < D; c += 16) {
+                    uint32_t v[16];
+                    ptx::tmem_ld_x16(tOg + c, v);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
+                    ptx::tmem_st_x16(tOg + c, v);
+                }
+            }
+            const uint64_t sc2 = pack2(p.scale_log2e, p.scale_log2e), nm2 = pack2(-m_run, -m_run);
+            uint64_t rs0 = 0ull, rs1 = 0ull;              // two zeros each
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                uint32_t pk[32];
+#pragma unroll
+                for (int j = 0; j < 32; j++) {
+                    const int e = h * 64 + 2 * j;
+                    float x0, x1, e0, e1;
+                    unpack2(fma2(pack2(sc[e], sc[e + 1]), sc2, nm2), x0, x1);     // masked: -inf stays -inf, 2^-inf = 0
+                    if (poly_pair(j)) ex2_poly2(x0, x1, e0, e1);
+                    else { e0 = ex2(x0); e1 = ex2(x1); }
+                    if (j & 1) rs1 = add2(rs1, pack2(e0, e1)); else rs0 = add2(rs0, pack2(e0, e1));
+                    pk[j] = pack_h2(e0, e1);
+                }
+                tmem_st_x32(tS + h * 32, pk);
+            }
+            ptx::tmem_st_wait();
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&p_full[g]);
+            float a0, a1;
+            unpack2(add2(rs0, rs1), a0, a1);
+            l_run = l_run * corr + (a0 + a1);
+        }
+        // ---------------- result ----------------
+        if (cnt > 0u && ok) ok = __all_sync(0xffffffffu, ptx::mbar_wait<64>(&o_full[g], 0u, abort_flag, p.err, 227));
+        if (cnt > 0u && ok) {
+            ptx::tc_fence_after_sync();
+            const uint32_t head = hk * p.G + hl;
+            const bool row_ok = hl < p.G && pos < p.M;
+            if (p.split) {
+                const size_t r = (size_t)blockIdx.z * p.Hq * p.M + (size_t)head * p.M + pos;
+                float* dst = p.part_o + r * D;
+                if (row_ok) p.part_ml[r] = make_float2(m_run, l_run);
+#pragma unroll
+                for (int c = 0; c < D; c += 32) {
+                    float v[32];
+                    tmem_ld_x32(tOg + c, v);
+                    ptx::tmem_ld_wait();
+                    if (row_ok) {
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    }
+                }
+            } else {
+                const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
+                __half* dst = p.out_tokens_major ? p.O + ((size_t)pos * p.Hq + head) * D : p.O + ((size_t)head * p.M + pos) * D;
+#pragma unroll
+                for (int c = 0; c < D; c += 32) {
+                    float v[32];
+                    tmem_ld_x32(tOg + c, v);
+                    ptx::tmem_ld_wait();
+                    if (row_ok) {
+#pragma unroll
+                        for (int j = 0; j < 32; j += 8)
+                            *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(pack_h2(v[j] * inv, v[j + 1] * inv), pack_h2(v[j + 2] * inv, v[j + 3] * inv),
+                                                                                pack_h2(v[j + 4] * inv, v[j + 5] * inv), pack_h2(v[j + 6] * inv, v[j + 7] * inv));
+                    }
+                }
+            }
+        }
+    }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (*abort_flag) {      // let loads that are still in flight land before the CTA gives its shared memory back
+        const long long c0 = clock64();
+        while (clock64() - c0 < 4000000LL) { }
+        __syncthreads();
+    }
+    if (warp == 8) { ptx::tc_fence_after_sync(); ptx::tmem_dealloc(tmem, 512); }
+}
+
+// Partial results of the splits of one row -> O: one warp per row, D / 32 values per lane.  The row's own tile says how many
+// splits it has.
+template <int D>
+__global__ void __launch_bounds__(256) combine_kernel(const Params p) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+    const uint32_t rows = p.Hq * p.M;
+    const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (r >= rows) return;
+    const uint32_t head = r / p.M, pos = r - head * p.M;
+    const uint32_t n = (key_tiles(pos / p.BP * p.BP, p.BP, p.M, p.Mkv, p.pos0) + p.tiles_per_split - 1u) / p.tiles_per_split;
+    // lane s holds split s's factor (at most 32 splits)
+    const float2 ml = lane < n ? p.part_ml[(size_t)lane * rows + r] : make_float2(-1e30f, 0.0f);
+    float m = ml.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float w = lane < n ? ex2(ml.x - m) : 0.0f;
+    float l = w * ml.y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    const float wn = l > 0.0f ? w / l : 0.0f;
+    constexpr int E = D / 32;
+    float acc[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) acc[e] = 0.0f;
+    for (uint32_t s = 0; s < n; s++) {
+        const float ws = __shfl_sync(0xffffffffu, wn, (int)s);
+        const float* src = p.part_o + ((size_t)s * rows + r) * D + lane * E;
+        float v[E];
+        if (E == 4) { const float4 t = __ldcg(reinterpret_cast<const float4*>(src)); v[0] = t.x; v[1] = t.y; v[E - 2] = t.z; v[E - 1] = t.w; }
+        else { const float2 t = __ldcg(reinterpret_cast<const float2*>(src)); v[0] = t.x; v[1] = t.y; }
+#pragma unroll
+        for (int e = 0; e < E; e++) acc[e] = fmaf(ws, v[e], acc[e]);
+    }
+    __half* dst = (p.out_tokens_major ? p.O + ((size_t)pos * p.Hq + head) * D : p.O + (size_t)r * D) + lane * E;
+    if (E == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_h2(acc[0], acc[1]), pack_h2(acc[E - 2], acc[E - 1]));
+    else *reinterpret_cast<uint32_t*>(dst) = pack_h2(acc[0], acc[1]);
+}
+
+// Q8_0 records (34 bytes: fp16 d, 32 codes; 2-byte aligned) of K and then V -> fp16, value = fp16(q * d), one rounding.  Eight
+// lanes per record: a warp reads 136 consecutive bytes and writes 256.
+__global__ void __launch_bounds__(256) dequant_q8_0_kernel(const uint8_t* __restrict__ K, const uint8_t* __restrict__ V, __half* __restrict__ out,
+                                                           size_t blocks) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+    const size_t i = (size_t)blockIdx.x * 256u + threadIdx.x;
+    const size_t b = i >> 3;
+    if (b >= 2 * blocks) return;
+    const uint8_t* blk = b < blocks ? K + b * 34 : V + (b - blocks) * 34;
+    const uint32_t part = (uint32_t)i & 7u;
+    const __half d = *reinterpret_cast<const __half*>(blk);
+    const uint16_t* cp = reinterpret_cast<const uint16_t*>(blk + 2u + 4u * part);
+    const uint32_t c = (uint32_t)cp[0] | ((uint32_t)cp[1] << 16);
+    __half v[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[e] = __hmul(__int2half_rn((int)(int8_t)(c >> (8 * e))), d);
+    uint2 o;
+    o.x = (uint32_t)__half_as_ushort(v[0]) | ((uint32_t)__half_as_ushort(v[1]) << 16);
+    o.y = (uint32_t)__half_as_ushort(v[2]) | ((uint32_t)__half_as_ushort(v[3]) << 16);
+    *reinterpret_cast<uint2*>(out + b * 32 + part * 4u) = o;
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+namespace {
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (EncodeTiledFn)f;
+    }();
+    return fn;
+}
+// fp16 [heads][rows][D] as a 3-D map, boxes of box_heads x box_rows x 64 d with the 128-byte swizzle; rows past the end read as zero
+bool make_map(CUtensorMap* m, const void* ptr, uint32_t D, uint32_t heads, uint32_t rows, uint32_t box_rows, uint32_t box_heads) {
+    cuuint64_t dims[3] = {D, rows, heads};
+    cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)rows * D * 2};
+    cuuint32_t box[3] = {64, box_rows, box_heads};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+uint32_t sm_count() {
+    static int n = 0;
+    if (!n) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); if (n <= 0) n = 148; }
+    return (uint32_t)n;
+}
+
+// Splits of the key range.  A step (128 keys against 256 query rows) is the unit; a CTA costs about FIXED steps on top of its
+// own, the pass over the partial results about COMBINE.  One CTA runs per SM, so items beyond a whole number of waves cost a
+// wave where all items are equally long (a chunk behind a long cache); a causal triangle from position 0 packs better than
+// that, its sum is what counts there.
+uint32_t choose_splits(uint32_t heads, uint32_t blocks, uint32_t n_first, uint32_t n_last) {
+    constexpr float FIXED = 3.0f, COMBINE = 5.0f;
+    const float sms = (float)sm_count();
+    uint32_t best = 1;
+    float best_cost = 0.0f;
+    for (uint32_t s = 1; s <= (uint32_t)MAX_SPLITS && s <= n_last; s++) {
+        const uint32_t len = (n_last + s - 1) / s;
+        if ((n_last + len - 1) / len != s) continue;                   // the last split would be empty
+        float cost;
+        if (2u * n_first >= n_last) {
+            const uint32_t items = heads * blocks * s;
+            cost = (float)((items + sm_count() - 1) / sm_count()) * ((float)len + FIXED);
+        } else {
+            const float steps = (float)heads * blocks * 0.5f * (float)(n_first + n_last);
+            const float items = (float)heads * blocks * (0.5f * (float)(s + 1));
+            const float even = (steps + items * FIXED) / sms + 0.5f * (float)len;
+            cost = even > (float)len + FIXED ? even : (float)len + FIXED;
+        }
+        if (s > 1) cost += COMBINE;
+        if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+    }
+    return best;
+}
+
+template <int D> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* launches) {
+    using C = Cfg<D>;
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(attn_ws_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        if (e != cudaSuccess) return e;
+        attr_set = true;
+    }
+    Params p;
+    p.G = a.Hq / a.Hkv; p.BP = (uint32_t)ROWS / p.G;
+    p.Hq = a.Hq; p.M = a.M; p.Mkv = a.Mkv; p.pos0 = a.pos0; p.scale_log2e = a.scale_log2e;
+    p.out_tokens_major = a.out_tokens_major; p.O = (__half*)a.O; p.err = bridge::g.err_word;
+    const uint32_t blocks = (a.M + 2 * p.BP - 1) / (2 * p.BP);
+    auto tiles = [&](uint64_t pos) {      // key tiles of a block whose last position is `pos`
+        const uint64_t last = (uint64_t)a.pos0 + (pos < a.M ? pos : a.M - 1);
+        return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / BK + 1);
+    };
+    const uint32_t n_last = tiles(a.M - 1), n_first = tiles(2ull * p.BP - 1);
+    const uint32_t splits = choose_splits(a.Hkv, blocks, n_first, n_last);
+    p.tiles_per_split = (n_last + splits - 1) / splits;
+    // scratch: the expanded cache, then the partial results
+    const size_t kv_elems = (size_t)a.Hkv * a.Mkv * D;
+    const size_t kv_bytes = a.kv_fp16 ? 0 : (2 * kv_elems * sizeof(__half) + 255) & ~(size_t)255;
+    const size_t rows = (size_t)a.Hq * a.M;
+    const size_t o_bytes = splits > 1 ? splits * rows * D * sizeof(float) : 0, ml_bytes = splits > 1 ? splits * rows * sizeof(float2) : 0;
+    if (kv_bytes + o_bytes + ml_bytes > 0 && !bridge::g.kv_fp16.ensure(kv_bytes + o_bytes + ml_bytes)) return cudaErrorMemoryAllocation;
+    uint8_t* scratch = static_cast<uint8_t*>(bridge::g.kv_fp16.p);
+    p.split = splits > 1;
+    p.part_o = reinterpret_cast<float*>(scratch + kv_bytes);
+    p.part_ml = reinterpret_cast<float2*>(scratch + kv_bytes + o_bytes);
+
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // a kernel's set-up may overlap the previous one's tail
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1; cfg.stream = stream;
+    *launches = 0;
+    const void *Kf = a.K, *Vf = a.V;
+    if (!a.kv_fp16) {
+        const size_t nb = kv_elems / 32;
+        cfg.gridDim = dim3((unsigned)((2 * nb * 8 + 255) / 256)); cfg.blockDim = dim3(256);
+        cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_q8_0_kernel, (const uint8_t*)a.K, (const uint8_t*)a.V, (__half*)scratch, nb);
+        if (e != cudaSuccess) return e;
+        Kf = scratch; Vf = scratch + kv_elems * sizeof(__half);
+        ++*launches;
+    }
+    CUtensorMap tmQ, tmK, tmV;
+    if (!make_map(&tmK, Kf, D, a.Hkv, a.Mkv, BK, 1) || !make_map(&tmV, Vf, D, a.Hkv, a.Mkv, BK, 1) || !make_map(&tmQ, a.Q, D, a.Hq, a.M, p.BP, p.G))
+        return cudaErrorInvalidValue;
+    cfg.gridDim = dim3(a.Hkv, blocks, splits); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = C::SMEM;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attn_ws_kernel<D>, tmQ, tmK, tmV, p);
+    if (e != cudaSuccess) return e;
+    ++*launches;
+    if (splits > 1) {
+        cfg.gridDim = dim3((unsigned)((rows + 7) / 8)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0;
+        e = cudaLaunchKernelEx(&cfg, combine_kernel<D>, p);
+        if (e != cudaSuccess) return e;
+        ++*launches;
+    }
+    return cudaSuccess;
+}
+
+}  // namespace
+
+bool usable(const Args& a) {
+    const uint32_t G = a.Hq / a.Hkv;
+    if ((a.D != 64 && a.D != 128) || G > (uint32_t)ROWS || !(a.scale_log2e > 0.0f) || (((uintptr_t)a.Q | (uintptr_t)a.O) & 15u)) return false;
+    if (a.kv_fp16 && (((uintptr_t)a.K | (uintptr_t)a.V) & 15u)) return false;
+    // grid dimensions, 32-bit row and position arithmetic
+    const uint32_t BP = (uint32_t)ROWS / G;
+    if ((a.M + 2 * BP - 1) / (2 * BP) > 65535u || (uint64_t)a.pos0 + a.M > 0x7fffffffu || (uint64_t)a.Hq * a.M > 0x7fffffffu || a.Mkv > 0x7fffff00u) return false;
+    return encode_fn() != nullptr;
+}
+
+cudaError_t launch(const Args& a, cudaStream_t stream, int* launches) {
+    return a.D == 128 ? launch_d<128>(a, stream, launches) : launch_d<64>(a, stream, launches);
+}
+
+}  // namespace ws
+}  // namespace attn
