@@ -43,6 +43,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Non-blocking look at a phase.  (try_wait may park the thread for a hardware-defined time, about 4 us on B200, before it
+// says no: a loop that only wants to know whether it may do something early must not use it.)
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait.  `abort_flag` lives in shared memory: the first waiter that runs out of time
 // sets it (and the global error word) so every other waiter of the CTA leaves at once.
 // mbarrier.try_wait itself parks the thread for a hardware-defined interval, so the loop is
