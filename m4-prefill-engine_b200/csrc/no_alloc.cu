@@ -111,12 +111,17 @@ int b200_bridge_gemm_scratch_static(void* X, size_t X_bytes, void* W, size_t W_b
     qg::GemmArgs a;
     memset(&a, 0, sizeof(a));
     a.format = format; a.X = X; a.W0 = W; a.Y = Y; a.M = M; a.N = N; a.K = K; a.layout = LAYOUT_STANDARD;
+    // Whether a shape is served is decided by what its launch needs at least; a split of K into unequal parts or a padded
+    // copy of the weights is used where the array has room for that too.
+    a.lean = 1;
     const size_t need = qg::workspace_floats(a);
     if (need > (size_t)B200_STATIC_SCRATCH_FLOATS) {
         set_error("b200_bridge_gemm_scratch_static: this shape needs " + std::to_string(need) +
                   " floats of split-K scratch, the static array holds " + std::to_string(B200_STATIC_SCRATCH_FLOATS));
         return -7;
     }
+    a.lean = 0;
+    if (qg::workspace_floats(a) > (size_t)B200_STATIC_SCRATCH_FLOATS) a.lean = 1;
     StaticScratch* sc = nullptr;
     cudaError_t e = scratch_address(dev, &sc);
     if (e != cudaSuccess) {

@@ -109,8 +109,9 @@ template <int FMT> struct Cfg {
 
 struct Params {
     uint32_t M, N, K;
+    uint32_t x_wrap;             // K after which the activation columns start over
     uint32_t T;                  // tokens per tile (multiple of 16)
-    uint32_t n_tok_tiles, n_w_tiles, k_splits, kchunks;   // kchunks: 256-element chunks per split
+    uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;    // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
     uint32_t raw_stages, b_stage_bytes, b_stages;         // ring depth of packed weights; bytes of one activation stage (T*128); activation ring depth
     uint32_t a_stages;                                    // ring depth of unpacked weight tiles (STAGES; more for CTA pairs)
     __half* Y;
@@ -186,7 +187,7 @@ template <int S> struct IntC { static constexpr int value = S; };
 template <class F, int... S>
 __device__ __forceinline__ void for_each_sub(F& f, std::integer_sequence<int, S...>) { (f(IntC<S>{}), ...); }
 
-struct Tile { uint32_t wt, tt, ks, id; };
+struct Tile { uint32_t wt, tt, ks, id, kc0, kcn; };     // kc0, kcn: first packed chunk of K and how many
 __device__ __forceinline__ Tile decode_tile(uint32_t idx, const Params& p) {
     Tile t;
     t.ks = idx % p.k_splits;
@@ -198,6 +199,8 @@ __device__ __forceinline__ Tile decode_tile(uint32_t idx, const Params& p) {
     // owner's NVLink port at a time) and the last, local tiles overlap the tail of the remote transfers
     if (p.tt_shift) { t.tt += p.tt_shift; if (t.tt >= p.n_tok_tiles) t.tt -= p.n_tok_tiles; }
     t.id = t.tt * p.n_w_tiles + t.wt;
+    t.kc0 = t.ks * p.chunks / p.k_splits;
+    t.kcn = (t.ks + 1u) * p.chunks / p.k_splits - t.kc0;
     return t;
 }
 
@@ -507,9 +510,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         t.ks = 0u; t.wt = 2u * (idx % n_wp) + pair_rank; t.tt = idx / n_wp;
         if (p.tt_shift) { t.tt += p.tt_shift; if (t.tt >= p.n_tok_tiles) t.tt -= p.n_tok_tiles; }
         t.id = t.tt * p.n_w_tiles + t.wt;
+        t.kc0 = 0u; t.kcn = p.chunks;
         return t;
     };
-    const uint32_t ksteps = p.kchunks * (uint32_t)C::SUBS;
     const uint32_t b_rows = PAIR ? p.T / 2u : p.T;                      // token rows of the activation tile this CTA loads
 
     if (threadIdx.x == 0) {
@@ -556,13 +559,13 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         bool ok = true;
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
-            for (uint32_t kc = 0; kc < p.kchunks; kc++) {
+            for (uint32_t kc = 0; kc < t.kcn; kc++) {
                 ok = __all_sync(0xffffffffu, ptx::mbar_wait<64>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(0, wtr, 0);
                     ptx::mbar_arrive_expect_tx(&raw_full[rs], RAW_TILE_BYTES);
-                    const int x = (int)((t.ks * p.kchunks + kc) * (ROW_BYTES / Cd::TMA_ELEM_BYTES));    // in elements of the map
+                    const int x = (int)((t.kc0 + kc) * (ROW_BYTES / Cd::TMA_ELEM_BYTES));    // in elements of the map
                     if (p.swiglu) {     // the maps of a SwiGLU launch have 64-row boxes: gate rows, then the same rows of up
                         const int y = (int)(t.wt * GATE_ROWS);
                         ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &tmW0, &raw_full[rs], x, y);
@@ -591,7 +594,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         uint32_t rows_seen = 0;               // bit o: owner o's rows are known to be there
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
-            const uint32_t k0 = t.ks * p.kchunks * (uint32_t)C::CHUNK;
+            const uint32_t k0 = t.kc0 * (uint32_t)C::CHUNK, ksteps = t.kcn * (uint32_t)C::SUBS;
             if (p.wait_rows.flags) {
                 // rows this CTA is about to load: wait until their owners have written them (system-scope acquire, then the
                 // proxy fence that orders the TMA reads behind it)
@@ -623,7 +626,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (lane == 0) {
                     QTR(1, xtr, 0);
                     ptx::mbar_arrive_expect_tx(&b_full[bs], b_rows * 128u);
-                    ptx::tma_load_2d(sB + bs * p.b_stage_bytes, &tmX, &b_full[bs], (int)(k0 + ks * KSTEP), (int)(t.tt * p.T + pair_rank * b_rows));
+                    ptx::tma_load_2d(sB + bs * p.b_stage_bytes, &tmX, &b_full[bs], (int)((k0 + ks * KSTEP) % p.x_wrap), (int)(t.tt * p.T + pair_rank * b_rows));
                     QTR(1, xtr, 1); xtr++;
                 }
                 __syncwarp();
@@ -635,6 +638,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         uint32_t bs = 0, bph = 0;
         bool ok = true;
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
+            const uint32_t ksteps = p.chunks * (uint32_t)C::SUBS;       // (pair launches do not split K)
             for (uint32_t ks = 0; ks < ksteps; ks++) {
                 ok = __all_sync(0xffffffffu, ptx::mbar_wait(&b_full[bs], bph, abort_flag, p.err, 109));
                 if (!ok) break;
@@ -659,6 +663,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             if (!ok) break;
             ptx::tc_fence_after_sync();
             if (lane == 0) QTRC(2, 200u + it, 0);
+            const uint32_t ksteps = tile_of(idx).kcn * (uint32_t)C::SUBS;
             for (uint32_t ks = 0; ks < ksteps; ks++) {
                 if (lane == 0) QTR(2, mtr, 0);
                 // (no tcgen05 fence here: the stage was written by TMA and by generic stores that were
@@ -723,7 +728,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 const uint32_t n = t.wt * (p.swiglu ? GATE_ROWS : W_TILE) + mrow_in_tile;
                 if (n < p.N) {
                     const uint32_t groups = (p.K / 256) * MW;
-                    const uint8_t* mp = (mat == 0 ? p.meta0 : p.meta1) + ((size_t)n * groups + (size_t)(t.ks * p.kchunks + kc) * MW) * 2;
+                    const uint8_t* mp = (mat == 0 ? p.meta0 : p.meta1) + ((size_t)n * groups + (size_t)(t.kc0 + kc) * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
                         const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
@@ -738,7 +743,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 }
             };
             (void)load_meta; (void)meta_next;
-            for (uint32_t kc = 0; ok && kc < p.kchunks; kc++) {
+            for (uint32_t kc = 0; ok && kc < t.kcn; kc++) {
                 // scales and biases kept outside the packed rows come straight from global memory, one chunk
                 // ahead of their use so the latency hides behind the unpacking of the current chunk
                 uint32_t meta[MW] = {};
@@ -746,7 +751,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (kc == 0) load_meta(0u, meta_next);
 #pragma unroll
                     for (int i = 0; i < MW; i++) meta[i] = meta_next[i];
-                    if (kc + 1 < p.kchunks) load_meta(kc + 1, meta_next);
+                    if (kc + 1 < t.kcn) load_meta(kc + 1, meta_next);
                 }
                 ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&raw_full[rs], rph, abort_flag, p.err, 106));
                 if (!ok) break;
@@ -1240,8 +1245,6 @@ int row_bytes_256(int fmt) {
     }
 }
 
-uint32_t chunk_elems(int fmt) { return fmt == QUANT_PRISM_Q2_0 ? 1024u : (uint32_t)KCHUNK; }
-
 int g_sm_count = 0;
 int sm_count() {
     if (!g_sm_count) {
@@ -1253,7 +1256,7 @@ int sm_count() {
     return g_sm_count;
 }
 
-struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, kchunks; };
+struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, chunks; };
 
 Plan make_plan(const GemmArgs& a) {
     const uint32_t tok_max = 256u;
@@ -1271,12 +1274,13 @@ Plan make_plan(const GemmArgs& a) {
         const uint32_t tiles = pl.n_tok_tiles * pl.n_w_tiles;
         const uint32_t sms = (uint32_t)sm_count();
         for (uint32_t s = 2; s <= 8; s *= 2) {
-            if (tiles * s > sms || chunks % s != 0 || chunks / s < 2) break;
+            if (tiles * s > sms || chunks / s < 2) break;
+            if (a.lean && chunks % s != 0) break;
             pl.k_splits = s;
         }
         if (pl.n_tok_tiles * pl.n_w_tiles > 4096) pl.k_splits = 1;
     }
-    pl.kchunks = chunks / pl.k_splits;
+    pl.chunks = chunks;
     return pl;
 }
 
@@ -1342,7 +1346,8 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
     const uint32_t t_cta = pair ? pl.T / 2u : pl.T;             // token rows of the activation tile one CTA loads
     g_last_pair = pair ? 1 : 0;
     CUtensorMap tmX, tmW0, tmW1, tmW2;
-    if (!make_map_2d(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.X, a.K, a.M, (uint64_t)a.K * 2, KSTEP, t_cta,
+    const uint32_t x_cols = a.x_cols ? a.x_cols : a.K;          // columns past the end read as zero
+    if (!make_map_2d(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.X, x_cols, a.M, (uint64_t)x_cols * 2, KSTEP, t_cta,
                      CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     const CUtensorMapSwizzle wsw = cdc::Codec<FMT>::RAW_SWIZZLE_128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE;
@@ -1367,7 +1372,8 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
 
     Params p;
     p.M = a.M; p.N = a.N; p.K = a.K;
-    p.T = pl.T; p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.kchunks = pl.kchunks;
+    p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
+    p.T = pl.T; p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
     p.swiglu = a.W1 ? 1u : 0u;
     // Row-wise epilogue: wherever every output row can take 16-byte stores (and, with a residual, 8-byte loads).  SwiGLU
     // tiles and split-K partial tiles have their own paths.
@@ -1509,6 +1515,8 @@ thread_local int g_last_launches = 0;
 
 }  // namespace
 
+uint32_t chunk_elems(int fmt) { return fmt == QUANT_PRISM_Q2_0 ? 1024u : (uint32_t)KCHUNK; }
+
 cudaError_t prepare_device() {
     cudaError_t e = set_kernel_attributes<QUANT_Q4_0>();
     if (e == cudaSuccess) e = set_kernel_attributes<QUANT_MLX_4BIT>();
@@ -1534,7 +1542,19 @@ bool fast_path_ok(const GemmArgs& a) {
     return encode_fn() != nullptr;
 }
 
+namespace {
+// what a launch on a padded copy looks like to the planners (the copy itself is not there yet)
+GemmArgs padded_probe(const GemmArgs& a) {
+    GemmArgs b = a;
+    padded_shape(a, b);
+    b.W0 = reinterpret_cast<const void*>(16);
+    if (a.W1) b.W1 = reinterpret_cast<const void*>(16);
+    return b;
+}
+}  // namespace
+
 size_t workspace_floats(const GemmArgs& a) {
+    if (pad_path_ok(a)) return workspace_floats(padded_probe(a)) + (padded_bytes(a) + 512) / sizeof(float);
     if (gemv_path_ok(a)) return 0;
     if (small_path_ok(a)) return small_scratch_floats(a);
     if (!fast_path_ok(a)) return 0;
@@ -1549,6 +1569,20 @@ cudaError_t launch(const GemmArgs& a, const Workspace& ws, cudaStream_t stream) 
     if (gemv_path_ok(a)) return launch_gemv(a, stream);
     if (small_path_ok(a)) return launch_small(a, ws, stream);
     if (fast_path_ok(a)) return dispatch_fast(a, ws, stream);
+    if (pad_path_ok(a) && ws.partial && ws.partial_floats >= workspace_floats(a)) {
+        // [padded copies][split-K scratch], both on 256-byte boundaries
+        const size_t bytes = padded_bytes(a);
+        uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws.partial) + 255) & ~(uintptr_t)255);
+        GemmArgs b;
+        cudaError_t e = launch_pad(a, base, b, stream);
+        if (e != cudaSuccess) return e;
+        Workspace rest = ws;
+        rest.partial = reinterpret_cast<float*>(base + bytes);
+        rest.partial_floats = ws.partial_floats - (size_t)(rest.partial - ws.partial);
+        e = launch(b, rest, stream);
+        g_last_launches = 2;
+        return e;
+    }
     if (a.scatter.world || a.n_extra) return cudaErrorInvalidValue;   // fused reduce-scatter and grouped launches exist on the tensor-core path only
     Params p;
     memset(&p, 0, sizeof(p));

@@ -14,11 +14,14 @@ struct GemmArgs {
     const void* W1;           // up matrix for SwiGLU, else nullptr
     void* Y;                  // fp16 out: [M][N], or [H][M][D] when layout == 1
     uint32_t M, N, K;
+    uint32_t x_cols, x_wrap;  // columns X really has (0: K), and the K after which the rows start over on the same columns
+                              // (0: never): rows that were padded to whole chunks and hold every weight as a sum of terms
     int layout;               // LayoutMode
     uint32_t H, D;            // direct-head split of N
     const void* residual;     // optional fp16 [M][N] added in the epilogue (standard layout only)
     float* partial_out;       // optional fp32 [M][N]: write raw accumulators instead of fp16 Y
     int force_generic;        // testing hook: use the CUDA-core fallback kernel
+    int lean;                 // little scratch: K split into equal parts only, no padded copy of the weights
     // Grouped launch: up to two more projections of the same X (same K, format, layout and D) run in the same
     // grid, their weight tiles queued behind those of W0.  n_extra == 0: off.  Plain fp16 outputs only.
     uint32_t n_extra;
@@ -66,6 +69,14 @@ struct Workspace {            // split-K scratch, owned by the caller
 // Sets the dynamic shared-memory attribute of every kernel instantiation on the current device (which also loads the
 // module image there).  Called once per device at initialisation; launches repeat it only for a device they have not seen.
 cudaError_t prepare_device();
+// K that is not a whole number of packed chunks (rows that TMA cannot address): the packed weights are copied into the
+// scratch with every row padded to whole chunks and the projection runs on the copy (qgemm_pad.cu).
+bool pad_path_ok(const GemmArgs& a);
+size_t padded_bytes(const GemmArgs& a);          // of all matrices of the launch, 256-byte aligned each
+cudaError_t launch_pad(const GemmArgs& a, void* dst, GemmArgs& padded, cudaStream_t stream);
+void padded_shape(const GemmArgs& a, GemmArgs& padded);      // K, x_cols, x_wrap of the launch on the copy
+uint32_t chunk_elems(int format);                // K elements per packed chunk of the tensor-core codecs
+
 // True if (format, shape, pointers) can take the TMA + tcgen05 path.
 bool fast_path_ok(const GemmArgs& a);
 // Floats of split-K scratch the launch will use (0 when it does not split).

@@ -1,0 +1,161 @@
+// Packed weights with rows padded to whole chunks, for K that is not a multiple of the codecs' chunk (256 elements; 1024 for
+// the 34-byte Prism blocks).
+//
+// The tensor-core kernels address packed rows through TMA maps, whose row stride has to be a multiple of 16 bytes: 18-byte
+// Q4_0 blocks give that every 256 elements only.  One pass copies the rows into scratch at a chunk-aligned stride; what lies
+// behind a row's last block is zero bytes, and the activation columns they meet read as zero (the map of X ends at the real
+// K).
+//
+// The kernel that such shapes ran on (one thread per output, fp32) multiplied with weights that were never rounded to fp16,
+// so the copy must not round them either.  A weight q * s (+ b) with a 4-bit q becomes a sum of terms that fp16 holds
+// exactly: s = sh + sl, sh its leading 7 significant bits, sl the remaining 4, so that q * sh, q * sl and b are exact; the
+// row holds the codes once per term with that term's scale and bias, and the activation columns start over for each.  Q4_0
+// takes two terms, the affine formats three; ternary weights are exact as they are.
+//
+// One launch and the packed bytes once or a few times more; K = 2080, N = 1100, 129 tokens took 1361 us on the CUDA cores and takes 23 us
+// (one token 13 us).
+// That kernel remains for activations that are not 16-byte aligned.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <cstring>
+
+#include "../../include/quant_router.h"
+#include "ptx.cuh"
+#include "qgemm.cuh"
+
+namespace qg {
+namespace {
+
+// A packed matrix is one to three planes of rows.  A plane is a run of records per row, `rec` bytes each, of which the 16-bit
+// field at `scale_at` is a scale and the one at `bias_at` a bias (-1: none); the rest are codes.
+struct Plane { uint64_t src, dst; uint32_t rows, src_row, dst_term; int32_t rec, scale_at, bias_at; };     // dst_term: bytes of one term of a padded row
+struct Planes { Plane p[3]; uint32_t n, terms; uint64_t bytes; };
+
+uint32_t padded_k(const GemmArgs& a) { const uint32_t c = chunk_elems(a.format); return (a.K + c - 1) / c * c; }
+
+bool planes_of(const GemmArgs& a, Planes& out) {
+    const uint64_t N = a.N;
+    const uint32_t K = a.K, Kp = padded_k(a);
+    memset(&out, 0, sizeof(out));
+    out.terms = 1;
+    auto add = [&](uint64_t src, uint32_t per, uint32_t rec, int scale_at, int bias_at) {      // one record of rec bytes per `per` elements
+        out.p[out.n++] = Plane{src, out.bytes, a.N, K / per * rec, Kp / per * rec, (int32_t)rec, scale_at, bias_at};
+        out.bytes += N * out.terms * (Kp / per * rec);
+        return K % per == 0;
+    };
+    bool ok = true;
+    switch (a.format) {
+        case QUANT_Q4_0: out.terms = 2; ok = add(0, 32, 18, 0, -1); break;
+        case QUANT_MLX_4BIT: out.terms = 3; ok = add(0, 32, 20, 0, 2); break;
+        case QUANT_TERNARY_1_58: ok = add(0, 32, 12, -1, -1); break;
+        case QUANT_PRISM_Q2_0: ok = add(0, 128, 34, -1, -1); break;
+        case QUANT_MLX_4BIT_G64: {
+            const uint64_t codes = N * (K / 2), plane = N * (K / 64) * 2;
+            out.terms = 3;
+            ok = add(0, 64, 32, -1, -1) && add(codes, 64, 2, 0, -1) && add(codes + plane, 64, 2, -1, 0);
+            break;
+        }
+        case QUANT_MLX_4BIT_PLANAR: {
+            const uint64_t n = N * (K / 32), scales = (n * 16 + 15) & ~(uint64_t)15, biases = (scales + n * 2 + 15) & ~(uint64_t)15;
+            out.terms = 3;
+            ok = add(0, 32, 16, -1, -1) && add(scales, 32, 2, 0, -1) && add(biases, 32, 2, -1, 0);
+            break;
+        }
+        case QUANT_TERNARY_ROW:
+            ok = add(0, 32, 8, -1, -1);
+            // one scale per row, behind the codes: a single row of N scales, copied as it is
+            out.p[out.n++] = Plane{N * (K / 4), out.bytes, 1u, a.N * 2u, a.N * 2u, 2, -1, -1};
+            out.bytes += N * 2;
+            break;
+        default: return false;
+    }
+    out.bytes = (out.bytes + 255) & ~(uint64_t)255;
+    return ok;
+}
+
+// scale of term t: leading 7 significant bits, the rest, nothing
+__device__ __forceinline__ uint16_t scale_term(uint16_t bits, uint32_t t) {
+    const bool finite = (bits & 0x7C00u) != 0x7C00u;
+    const uint16_t hi = finite ? (uint16_t)(bits & 0xFFF0u) : bits;
+    if (t == 0u) return hi;
+    if (t == 1u && finite) return __half_as_ushort(__hsub(__ushort_as_half(bits), __ushort_as_half(hi)));      // exact
+    return 0u;
+}
+
+// One thread writes eight bytes of a padded row (plane blockIdx.y of matrix blockIdx.z), or what is left of them.
+__global__ void __launch_bounds__(256) pad_rows_kernel(const uint8_t* __restrict__ w0, const uint8_t* __restrict__ w1, uint8_t* __restrict__ dst, const Planes pl) {
+    ptx::grid_dependency_wait();           // the scratch may still be read by the launch before
+    ptx::launch_dependents();
+    const Plane p = pl.p[blockIdx.y];
+    const uint32_t terms = pl.terms, dst_row = p.dst_term * terms, per_row = (dst_row + 7u) / 8u;
+    const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
+    if (i >= (uint64_t)p.rows * per_row) return;
+    const uint32_t row = (uint32_t)(i / per_row), b0 = (uint32_t)(i - (uint64_t)row * per_row) * 8u;
+    const uint8_t* s = (blockIdx.z ? w1 : w0) + p.src + (uint64_t)row * p.src_row;
+    uint8_t* d = dst + blockIdx.z * pl.bytes + p.dst + (uint64_t)row * dst_row + b0;
+    uint16_t v[4];
+#pragma unroll
+    for (uint32_t e = 0; e < 4u; e++) {
+        const uint32_t b = b0 + 2u * e, t = b / p.dst_term, off = b - t * p.dst_term;
+        v[e] = b < dst_row && off < p.src_row ? *reinterpret_cast<const uint16_t*>(s + off) : (uint16_t)0;
+        const int32_t field = (int32_t)(off % (uint32_t)p.rec);
+        if (terms > 1u && field == p.scale_at) v[e] = scale_term(v[e], t);
+        if (terms > 1u && field == p.bias_at && t + 1u != terms) v[e] = 0u;
+    }
+    if (dst_row % 8u == 0u) {              // (rows of whole chunks: every store is 8-byte aligned)
+        *reinterpret_cast<uint2*>(d) = make_uint2((uint32_t)v[0] | ((uint32_t)v[1] << 16), (uint32_t)v[2] | ((uint32_t)v[3] << 16));
+    } else {
+#pragma unroll
+        for (uint32_t e = 0; e < 4u; e++)
+            if (b0 + 2u * e < dst_row) reinterpret_cast<uint16_t*>(d)[e] = v[e];
+    }
+}
+
+}  // namespace
+
+bool pad_path_ok(const GemmArgs& a) {
+    if (a.force_generic || a.lean || a.x_cols || a.scatter.world || a.n_extra || a.wait_rows.flags || a.post[0] || a.post[1] || a.post[2]) return false;
+    if (a.M == 0 || a.N == 0 || a.K == 0 || a.K % 8 != 0 || a.K % chunk_elems(a.format) == 0 || a.K > (1u << 24)) return false;
+    if (((uintptr_t)a.X & 15u) || ((uintptr_t)a.W0 & 1u) || ((uintptr_t)a.W1 & 1u)) return false;
+    Planes pl;
+    return planes_of(a, pl);
+}
+
+void padded_shape(const GemmArgs& a, GemmArgs& padded) {
+    Planes pl;
+    planes_of(a, pl);
+    padded.x_cols = a.K; padded.x_wrap = padded_k(a); padded.K = pl.terms * padded.x_wrap;
+}
+
+size_t padded_bytes(const GemmArgs& a) {
+    Planes pl;
+    return planes_of(a, pl) ? (size_t)pl.bytes * (a.W1 ? 2 : 1) : 0;
+}
+
+cudaError_t launch_pad(const GemmArgs& a, void* dst, GemmArgs& padded, cudaStream_t stream) {
+    Planes pl;
+    if (!planes_of(a, pl)) return cudaErrorInvalidValue;
+    uint64_t most = 0;
+    for (uint32_t i = 0; i < pl.n; i++) {
+        const uint64_t n = (uint64_t)pl.p[i].rows * ((pl.p[i].dst_term * pl.terms + 7u) / 8u);
+        if (n > most) most = n;
+    }
+    padded = a;
+    padded_shape(a, padded);
+    padded.W0 = dst;
+    if (a.W1) padded.W1 = static_cast<uint8_t*>(dst) + pl.bytes;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)((most + 255) / 256), pl.n, a.W1 ? 2 : 1);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, pad_rows_kernel, (const uint8_t*)a.W0, (const uint8_t*)a.W1, (uint8_t*)dst, pl);
+}
+
+}  // namespace qg

@@ -56,7 +56,8 @@ __device__ unsigned long long g_qs_trace[8][64];
 
 struct Params {
     uint32_t M, N, K, T;
-    uint32_t n_tok_tiles, n_w_tiles, k_splits, kchunks;      // kchunks: packed chunks per split
+    uint32_t x_wrap;             // K after which the activation columns start over
+    uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;       // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
     __half* Y;
     const __half* residual;
     uint32_t layout, D;
@@ -146,7 +147,8 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t ks = blockIdx.x % p.k_splits;                    // == rank inside the cluster
     const uint32_t tile = blockIdx.x / p.k_splits;
     const uint32_t wt = tile % p.n_w_tiles, tt = tile / p.n_w_tiles;
-    const uint32_t ksteps = p.kchunks * (uint32_t)SUBS;
+    const uint32_t kc0 = ks * p.chunks / p.k_splits, kcn = (ks + 1u) * p.chunks / p.k_splits - kc0;     // this split's packed chunks
+    const uint32_t ksteps = kcn * (uint32_t)SUBS;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < RAW_STAGES; i++) { ptx::mbar_init(&raw_full[i], 1); ptx::mbar_init(&raw_empty[i], UNPACK_WARPS); }
@@ -175,7 +177,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         uint32_t rs = 0, rph = 0, bs = 0, bph = 0, raw_next = 0;
         bool ok = true;
         auto issue_raw = [&](bool block) {       // request chunk raw_next if its stage is free (block: wait for it)
-            if (raw_next >= p.kchunks) return;
+            if (raw_next >= kcn) return;
             // (a look that never parks: with try_wait here every activation tile behind a full packed ring was held up by
             // about 4 us -- K = 4096, N = 14336, 33 tokens 74.6 us instead of 19.5)
             bool free_now = ptx::mbar_test_wait(&raw_empty[rs], rph ^ 1u);
@@ -186,14 +188,14 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 QST(1, raw_next);
                 ptx::mbar_arrive_expect_tx(&raw_full[rs], RAW_TILE_BYTES);
                 ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &tmW, &raw_full[rs],
-                                 (int)((ks * p.kchunks + raw_next) * (ROW_BYTES / Cd::TMA_ELEM_BYTES)), (int)(wt * W_TILE));
+                                 (int)((kc0 + raw_next) * (ROW_BYTES / Cd::TMA_ELEM_BYTES)), (int)(wt * W_TILE));
             }
             __syncwarp();
             raw_next++;
             if (++rs == RAW_STAGES) { rs = 0; rph ^= 1u; }
         };
         for (int i = 0; i < RAW_STAGES; i++) issue_raw(false);
-        for (uint32_t kc = 0; ok && kc < p.kchunks; kc++) {
+        for (uint32_t kc = 0; ok && kc < kcn; kc++) {
             if (raw_next <= kc) issue_raw(true);              // the chunk these activation tiles belong to must be on its way
             for (uint32_t s = 0; ok && s < (uint32_t)SUBS; s++) {
                 ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 112));
@@ -201,7 +203,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 if (lane == 0) {
                     ptx::mbar_arrive_expect_tx(&b_full[bs], b_stage_bytes);
                     ptx::tma_load_2d(sB + bs * b_stage_bytes, &tmX, &b_full[bs],
-                                     (int)((ks * p.kchunks + kc) * Cd::CHUNK + s * KSTEP), (int)(tt * p.T));
+                                     (int)(((kc0 + kc) * Cd::CHUNK + s * KSTEP) % p.x_wrap), (int)(tt * p.T));
                 }
                 __syncwarp();
                 if (++bs == B_STAGES) { bs = 0; bph ^= 1u; }
@@ -243,7 +245,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         const uint32_t lane_base = (quad * 32u) << 16;
         uint32_t rs = 0, rph = 0;
         bool ok = true;
-        for (uint32_t kc = 0; ok && kc < p.kchunks; kc++) {
+        for (uint32_t kc = 0; ok && kc < kcn; kc++) {
             // planar layouts: this chunk's scales and biases come straight from their planes in global memory, requested
             // before the wait for the packed bytes
             uint32_t meta[MW] = {};
@@ -251,7 +253,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 const uint32_t n = wt * W_TILE + row;
                 if (n < p.N) {
                     const uint32_t groups = (p.K / 256u) * MW;
-                    const uint8_t* mp = p.meta0 + ((size_t)n * groups + (size_t)(ks * p.kchunks + kc) * MW) * 2;
+                    const uint8_t* mp = p.meta0 + ((size_t)n * groups + (size_t)(kc0 + kc) * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
                         const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
@@ -417,7 +419,7 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, uint64_t 
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, kchunks; size_t smem; };
+struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, chunks; size_t smem; };
 
 // alignment slack + activation ring + packed ring + barrier block
 template <int FMT> size_t smem_bytes(uint32_t T) {
@@ -442,10 +444,11 @@ template <int FMT> bool make_plan(const GemmArgs& a, Plan& pl) {
     // divide evenly among the CTAs of a cluster
     pl.k_splits = 1;
     for (uint32_t s = 2; s <= 8; s *= 2) {
-        if (tiles * s > 2u * (uint32_t)sms() || chunks % s != 0 || pl.T % s != 0) break;
+        if (tiles * s > 2u * (uint32_t)sms() || chunks < s || pl.T % s != 0) break;
+        if (a.lean && chunks % s != 0) break;
         pl.k_splits = s;
     }
-    pl.kchunks = chunks / pl.k_splits;
+    pl.chunks = chunks;
     // at least 80 KB, so that no more than two CTAs share an SM: each holds 256 of the SM's 512 tensor-memory columns, and a
     // third CTA would sit in tcgen05.alloc until one of the others leaves
     pl.smem = smem_bytes<FMT>(pl.T);
@@ -466,16 +469,17 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
     if (pl.k_splits > 1 && (!ws.partial || ws.partial_floats < (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE))
         return cudaErrorInvalidValue;
     const uint64_t w_row_bytes = (uint64_t)(a.K / Cd::CHUNK) * Cd::ROW_BYTES;
+    const uint32_t x_cols = a.x_cols ? a.x_cols : a.K;          // columns past the end read as zero
     CUtensorMap tmX, tmW;
-    if (!make_map(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.X, a.K, a.M, (uint64_t)a.K * 2, KSTEP, pl.T, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (!make_map(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.X, x_cols, a.M, (uint64_t)x_cols * 2, KSTEP, pl.T, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     constexpr int EB = Cd::TMA_ELEM_BYTES;
     if (!make_map(&tmW, EB == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, a.W0, w_row_bytes / EB, a.N, w_row_bytes,
                   Cd::ROW_BYTES / EB, W_TILE, Cd::RAW_SWIZZLE_128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE))
         return cudaErrorInvalidValue;
     Params p;
-    p.M = a.M; p.N = a.N; p.K = a.K; p.T = pl.T;
-    p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.kchunks = pl.kchunks;
+    p.M = a.M; p.N = a.N; p.K = a.K; p.T = pl.T; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
+    p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
     p.Y = (__half*)a.Y; p.residual = (const __half*)a.residual; p.layout = (uint32_t)a.layout; p.D = a.D ? a.D : 2;
     p.err = ws.err; p.scratch = ws.partial;
     p.meta0 = (const uint8_t*)a.W0 + (size_t)a.N * w_row_bytes;

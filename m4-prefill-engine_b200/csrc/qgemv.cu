@@ -27,7 +27,7 @@ constexpr int XSTRIDE = 257;                 // fp32 words per 256-element activ
 
 struct GvParams {
     const __half* X; const uint8_t* W; __half* Y;
-    uint32_t M, N, K, chunks;                // chunks = K / 256
+    uint32_t M, N, K, x_cols, x_wrap, chunks;    // chunks = K / 256; X has x_cols columns and starts over every x_wrap of K
     uint32_t rows_per_warp, lanes_per_row;   // chunks < 32: 32 / chunks rows per warp; else 1 row, 32 lanes
     const uint8_t* meta;                     // planar layouts: scale / bias planes behind the packed plane
     const __half* row_scale;                 // per-row scale (integer-valued codecs)
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(GV_THREADS) qgemv_kernel(const GvParams p) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t i = tid; i < M * p.K; i += GV_THREADS) {
         const uint32_t m = i / p.K, k = i % p.K;
-        sx[(size_t)m * p.chunks * XSTRIDE + (k >> 8) * XSTRIDE + (k & 255u)] = __half2float(p.X[(size_t)m * p.K + k]);
+        sx[(size_t)m * p.chunks * XSTRIDE + (k >> 8) * XSTRIDE + (k & 255u)] = k % p.x_wrap < p.x_cols ? __half2float(p.X[(size_t)m * p.x_cols + k % p.x_wrap]) : 0.0f;
     }
     __syncthreads();
     const uint32_t warps_total = gridDim.x * (GV_THREADS / 32), gw = blockIdx.x * (GV_THREADS / 32) + warp;
@@ -115,7 +115,7 @@ cudaError_t launch_gemv_m(const GemmArgs& a, cudaStream_t stream) {
     using Cd = cdc::Codec<FMT>;
     GvParams p;
     p.X = (const __half*)a.X; p.W = (const uint8_t*)a.W0; p.Y = (__half*)a.Y;
-    p.M = a.M; p.N = a.N; p.K = a.K; p.chunks = a.K / 256;
+    p.M = a.M; p.N = a.N; p.K = a.K; p.chunks = a.K / 256; p.x_cols = a.x_cols ? a.x_cols : a.K; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
     if (p.chunks >= 32) { p.rows_per_warp = 1; p.lanes_per_row = 32; }
     else { uint32_t lp = 1; while (lp < p.chunks) lp <<= 1; p.lanes_per_row = lp; p.rows_per_warp = 32 / lp; }
     const size_t plane = (size_t)a.N * p.chunks * Cd::ROW_BYTES;

@@ -95,18 +95,25 @@ bool TransformerLayerCoordinator::initialize_pipelines(const void*) {
         ok = dev_alloc(&impl_->rope_table, (size_t)c.M * (c.D / 2) * 8) &&
              lops::build_rope_table(impl_->rope_table, c.M, c.D, c.rope_theta, 0, impl_->stream) == cudaSuccess;
     }
-    // split-K scratch: sized for the largest projection of this layer (tokens <= 256 per tile)
+    // scratch (split K, padded copies): sized for the largest projection of this layer, each probed with the outputs it has
     if (ok) {
         size_t need = 0;
-        const uint32_t ns[4] = {hq * c.D, hkv * c.D, c.K, f};
-        const uint32_t ks[4] = {c.K, c.K, hq * c.D, c.K};
-        for (int i = 0; i < 4; i++) {
+        const void* at16 = (const void*)16;                 // alignment probes only
+        auto probe = [&](uint32_t n, uint32_t k, bool dual, bool residual, bool partial) {
             qg::GemmArgs a; memset(&a, 0, sizeof(a));
-            a.format = c.weight_format; a.M = c.M; a.N = ns[i]; a.K = ks[i];
-            a.X = (const void*)16; a.W0 = (const void*)16; a.Y = (void*)16;   // alignment probes only
-            size_t w = qg::workspace_floats(a);
+            a.format = c.weight_format; a.M = c.M; a.N = n; a.K = k; a.D = c.D;
+            a.X = at16; a.W0 = at16; a.W1 = dual ? at16 : nullptr; a.Y = (void*)16;
+            a.residual = residual ? at16 : nullptr; a.partial_out = partial ? (float*)16 : nullptr;
+            const size_t w = qg::workspace_floats(a);
             if (w > need) need = w;
+        };
+        for (int form = 0; form < 3; form++) {              // plain, residual, fp32 partial sums
+            probe(hq * c.D, c.K, false, form == 1, form == 2);
+            probe(hkv * c.D, c.K, false, form == 1, form == 2);
+            probe(c.K, hq * c.D, false, form == 1, form == 2);
+            probe(c.K, f, false, form == 1, form == 2);
         }
+        probe(f, c.K, true, false, false);
         {   // the grouped Q + K + V launch
             qg::GemmArgs a; memset(&a, 0, sizeof(a));
             a.format = c.weight_format; a.M = c.M; a.N = hq * c.D; a.K = c.K; a.layout = LAYOUT_DIRECT_HEAD; a.H = hq; a.D = c.D;
@@ -116,8 +123,6 @@ bool TransformerLayerCoordinator::initialize_pipelines(const void*) {
             const size_t w = qg::workspace_floats(a);
             if (w > need) need = w;
         }
-        { qg::GemmArgs a; memset(&a, 0, sizeof(a)); a.format = c.weight_format; a.M = c.M; a.N = c.K; a.K = f;
-          a.X = (const void*)16; a.W0 = (const void*)16; a.Y = (void*)16; size_t w = qg::workspace_floats(a); if (w > need) need = w; }
         impl_->ws_floats = need;
         if (need) ok = dev_alloc((void**)&impl_->ws, need * 4);
         if (ok) ok = dev_alloc((void**)&impl_->counters, 4096 * 4 + 64);
