@@ -1,6 +1,6 @@
-// Few-token projection: Y[m][n] = sum_k X[m][k] * dequant(W)[n][k] for up to 128 tokens where one launch has too few
-// output tiles to fill the GPU (the decode-like shapes M = 33 / 127 / 128 of the router sweep,
-// bench_universal_router.mm:764-773, and every projection of a short prefill).  HBM-bound: the packed weights are
+// Few-token projection: Y[m][n] = sum_k X[m][k] * dequant(W)[n][k] for up to 128 tokens (the decode-like shapes M = 33 /
+// 127 / 128 of the router sweep, bench_universal_router.mm:764-773, and every projection of a short prefill: up to three
+// matrices in one launch, and the dual gate / up projection with SwiGLU).  HBM-bound: the packed weights are
 // read once, so what matters is how fast an SM turns packed bytes into MMA operands.
 //
 // Differences from the persistent kernel in qgemm.cu, all aimed at that:
@@ -39,11 +39,13 @@ constexpr int A_STAGES = 4;          // ring of unpacked-weight stages in tensor
 constexpr int A_COLS = KSTEP / 2;    // fp16 pairs: 32 columns per stage
 constexpr int ACC_COL = A_STAGES * A_COLS;   // accumulator behind the A ring (columns 128 ..)
 constexpr int TMEM_COLS = 256;
-constexpr int RAW_STAGES = 2, B_STAGES = 4;
+constexpr int MAX_RAW_STAGES = 6, MAX_B_STAGES = 4;   // ring depths are chosen per launch (stages_for)
 constexpr int UNPACK_WARPS = 4;      // one per lane quadrant (a second group of four measured slower: 2080 against 550 cycles per sub-tile)
 constexpr int THREADS = (UNPACK_WARPS + 2) * 32;    // warps 0-3 unpack + epilogue, warp 4 copies, warp 5 issues MMAs
 constexpr int COPY_WARP = UNPACK_WARPS, MMA_WARP = UNPACK_WARPS + 1;
 constexpr int MAX_T = 128;
+constexpr int GATE_ROWS = W_TILE / 2;    // SwiGLU tile: 64 gate rows and the same 64 up rows
+constexpr size_t SMEM_LIMIT = 112 * 1024; // two CTAs per SM
 
 // Development aid: with -DQS_TRACE the first CTA records clock64() stamps at its synchronisation points into a device
 // array that b200_debug_small_trace copies out.  Compiled out otherwise.
@@ -58,14 +60,19 @@ struct Params {
     uint32_t M, N, K, T;
     uint32_t x_wrap;             // K after which the activation columns start over
     uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;       // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
-    __half* Y;
+    uint32_t raw_stages, b_stages;
+    uint32_t swiglu;             // tiles of 64 gate rows (matrix 0) and their 64 up rows (matrix 1); output silu(g) * u
+    // grouped launch: weight tiles [0, tiles[0]) belong to matrix 0, the next tiles[1] to matrix 1, ...
+    uint32_t groups, tiles[3], grp_N[3];
+    __half* grp_Y[3];
     const __half* residual;
     uint32_t layout, D;
     int* err;
-    float* scratch;              // [k_splits][tiles][T][128] partial tiles (k_splits > 1)
-    const uint8_t* meta0;
-    const __half* row_scale0;
+    float* scratch;              // [k_splits][tiles][T][128] partial tiles (k_splits > 1, or SwiGLU)
+    const uint8_t *meta0, *meta1;
+    const __half *row_scale0, *row_scale1;
 };
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
 __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
@@ -117,7 +124,8 @@ __device__ __forceinline__ void for_each_sub(F& f, std::integer_sequence<int, S.
 
 template <int FMT>
 __global__ void __launch_bounds__(THREADS, 2)
-qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Params p) {
+qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW0,
+                   const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2, const Params p) {
     using Cd = cdc::Codec<FMT>;
     constexpr int ROW_BYTES = Cd::ROW_BYTES;
     constexpr int RAW_TILE_BYTES = ROW_BYTES * W_TILE;
@@ -130,15 +138,15 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t pad = (1024u - (ptx::smem_u32(smem_dyn) & 1023u)) & 1023u;
     uint8_t* sB = smem_dyn + pad;                                   // [B_STAGES][T rows of 128 bytes], 128-byte swizzle
     const uint32_t b_stage_bytes = p.T * 128u;
-    uint8_t* sRaw = sB + B_STAGES * b_stage_bytes;                  // [RAW_STAGES][128 rows][ROW_BYTES]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + RAW_STAGES * RAW_TILE_BYTES);
+    uint8_t* sRaw = sB + p.b_stages * b_stage_bytes;                // [raw_stages][128 rows][ROW_BYTES]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + p.raw_stages * RAW_TILE_BYTES);
     uint64_t* raw_full = bars;
-    uint64_t* raw_empty = raw_full + RAW_STAGES;
-    uint64_t* a_full = raw_empty + RAW_STAGES;
+    uint64_t* raw_empty = raw_full + MAX_RAW_STAGES;
+    uint64_t* a_full = raw_empty + MAX_RAW_STAGES;
     uint64_t* a_empty = a_full + A_STAGES;
     uint64_t* b_full = a_empty + A_STAGES;
-    uint64_t* b_empty = b_full + B_STAGES;
-    uint64_t* acc_full = b_empty + B_STAGES;
+    uint64_t* b_empty = b_full + MAX_B_STAGES;
+    uint64_t* acc_full = b_empty + MAX_B_STAGES;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
     volatile uint32_t* abort_flag = tmem_holder + 1;
 
@@ -147,13 +155,18 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t ks = blockIdx.x % p.k_splits;                    // == rank inside the cluster
     const uint32_t tile = blockIdx.x / p.k_splits;
     const uint32_t wt = tile % p.n_w_tiles, tt = tile / p.n_w_tiles;
+    // grouped launch: this tile's matrix, and the tile's place in it
+    uint32_t gi = 0u, wl = wt;
+    if (p.groups > 1u && wl >= p.tiles[0]) { wl -= p.tiles[0]; gi = 1u; if (wl >= p.tiles[1]) { wl -= p.tiles[1]; gi = 2u; } }
+    const uint32_t N = p.grp_N[gi];
+    __half* const Y = p.grp_Y[gi];
     const uint32_t kc0 = ks * p.chunks / p.k_splits, kcn = (ks + 1u) * p.chunks / p.k_splits - kc0;     // this split's packed chunks
     const uint32_t ksteps = kcn * (uint32_t)SUBS;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < RAW_STAGES; i++) { ptx::mbar_init(&raw_full[i], 1); ptx::mbar_init(&raw_empty[i], UNPACK_WARPS); }
+        for (int i = 0; i < MAX_RAW_STAGES; i++) { ptx::mbar_init(&raw_full[i], 1); ptx::mbar_init(&raw_empty[i], UNPACK_WARPS); }
         for (int i = 0; i < A_STAGES; i++) { ptx::mbar_init(&a_full[i], 4); ptx::mbar_init(&a_empty[i], 1); }
-        for (int i = 0; i < B_STAGES; i++) { ptx::mbar_init(&b_full[i], 1); ptx::mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < MAX_B_STAGES; i++) { ptx::mbar_init(&b_full[i], 1); ptx::mbar_init(&b_empty[i], 1); }
         ptx::mbar_init(acc_full, 1);
         *abort_flag = 0u;
         ptx::fence_barrier_init();
@@ -173,7 +186,8 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         // ---------------- copies: packed weight chunks run ahead of the activation tiles ----------------
         // (the packed bytes are what the launch waits for: every chunk that has a free stage is requested before the
         // activation tiles of the chunk in front of it)
-        if (lane == 0) { ptx::prefetch_tensormap(&tmW); ptx::prefetch_tensormap(&tmX); }
+        const CUtensorMap* tmW = gi == 0u ? &tmW0 : (gi == 1u ? &tmW1 : &tmW2);
+        if (lane == 0) { ptx::prefetch_tensormap(tmW); ptx::prefetch_tensormap(&tmX); }
         uint32_t rs = 0, rph = 0, bs = 0, bph = 0, raw_next = 0;
         bool ok = true;
         auto issue_raw = [&](bool block) {       // request chunk raw_next if its stage is free (block: wait for it)
@@ -187,14 +201,19 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             if (lane == 0) {
                 QST(1, raw_next);
                 ptx::mbar_arrive_expect_tx(&raw_full[rs], RAW_TILE_BYTES);
-                ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &tmW, &raw_full[rs],
-                                 (int)((kc0 + raw_next) * (ROW_BYTES / Cd::TMA_ELEM_BYTES)), (int)(wt * W_TILE));
+                const int x = (int)((kc0 + raw_next) * (ROW_BYTES / Cd::TMA_ELEM_BYTES));
+                if (p.swiglu) {          // 64-row boxes: gate rows, then the same rows of up
+                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &tmW0, &raw_full[rs], x, (int)(wt * GATE_ROWS));
+                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES + GATE_ROWS * ROW_BYTES, &tmW1, &raw_full[rs], x, (int)(wt * GATE_ROWS));
+                } else {
+                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, tmW, &raw_full[rs], x, (int)(wl * W_TILE));
+                }
             }
             __syncwarp();
             raw_next++;
-            if (++rs == RAW_STAGES) { rs = 0; rph ^= 1u; }
+            if (++rs == p.raw_stages) { rs = 0; rph ^= 1u; }
         };
-        for (int i = 0; i < RAW_STAGES; i++) issue_raw(false);
+        for (uint32_t i = 0; i < p.raw_stages; i++) issue_raw(false);
         for (uint32_t kc = 0; ok && kc < kcn; kc++) {
             if (raw_next <= kc) issue_raw(true);              // the chunk these activation tiles belong to must be on its way
             for (uint32_t s = 0; ok && s < (uint32_t)SUBS; s++) {
@@ -206,7 +225,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                                      (int)(((kc0 + kc) * Cd::CHUNK + s * KSTEP) % p.x_wrap), (int)(tt * p.T));
                 }
                 __syncwarp();
-                if (++bs == B_STAGES) { bs = 0; bph ^= 1u; }
+                if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
                 issue_raw(false);                             // a packed stage may have been released meanwhile
             }
         }
@@ -234,7 +253,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             }
             __syncwarp();
             if (++as == A_STAGES) { as = 0; aph ^= 1u; }
-            if (++bs == B_STAGES) { bs = 0; bph ^= 1u; }
+            if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
         }
         if (ok && ptx::elect_one()) ptx::umma_commit(acc_full);
         __syncwarp();
@@ -250,10 +269,10 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             // before the wait for the packed bytes
             uint32_t meta[MW] = {};
             if (Cd::META_WORDS != 0) {
-                const uint32_t n = wt * W_TILE + row;
+                const uint32_t n = p.swiglu ? wt * GATE_ROWS + (row & 63u) : wt * W_TILE + row;
                 if (n < p.N) {
                     const uint32_t groups = (p.K / 256u) * MW;
-                    const uint8_t* mp = p.meta0 + ((size_t)n * groups + (size_t)(kc0 + kc) * MW) * 2;
+                    const uint8_t* mp = (p.swiglu && row >= 64u ? p.meta1 : p.meta0) + ((size_t)n * groups + (size_t)(kc0 + kc) * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
                         const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
@@ -295,7 +314,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             for_each_sub(sub_tile, std::make_integer_sequence<int, SUBS>{});
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&raw_empty[rs]);         // after the stores that consumed every loaded register
-            if (++rs == RAW_STAGES) { rs = 0; rph ^= 1u; }
+            if (++rs == p.raw_stages) { rs = 0; rph ^= 1u; }
         }
     }
 
@@ -312,11 +331,11 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (warp < 4 && !bad) {
         ptx::tc_fence_after_sync();
         const uint32_t f = warp * 32u + lane;                       // feature row of the tile
-        const uint32_t n = wt * W_TILE + f;
+        const uint32_t n = p.swiglu ? wt * GATE_ROWS + (f & 63u) : wl * W_TILE + f;
         float rsc = 1.0f;
-        if (Cd::ROW_SCALE) rsc = n < p.N ? __half2float(p.row_scale0[n]) : 0.0f;
+        if (Cd::ROW_SCALE) rsc = n < N ? __half2float((p.swiglu && f >= 64u ? p.row_scale1 : p.row_scale0)[n]) : 0.0f;
         const uint32_t taddr = tmem_base + ((warp * 32u) << 16) + ACC_COL;
-        if (p.k_splits > 1u) {
+        if (p.k_splits > 1u || p.swiglu) {
             // [split][tile][token column][feature]: a warp's store covers 32 consecutive features of one column
             float* dst = p.scratch + ((size_t)ks * n_tiles + tile) * tile_floats + f;
             for (uint32_t c0 = 0; c0 < p.T; c0 += 16) {
@@ -334,15 +353,15 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 uint32_t v[16];
                 ptx::tmem_ld_x16(taddr + c0, v);
                 ptx::tmem_ld_wait();
-                if (n >= p.N) continue;
+                if (n >= N) continue;
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const uint32_t tok = tok0 + c0 + j;
                     if (tok >= p.M) break;
                     float a = Cd::ROW_SCALE ? __uint_as_float(v[j]) * rsc : __uint_as_float(v[j]);
-                    const size_t o = p.layout == 1 ? ((size_t)(n / p.D) * p.M + tok) * p.D + (n % p.D) : (size_t)tok * p.N + n;
+                    const size_t o = p.layout == 1 ? ((size_t)(n / p.D) * p.M + tok) * p.D + (n % p.D) : (size_t)tok * N + n;
                     if (p.residual) a += __half2float(p.residual[o]);
-                    p.Y[o] = __float2half_rn(a);
+                    Y[o] = __float2half_rn(a);
                 }
             }
         }
@@ -351,28 +370,38 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // every partial tile of the cluster is written (release / acquire at cluster scope covers the global stores)
     cluster_sync_all();
     if (threadIdx.x == 0) QST(0, 6);
-    if (!bad && p.k_splits > 1u) {
+    if (!bad && (p.k_splits > 1u || p.swiglu)) {
         // this CTA's token columns [ks * cols, (ks + 1) * cols): sum over the splits in split order, write fp16
         const uint32_t cols = p.T / p.k_splits;
         const float* base = p.scratch + (size_t)tile * tile_floats + (size_t)(ks * cols) * W_TILE;
         const size_t split_stride = (size_t)n_tiles * tile_floats;
         const uint32_t tok0 = tt * p.T + ks * cols;
-        for (uint32_t i = threadIdx.x; i < cols * (W_TILE / 4); i += THREADS) {
-            const uint32_t cl = i / (W_TILE / 4), f = (i % (W_TILE / 4)) * 4u;
-            const uint32_t tok = tok0 + cl, n = wt * W_TILE + f;
-            if (tok >= p.M || n >= p.N) continue;
-            float4 acc = __ldcg(reinterpret_cast<const float4*>(base + (size_t)cl * W_TILE + f));
+        auto sum4 = [&](const float* at) {
+            float4 acc = __ldcg(reinterpret_cast<const float4*>(at));
             for (uint32_t s = 1; s < p.k_splits; s++) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(base + s * split_stride + (size_t)cl * W_TILE + f));
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(at + s * split_stride));
                 acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
             }
+            return acc;
+        };
+        // four features per thread; a SwiGLU tile's features 64 .. 127 are the up projections of 0 .. 63
+        const uint32_t quads = p.swiglu ? GATE_ROWS / 4 : W_TILE / 4;
+        for (uint32_t i = threadIdx.x; i < cols * quads; i += THREADS) {
+            const uint32_t cl = i / quads, f = (i % quads) * 4u;
+            const uint32_t tok = tok0 + cl, n = p.swiglu ? wt * GATE_ROWS + f : wl * W_TILE + f;
+            if (tok >= p.M || n >= N) continue;
+            const float4 acc = sum4(base + (size_t)cl * W_TILE + f);
             float a[4] = {acc.x, acc.y, acc.z, acc.w};
+            if (p.swiglu) {
+                const float4 u = sum4(base + (size_t)cl * W_TILE + GATE_ROWS + f);
+                a[0] = silu_mul(a[0], u.x); a[1] = silu_mul(a[1], u.y); a[2] = silu_mul(a[2], u.z); a[3] = silu_mul(a[3], u.w);
+            }
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                if (n + e >= p.N) break;
-                const size_t o = p.layout == 1 ? ((size_t)((n + e) / p.D) * p.M + tok) * p.D + ((n + e) % p.D) : (size_t)tok * p.N + n + e;
+                if (n + e >= N) break;
+                const size_t o = p.layout == 1 ? ((size_t)((n + e) / p.D) * p.M + tok) * p.D + ((n + e) % p.D) : (size_t)tok * N + n + e;
                 if (p.residual) a[e] += __half2float(p.residual[o]);
-                p.Y[o] = __float2half_rn(a[e]);
+                Y[o] = __float2half_rn(a[e]);
             }
         }
     }
@@ -419,11 +448,20 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, uint64_t 
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, chunks; size_t smem; };
+struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, chunks, raw_stages, b_stages; size_t smem; };
 
 // alignment slack + activation ring + packed ring + barrier block
-template <int FMT> size_t smem_bytes(uint32_t T) {
-    return 1024 + (size_t)B_STAGES * T * 128 + (size_t)RAW_STAGES * cdc::Codec<FMT>::ROW_BYTES * W_TILE + 256;
+template <int FMT> size_t smem_bytes(uint32_t T, uint32_t raw_stages, uint32_t b_stages) {
+    return 1024 + (size_t)b_stages * T * 128 + (size_t)raw_stages * cdc::Codec<FMT>::ROW_BYTES * W_TILE + 256;
+}
+// Packed chunks in flight cover the latency of HBM: at least three of them where two CTAs still fit an SM, the fourth
+// activation stage giving way; what is left over goes to further chunks.
+template <int FMT> void stages_for(uint32_t T, uint32_t chunks, uint32_t& raw, uint32_t& b) {
+    b = MAX_B_STAGES;
+    while (b > 2u && smem_bytes<FMT>(T, 2, b) > SMEM_LIMIT) b--;          // (the 272-byte rows at 128 tokens: two)
+    if (b > 3u && smem_bytes<FMT>(T, 3, b) > SMEM_LIMIT && smem_bytes<FMT>(T, 3, b - 1) <= SMEM_LIMIT) b--;
+    raw = 2;
+    while (raw < (uint32_t)MAX_RAW_STAGES && raw < chunks && smem_bytes<FMT>(T, raw + 1, b) <= SMEM_LIMIT) raw++;
 }
 
 int g_sms = 0;
@@ -434,10 +472,13 @@ int sms() {
 
 template <int FMT> bool make_plan(const GemmArgs& a, Plan& pl) {
     using Cd = cdc::Codec<FMT>;
+    static_assert(1024 + 2 * MAX_T * 128 + 2 * Cd::ROW_BYTES * W_TILE + 256 <= SMEM_LIMIT, "two stages of each ring fit half an SM");
     pl.n_tok_tiles = (a.M + MAX_T - 1) / MAX_T;
     const uint32_t per = (a.M + pl.n_tok_tiles - 1) / pl.n_tok_tiles;
     pl.T = (per + 15u) & ~15u;
-    pl.n_w_tiles = (a.N + W_TILE - 1) / W_TILE;
+    const uint32_t rows_per_tile = a.W1 ? GATE_ROWS : W_TILE;        // output features per tile
+    pl.n_w_tiles = (a.N + rows_per_tile - 1) / rows_per_tile;
+    for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) pl.n_w_tiles += (a.N_extra[e] + W_TILE - 1) / W_TILE;
     const uint32_t chunks = a.K / Cd::CHUNK;
     const uint32_t tiles = pl.n_tok_tiles * pl.n_w_tiles;
     // split K while all CTAs still fit on the GPU at two per SM, every split keeps a whole chunk, and the token columns
@@ -446,19 +487,21 @@ template <int FMT> bool make_plan(const GemmArgs& a, Plan& pl) {
     for (uint32_t s = 2; s <= 8; s *= 2) {
         if (tiles * s > 2u * (uint32_t)sms() || chunks < s || pl.T % s != 0) break;
         if (a.lean && chunks % s != 0) break;
+        if (a.n_extra && chunks / s < 2) break;       // grouped launches: the persistent kernel's rule, so that both split alike
         pl.k_splits = s;
     }
     pl.chunks = chunks;
     // at least 80 KB, so that no more than two CTAs share an SM: each holds 256 of the SM's 512 tensor-memory columns, and a
     // third CTA would sit in tcgen05.alloc until one of the others leaves
-    pl.smem = smem_bytes<FMT>(pl.T);
+    stages_for<FMT>(pl.T, (chunks + pl.k_splits - 1) / pl.k_splits, pl.raw_stages, pl.b_stages);
+    pl.smem = smem_bytes<FMT>(pl.T, pl.raw_stages, pl.b_stages);
     if (pl.smem < 80 * 1024) pl.smem = 80 * 1024;
     return tiles * pl.k_splits <= 65535u * 8u;
 }
 
 template <int FMT> size_t scratch_floats_fmt(const GemmArgs& a) {
     Plan pl;
-    if (!make_plan<FMT>(a, pl) || pl.k_splits <= 1) return 0;
+    if (!make_plan<FMT>(a, pl) || (pl.k_splits <= 1 && !a.W1)) return 0;
     return (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE;
 }
 
@@ -466,24 +509,40 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
     using Cd = cdc::Codec<FMT>;
     Plan pl;
     if (!make_plan<FMT>(a, pl)) return cudaErrorInvalidValue;
-    if (pl.k_splits > 1 && (!ws.partial || ws.partial_floats < (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE))
+    if ((pl.k_splits > 1 || a.W1) && (!ws.partial || ws.partial_floats < (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE))
         return cudaErrorInvalidValue;
     const uint64_t w_row_bytes = (uint64_t)(a.K / Cd::CHUNK) * Cd::ROW_BYTES;
     const uint32_t x_cols = a.x_cols ? a.x_cols : a.K;          // columns past the end read as zero
-    CUtensorMap tmX, tmW;
+    CUtensorMap tmX, tmW0, tmW1, tmW2;
     if (!make_map(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.X, x_cols, a.M, (uint64_t)x_cols * 2, KSTEP, pl.T, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     constexpr int EB = Cd::TMA_ELEM_BYTES;
-    if (!make_map(&tmW, EB == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, a.W0, w_row_bytes / EB, a.N, w_row_bytes,
-                  Cd::ROW_BYTES / EB, W_TILE, Cd::RAW_SWIZZLE_128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE))
-        return cudaErrorInvalidValue;
+    auto weight_map = [&](CUtensorMap* m, const void* w, uint32_t n) {
+        return make_map(m, EB == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, w, w_row_bytes / EB, n, w_row_bytes,
+                        Cd::ROW_BYTES / EB, a.W1 ? GATE_ROWS : W_TILE, Cd::RAW_SWIZZLE_128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
+    };
+    // second and third map: the up matrix of a SwiGLU launch, or the extra matrices of a grouped one
+    if (!weight_map(&tmW0, a.W0, a.N)) return cudaErrorInvalidValue;
+    tmW1 = tmW0; tmW2 = tmW0;
+    if (a.W1 && !weight_map(&tmW1, a.W1, a.N)) return cudaErrorInvalidValue;
+    if (a.n_extra > 0 && !weight_map(&tmW1, a.W_extra[0], a.N_extra[0])) return cudaErrorInvalidValue;
+    if (a.n_extra > 1 && !weight_map(&tmW2, a.W_extra[1], a.N_extra[1])) return cudaErrorInvalidValue;
     Params p;
     p.M = a.M; p.N = a.N; p.K = a.K; p.T = pl.T; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
     p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
-    p.Y = (__half*)a.Y; p.residual = (const __half*)a.residual; p.layout = (uint32_t)a.layout; p.D = a.D ? a.D : 2;
+    p.raw_stages = pl.raw_stages; p.b_stages = pl.b_stages; p.swiglu = a.W1 ? 1u : 0u;
+    p.groups = 1u + a.n_extra;
+    p.tiles[0] = (a.N + W_TILE - 1) / W_TILE; p.grp_N[0] = a.N; p.grp_Y[0] = (__half*)a.Y;
+    for (uint32_t e = 0; e < 2u; e++) {
+        const bool on = e < a.n_extra;
+        p.tiles[1 + e] = on ? (a.N_extra[e] + W_TILE - 1) / W_TILE : 0u;
+        p.grp_N[1 + e] = on ? a.N_extra[e] : 0u; p.grp_Y[1 + e] = on ? (__half*)a.Y_extra[e] : nullptr;
+    }
+    p.residual = (const __half*)a.residual; p.layout = (uint32_t)a.layout; p.D = a.D ? a.D : 2;
     p.err = ws.err; p.scratch = ws.partial;
     p.meta0 = (const uint8_t*)a.W0 + (size_t)a.N * w_row_bytes;
-    p.row_scale0 = (const __half*)p.meta0;
+    p.meta1 = a.W1 ? (const uint8_t*)a.W1 + (size_t)a.N * w_row_bytes : p.meta0;
+    p.row_scale0 = (const __half*)p.meta0; p.row_scale1 = (const __half*)p.meta1;
     static uint64_t attr_mask = 0;
     static std::mutex mu;
     {
@@ -491,7 +550,7 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
         cudaGetDevice(&dev);
         std::lock_guard<std::mutex> lock(mu);
         if (!(dev >= 0 && dev < 64 && ((attr_mask >> dev) & 1u))) {
-            cudaError_t e = cudaFuncSetAttribute(qgemm_small_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<FMT>(MAX_T));
+            cudaError_t e = cudaFuncSetAttribute(qgemm_small_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 64) attr_mask |= 1ull << dev;
         }
@@ -508,7 +567,7 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // prologue may overlap the previous kernel's tail
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, qgemm_small_kernel<FMT>, tmX, tmW, p);
+    return cudaLaunchKernelEx(&cfg, qgemm_small_kernel<FMT>, tmX, tmW0, tmW1, tmW2, p);
 }
 
 int g_mode = 1;
@@ -526,7 +585,12 @@ extern "C" int b200_debug_small_trace(unsigned long long* out) {
 
 bool small_path_ok(const GemmArgs& a) {
     if (small::g_mode == 0 || a.force_generic) return false;
-    if (a.W1 || a.partial_out || a.scatter.world || a.n_extra || a.post[0] || a.post[1] || a.post[2]) return false;
+    if (a.partial_out || a.scatter.world || a.wait_rows.flags || a.post[0] || a.post[1] || a.post[2]) return false;
+    if (a.W1 && (((uintptr_t)a.W1 & 15u) || a.residual || a.layout != 0 || a.n_extra)) return false;
+    // (matrices of a grouped launch: plain block formats, as on the persistent kernel)
+    if (a.n_extra && (a.n_extra > 2 || a.residual || a.format == QUANT_TERNARY_ROW || a.format == QUANT_MLX_4BIT_G64 || a.format == QUANT_MLX_4BIT_PLANAR)) return false;
+    for (uint32_t e = 0; e < a.n_extra && e < 2u; e++)
+        if (!a.W_extra[e] || ((uintptr_t)a.W_extra[e] & 15u) || !a.Y_extra[e] || a.N_extra[e] == 0) return false;
     if (a.M == 0 || a.N == 0 || a.K == 0) return false;
     if (((uintptr_t)a.X & 15u) || ((uintptr_t)a.W0 & 15u) || ((uintptr_t)a.Y & 3u)) return false;
     if (a.residual && (a.layout != 0 || ((uintptr_t)a.residual & 1u))) return false;
@@ -539,14 +603,12 @@ bool small_path_ok(const GemmArgs& a) {
         default: return false;
     }
     if (a.K % chunk != 0) return false;
-    // worthwhile where the persistent kernel would leave SMs idle: fewer output tiles (at its tile height) than SMs
-    const uint32_t big_tiles = ((a.M + 255u) / 256u) * ((a.N + 127u) / 128u);
-    int dev = 0, n_sm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-    // (one token tile of up to 128 tokens: with two, every weight tile would be unpacked twice)
+    // One token tile of up to 128 tokens (with two, every weight tile would be unpacked twice), and at most two tiles per SM:
+    // beyond that the persistent kernel, which starts on the next tile while the last one drains, is as fast.
     if (small::g_mode == 2) return true;
-    return a.M <= (uint32_t)small::MAX_T && big_tiles < (uint32_t)n_sm;
+    uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
+    for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) tiles += (a.N_extra[e] + 127u) / 128u;
+    return a.M <= (uint32_t)small::MAX_T && tiles <= 2u * (uint32_t)small::sms();
 }
 
 #define QG_SMALL_DISPATCH(EXPR)                                                            \
