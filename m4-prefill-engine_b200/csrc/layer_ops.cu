@@ -6,17 +6,36 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <mutex>
 
 #include "../../include/b200_bridge.h"
 #include "bridge_state.cuh"
 #include "layer_ops.cuh"
+#include "ptx.cuh"
 
 namespace lops {
+
+// Every kernel of this file that a layer runs is launched so that its CTAs may be placed while the kernel in front of it
+// drains (programmatic stream serialization); it touches memory only behind grid_dependency_wait, and lets the next kernel do
+// the same from its own start.
+template <class... P, class... A>
+static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // one CTA of 256 threads per row; each thread walks 8-element vectors
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* __restrict__ X, const __half* __restrict__ W,
                                                       __half* __restrict__ Y, uint32_t K, float eps) {
+    ptx::launch_dependents();
+    ptx::grid_dependency_wait();
     const __half* x = X + (size_t)blockIdx.x * K;
     __half* y = Y + (size_t)blockIdx.x * K;
     float ss = 0.0f;
@@ -165,6 +184,8 @@ __global__ void add_residual_f16_kernel(const __half* __restrict__ A, const __ha
 __global__ void __launch_bounds__(256) rmsnorm_add_kernel(const __half* A, const __half* __restrict__ B,
                                                           const __half* __restrict__ W, __half* __restrict__ S, __half* Y,
                                                           uint32_t K, float eps) {
+    ptx::launch_dependents();
+    ptx::grid_dependency_wait();
     const size_t row = (size_t)blockIdx.x * K;
     float ss = 0.0f;
     for (uint32_t i = threadIdx.x; i < K / 8; i += blockDim.x) {
@@ -209,16 +230,14 @@ __global__ void __launch_bounds__(256) rmsnorm_add_kernel(const __half* A, const
 }
 
 cudaError_t rmsnorm(const void* X, const void* weight, void* Y, uint32_t M, uint32_t K, float eps, cudaStream_t s) {
-    rmsnorm_kernel<<<M, 256, 0, s>>>((const __half*)X, (const __half*)weight, (__half*)Y, K, eps);
-    return cudaGetLastError();
+    return launch_pdl(rmsnorm_kernel, dim3(M), 256, s, (const __half*)X, (const __half*)weight, (__half*)Y, K, eps);
 }
 cudaError_t rmsnorm_add(const void* A, const void* B, const void* weight, void* S, void* Y, uint32_t M, uint32_t K, float eps,
                         cudaStream_t s) {
     if (K % 8 != 0 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(weight) |
                         reinterpret_cast<uintptr_t>(S) | reinterpret_cast<uintptr_t>(Y)) & 15u))
         return cudaErrorInvalidValue;
-    rmsnorm_add_kernel<<<M, 256, 0, s>>>((const __half*)A, (const __half*)B, (const __half*)weight, (__half*)S, (__half*)Y, K, eps);
-    return cudaGetLastError();
+    return launch_pdl(rmsnorm_add_kernel, dim3(M), 256, s, (const __half*)A, (const __half*)B, (const __half*)weight, (__half*)S, (__half*)Y, K, eps);
 }
 cudaError_t rope(void* X, uint32_t H, uint32_t M, uint32_t D, float theta, uint32_t pos0, cudaStream_t s) {
     if (D % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 3u) == 0) {
@@ -231,99 +250,109 @@ cudaError_t rope(void* X, uint32_t H, uint32_t M, uint32_t D, float theta, uint3
     return cudaGetLastError();
 }
 // Everything between the Q/K/V projections and attention in one pass: rotary embedding on Q and K (in place for Q),
-// K and V compressed to Q8_0 records.  One warp per token walks that token's rows of all heads: a row of D = 128 fp16 is
-// 8 bytes per lane, the rotation partner (i +- D/2) sits 16 lanes away, the 32 values of a Q8_0 record are those of 8
-// neighbouring lanes, and the token's (cos, sin) values are read from the table once and reused for every head.
+// K and V compressed to Q8_0 records and overwritten by the values those give back.  A warp takes one token and one batch of
+// four rows -- four Q heads, or K and V of two kv heads (blockIdx.y: first the batches of Q, then those of K and V) -- so
+// that its four loads are in flight together and a 33-token launch still has a hundred CTAs.  (One warp per token walking all
+// heads was a chain of memory latencies: 16.4 us between events for 33 tokens of the 8B shape, 7.2 now; 20.5 -> 16.4 for 2048.)  Lane l holds elements E l .. E l + E - 1 of a row, E = D / 32;
+// the rotation partner (i +- D/2) sits 16 lanes away and the 32 values of a Q8_0 record are those of 32 / E neighbouring lanes.
 // Arithmetic is that of rope_heads_kernel and of attn::quantize_q8_0_kernel, bit for bit.
-__global__ void __launch_bounds__(128) kv_post_d128_kernel(__half* __restrict__ Q, const __half* __restrict__ Kin, const __half* __restrict__ Vin,
-                                                           uint8_t* __restrict__ Kq, uint8_t* __restrict__ Vq, __half* __restrict__ Kout,
-                                                           __half* __restrict__ Vout, const float2* __restrict__ table, uint32_t Hq, uint32_t Hkv,
-                                                           uint32_t M, int rope, int q8, int dq) {
-    constexpr uint32_t D = 128, HALF = 64;
+template <int D>
+__global__ void __launch_bounds__(128) kv_post_kernel(__half* Q, __half* K, __half* V, uint8_t* __restrict__ Kq, uint8_t* __restrict__ Vq,
+                                                      const float2* __restrict__ table, uint32_t Hq, uint32_t Hkv, uint32_t M, int rope, int q8, int dq) {
+    constexpr int E = D / 32, W = E / 2;          // elements and 32-bit words per lane
+    ptx::launch_dependents();
+    ptx::grid_dependency_wait();
     const uint32_t m = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (m >= M) return;
+    const uint32_t q_batches = rope ? (Hq + 3u) / 4u : 0u;
+    const bool is_q = blockIdx.y < q_batches;
+    // row u of the batch: its head, and the matrix it belongs to
+    uint32_t head[4];
+    __half* base[4];
+    bool on[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4u; u++) {
+        head[u] = is_q ? blockIdx.y * 4u + u : (blockIdx.y - q_batches) * 2u + (u >> 1);
+        base[u] = is_q ? Q : ((u & 1u) ? V : K);
+        on[u] = head[u] < (is_q ? Hq : Hkv);
+    }
+    uint32_t w[4][W];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (on[u]) {
+            const __half* src = base[u] + ((size_t)head[u] * M + m) * D + lane * E;
+            if (W == 2) { const uint2 t = *reinterpret_cast<const uint2*>(src); w[u][0] = t.x; w[u][W - 1] = t.y; }
+            else w[u][0] = *reinterpret_cast<const uint32_t*>(src);
+        }
     const bool upper = lane >= 16u;
-    float2 cs[4];
+    float2 cs[E];
     if (rope) {
-        const float4* t4 = reinterpret_cast<const float4*>(table + (size_t)m * HALF + (lane & 15u) * 4u);
-        const float4 a = __ldg(t4), b = __ldg(t4 + 1);
-        cs[0] = make_float2(a.x, a.y); cs[1] = make_float2(a.z, a.w); cs[2] = make_float2(b.x, b.y); cs[3] = make_float2(b.z, b.w);
+        const float4* t4 = reinterpret_cast<const float4*>(table + (size_t)m * (D / 2) + (lane & 15u) * E);
+#pragma unroll
+        for (int e = 0; e < W; e++) { const float4 t = __ldg(t4 + e); cs[2 * e] = make_float2(t.x, t.y); cs[2 * e + 1] = make_float2(t.z, t.w); }
     }
-    auto rotate = [&](uint2 w) {
-        uint2 pw;
-        pw.x = __shfl_xor_sync(0xffffffffu, w.x, 16); pw.y = __shfl_xor_sync(0xffffffffu, w.y, 16);
-        const float2 x01 = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), x23 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-        const float2 y01 = __half22float2(*reinterpret_cast<const __half2*>(&pw.x)), y23 = __half22float2(*reinterpret_cast<const __half2*>(&pw.y));
-        const float x[4] = {x01.x, x01.y, x23.x, x23.y}, y[4] = {y01.x, y01.y, y23.x, y23.y};
-        float r[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++)      // lower half: a*c - b*s with (a, b) = (x, y); upper half: b*c + a*s with (a, b) = (y, x)
-            r[e] = upper ? __fmaf_rn(x[e], cs[e].x, __fmul_rn(y[e], cs[e].y)) : __fmaf_rn(x[e], cs[e].x, -__fmul_rn(y[e], cs[e].y));
-        const __half2 h01 = __floats2half2_rn(r[0], r[1]), h23 = __floats2half2_rn(r[2], r[3]);
-        uint2 o;
-        o.x = *reinterpret_cast<const uint32_t*>(&h01); o.y = *reinterpret_cast<const uint32_t*>(&h23);
-        return o;
-    };
-    // rec_row: the four records of this (head, token) row; dq_row (optional): the row's values as the cache will give them
-    // back, fp16(q * fp16(d)) -- what attention over the Q8_0 cache multiplies with
-    auto quantise = [&](uint2 w, uint8_t* rec_row, __half* dq_row) {
-        const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), f23 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-        const float v[4] = {f01.x, f01.y, f23.x, f23.y};
-        float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-        const float d = __fdiv_rn(amax, 127.0f);
-        const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-        uint16_t* o = reinterpret_cast<uint16_t*>(rec_row + (lane >> 3) * 34u);
-        const __half dh = __float2half_rn(d);
-        if ((lane & 7u) == 0u) o[0] = __half_as_ushort(dh);
-        uint32_t back[2];
+    for (int u = 0; u < 4; u++) {
+        if (!on[u]) continue;                     // (the same for every lane of the warp)
+        const bool is_v = !is_q && (u & 1);
+        __half* dst = base[u] + ((size_t)head[u] * M + m) * D + lane * E;
+        if (rope && !is_v) {
+            uint32_t r[W];
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-            int q0 = (int)roundf(__fmul_rn(v[2 * e], id)), q1 = (int)roundf(__fmul_rn(v[2 * e + 1], id));
-            q0 = max(-128, min(127, q0)); q1 = max(-128, min(127, q1));
-            o[1 + (lane & 7u) * 2u + e] = (uint16_t)((uint32_t)(uint8_t)(int8_t)q0 | ((uint32_t)(uint8_t)(int8_t)q1 << 8));
-            back[e] = (uint32_t)__half_as_ushort(__hmul(__int2half_rn(q0), dh)) | ((uint32_t)__half_as_ushort(__hmul(__int2half_rn(q1), dh)) << 16);
+            for (int i = 0; i < W; i++) {
+                const uint32_t pw = __shfl_xor_sync(0xffffffffu, w[u][i], 16);
+                const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&w[u][i])), y = __half22float2(*reinterpret_cast<const __half2*>(&pw));
+                const float2 c0 = cs[2 * i], c1 = cs[2 * i + 1];
+                // lower half: a*c - b*s with (a, b) = (x, y); upper half: b*c + a*s with (a, b) = (y, x)
+                const float r0 = upper ? __fmaf_rn(x.x, c0.x, __fmul_rn(y.x, c0.y)) : __fmaf_rn(x.x, c0.x, -__fmul_rn(y.x, c0.y));
+                const float r1 = upper ? __fmaf_rn(x.y, c1.x, __fmul_rn(y.y, c1.y)) : __fmaf_rn(x.y, c1.x, -__fmul_rn(y.y, c1.y));
+                const __half2 h = __floats2half2_rn(r0, r1);
+                r[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+#pragma unroll
+            for (int i = 0; i < W; i++) w[u][i] = r[i];
         }
-        if (dq_row) *reinterpret_cast<uint2*>(dq_row + lane * 4u) = make_uint2(back[0], back[1]);
-    };
-    if (rope) {
-        // heads in batches of four: the loads of a batch are issued before its first store
-        for (uint32_t h0 = 0; h0 < Hq; h0 += 4) {
-            uint2 w[4];
+        bool write = rope && !is_v;
+        if (!is_q && q8) {
+            float v[E], amax = 0.0f;
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (h0 + u < Hq) w[u] = *reinterpret_cast<const uint2*>(Q + ((size_t)(h0 + u) * M + m) * D + lane * 4u);
+            for (int i = 0; i < W; i++) { const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[u][i])); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (h0 + u < Hq) *reinterpret_cast<uint2*>(Q + ((size_t)(h0 + u) * M + m) * D + lane * 4u) = rotate(w[u]);
+            for (int e = 0; e < E; e++) amax = fmaxf(amax, fabsf(v[e]));
+#pragma unroll
+            for (int o = 1; o < 32 / E; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            const float d = __fdiv_rn(amax, 127.0f);
+            const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+            const uint32_t part = lane % (32u / E);          // this lane's place in its record
+            uint16_t* o = reinterpret_cast<uint16_t*>((is_v ? Vq : Kq) + (((size_t)head[u] * M + m) * (D / 32) + lane / (32u / E)) * 34u);
+            const __half dh = __float2half_rn(d);
+            if (part == 0u) o[0] = __half_as_ushort(dh);
+#pragma unroll
+            for (int i = 0; i < W; i++) {
+                int q0 = (int)roundf(__fmul_rn(v[2 * i], id)), q1 = (int)roundf(__fmul_rn(v[2 * i + 1], id));
+                q0 = max(-128, min(127, q0)); q1 = max(-128, min(127, q1));
+                o[1u + part * W + i] = (uint16_t)((uint32_t)(uint8_t)(int8_t)q0 | ((uint32_t)(uint8_t)(int8_t)q1 << 8));
+                w[u][i] = (uint32_t)__half_as_ushort(__hmul(__int2half_rn(q0), dh)) | ((uint32_t)__half_as_ushort(__hmul(__int2half_rn(q1), dh)) << 16);
+            }
+            write = dq;
         }
-    }
-    for (uint32_t h = 0; h < Hkv; h++) {
-        const size_t row = ((size_t)h * M + m);
-        uint2 k = *reinterpret_cast<const uint2*>(Kin + row * D + lane * 4u);
-        const uint2 v = *reinterpret_cast<const uint2*>(Vin + row * D + lane * 4u);
-        if (rope) k = rotate(k);
-        if (q8) {
-            quantise(k, Kq + row * (D / 32u) * 34u, dq ? Kout + row * D : nullptr);
-            quantise(v, Vq + row * (D / 32u) * 34u, dq ? Vout + row * D : nullptr);
-        } else if (rope) {
-            *reinterpret_cast<uint2*>(Kout + row * D + lane * 4u) = k;
+        if (write) {
+            if (W == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(w[u][0], w[u][W - 1]);
+            else *reinterpret_cast<uint32_t*>(dst) = w[u][0];
         }
     }
 }
 
 cudaError_t kv_post(void* Q, void* K, void* V, void* Kq, void* Vq, const void* rope_table, uint32_t Hq, uint32_t Hkv,
                     uint32_t M, uint32_t D, bool rope, bool q8, bool dequant_in_place, cudaStream_t s) {
-    if (D != 128 || (rope && !rope_table) || (q8 && (!Kq || !Vq))) return cudaErrorInvalidValue;
+    if ((D != 64 && D != 128) || (rope && !rope_table) || (q8 && (!Kq || !Vq))) return cudaErrorInvalidValue;
     if (((reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V)) & 7u) ||
         (reinterpret_cast<uintptr_t>(rope_table) & 15u))
         return cudaErrorInvalidValue;
-    kv_post_d128_kernel<<<(M + 3) / 4, 128, 0, s>>>((__half*)Q, (const __half*)K, (const __half*)V, (uint8_t*)Kq, (uint8_t*)Vq, (__half*)K,
-                                                   (__half*)V, (const float2*)rope_table, Hq, Hkv, M, rope ? 1 : 0, q8 ? 1 : 0,
-                                                   (q8 && dequant_in_place) ? 1 : 0);
-    return cudaGetLastError();
+    const uint32_t batches = (rope ? (Hq + 3) / 4 : 0) + (Hkv + 1) / 2;
+    if (batches > 65535u) return cudaErrorInvalidValue;
+    return launch_pdl(D == 128 ? kv_post_kernel<128> : kv_post_kernel<64>, dim3((M + 3) / 4, batches), 128, s, (__half*)Q, (__half*)K, (__half*)V,
+                      (uint8_t*)Kq, (uint8_t*)Vq, (const float2*)rope_table, Hq, Hkv, M, rope ? 1 : 0, q8 ? 1 : 0, (q8 && dequant_in_place) ? 1 : 0);
 }
 
 cudaError_t build_rope_table(void* table, uint32_t M, uint32_t D, float theta, uint32_t pos0, cudaStream_t s) {
