@@ -381,37 +381,49 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (cnt > 0u && ok) ok = __all_sync(0xffffffffu, ptx::mbar_wait<64>(&o_full[g], 0u, abort_flag, p.err, 227));
         if (cnt > 0u && ok) {
             ptx::tc_fence_after_sync();
+            // Rows leave through the tile's Q buffer, which nothing reads any more: a thread deposits the 16-byte chunks of its
+            // row (chunk c of row r at c ^ (r & 7): no bank conflict either way), then the warp moves its own 32 rows with whole
+            // rows per store.  (Stores straight from the accumulator touch 32 rows each: about 4 us per CTA for fp32 partials.)
+            constexpr uint32_t CH = D / 8;                           // chunks of a row per pass: D fp16, or D / 2 fp32
             const uint32_t head = hk * p.G + hl;
             const bool row_ok = hl < p.G && pos < p.M;
-            if (p.split) {
-                const size_t r = (size_t)blockIdx.z * p.Hq * p.M + (size_t)head * p.M + pos;
-                float* dst = p.part_o + r * D;
-                if (row_ok) p.part_ml[r] = make_float2(m_run, l_run);
-#pragma unroll
-                for (int c = 0; c < D; c += 32) {
+            const size_t r = (size_t)head * p.M + pos;
+            const size_t split_row = (size_t)blockIdx.z * p.Hq * p.M + r;
+            uint8_t* dst = p.split ? reinterpret_cast<uint8_t*>(p.part_o + split_row * D)
+                                   : reinterpret_cast<uint8_t*>(p.O + (p.out_tokens_major ? ((size_t)pos * p.Hq + head) * D : r * D));
+            if (!row_ok) dst = nullptr;
+            if (p.split && row_ok) p.part_ml[split_row] = make_float2(m_run, l_run);
+            const float inv = p.split ? 1.0f : (l_run > 0.0f ? 1.0f / l_run : 0.0f);
+            uint8_t* stage = sQ + g * C::TILE;
+            const uint32_t row0 = (warp & 3u) * 32u;
+            const uint32_t cols = p.split ? D / 2u : (uint32_t)D;    // accumulator columns per pass
+            for (uint32_t c0 = 0; c0 < (uint32_t)D; c0 += cols) {
+                for (uint32_t c = 0; c < cols; c += 32u) {
                     float v[32];
-                    tmem_ld_x32(tOg + c, v);
+                    tmem_ld_x32(tOg + c0 + c, v);
                     ptx::tmem_ld_wait();
-                    if (row_ok) {
+                    if (p.split) {
 #pragma unroll
-                        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                        for (uint32_t j = 0; j < 8u; j++)
+                            *reinterpret_cast<float4*>(stage + row * (CH * 16u) + (((c / 4u + j) ^ (row & 7u)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < 4u; j++)
+                            *reinterpret_cast<uint4*>(stage + row * (CH * 16u) + (((c / 8u + j) ^ (row & 7u)) << 4)) =
+                                make_uint4(pack_h2(v[8 * j] * inv, v[8 * j + 1] * inv), pack_h2(v[8 * j + 2] * inv, v[8 * j + 3] * inv),
+                                           pack_h2(v[8 * j + 4] * inv, v[8 * j + 5] * inv), pack_h2(v[8 * j + 6] * inv, v[8 * j + 7] * inv));
                     }
                 }
-            } else {
-                const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-                __half* dst = p.out_tokens_major ? p.O + ((size_t)pos * p.Hq + head) * D : p.O + ((size_t)head * p.M + pos) * D;
-#pragma unroll
-                for (int c = 0; c < D; c += 32) {
-                    float v[32];
-                    tmem_ld_x32(tOg + c, v);
-                    ptx::tmem_ld_wait();
-                    if (row_ok) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 8)
-                            *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(pack_h2(v[j] * inv, v[j + 1] * inv), pack_h2(v[j + 2] * inv, v[j + 3] * inv),
-                                                                                pack_h2(v[j + 4] * inv, v[j + 5] * inv), pack_h2(v[j + 6] * inv, v[j + 7] * inv));
-                    }
+                __syncwarp();
+                const uint32_t ch = lane % CH;
+#pragma unroll 4
+                for (uint32_t j = lane / CH; j < 32u; j += 32u / CH) {
+                    uint8_t* d = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, (unsigned long long)dst, (int)j));
+                    const uint32_t rr = row0 + j;
+                    const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * (CH * 16u) + ((ch ^ (rr & 7u)) << 4));
+                    if (d) *reinterpret_cast<uint4*>(d + c0 * 4u + ch * 16u) = w;        // (c0 > 0 only for fp32 rows)
                 }
+                __syncwarp();
             }
         }
     }
@@ -464,27 +476,33 @@ __global__ void __launch_bounds__(256) combine_kernel(const Params p) {
     else *reinterpret_cast<uint32_t*>(dst) = pack_h2(acc[0], acc[1]);
 }
 
-// Q8_0 records (34 bytes: fp16 d, 32 codes; 2-byte aligned) of K and then V -> fp16, value = fp16(q * d), one rounding.  Eight
-// lanes per record: a warp reads 136 consecutive bytes and writes 256.
-__global__ void __launch_bounds__(256) dequant_q8_0_kernel(const uint8_t* __restrict__ K, const uint8_t* __restrict__ V, __half* __restrict__ out,
-                                                           size_t blocks) {
+// Q8_0 records (34 bytes: fp16 d, 32 codes; 2-byte aligned) of K and then V -> fp16, value = fp16(q * d), one rounding.  A
+// thread takes half a record (16 codes, two 16-byte stores); the integer becomes fp16 through the mantissa: 0x6400 | (q + 128)
+// is 1152 + q.
+constexpr uint32_t DEQUANT_THREADS = 256;
+__global__ void __launch_bounds__(DEQUANT_THREADS) dequant_q8_0_kernel(const uint8_t* __restrict__ K, const uint8_t* __restrict__ V, __half* __restrict__ out,
+                                                                       size_t blocks) {
     ptx::grid_dependency_wait();
     ptx::launch_dependents();
-    const size_t i = (size_t)blockIdx.x * 256u + threadIdx.x;
-    const size_t b = i >> 3;
+    const size_t i = (size_t)blockIdx.x * DEQUANT_THREADS + threadIdx.x;
+    const size_t b = i >> 1;
     if (b >= 2 * blocks) return;
-    const uint8_t* blk = b < blocks ? K + b * 34 : V + (b - blocks) * 34;
-    const uint32_t part = (uint32_t)i & 7u;
-    const __half d = *reinterpret_cast<const __half*>(blk);
-    const uint16_t* cp = reinterpret_cast<const uint16_t*>(blk + 2u + 4u * part);
-    const uint32_t c = (uint32_t)cp[0] | ((uint32_t)cp[1] << 16);
-    __half v[4];
+    const uint16_t* blk = reinterpret_cast<const uint16_t*>(b < blocks ? K + b * 34 : V + (b - blocks) * 34);
+    const uint16_t* c = blk + 1 + ((uint32_t)i & 1u) * 8u;
+    uint16_t q[8];
 #pragma unroll
-    for (int e = 0; e < 4; e++) v[e] = __hmul(__int2half_rn((int)(int8_t)(c >> (8 * e))), d);
-    uint2 o;
-    o.x = (uint32_t)__half_as_ushort(v[0]) | ((uint32_t)__half_as_ushort(v[1]) << 16);
-    o.y = (uint32_t)__half_as_ushort(v[2]) | ((uint32_t)__half_as_ushort(v[3]) << 16);
-    *reinterpret_cast<uint2*>(out + b * 32 + part * 4u) = o;
+    for (int e = 0; e < 8; e++) q[e] = __ldg(c + e);
+    const __half2 d2 = __half2half2(__ushort_as_half(__ldg(blk))), off = __half2half2(__ushort_as_half((unsigned short)0x6480));      // 1152
+    uint32_t o[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const uint32_t x = (__byte_perm((uint32_t)q[e], 0u, 0x4140u) ^ 0x00800080u) | 0x64006400u;
+        const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&x), off), d2);
+        o[e] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+    uint4* dst = reinterpret_cast<uint4*>(out + b * 32 + ((uint32_t)i & 1u) * 16u);
+    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -590,7 +608,7 @@ template <int D> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* l
     const void *Kf = a.K, *Vf = a.V;
     if (!a.kv_fp16) {
         const size_t nb = kv_elems / 32;
-        cfg.gridDim = dim3((unsigned)((2 * nb * 8 + 255) / 256)); cfg.blockDim = dim3(256);
+        cfg.gridDim = dim3((unsigned)((4 * nb + DEQUANT_THREADS - 1) / DEQUANT_THREADS)); cfg.blockDim = dim3(DEQUANT_THREADS);
         cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_q8_0_kernel, (const uint8_t*)a.K, (const uint8_t*)a.V, (__half*)scratch, nb);
         if (e != cudaSuccess) return e;
         Kf = scratch; Vf = scratch + kv_elems * sizeof(__half);
