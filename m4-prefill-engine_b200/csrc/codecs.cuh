@@ -192,17 +192,20 @@ template <> struct Codec<QUANT_Q4_K> : CodecDefaults {
             else       mn = (byte_at(r, 4 + j + 4) >> 4) | ((sj >> 6) << 4);
             // (sc, mn) as exact fp16.  q*sc <= 945 is exact in fp16, so w = fma(q*sc, d, -m_sub) rounds the
             // product once (tighter than the reference's fp16 d*sc, which rounds the sub-scale first);
-            // m_sub = dmin*mn is rounded once as in the reference.
+            // m_sub = dmin*mn is rounded once as in the reference.  The integer and its scale are one multiply-add: the
+            // nibble arrives as 1024 + q (64 + q), and 1024*sc (64*sc) has at most six significant bits, so
+            // (1024 + q)*sc - 1024*sc is q*sc exactly.
             const uint32_t scm = h2sub((sc | (mn << 16)) | H2_1024, H2_1024);
             const uint32_t sc2 = prmt(scm, 0u, 0x1010u);
             const uint32_t negm2 = prmt(h2mul(scm, d_dmin), 0u, 0x3232u) ^ 0x80008000u;
             const uint32_t d2 = prmt(d_dmin, 0u, 0x1010u);
+            const uint32_t sc1024 = h2mul(sc2, H2_1024) ^ 0x80008000u, sc64 = h2mul(sc2, H2_64) ^ 0x80008000u;
 #pragma unroll
             for (int p = 0; p < 8; p++) {
                 uint32_t lo, hi;
                 nib_pairs(spread_pair(r, 16 + 16 * j + 2 * p), lo, hi);
-                out[16 * bi + p] = h2fma(h2mul(h2sub(lo, H2_1024), sc2), d2, negm2);
-                out[16 * bi + 8 + p] = h2fma(h2mul(h2sub(hi, H2_64), sc2), d2, negm2);
+                out[16 * bi + p] = h2fma(h2fma(lo, sc2, sc1024), d2, negm2);
+                out[16 * bi + 8 + p] = h2fma(h2fma(hi, sc2, sc64), d2, negm2);
             }
         }
     }
