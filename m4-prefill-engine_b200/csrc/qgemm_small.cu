@@ -608,7 +608,14 @@ bool small_path_ok(const GemmArgs& a) {
     if (small::g_mode == 2) return true;
     uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
     for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) tiles += (a.N_extra[e] + 127u) / 128u;
-    return a.M <= (uint32_t)small::MAX_T && tiles <= 2u * (uint32_t)small::sms();
+    if (a.M > (uint32_t)small::MAX_T || tiles > 2u * (uint32_t)small::sms()) return false;
+    // SwiGLU tiles pass through the scratch buffer even unsplit, which grows with the tokens, and from 113 tokens on the
+    // persistent kernel pairs its CTAs: a short K does not make up for it (F = 8192, 128 tokens, K = 512 / 1024: 13.2 / 14.9
+    // against 10.2 / 13.0 us there; 64 tokens, K = 512 / 1024: 9.6 / 11.0 against 9.1 / 11.5; F = 14336, K = 4096, 128 tokens: 44.5
+    // against 47.5, the variable-rate codec 75.8 against 72.2).
+    const uint32_t T = (a.M + 15u) & ~15u;
+    if (a.W1 && (a.K < T * T / 4u || (T == (uint32_t)small::MAX_T && a.format == QUANT_VAR_RATE_AFFINE))) return false;
+    return true;
 }
 
 #define QG_SMALL_DISPATCH(EXPR)                                                            \
