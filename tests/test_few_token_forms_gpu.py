@@ -44,7 +44,7 @@ def test_unequal_splits(bridge, fmt, M):
         check(run_gemm(bridge, fmt, X, W, N, ex=True), o.gemm_f64(fmt, X, W, N), f"{chunks} chunks fmt {fmt} M {M}", rms_factor=rms_factor(fmt))
 
 
-@pytest.mark.parametrize("M", [129, 300])
+@pytest.mark.parametrize("M", [129, 300, 1000])       # token tiles shortened to fill the SMs
 def test_unequal_splits_persistent(bridge, M):
     for chunks, N in ((5, 130), (9, 256), (17, 64)):
         X, W = o.baseline_inputs(o.Q4_0, M, chunks * 256, N, 33)
