@@ -125,9 +125,12 @@ int b200_bridge_unregister_weights(const void* host_ptr);
 
 /* 0 if no kernel has reported a fault since init; otherwise the first code reported: a bounded wait ran out inside a
  * projection kernel (101..110; 109 the CTA-pair relay, 110 rows another rank had not written), the few-token projection
- * kernel (111..117), an attention kernel (201..204, 210..217) or the peer exchange (301, 302); 401: a token id outside the
+ * kernel (111..117), an attention kernel (201..204, 220..227) or the peer exchange (301, 302); 401: a token id outside the
  * embedding table. */
 int b200_bridge_device_error(void);
+/* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
+ * holds now, without a wait on the host.  -6 if that is not possible (a stream under capture). */
+int b200_bridge_wait_stream(void* stream);
 const char* b200_bridge_last_error_string(void);
 
 /* Kernels enqueued by this library since init (launch accounting for benchmarks). */

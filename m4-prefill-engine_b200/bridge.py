@@ -78,6 +78,8 @@ def bind(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.b200_bridge_register_weights.restype = _i
     lib.b200_bridge_unregister_weights.argtypes = [_vp]
     lib.b200_bridge_unregister_weights.restype = _i
+    lib.b200_bridge_wait_stream.argtypes = [_vp]
+    lib.b200_bridge_wait_stream.restype = _i
     lib.b200_bridge_device_error.argtypes = []
     lib.b200_bridge_device_error.restype = _i
     lib.b200_bridge_last_error_string.argtypes = []
@@ -115,6 +117,12 @@ _OPTIONAL = {
 
 def _addr(t: torch.Tensor) -> tuple[int, int]:
     return t.data_ptr(), t.numel() * t.element_size()
+
+
+def _current_stream() -> int:
+    """cudaStream_t of torch's current stream (the raw accessor where this torch has it: a tenth of the cost of the object)."""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
 
 
 class B200Bridge:
@@ -156,9 +164,11 @@ class B200Bridge:
         return bool(self._lib.m4_bridge_is_initialized())
 
     def _wait_torch(self, *tensors: torch.Tensor) -> None:
-        # inputs produced on torch's stream must be complete before the bridge stream reads them
-        if any(t.is_cuda for t in tensors):
-            torch.cuda.current_stream().synchronize()
+        # inputs produced on torch's stream must be complete before the bridge stream reads them: the GPU waits, the host
+        # only where it cannot (a stream under capture, another device, a bridge that is not up)
+        if any(t.is_cuda for t in tensors if t is not None):
+            if self._lib.b200_bridge_wait_stream(_current_stream()) != 0:
+                torch.cuda.current_stream().synchronize()
 
     def dispatch_gemm(self, X, W, Y, format, M=None, K=None, N=None, check_finite: bool = False) -> int:
         Xc, xp, xb = self.extract_buffer_address_and_size(X)

@@ -99,6 +99,7 @@ const void* stage_in(const void* ptr, size_t bytes, StageSlot& sl, DevBuf& buf, 
         if (g.main_d2h_pending) cudaStreamWaitEvent(g.stream_in, g.ev_main_d2h, 0);
     }
     if (!buf.ensure(bytes)) { *rc = -5; return nullptr; }
+    g.copies = true; g.copy_seq++;
     if (cudaMemcpyAsync(buf.p, ptr, bytes, cudaMemcpyHostToDevice, g.stream_in) != cudaSuccess) { cudaGetLastError(); *rc = -5; return nullptr; }
     g.h2d_bytes += bytes;
     *staged = true;
@@ -182,6 +183,7 @@ int run_gemm(void* X, size_t Xb, void* W0, void* W1, size_t Wb, void* Y, size_t 
         g.slot_seq++;
     }
     if (host_dst) {
+        g.copies = true; g.copy_seq++;
         cudaStreamWaitEvent(g.stream_out, sl.ev_kernel, 0);
         if (cudaMemcpyAsync(host_dst, a.Y, y_bytes, cudaMemcpyDeviceToHost, g.stream_out) != cudaSuccess) { cudaGetLastError(); return -5; }
         cudaEventRecord(sl.ev_out, g.stream_out);
@@ -225,7 +227,9 @@ bool m4_bridge_init(const char*) {
     if (cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&g.stream_in, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&g.stream_out, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); return false; }
-    bool ev_ok = cudaEventCreateWithFlags(&g.ev_main_d2h, cudaEventDisableTiming) == cudaSuccess;
+    bool ev_ok = cudaEventCreateWithFlags(&g.ev_main_d2h, cudaEventDisableTiming) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&g.ev_caller, cudaEventDisableTiming) == cudaSuccess;
+    g.copies = false;
     for (StageSlot& sl : g.slots) {
         ev_ok = ev_ok && cudaEventCreateWithFlags(&sl.ev_in, cudaEventDisableTiming) == cudaSuccess &&
                 cudaEventCreateWithFlags(&sl.ev_kernel, cudaEventDisableTiming) == cudaSuccess &&
@@ -398,17 +402,21 @@ void m4_bridge_synchronize(void) {
     // only be cleared for copies that were already enqueued when the wait began: their events are recorded under the
     // lock before the wait and queried afterwards.  A copy enqueued by another thread in between keeps its mark.
     cudaStream_t s, si, so;
-    uint64_t seq_before;
+    uint64_t seq_before, copy_seq_before;
+    bool copies;
     {
         std::lock_guard<std::mutex> lock(g.mu);
         if (!g.initialized) return;
         s = g.stream; si = g.stream_in; so = g.stream_out;
         seq_before = g.dispatch_seq;
+        copies = g.copies; copy_seq_before = g.copy_seq;
     }
-    cudaError_t e = sync_all_streams(s, si, so);
+    // (callers that hand in device pointers never use the copy streams: one wait instead of three)
+    cudaError_t e = copies ? sync_all_streams(s, si, so) : cudaStreamSynchronize(s);
     {
         std::lock_guard<std::mutex> lock(g.mu);
         if (g.initialized) {
+            if (copies && g.copy_seq == copy_seq_before) g.copies = false;
             for (StageSlot& sl : g.slots)
                 if (sl.out_pending && (sl.out_seq <= seq_before || cudaEventQuery(sl.ev_out) == cudaSuccess)) {
                     sl.out_pending = false; sl.out_ptr = nullptr; sl.out_bytes = 0;
@@ -446,6 +454,7 @@ void m4_bridge_shutdown(void) {
         sl.ev_in = sl.ev_kernel = sl.ev_out = nullptr; sl.used = false; sl.out_pending = false;
     }
     cudaEventDestroy(g.ev_main_d2h); g.ev_main_d2h = nullptr;
+    cudaEventDestroy(g.ev_caller); g.ev_caller = nullptr;
     cudaStreamDestroy(g.stream_in); cudaStreamDestroy(g.stream_out); g.stream_in = g.stream_out = nullptr;
     g.stage_x.release(); g.stage_w0.release(); g.stage_w1.release(); g.stage_y.release(); g.stage_res.release();
     g.stage_aux0.release(); g.stage_aux1.release(); g.stage_aux2.release();
@@ -458,6 +467,23 @@ void m4_bridge_shutdown(void) {
     cudaStreamDestroy(g.stream); g.stream = nullptr;
     static_scratch_forget();
     g.initialized = false;
+}
+
+/* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
+ * holds now.  -6 if that is not possible (a stream that is being captured): wait on the host instead. */
+int b200_bridge_wait_stream(void* stream) {
+    std::lock_guard<std::mutex> lock(g.mu);
+    if (!g.initialized) return -1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { cudaGetLastError(); return -6; }
+    if (cudaStreamQuery((cudaStream_t)stream) == cudaSuccess) return 0;         // nothing to wait for: one call instead of three
+    cudaGetLastError();
+    if (cudaEventRecord(g.ev_caller, (cudaStream_t)stream) != cudaSuccess || cudaStreamWaitEvent(g.stream, g.ev_caller, 0) != cudaSuccess ||
+        cudaStreamWaitEvent(g.stream_in, g.ev_caller, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return -6;
+    }
+    return 0;
 }
 
 int b200_bridge_device_error(void) {

@@ -40,6 +40,9 @@ struct State {
     cudaStream_t stream_out = nullptr;   // device -> host copies of the projection entry points
     StageSlot slots[2];
     uint64_t slot_seq = 0;
+    cudaEvent_t ev_caller = nullptr;     // last position of a caller's stream that the bridge's streams wait for
+    bool copies = false;                 // work may be under way on the copy streams
+    uint64_t copy_seq = 0;               // counts what is enqueued there
     cudaEvent_t ev_main_d2h = nullptr;   // last copy back issued on the main stream by another entry point
     bool main_d2h_pending = false;
     uint64_t main_d2h_seq = 0;

@@ -168,8 +168,7 @@ class TransformerLayerCoordinator:
 
     def forward(self, X_in, W_q, W_k, W_v, W_o, W_gate, W_up, W_down, X_out) -> None:
         ts = (X_in, W_q, W_k, W_v, W_o, W_gate, W_up, W_down, X_out)
-        if any(t.is_cuda for t in ts):
-            torch.cuda.current_stream().synchronize()
+        self.bridge._wait_torch(*ts)
         rc = self.lib.b200_layer_forward(self._h, *[t.data_ptr() for t in ts])
         if rc:
             raise RuntimeError(f"b200_layer_forward failed with status code {rc}")

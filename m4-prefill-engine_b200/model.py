@@ -235,8 +235,7 @@ class TransformerModel:
             raise IndexError(f"Token ID out of vocabulary bounds [0, {self.config.vocab_size})")
         if want_logits and logits is None:
             logits = torch.empty(self.M, self.vocab_rows, dtype=torch.float16, device="cuda")
-        if any(t is not None and t.is_cuda for t in (tokens, logits, hidden)):
-            torch.cuda.current_stream().synchronize()
+        self.bridge._wait_torch(tokens, logits, hidden)
         rc = self.lib.b200_model_forward(self._h, tokens.data_ptr(), self.M, logits.data_ptr() if logits is not None else None,
                                          hidden.data_ptr() if hidden is not None else None)
         if rc == -8:

@@ -147,13 +147,13 @@ class M4QuantizedLinear(torch.nn.Module):
             x = x.to(torch.float16)
         x = x.to(dev)
         if x.dim() == 1:
-            y = torch.zeros((N,), dtype=torch.float16, device=dev)
+            y = torch.empty((N,), dtype=torch.float16, device=dev)      # the projection writes every element
             m4_bridge_dispatch_gemv(x, self.weight, y, self.format, K, N, check_finite=check_finite)
             m4_bridge_synchronize()
             return y
         x2 = x.reshape(-1, K)
         m = x2.shape[0]
-        y2 = torch.zeros((m, N), dtype=torch.float16, device=dev)
+        y2 = torch.empty((m, N), dtype=torch.float16, device=dev)
         if m == 1:
             m4_bridge_dispatch_gemv(x2, self.weight, y2, self.format, K, N, check_finite=check_finite)
         else:

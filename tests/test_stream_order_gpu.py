@@ -1,0 +1,51 @@
+"""The bridge's work is ordered behind the caller's stream on the GPU, without a wait on the host."""
+import pytest
+import torch
+
+import oracle as o
+from gpu_util import dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_inputs_still_being_produced(bridge, side):
+    """X is overwritten by torch work that is still queued (tens of milliseconds of it) when the projection is dispatched, on the
+    default stream and on a side stream; the projection reads what that work leaves."""
+    M, K, N = 40, 512, 256
+    X, W = o.baseline_inputs(o.Q4_0, M, K, N, 5)
+    Xf, Wd = dev(X), dev(W)
+    want = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    bridge.dispatch_gemm(Xf, Wd, want, o.Q4_0)
+    bridge.synchronize()
+    stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    with torch.cuda.stream(stream):
+        a = torch.tanh(torch.randn(4096, 4096, device="cuda"))
+        a = torch.tanh(a @ a)                       # libraries and modules are loaded before the queue is filled
+        (Xf + (a.sum() * 0).to(torch.float16)).clone()
+        x = torch.zeros_like(Xf)
+        got = torch.empty_like(want)
+        torch.cuda.synchronize()
+        for _ in range(60):
+            a = torch.tanh(a @ a)
+        x.copy_(Xf + (a.sum() * 0).to(torch.float16))
+        busy = not stream.query()
+        bridge.dispatch_gemm(x, Wd, got, o.Q4_0)
+        still = not stream.query()
+        bridge.synchronize()
+    assert busy and still, "the dispatch waited on the host"
+    assert torch.equal(got, want)
+
+
+def test_stream_under_capture_is_refused(bridge):
+    s = torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    t = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        rc = bridge.lib.b200_bridge_wait_stream(torch.cuda.current_stream().cuda_stream)
+        t.add_(1)
+    assert rc == -6
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(t.sum()) == 8.0
