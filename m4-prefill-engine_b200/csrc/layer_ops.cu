@@ -18,7 +18,8 @@ namespace lops {
 
 // Every kernel of this file that a layer runs is launched so that its CTAs may be placed while the kernel in front of it
 // drains (programmatic stream serialization); it touches memory only behind grid_dependency_wait, and lets the next kernel do
-// the same from its own start.
+// the same from its own start.  The plain normalisation, which opens a layer, lets its successors be placed only once its own
+// wait is over: from there on no kernel of the layer writes packed weights, and the projections may fetch theirs early.
 template <class... P, class... A>
 static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg;
@@ -34,8 +35,8 @@ static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads,
 // one CTA of 256 threads per row; each thread walks 8-element vectors
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* __restrict__ X, const __half* __restrict__ W,
                                                       __half* __restrict__ Y, uint32_t K, float eps) {
-    ptx::launch_dependents();
     ptx::grid_dependency_wait();
+    ptx::launch_dependents();
     const __half* x = X + (size_t)blockIdx.x * K;
     __half* y = Y + (size_t)blockIdx.x * K;
     float ss = 0.0f;

@@ -109,6 +109,7 @@ template <int FMT> struct Cfg {
 
 struct Params {
     uint32_t M, N, K;
+    uint32_t early;              // packed weights may be fetched before the preceding kernel has finished
     uint32_t x_wrap;             // K after which the activation columns start over
     uint32_t T;                  // tokens per tile (multiple of 16)
     uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;    // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
@@ -536,8 +537,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
     // Everything above touched only this CTA's shared and tensor memory; global memory (inputs another kernel may
-    // still be writing, the split-K scratch the previous launch may still be using) is first touched below.
-    ptx::grid_dependency_wait();
+    // still be writing, the split-K scratch the previous launch may still be using) is first touched below -- except for packed
+    // weights that the preceding kernels are known not to write: the roles that touch anything else wait then.
+    if (!p.early) ptx::grid_dependency_wait();
     if (threadIdx.x == 0) QTRC(7, 0u, 0);
     QCTA(1);
 
@@ -588,6 +590,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     } else if (pre_epi && wq == 2u && wg == 2u) {
         // ---------------- activation producer ----------------
         if (lane == 0) ptx::prefetch_tensormap(&tmX);
+        if (p.early) ptx::grid_dependency_wait();
         uint32_t bs = 0, bph = 0, xtr = 0;
         (void)xtr;
         bool ok = true;
@@ -810,6 +813,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // ---------------- epilogue: tensor memory -> fp16 (or fp32 partials) ----------------
         const uint32_t q = warp - C::EPI_WARP0;               // == warp % 4: the TMEM lane quadrant
         const uint32_t et = threadIdx.x - C::EPI_WARP0 * 32;  // 0..127
+        if (p.early) ptx::grid_dependency_wait();
         uint32_t it = 0, xb_i = 0;
         // Fused reduce-scatter: every epilogue warp counts the tiles it has stored per owning rank (eight counters per warp
         // in shared memory).  After its last tile the warp fences its peer stores at system scope once -- a system-scope
@@ -1034,6 +1038,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     }
 
     // ---------------- teardown ----------------
+    if (p.early) ptx::grid_dependency_wait();      // (long over; the fix-up below is every warp's work)
     ptx::tc_fence_before_sync();
     __syncthreads();
     if (threadIdx.x == 0) QTRC(7, 0u, 1);
@@ -1386,6 +1391,7 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
     Params p;
     p.M = a.M; p.N = a.N; p.K = a.K;
     p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
+    p.early = a.early_weights ? 1u : 0u;
     p.T = pl.T; p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
     p.swiglu = a.W1 ? 1u : 0u;
     // Row-wise epilogue: wherever every output row can take 16-byte stores (and, with a residual, 8-byte loads).  SwiGLU

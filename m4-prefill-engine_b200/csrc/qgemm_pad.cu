@@ -143,6 +143,7 @@ cudaError_t launch_pad(const GemmArgs& a, void* dst, GemmArgs& padded, cudaStrea
         if (n > most) most = n;
     }
     padded = a;
+    padded.early_weights = 0;                    // this kernel writes them
     padded_shape(a, padded);
     padded.W0 = dst;
     if (a.W1) padded.W1 = static_cast<uint8_t*>(dst) + pl.bytes;

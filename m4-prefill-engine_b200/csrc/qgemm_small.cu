@@ -61,6 +61,7 @@ struct Params {
     uint32_t x_wrap;             // K after which the activation columns start over
     uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;       // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
     uint32_t raw_stages, b_stages;
+    uint32_t early;              // packed weights may be fetched before the preceding kernel has finished
     uint32_t swiglu;             // tiles of 64 gate rows (matrix 0) and their 64 up rows (matrix 1); output silu(g) * u
     // grouped launch: weight tiles [0, tiles[0]) belong to matrix 0, the next tiles[1] to matrix 1, ...
     uint32_t groups, tiles[3], grp_N[3];
@@ -178,8 +179,10 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (threadIdx.x == 0) QST(0, 1);
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
-    // everything above touched only this CTA's shared and tensor memory; global memory is first touched below
-    ptx::grid_dependency_wait();
+    // Everything above touched only this CTA's shared and tensor memory.  Global memory is first touched below -- or, where the
+    // preceding kernels are known not to write the weights, by the copies of packed chunks: they then stream in while the
+    // preceding kernel drains, and the wait stands in front of the first activation tile and of the results.
+    if (!p.early) ptx::grid_dependency_wait();
     if (threadIdx.x == 0) QST(0, 2);
 
     if (warp == COPY_WARP) {
@@ -214,6 +217,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             if (++rs == p.raw_stages) { rs = 0; rph ^= 1u; }
         };
         for (uint32_t i = 0; i < p.raw_stages; i++) issue_raw(false);
+        if (p.early) ptx::grid_dependency_wait();
         for (uint32_t kc = 0; ok && kc < kcn; kc++) {
             if (raw_next <= kc) issue_raw(true);              // the chunk these activation tiles belong to must be on its way
             for (uint32_t s = 0; ok && s < (uint32_t)SUBS; s++) {
@@ -319,6 +323,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
 
     // ---------------- partial tiles meet in the scratch buffer, the cluster shares out the sums ----------------
+    if (p.early) ptx::grid_dependency_wait();      // (long over; orders this thread's stores behind it)
     if (warp < 4) {
         // the accumulator is complete once every MMA has; a failed wait sets the abort flag, the barrier is still reached
         ptx::mbar_wait<64>(acc_full, 0u, abort_flag, p.err, 117);
@@ -530,7 +535,7 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
     Params p;
     p.M = a.M; p.N = a.N; p.K = a.K; p.T = pl.T; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
     p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
-    p.raw_stages = pl.raw_stages; p.b_stages = pl.b_stages; p.swiglu = a.W1 ? 1u : 0u;
+    p.raw_stages = pl.raw_stages; p.b_stages = pl.b_stages; p.early = a.early_weights ? 1u : 0u; p.swiglu = a.W1 ? 1u : 0u;
     p.groups = 1u + a.n_extra;
     p.tiles[0] = (a.N + W_TILE - 1) / W_TILE; p.grp_N[0] = a.N; p.grp_Y[0] = (__half*)a.Y;
     for (uint32_t e = 0; e < 2u; e++) {

@@ -205,12 +205,14 @@ void TransformerLayerCoordinator::forward(cudaStream_t stream, const void* X_in,
     qg::Workspace ws;
     ws.partial = im.ws; ws.partial_floats = im.ws_floats; ws.counters = im.counters; ws.err = im.err;
 
+    // the normalisation at the start of the layer waits for everything before it (see lops::rmsnorm)
+    const int early = c.rms_eps > 0.0f && c.tp_size == 1 ? 1 : 0;
     auto gemm = [&](const KernelBinding& kb, const void* X, const void* W0, const void* W1, void* Y, uint32_t N, uint32_t K,
                     uint32_t H, const void* residual, float* partial_out) {
         if (status_) return;
         qg::GemmArgs a; memset(&a, 0, sizeof(a));
         a.format = kb.format; a.X = X; a.W0 = W0; a.W1 = W1; a.Y = Y; a.M = c.M; a.N = N; a.K = K;
-        a.layout = kb.layout; a.H = H; a.D = c.D; a.residual = residual; a.partial_out = partial_out;
+        a.layout = kb.layout; a.H = H; a.D = c.D; a.residual = residual; a.partial_out = partial_out; a.early_weights = early;
         if (qg::launch(a, ws, stream) != cudaSuccess) { status_ = -6; return; }
         launches_ += (uint32_t)qg::last_launch_count();
     };
@@ -245,6 +247,7 @@ void TransformerLayerCoordinator::forward(cudaStream_t stream, const void* X_in,
         a.layout = im.head_binding.layout; a.H = hq; a.D = c.D;
         a.n_extra = 2; a.W_extra[0] = W_k; a.W_extra[1] = W_v; a.Y_extra[0] = im.k; a.Y_extra[1] = im.v;
         a.N_extra[0] = a.N_extra[1] = hkv * c.D;
+        a.early_weights = early;
         if (fuse) {
             const uint32_t rope = c.rope_theta > 0.0f ? 1u : 0u, q8 = c.kv_q8_0 ? 2u : 0u;
             a.post[0] = rope; a.post[1] = rope | q8; a.post[2] = q8;

@@ -157,6 +157,7 @@ int TransformerModel::forward(cudaStream_t stream, const int32_t* tokens, void* 
         qg::GemmArgs a; memset(&a, 0, sizeof(a));
         a.format = im.head_binding.format; a.X = x; a.W0 = im.lm_head; a.Y = logits; a.M = c.M; a.N = im.vocab_rows; a.K = c.K;
         a.layout = im.head_binding.layout;
+        a.early_weights = c.rms_eps > 0.0f && c.tp_size == 1 ? 1 : 0;      // behind the final normalisation
         qg::Workspace ws;
         ws.partial = im.ws; ws.partial_floats = im.ws_floats; ws.counters = im.counters; ws.err = im.err;
         if (qg::launch(a, ws, stream) != cudaSuccess) { cudaGetLastError(); return -6; }
