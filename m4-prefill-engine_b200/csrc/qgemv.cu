@@ -1,152 +1,191 @@
-// Single-token projection on CUDA cores: the decode-like end of the path (m4_bridge_dispatch_gemv, and
-// m4_bridge_dispatch_gemm with M = 1; reference: gemv_q4_0 and friends, quant_router_kernels.metal:930-1144).
-// With one token the projection is a stream over the packed weights (9.4 MB at the 8B shape) with a few
-// multiply-adds per weight: HBM-bound byte work that gains nothing from the tensor core (its 128-row tiles spend
-// 16 dependent unpack-and-MMA steps per CTA on latency).  Here one lane owns one 256-element chunk of one weight
-// row: it loads the chunk's packed bytes (the codecs' ROW_BYTES, 16-byte loads), unpacks them with the same
-// register-level codecs as the tensor-core kernel (bit-identical fp16 weights), multiplies with the activations kept
-// as fp32 in shared memory (chunk stride 257 words: conflict-free) and accumulates in fp32; the lanes of a row are
-// reduced with shuffles.  The kernel is written for M tokens (every weight is unpacked once and used M times), but
-// measured on B200 it only beats the tensor-core path at M = 1 (8.3 us against 12.6 us at K = N = 4096; 12.6 us at
-// M = 2, 16.5 us at M = 3: fp32 multiply-adds on CUDA cores), so only M = 1 is dispatched here.
+// Single-token projection: the decode-like end of the path (m4_bridge_dispatch_gemv, and m4_bridge_dispatch_gemm with M = 1;
+// reference: gemv_q4_0 and friends, quant_router_kernels.metal:930-1144).
+//
+// With one token the projection is a stream over the packed weights (9.4 MB at K = N = 4096) and what costs is instructions:
+// unpacking a weight takes about two, and converting it to fp32, reading its activation and multiplying took three more.  Here
+// the unpacked fp16 pairs go straight into warp-level MMAs (m16n8k16, fp32 accumulators): a warp works on 16 rows, lane 4 g + t
+// on rows g and g + 8 with every fourth chunk of 256 elements.  The sum over K does not care about the order of K, so a lane's
+// own pairs are the A fragment as they come out of the codec, and the B fragment is the activation pairs of the same elements
+// (all eight columns alike); the MMA adds up the four lanes of a row.  The eight fragments' worth of K that one row's four lanes
+// do not cover are other warps' chunks; they meet in shared memory.  (128-row tiles of tcgen05 would spend their time on
+// latency here: K = N = 4096 takes 9.5 us on the few-token kernel.)
+// Weights are those of the tensor-core kernels bit for bit (the same register-level codecs).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 
 #include "codecs.cuh"
+#include "ptx.cuh"
 #include "qgemm.cuh"
 
 namespace qg {
 
 namespace {
 
-constexpr int GV_THREADS = 256;
-constexpr int GV_MAX_M = 8;
-constexpr int XSTRIDE = 257;                 // fp32 words per 256-element activation chunk in shared memory
+constexpr int GV_MAX_WARPS = 8;
+constexpr uint32_t X_CHUNK = 512 + 16;       // bytes of one activation chunk in shared memory: the four lanes of a row read
+                                             // four neighbouring chunks at once, on different banks
 
 struct GvParams {
     const __half* X; const uint8_t* W; __half* Y;
-    uint32_t M, N, K, x_cols, x_wrap, chunks;    // chunks = K / 256; X has x_cols columns and starts over every x_wrap of K
-    uint32_t rows_per_warp, lanes_per_row;   // chunks < 32: 32 / chunks rows per warp; else 1 row, 32 lanes
+    uint32_t N, K, x_cols, x_wrap, chunks;       // chunks = K / 256; X has x_cols columns and starts over every x_wrap of K
     const uint8_t* meta;                     // planar layouts: scale / bias planes behind the packed plane
     const __half* row_scale;                 // per-row scale (integer-valued codecs)
+    uint32_t early;                          // packed weights may be fetched before the preceding kernel has finished
 };
 
-template <int FMT, int M>
-__global__ void __launch_bounds__(GV_THREADS) qgemv_kernel(const GvParams p) {
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// R: rows per lane, 8 R rows per warp and CTA (R == 1 leaves the fragment's rows 8 .. 15 zero)
+template <int FMT, int R>
+__global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams p) {
     using Cd = cdc::Codec<FMT>;
-    constexpr int RB = Cd::ROW_BYTES;
-    extern __shared__ float sx[];            // [M][chunks][XSTRIDE]
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (uint32_t i = tid; i < M * p.K; i += GV_THREADS) {
-        const uint32_t m = i / p.K, k = i % p.K;
-        sx[(size_t)m * p.chunks * XSTRIDE + (k >> 8) * XSTRIDE + (k & 255u)] = k % p.x_wrap < p.x_cols ? __half2float(p.X[(size_t)m * p.x_cols + k % p.x_wrap]) : 0.0f;
-    }
-    __syncthreads();
-    const uint32_t warps_total = gridDim.x * (GV_THREADS / 32), gw = blockIdx.x * (GV_THREADS / 32) + warp;
-    const uint32_t sub = lane / p.lanes_per_row, l = lane % p.lanes_per_row;       // row within the warp's group, lane within the row
+    constexpr uint32_t ROWS = 8u * R;
+    constexpr int RB = Cd::ROW_BYTES, MW = Cd::META_WORDS > 0 ? Cd::META_WORDS : 4;
+    extern __shared__ __align__(16) uint8_t sx[];            // [chunks][X_CHUNK]
+    __shared__ float part[GV_MAX_WARPS][ROWS];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = blockDim.x >> 5;
+    const uint32_t g = lane >> 2, t = lane & 3u;
     const size_t row_bytes = (size_t)p.chunks * RB;
-    for (uint32_t n0 = gw * p.rows_per_warp; n0 < p.N; n0 += warps_total * p.rows_per_warp) {
-        const uint32_t n = n0 + sub;
-        float acc[M];
+    const uint32_t n0 = blockIdx.x * ROWS;
+    ptx::launch_dependents();
+    if (!p.early) ptx::grid_dependency_wait();
+
+    // packed bytes (and planar scales) of rows g, g + 8 and chunk c; rows past N repeat the last one, chunks past the end are zero
+    uint32_t r[R][RB / 4], meta[R][MW];
+    auto load = [&](uint32_t c, uint32_t (&r)[R][RB / 4], uint32_t (&meta)[R][MW]) {
 #pragma unroll
-        for (int m = 0; m < M; m++) acc[m] = 0.0f;
-        if (n < p.N) {
-            for (uint32_t c = l; c < p.chunks; c += p.lanes_per_row) {
-                uint32_t r[RB / 4];
+        for (int h = 0; h < R; h++) {
+            const uint32_t n = min(n0 + g + 8u * h, p.N - 1u);
+            if (c < p.chunks) {
                 const uint4* src = reinterpret_cast<const uint4*>(p.W + (size_t)n * row_bytes + (size_t)c * RB);
 #pragma unroll
                 for (int i = 0; i < RB / 16; i++) {
                     const uint4 v = __ldg(src + i);
-                    r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
+                    r[h][4 * i] = v.x; r[h][4 * i + 1] = v.y; r[h][4 * i + 2] = v.z; r[h][4 * i + 3] = v.w;
                 }
-                constexpr int MW = Cd::META_WORDS > 0 ? Cd::META_WORDS : 4;
-                uint32_t meta[MW] = {};
-                if (Cd::META_WORDS != 0) {           // one scale and one bias per 64 (4 words) or 32 (8 words) elements, two planes
+                if (Cd::META_WORDS != 0) {       // one scale and one bias per 64 (4 words) or 32 (8 words) elements, two planes
                     const uint32_t groups = (p.K / 256) * MW;
                     const uint8_t* mp = p.meta + ((size_t)n * groups + (size_t)c * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
-                        const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
-                        const uint2 bi = __ldg(reinterpret_cast<const uint2*>(bp));
-                        meta[0] = sc.x; meta[1] = sc.y; meta[2] = bi.x; meta[3] = bi.y;
+                        const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp)), bi = __ldg(reinterpret_cast<const uint2*>(bp));
+                        meta[h][0] = sc.x; meta[h][1] = sc.y; meta[h][2] = bi.x; meta[h][3] = bi.y;
                     } else {
-                        const uint4 sc = __ldg(reinterpret_cast<const uint4*>(mp));
-                        const uint4 bi = __ldg(reinterpret_cast<const uint4*>(bp));
-                        meta[0] = sc.x; meta[1] = sc.y; meta[2] = sc.z; meta[3] = sc.w;
-                        meta[MW - 4] = bi.x; meta[MW - 3] = bi.y; meta[MW - 2] = bi.z; meta[MW - 1] = bi.w;
+                        const uint4 sc = __ldg(reinterpret_cast<const uint4*>(mp)), bi = __ldg(reinterpret_cast<const uint4*>(bp));
+                        meta[h][0] = sc.x; meta[h][1] = sc.y; meta[h][2] = sc.z; meta[h][3] = sc.w;
+                        meta[h][MW - 4] = bi.x; meta[h][MW - 3] = bi.y; meta[h][MW - 2] = bi.z; meta[h][MW - 1] = bi.w;
                     }
                 }
-                const float* xc = sx + (size_t)c * XSTRIDE;
+            } else {
 #pragma unroll
-                for (int s = 0; s < 4; s++) {
-                    uint32_t o[32];
-                    Cd::dequant64(r, s, o, meta);
+                for (int i = 0; i < RB / 4; i++) r[h][i] = 0u;
 #pragma unroll
-                    for (int i = 0; i < 32; i++) {
-                        const float2 w = __half22float2(*reinterpret_cast<const __half2*>(&o[i]));
-#pragma unroll
-                        for (int m = 0; m < M; m++) {
-                            const float* xm = xc + (size_t)m * p.chunks * XSTRIDE + s * 64 + 2 * i;
-                            acc[m] = fmaf(w.x, xm[0], acc[m]);
-                            acc[m] = fmaf(w.y, xm[1], acc[m]);
-                        }
-                    }
-                }
+                for (int i = 0; i < MW; i++) meta[h][i] = 0u;
             }
         }
-        // lanes of one row: lanes_per_row is a power of two and rows are lane-aligned groups
-#pragma unroll
-        for (int m = 0; m < M; m++)
-            for (uint32_t off = p.lanes_per_row >> 1; off > 0; off >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], off);
-        if (l == 0 && n < p.N) {
-            const float rs = Cd::ROW_SCALE ? __half2float(p.row_scale[n]) : 1.0f;
-#pragma unroll
-            for (int m = 0; m < M; m++) p.Y[(size_t)m * p.N + n] = __float2half_rn(Cd::ROW_SCALE ? acc[m] * rs : acc[m]);
+    };
+    load(warp * 4u + t, r, meta);                     // under way while the activations are staged
+    if (p.early) ptx::grid_dependency_wait();
+
+    // activations: fp16, columns past x_cols (of every period of x_wrap) are zero
+    if ((reinterpret_cast<uintptr_t>(p.X) & 15u) == 0 && p.x_cols % 8u == 0u) {
+        for (uint32_t i = tid; i < p.K / 8u; i += blockDim.x) {
+            const uint32_t k = i * 8u, col = p.x_wrap == p.K ? k : k % p.x_wrap;
+            const uint4 v = col < p.x_cols ? __ldg(reinterpret_cast<const uint4*>(p.X + col)) : make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(sx + (k >> 8) * X_CHUNK + (k & 255u) * 2u) = v;
         }
+    } else {
+        for (uint32_t k = tid; k < p.K; k += blockDim.x) {
+            const uint32_t col = k % p.x_wrap;
+            *reinterpret_cast<__half*>(sx + (k >> 8) * X_CHUNK + (k & 255u) * 2u) = col < p.x_cols ? p.X[col] : __half(0.0f);
+        }
+    }
+    __syncthreads();
+
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (uint32_t c0 = warp * 4u; c0 < p.chunks; c0 += warps * 4u) {
+        const uint32_t c = c0 + t;
+        // (a lane without a chunk multiplies what its codec makes of zero bytes, a finite number, with zeros)
+        const uint8_t* xc = sx + (c < p.chunks ? c : 0u) * X_CHUNK;
+        const uint32_t keep = c < p.chunks ? 0xffffffffu : 0u;
+        // short rows leave the registers to fetch the next chunk while this one is multiplied
+        constexpr bool AHEAD = RB <= 96 && Cd::META_WORDS == 0;
+        const bool more = c0 + warps * 4u < p.chunks;
+        uint32_t rn[AHEAD ? R : 1][AHEAD ? RB / 4 : 1], mn[AHEAD ? R : 1][AHEAD ? MW : 1];
+        if constexpr (AHEAD) { if (more) load(c + warps * 4u, rn, mn); }
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            uint32_t a[R][32];
+#pragma unroll
+            for (int h = 0; h < R; h++) Cd::dequant64(r[h], s, a[h], meta[h]);
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const uint4 x = *reinterpret_cast<const uint4*>(xc + s * 128 + q * 16);
+                mma16816(acc, a[0][4 * q], R == 2 ? a[R - 1][4 * q] : 0u, a[0][4 * q + 1], R == 2 ? a[R - 1][4 * q + 1] : 0u, x.x & keep, x.y & keep);
+                mma16816(acc, a[0][4 * q + 2], R == 2 ? a[R - 1][4 * q + 2] : 0u, a[0][4 * q + 3], R == 2 ? a[R - 1][4 * q + 3] : 0u, x.z & keep, x.w & keep);
+            }
+        }
+        if constexpr (AHEAD) {
+            if (more) {
+#pragma unroll
+                for (int h = 0; h < R; h++)
+#pragma unroll
+                    for (int i = 0; i < RB / 4; i++) r[h][i] = rn[h][i];
+            }
+        } else if (more) load(c + warps * 4u, r, meta);
+    }
+    // every column of the accumulator is the same: rows g (acc[0]) and g + 8 (acc[2])
+    if (t == 0u) { part[warp][g] = acc[0]; if (R == 2) part[warp][ROWS - 8u + g] = acc[2]; }
+    __syncthreads();
+    if (tid < ROWS && n0 + tid < p.N) {
+        float sum = 0.0f;
+        for (uint32_t w = 0; w < warps; w++) sum += part[w][tid];
+        p.Y[n0 + tid] = __float2half_rn(Cd::ROW_SCALE ? sum * __half2float(p.row_scale[n0 + tid]) : sum);
     }
 }
 
-int g_gv_sms = 0;
-
-template <int FMT, int M>
-cudaError_t launch_gemv_m(const GemmArgs& a, cudaStream_t stream) {
+template <int FMT, int R>
+cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
     using Cd = cdc::Codec<FMT>;
     GvParams p;
     p.X = (const __half*)a.X; p.W = (const uint8_t*)a.W0; p.Y = (__half*)a.Y;
-    p.M = a.M; p.N = a.N; p.K = a.K; p.chunks = a.K / 256; p.x_cols = a.x_cols ? a.x_cols : a.K; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
-    if (p.chunks >= 32) { p.rows_per_warp = 1; p.lanes_per_row = 32; }
-    else { uint32_t lp = 1; while (lp < p.chunks) lp <<= 1; p.lanes_per_row = lp; p.rows_per_warp = 32 / lp; }
-    const size_t plane = (size_t)a.N * p.chunks * Cd::ROW_BYTES;
-    p.meta = (const uint8_t*)a.W0 + plane;
+    p.N = a.N; p.K = a.K; p.chunks = a.K / 256; p.x_cols = a.x_cols ? a.x_cols : a.K; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
+    p.meta = (const uint8_t*)a.W0 + (size_t)a.N * p.chunks * Cd::ROW_BYTES;
     p.row_scale = (const __half*)p.meta;
-    const size_t smem = (size_t)M * p.chunks * XSTRIDE * sizeof(float);
+    p.early = a.early_weights ? 1u : 0u;
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    if (!g_gv_sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_gv_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g_gv_sms <= 0) g_gv_sms = 148;
-    }
-    // as many CTAs as fit per SM given the activation copy each keeps in shared memory, but no more warps than rows
-    uint32_t per_sm = smem ? (uint32_t)((220 * 1024) / (smem + 1024)) : 8u;
-    per_sm = per_sm < 1u ? 1u : (per_sm > 8u ? 8u : per_sm);
-    uint32_t grid = (uint32_t)g_gv_sms * per_sm;
-    const uint32_t need = (a.N + p.rows_per_warp * (GV_THREADS / 32) - 1) / (p.rows_per_warp * (GV_THREADS / 32));
-    if (grid > need) grid = need;
-    qgemv_kernel<FMT, M><<<grid, GV_THREADS, smem, stream>>>(p);
-    return cudaGetLastError();
+    const uint32_t groups = (p.chunks + 3u) / 4u;            // a warp takes four chunks at a time
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((a.N + 8 * R - 1) / (8 * R));
+    const uint32_t rounds = (groups + GV_MAX_WARPS - 1) / GV_MAX_WARPS;
+    cfg.blockDim = dim3(32u * ((groups + rounds - 1) / rounds));      // every warp the same number of rounds, as far as that goes
+    cfg.dynamicSmemBytes = (size_t)p.chunks * X_CHUNK;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, R>, p);
 }
 
 template <int FMT>
-cudaError_t launch_gemv_fmt(const GemmArgs& a, cudaStream_t s) {
-    return a.M == 1 ? launch_gemv_m<FMT, 1>(a, s) : cudaErrorInvalidValue;
+cudaError_t launch_gemv_fmt(const GemmArgs& a, cudaStream_t stream) {
+    // Two rows per lane fill the fragment; the variable-rate codec's two rows take 179 registers, one row 124 (K = 4096, N = 14336:
+    // 31.3 against 23.5 us), and the codebook's 177 cost more than they give once a warp loops over K (K = 14336: 25.8 against 24.9).
+    const bool one = FMT == QUANT_VAR_RATE_AFFINE || (FMT == QUANT_EXL3 && a.K > 256u * 4u * GV_MAX_WARPS);
+    return one ? launch_gemv_rows<FMT, 1>(a, stream) : launch_gemv_rows<FMT, 2>(a, stream);
 }
 
 }  // namespace
@@ -155,7 +194,7 @@ bool gemv_path_ok(const GemmArgs& a) {
     if (a.force_generic || a.M != 1 || a.W1 || a.residual || a.partial_out || a.layout != 0 || a.scatter.world || a.n_extra) return false;
     if (a.K == 0 || a.K % 256 != 0 || a.N == 0) return false;
     if (((uintptr_t)a.W0 & 15u) || ((uintptr_t)a.X & 1u)) return false;
-    if ((size_t)a.M * (a.K / 256) * XSTRIDE * sizeof(float) > 200 * 1024) return false;
+    if ((size_t)(a.K / 256) * 257 * sizeof(float) > 200 * 1024) return false;      // (longer rows go to the few-token kernel)
     switch (a.format) {
         case QUANT_Q4_0: case QUANT_MLX_4BIT: case QUANT_Q4_K: case QUANT_TERNARY_1_58: case QUANT_VAR_RATE_AFFINE: case QUANT_EXL3:
         case QUANT_MLX_4BIT_G64: case QUANT_TERNARY_ROW: case QUANT_MLX_4BIT_PLANAR: return true;
