@@ -20,8 +20,9 @@
 //     boxes into one packed stage), so unpacking, MMA shape and tile width are those of the plain
 //     projection; the epilogue pairs each gate lane with its up lane through shared memory;
 //   * two accumulator buffers in tensor memory overlap a tile's epilogue with the next tile;
-//   * for few tokens the K range is split across CTAs; partial tiles meet in a scratch buffer
-//     and the last CTA of a tile adds them in split order (deterministic) and writes Y.
+//   * for few tokens the K range is split across CTAs; partial tiles meet in a scratch buffer and
+//     are added in split order (deterministic): by all CTAs of a tile, which form a thread-block
+//     cluster, or by the last of them where that many clusters do not fit the GPU at once.
 //
 // Every mbarrier wait is bounded (ptx::mbar_wait): on expiry the CTA records a code in the
 // error word, stops issuing work, lets outstanding copies land, frees tensor memory and exits.
@@ -120,6 +121,7 @@ struct Params {
     float* partial_out;
     uint32_t layout, H, D;
     float* ws_partial;
+    uint32_t split_cluster;      // the splits of a tile are one cluster and share out the sums
     uint32_t* ws_counters;
     int* err;
     // planar layouts: per-64 scale plane followed by the bias plane (meta), or one fp16 scale per row
@@ -1023,7 +1025,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             __syncwarp();
             if (lane == 0) { if (PAIR && pair_rank == 1u) ptx::mbar_arrive_cluster(&tm_empty[buf], 0u); else ptx::mbar_arrive(&tm_empty[buf]); }
             if (et == 0) QTRC(6, it, 1);
-            if (p.k_splits > 1) {
+            if (p.k_splits > 1 && !p.split_cluster) {
                 // count this partial tile in; the CTA that completes the count adds the partial tiles after the
                 // role loops have ended (every CTA of a split launch owns exactly one work item)
                 __threadfence();
@@ -1056,7 +1058,20 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         ptx::tc_fence_after_sync();
         if (PAIR) ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS); else ptx::tmem_dealloc(tmem_base, TMEM_COLS);
     }
-    if (p.k_splits > 1 && *last_flag && !*abort_flag) {
+    if (!PAIR && p.split_cluster) {
+        // Split-K fix-up by every CTA of the tile, each a share of the rows (the barrier orders every CTA's partial tile before it;
+        // every thread of every CTA gets here on every path).  One CTA adding alone took 2 to 4.5 us.
+        ptx::cluster_sync_all();
+        if (!*abort_flag) {
+            const Tile t = decode_tile(blockIdx.x, p);
+            const uint32_t i = t.ks * (uint32_t)C::THREADS + threadIdx.x, n = p.k_splits * (uint32_t)C::THREADS;
+            switch (p.k_splits) {
+                case 2: splitk_fixup<2>(p, t, i, n); break;
+                case 4: splitk_fixup<4>(p, t, i, n); break;
+                default: splitk_fixup<8>(p, t, i, n); break;
+            }
+        }
+    } else if (p.k_splits > 1 && *last_flag && !*abort_flag) {
         // Split-K fix-up by the whole CTA: the partial tiles of this output tile are complete (this CTA's arrival
         // completed the count), every warp is idle by now, and 16 float4 loads per thread keep enough bytes in
         // flight to cover the L2 latency in one or two rounds.  The sum runs in split order, so the result does not
@@ -1352,6 +1367,24 @@ template <int FMT> int max_pairs() {
     return n;
 }
 
+// Clusters of `splits` CTAs (one CTA per SM) that can be resident at once, asked of the runtime once per format and size.
+template <int FMT> uint32_t max_split_clusters(uint32_t splits) {
+    static int known[9] = {};
+    if (known[splits] == 0) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3((unsigned)sm_count() / splits * splits); cfg.blockDim = dim3(Cfg<FMT>::THREADS); cfg.dynamicSmemBytes = SMEM_BYTES;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        int c = 0;
+        if (cudaOccupancyMaxActiveClusters(&c, qgemm_kernel<FMT, false, false>, &cfg) != cudaSuccess || c <= 0) { cudaGetLastError(); c = -1; }
+        known[splits] = c;
+    }
+    return known[splits] > 0 ? (uint32_t)known[splits] : 0u;
+}
+
 template <int FMT>
 cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t stream) {
     using C = Cfg<FMT>;
@@ -1392,6 +1425,7 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
     p.M = a.M; p.N = a.N; p.K = a.K;
     p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
     p.early = a.early_weights ? 1u : 0u;
+    p.split_cluster = 0u;
     p.T = pl.T; p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
     p.swiglu = a.W1 ? 1u : 0u;
     // Row-wise epilogue: wherever every output row can take 16-byte stores (and, with a residual, 8-byte loads).  SwiGLU
@@ -1508,6 +1542,12 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
             if (a.residual) return cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, true, true>, tmX, tmW0, tmW1, tmW2, p);
             return cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, false, true>, tmX, tmW0, tmW1, tmW2, p);
         }
+    }
+    p.split_cluster = pl.k_splits > 1 && pl.n_tok_tiles * pl.n_w_tiles <= max_split_clusters<FMT>(pl.k_splits) ? 1u : 0u;
+    if (p.split_cluster) {
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = pl.k_splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
     }
     // (the split-K fix-up adds the residual outside the epilogue loop: only unsplit residual launches need the RESID build)
     if (a.residual && pl.k_splits == 1) return cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, true, false>, tmX, tmW0, tmW1, tmW2, p);
