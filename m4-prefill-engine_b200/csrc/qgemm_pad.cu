@@ -12,7 +12,7 @@
 // row holds the codes once per term with that term's scale and bias, and the activation columns start over for each.  Q4_0
 // takes two terms, the affine formats three; ternary weights are exact as they are.
 //
-// One launch and the packed bytes once or a few times more; K = 2080, N = 1100, 129 tokens took 1361 us on the CUDA cores and takes 23 us
+// One launch and the packed bytes once or a few times more; K = 2080, N = 1100, 129 tokens took 1361 us on the CUDA cores and takes 17 us
 // (one token 13 us).
 // That kernel remains for activations that are not 16-byte aligned.
 #include <cuda_fp16.h>
@@ -75,6 +75,12 @@ bool planes_of(const GemmArgs& a, Planes& out) {
     return ok;
 }
 
+// bytes a thread writes at a time: rows and terms start on such a boundary (whole blocks and codes: 16; planes of scales: 8; the
+// single row of per-row scales, whose length is N: 2)
+__host__ __device__ inline uint32_t unit_of(const Plane& p) {
+    return p.dst_term % 16u == 0u && p.dst % 16u == 0u ? 16u : (p.dst_term % 8u == 0u && p.dst % 8u == 0u ? 8u : 2u);
+}
+
 // scale of term t: leading 7 significant bits, the rest, nothing
 __device__ __forceinline__ uint16_t scale_term(uint16_t bits, uint32_t t) {
     const bool finite = (bits & 0x7C00u) != 0x7C00u;
@@ -84,33 +90,71 @@ __device__ __forceinline__ uint16_t scale_term(uint16_t bits, uint32_t t) {
     return 0u;
 }
 
-// One thread writes eight bytes of a padded row (plane blockIdx.y of matrix blockIdx.z), or what is left of them.
-__global__ void __launch_bounds__(256) pad_rows_kernel(const uint8_t* __restrict__ w0, const uint8_t* __restrict__ w1, uint8_t* __restrict__ dst, const Planes pl) {
+// A thread owns UNIT bytes at one place of a padded row (plane blockIdx.z % n of matrix blockIdx.z / n) and walks down the rows:
+// where it stands in a term, in a record and in its source row is worked out once.  Source rows are only 2-byte aligned in
+// general; whole units come in with 4-byte loads, shifted by a half word where the row asks for it.
+template <int UNIT>
+__device__ __forceinline__ void pad_plane(const Plane& p, const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, uint32_t terms) {
+    constexpr int H = UNIT / 2;                                  // 16-bit fields per unit
+    const uint32_t dst_row = p.dst_term * terms;
+    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) * UNIT;
+    if (b >= dst_row) return;
+    const uint32_t t = b / p.dst_term, off = b - t * p.dst_term;
+    const uint32_t field0 = off % (uint32_t)p.rec;
+    const bool whole = UNIT >= 8 && off + UNIT <= p.src_row;
+    for (uint32_t row = blockIdx.y; row < p.rows; row += gridDim.y) {
+        const uint8_t* s = src + (uint64_t)row * p.src_row + off;
+        uint32_t v[(H + 1) / 2];
+        const bool odd = (reinterpret_cast<uintptr_t>(s) & 2u) != 0;
+        if (whole && !odd) {
+#pragma unroll
+            for (int i = 0; i < H / 2; i++) v[i] = __ldg(reinterpret_cast<const uint32_t*>(s) + i);
+        } else if (whole && odd && (row > 0u || off > 0u) && (row + 1u < p.rows || off + UNIT + 2u <= p.src_row)) {
+            // the words around it also hold the field before and the field behind, both inside the matrix
+            uint32_t w[H / 2 + 1];
+#pragma unroll
+            for (int i = 0; i <= H / 2; i++) w[i] = __ldg(reinterpret_cast<const uint32_t*>(s - 2) + i);
+#pragma unroll
+            for (int i = 0; i < H / 2; i++) v[i] = __funnelshift_r(w[i], w[i + 1], 16);
+        } else {
+#pragma unroll
+            for (int i = 0; i < (H + 1) / 2; i++) {
+                const uint32_t o = off + 4u * i;
+                const uint32_t lo = o < p.src_row ? *reinterpret_cast<const uint16_t*>(s + 4 * i) : 0u;
+                const uint32_t hi = H > 1 && o + 2u < p.src_row ? *reinterpret_cast<const uint16_t*>(s + 4 * i + 2) : 0u;
+                v[i] = lo | (hi << 16);
+            }
+        }
+        if (terms > 1u) {
+            int32_t field = (int32_t)field0;
+#pragma unroll
+            for (int e = 0; e < H; e++) {
+                const uint32_t x = (v[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
+                uint32_t y = x;
+                if (field == p.scale_at) y = scale_term((uint16_t)x, t);
+                if (field == p.bias_at && t + 1u != terms) y = 0u;
+                v[e >> 1] ^= (x ^ y) << (16 * (e & 1));
+                field += 2;
+                if (field == p.rec) field = 0;
+            }
+        }
+        uint8_t* d = dst + (uint64_t)row * dst_row + b;
+        if constexpr (UNIT == 16) *reinterpret_cast<uint4*>(d) = make_uint4(v[0], v[1], v[2], v[3]);
+        else if constexpr (UNIT == 8) *reinterpret_cast<uint2*>(d) = make_uint2(v[0], v[1]);
+        else *reinterpret_cast<uint16_t*>(d) = (uint16_t)v[0];
+    }
+}
+
+__global__ void __launch_bounds__(128) pad_rows_kernel(const uint8_t* __restrict__ w0, const uint8_t* __restrict__ w1, uint8_t* __restrict__ dst, const Planes pl) {
     ptx::grid_dependency_wait();           // the scratch may still be read by the launch before
     ptx::launch_dependents();
-    const Plane p = pl.p[blockIdx.y];
-    const uint32_t terms = pl.terms, dst_row = p.dst_term * terms, per_row = (dst_row + 7u) / 8u;
-    const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
-    if (i >= (uint64_t)p.rows * per_row) return;
-    const uint32_t row = (uint32_t)(i / per_row), b0 = (uint32_t)(i - (uint64_t)row * per_row) * 8u;
-    const uint8_t* s = (blockIdx.z ? w1 : w0) + p.src + (uint64_t)row * p.src_row;
-    uint8_t* d = dst + blockIdx.z * pl.bytes + p.dst + (uint64_t)row * dst_row + b0;
-    uint16_t v[4];
-#pragma unroll
-    for (uint32_t e = 0; e < 4u; e++) {
-        const uint32_t b = b0 + 2u * e, t = b / p.dst_term, off = b - t * p.dst_term;
-        v[e] = b < dst_row && off < p.src_row ? *reinterpret_cast<const uint16_t*>(s + off) : (uint16_t)0;
-        const int32_t field = (int32_t)(off % (uint32_t)p.rec);
-        if (terms > 1u && field == p.scale_at) v[e] = scale_term(v[e], t);
-        if (terms > 1u && field == p.bias_at && t + 1u != terms) v[e] = 0u;
-    }
-    if (dst_row % 8u == 0u) {              // (rows of whole chunks: every store is 8-byte aligned)
-        *reinterpret_cast<uint2*>(d) = make_uint2((uint32_t)v[0] | ((uint32_t)v[1] << 16), (uint32_t)v[2] | ((uint32_t)v[3] << 16));
-    } else {
-#pragma unroll
-        for (uint32_t e = 0; e < 4u; e++)
-            if (b0 + 2u * e < dst_row) reinterpret_cast<uint16_t*>(d)[e] = v[e];
-    }
+    const uint32_t which = blockIdx.z % pl.n, matrix = blockIdx.z / pl.n;
+    const Plane p = pl.p[which];
+    const uint8_t* src = (matrix ? w1 : w0) + p.src;
+    uint8_t* out = dst + matrix * pl.bytes + p.dst;
+    if (unit_of(p) == 16u) pad_plane<16>(p, src, out, pl.terms);
+    else if (unit_of(p) == 8u) pad_plane<8>(p, src, out, pl.terms);
+    else pad_plane<2>(p, src, out, pl.terms);
 }
 
 }  // namespace
@@ -137,10 +181,11 @@ size_t padded_bytes(const GemmArgs& a) {
 cudaError_t launch_pad(const GemmArgs& a, void* dst, GemmArgs& padded, cudaStream_t stream) {
     Planes pl;
     if (!planes_of(a, pl)) return cudaErrorInvalidValue;
-    uint64_t most = 0;
+    uint32_t across = 0, rows = 0;
     for (uint32_t i = 0; i < pl.n; i++) {
-        const uint64_t n = (uint64_t)pl.p[i].rows * ((pl.p[i].dst_term * pl.terms + 7u) / 8u);
-        if (n > most) most = n;
+        const uint32_t units = (pl.p[i].dst_term * pl.terms + unit_of(pl.p[i]) - 1u) / unit_of(pl.p[i]);
+        if (units > across) across = units;
+        if (pl.p[i].rows > rows) rows = pl.p[i].rows;
     }
     padded = a;
     padded.early_weights = 0;                    // this kernel writes them
@@ -149,8 +194,12 @@ cudaError_t launch_pad(const GemmArgs& a, void* dst, GemmArgs& padded, cudaStrea
     if (a.W1) padded.W1 = static_cast<uint8_t*>(dst) + pl.bytes;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)((most + 255) / 256), pl.n, a.W1 ? 2 : 1);
-    cfg.blockDim = dim3(256);
+    // one row per thread while that does not fill the GPU (148 SMs of 2048 threads), then up to eight
+    const uint64_t fills = (uint64_t)across * rows / (148u * 2048u);
+    const uint32_t per = fills < 1u ? 1u : (fills > 8u ? 8u : (uint32_t)fills);
+    const uint32_t down = (rows + per - 1u) / per;
+    cfg.gridDim = dim3((across + 127u) / 128u, down < 65535u ? down : 65535u, pl.n * (a.W1 ? 2u : 1u));
+    cfg.blockDim = dim3(128);
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
