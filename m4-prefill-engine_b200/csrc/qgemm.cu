@@ -1371,6 +1371,7 @@ template <int FMT> int max_pairs() {
 template <int FMT> uint32_t max_split_clusters(uint32_t splits) {
     static int known[9] = {};
     if (known[splits] == 0) {
+        if (set_kernel_attributes<FMT>() != cudaSuccess) { cudaGetLastError(); return 0u; }
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3((unsigned)sm_count() / splits * splits); cfg.blockDim = dim3(Cfg<FMT>::THREADS); cfg.dynamicSmemBytes = SMEM_BYTES;
@@ -1611,6 +1612,13 @@ GemmArgs padded_probe(const GemmArgs& a) {
     return b;
 }
 }  // namespace
+
+bool persistent_splits_poorly(const GemmArgs& a) {
+    if (row_bytes_256(a.format) == 0 || a.K % chunk_elems(a.format) != 0) return false;
+    const Plan pl = make_plan(a);
+    // (the cluster capacity is that of one CTA per SM: the same for every format)
+    return pl.k_splits == 8u || (pl.k_splits > 1u && pl.n_tok_tiles * pl.n_w_tiles > max_split_clusters<QUANT_Q4_0>(pl.k_splits));
+}
 
 size_t workspace_floats(const GemmArgs& a) {
     if (pad_path_ok(a)) return workspace_floats(padded_probe(a)) + (padded_bytes(a) + 512) / sizeof(float);

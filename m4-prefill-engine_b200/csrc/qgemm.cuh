@@ -93,6 +93,8 @@ cudaError_t launch(const GemmArgs& a, const Workspace& ws, cudaStream_t stream);
 // CTAs share out the sum of the partial tiles.  Taken for M <= 128 where the persistent kernel would leave SMs idle.
 bool small_path_ok(const GemmArgs& a);
 size_t small_scratch_floats(const GemmArgs& a);
+// The persistent kernel would split this launch's K eight ways, or into more clusters than the GPU holds at once.
+bool persistent_splits_poorly(const GemmArgs& a);
 cudaError_t launch_small(const GemmArgs& a, const Workspace& ws, cudaStream_t stream);
 void set_small_kernel_enabled(int mode);     // testing hook: 0 routes those shapes to the persistent kernel again, 1 default,
                                              // 2 takes every shape the kernel can compute (any number of token tiles)

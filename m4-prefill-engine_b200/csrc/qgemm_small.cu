@@ -608,12 +608,17 @@ bool small_path_ok(const GemmArgs& a) {
         default: return false;
     }
     if (a.K % chunk != 0) return false;
-    // One token tile of up to 128 tokens (with two, every weight tile would be unpacked twice), and at most two tiles per SM:
-    // beyond that the persistent kernel, which starts on the next tile while the last one drains, is as fast.
     if (small::g_mode == 2) return true;
+    // More than one token tile unpacks every weight tile more than once, which costs nothing where most of the GPU would idle: a
+    // projection that the persistent kernel splits eight ways, or into more clusters than fit (its CTAs take an SM each), has
+    // its work in twice as many CTAs here (K = 4096: 160 tokens N = 2048 19.3 -> 12.3 us, 200 tokens N = 1100 16.3 -> 12.8, 300 tokens
+    // N = 1000 19.2 -> 13.7; 300 tokens K = N = 2304 17.1 -> 14.5; 140 tokens K = 5120 N = 640 10.7 -> 11.2).
+    if (a.M > (uint32_t)small::MAX_T) return !a.W1 && !a.n_extra && !a.lean && persistent_splits_poorly(a);
+    // One token tile: at most two weight tiles per SM.  Beyond that the persistent kernel, which starts on the next tile while the
+    // last one drains, is as fast.
     uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
     for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) tiles += (a.N_extra[e] + 127u) / 128u;
-    if (a.M > (uint32_t)small::MAX_T || tiles > 2u * (uint32_t)small::sms()) return false;
+    if (tiles > 2u * (uint32_t)small::sms()) return false;
     // SwiGLU tiles pass through the scratch buffer even unsplit, which grows with the tokens, and from 113 tokens on the
     // persistent kernel pairs its CTAs: a short K does not make up for it (F = 8192, 128 tokens, K = 512 / 1024: 13.2 / 14.9
     // against 10.2 / 13.0 us there; 64 tokens, K = 512 / 1024: 9.6 / 11.0 against 9.1 / 11.5; F = 14336, K = 4096, 128 tokens: 44.5

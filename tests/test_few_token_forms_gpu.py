@@ -44,11 +44,21 @@ def test_unequal_splits(bridge, fmt, M):
         check(run_gemm(bridge, fmt, X, W, N, ex=True), o.gemm_f64(fmt, X, W, N), f"{chunks} chunks fmt {fmt} M {M}", rms_factor=rms_factor(fmt))
 
 
-@pytest.mark.parametrize("M", [129, 300, 1000])       # token tiles shortened to fill the SMs
-def test_unequal_splits_persistent(bridge, M):
-    for chunks, N in ((5, 130), (9, 256), (17, 64)):
-        X, W = o.baseline_inputs(o.Q4_0, M, chunks * 256, N, 33)
-        check(run_gemm(bridge, o.Q4_0, X, W, N), o.gemm_f64(o.Q4_0, X, W, N), f"{chunks} chunks M {M}")
+@pytest.mark.parametrize("M", [129, 300, 1000])
+@pytest.mark.parametrize("small", [0, 1])
+def test_unequal_splits_many_tokens(bridge, M, small):
+    """Several token tiles: the persistent kernel (shortened token tiles, splits summed by a cluster or by the last CTA) and the
+    shapes that go to the few-token kernel instead."""
+    bridge.lib.b200_bridge_enable_small_kernel(small)
+    try:
+        for chunks, N in ((5, 130), (9, 256), (17, 64), (16, 2304), (32, 1100)):
+            X, W = o.baseline_inputs(o.Q4_0, M, chunks * 256, N, 33)
+            check(run_gemm(bridge, o.Q4_0, X, W, N), o.gemm_f64(o.Q4_0, X, W, N), f"{chunks} chunks M {M} N {N}")
+        R = np.random.default_rng(6).standard_normal((M, 1100)).astype(np.float16)
+        Y = run_gemm(bridge, o.Q4_0, X, W, N, residual=R)
+        check(Y, o.gemm_f64(o.Q4_0, X, W, N) + R.astype(np.float64), f"residual M {M}")
+    finally:
+        bridge.lib.b200_bridge_enable_small_kernel(1)
 
 
 @pytest.mark.parametrize("M", [1, 33, 128])
