@@ -32,7 +32,29 @@ static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// one CTA of 256 threads per row; each thread walks 8-element vectors
+// One CTA of 256 threads per row, 8-element vectors.  Rows of up to KEEP * 2048 elements stay in registers between the sum and the
+// scaling, and their weights are on the way during the reduction; longer rows are read a second time.
+constexpr int KEEP = 4;
+__device__ __forceinline__ void add_squares(float& ss, const uint4& v) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; j++) { const float2 f = __half22float2(h[j]); ss += f.x * f.x + f.y * f.y; }
+}
+__device__ __forceinline__ uint4 scale_row(const uint4& v, const uint4& w, float r) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+    const __half2* wh = reinterpret_cast<const __half2*>(&w);
+    uint4 o;
+    __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float2 f = __half22float2(h[j]), g = __half22float2(wh[j]);
+        const __half2 n = __floats2half2_rn(f.x * r, f.y * r);          // rounded to fp16 first, as the reference does
+        const float2 nf = __half22float2(n);
+        oh[j] = __floats2half2_rn(nf.x * g.x, nf.y * g.y);
+    }
+    return o;
+}
+
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* __restrict__ X, const __half* __restrict__ W,
                                                       __half* __restrict__ Y, uint32_t K, float eps) {
     ptx::grid_dependency_wait();
@@ -41,15 +63,26 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* __restrict__
     __half* y = Y + (size_t)blockIdx.x * K;
     float ss = 0.0f;
     const bool vec = (K % 8 == 0) && ((((uintptr_t)x | (uintptr_t)y | (uintptr_t)W) & 15u) == 0);
-    if (vec) {
-        for (uint32_t i = threadIdx.x; i < K / 8; i += blockDim.x) {
-            uint4 v = reinterpret_cast<const uint4*>(x)[i];
-            const __half2* h = reinterpret_cast<const __half2*>(&v);
+    const uint32_t nv = K / 8u;
+    const bool keep = vec && nv <= (uint32_t)KEEP * 256u;
+    uint4 xv[KEEP], wv[KEEP];
+    if (keep) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) { float2 f = __half22float2(h[j]); ss += f.x * f.x + f.y * f.y; }
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + 256u * u;
+            if (i < nv) xv[u] = reinterpret_cast<const uint4*>(x)[i];
         }
+#pragma unroll
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + 256u * u;
+            if (i < nv) wv[u] = reinterpret_cast<const uint4*>(W)[i];
+        }
+#pragma unroll
+        for (int u = 0; u < KEEP; u++) if (threadIdx.x + 256u * u < nv) add_squares(ss, xv[u]);
+    } else if (vec) {
+        for (uint32_t i = threadIdx.x; i < nv; i += 256u) add_squares(ss, reinterpret_cast<const uint4*>(x)[i]);
     } else {
-        for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) { float f = __half2float(x[i]); ss += f * f; }
+        for (uint32_t i = threadIdx.x; i < K; i += 256u) { float f = __half2float(x[i]); ss += f * f; }
     }
     __shared__ float red[8];
 #pragma unroll
@@ -60,23 +93,17 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* __restrict__
 #pragma unroll
     for (int i = 0; i < 8; i++) tot += red[i];
     const float r = 1.0f / sqrtf(tot / (float)K + eps);
-    if (vec) {
-        for (uint32_t i = threadIdx.x; i < K / 8; i += blockDim.x) {
-            uint4 v = reinterpret_cast<const uint4*>(x)[i], w = reinterpret_cast<const uint4*>(W)[i], o;
-            const __half2* h = reinterpret_cast<const __half2*>(&v);
-            const __half2* wh = reinterpret_cast<const __half2*>(&w);
-            __half2* oh = reinterpret_cast<__half2*>(&o);
+    if (keep) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                float2 f = __half22float2(h[j]), g = __half22float2(wh[j]);
-                __half2 n = __floats2half2_rn(f.x * r, f.y * r);          // rounded to fp16 first, as the reference does
-                float2 nf = __half22float2(n);
-                oh[j] = __floats2half2_rn(nf.x * g.x, nf.y * g.y);
-            }
-            reinterpret_cast<uint4*>(y)[i] = o;
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + 256u * u;
+            if (i < nv) reinterpret_cast<uint4*>(y)[i] = scale_row(xv[u], wv[u], r);
         }
+    } else if (vec) {
+        for (uint32_t i = threadIdx.x; i < nv; i += 256u)
+            reinterpret_cast<uint4*>(y)[i] = scale_row(reinterpret_cast<const uint4*>(x)[i], reinterpret_cast<const uint4*>(W)[i], r);
     } else {
-        for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) {
+        for (uint32_t i = threadIdx.x; i < K; i += 256u) {
             __half n = __float2half_rn(__half2float(x[i]) * r);
             y[i] = __float2half_rn(__half2float(n) * __half2float(W[i]));
         }
@@ -188,21 +215,44 @@ __global__ void __launch_bounds__(256) rmsnorm_add_kernel(const __half* A, const
     ptx::launch_dependents();
     ptx::grid_dependency_wait();
     const size_t row = (size_t)blockIdx.x * K;
+    const uint32_t nv = K / 8u;
+    const bool keep = nv <= (uint32_t)KEEP * 256u;
     float ss = 0.0f;
-    for (uint32_t i = threadIdx.x; i < K / 8; i += blockDim.x) {
-        const uint4 a = reinterpret_cast<const uint4*>(A + row)[i], b = reinterpret_cast<const uint4*>(B + row)[i];
-        uint4 o;
+    auto add = [](const uint4& a, const uint4& b) {
         const __half2* ah = reinterpret_cast<const __half2*>(&a);
         const __half2* bh = reinterpret_cast<const __half2*>(&b);
+        uint4 o;
         __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const float2 fa = __half22float2(ah[j]), fb = __half22float2(bh[j]);
             oh[j] = __floats2half2_rn(fa.x + fb.x, fa.y + fb.y);
-            const float2 f = __half22float2(oh[j]);
-            ss += f.x * f.x + f.y * f.y;
         }
-        reinterpret_cast<uint4*>(S + row)[i] = o;
+        return o;
+    };
+    uint4 sv[KEEP], bv[KEEP];
+    if (keep) {
+#pragma unroll
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + 256u * u;
+            if (i < nv) { sv[u] = reinterpret_cast<const uint4*>(A + row)[i]; bv[u] = reinterpret_cast<const uint4*>(B + row)[i]; }
+        }
+#pragma unroll
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + 256u * u;
+            if (i < nv) {
+                sv[u] = add(sv[u], bv[u]);
+                add_squares(ss, sv[u]);
+                reinterpret_cast<uint4*>(S + row)[i] = sv[u];
+                bv[u] = reinterpret_cast<const uint4*>(W)[i];           // the weights, during the reduction
+            }
+        }
+    } else {
+        for (uint32_t i = threadIdx.x; i < nv; i += 256u) {
+            const uint4 o = add(reinterpret_cast<const uint4*>(A + row)[i], reinterpret_cast<const uint4*>(B + row)[i]);
+            add_squares(ss, o);
+            reinterpret_cast<uint4*>(S + row)[i] = o;
+        }
     }
     __shared__ float red[8];
 #pragma unroll
@@ -213,20 +263,15 @@ __global__ void __launch_bounds__(256) rmsnorm_add_kernel(const __half* A, const
 #pragma unroll
     for (int i = 0; i < 8; i++) tot += red[i];
     const float r = 1.0f / sqrtf(tot / (float)K + eps);
-    for (uint32_t i = threadIdx.x; i < K / 8; i += blockDim.x) {
-        const uint4 v = reinterpret_cast<const uint4*>(S + row)[i], w = reinterpret_cast<const uint4*>(W)[i];
-        uint4 o;
-        const __half2* h = reinterpret_cast<const __half2*>(&v);
-        const __half2* wh = reinterpret_cast<const __half2*>(&w);
-        __half2* oh = reinterpret_cast<__half2*>(&o);
+    if (keep) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 f = __half22float2(h[j]), g = __half22float2(wh[j]);
-            const __half2 n = __floats2half2_rn(f.x * r, f.y * r);            // rounded to fp16 first, as in rmsnorm_kernel
-            const float2 nf = __half22float2(n);
-            oh[j] = __floats2half2_rn(nf.x * g.x, nf.y * g.y);
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + 256u * u;
+            if (i < nv) reinterpret_cast<uint4*>(Y + row)[i] = scale_row(sv[u], bv[u], r);
         }
-        reinterpret_cast<uint4*>(Y + row)[i] = o;
+    } else {
+        for (uint32_t i = threadIdx.x; i < nv; i += 256u)
+            reinterpret_cast<uint4*>(Y + row)[i] = scale_row(reinterpret_cast<const uint4*>(S + row)[i], reinterpret_cast<const uint4*>(W)[i], r);
     }
 }
 
