@@ -1295,7 +1295,8 @@ Plan make_plan(const GemmArgs& a) {
         const uint32_t sms = (uint32_t)sm_count();
         for (uint32_t s = 2; s <= 8; s *= 2) {
             if (tiles * s > sms || chunks / s < 2) break;
-            if (a.lean && chunks % s != 0) break;
+            // (K/V post-operations need whole sums: which launches have them is a contract of the entry points, by equal parts)
+            if ((a.lean || a.post[0] || a.post[1] || a.post[2]) && chunks % s != 0) break;
             pl.k_splits = s;
         }
         if (pl.n_tok_tiles * pl.n_w_tiles > 4096) pl.k_splits = 1;

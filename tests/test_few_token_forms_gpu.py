@@ -80,3 +80,25 @@ def test_grouped_few_tokens(bridge, M, layout):
             got = y.cpu().numpy()
             got = got.transpose(1, 0, 2).reshape(M, n) if layout else got
             check(got, o.gemm_f64(fmt, X, w, n), f"grouped fmt {fmt} M {M} N {n}", rms_factor=rms_factor(fmt))
+
+
+@pytest.mark.parametrize("chunks", [3, 5, 9])
+def test_fused_qkv_of_odd_chunk_counts(bridge, chunks):
+    """The fused Q/K/V epilogue needs whole sums: a K of an odd number of chunks, which other launches split unequally, stays
+    unsplit there and is served."""
+    L, M, Hq, Hkv, D, K = bridge.lib, 200, 4, 2, 64, chunks * 256
+    X, Wq = o.baseline_inputs(o.Q4_0, M, K, Hq * D, 51)
+    Wk, Wv = (o.baseline_inputs(o.Q4_0, M, K, Hkv * D, s)[1] for s in (52, 53))
+    Xd, Wd = dev(X), [dev(w) for w in (Wq, Wk, Wv)]
+    Q, Kc, Vc = (torch.full((h, M, D), float("nan"), dtype=torch.float16, device="cuda") for h in (Hq, Hkv, Hkv))
+    torch.cuda.synchronize()
+    assert L.b200_bridge_dispatch_qkv_fused(Xd.data_ptr(), *[w.data_ptr() for w in Wd], Q.data_ptr(), Kc.data_ptr(), Vc.data_ptr(), o.Q4_0, M, K, Hq, Hkv, D,
+                                            ctypes.c_float(10000.0), 0, 0, M) == 0
+    bridge.synchronize()
+    for got, w, h, rope in ((Q, Wq, Hq, True), (Kc, Wk, Hkv, True), (Vc, Wv, Hkv, False)):
+        y = o.gemm(o.Q4_0, X, w, h * D, direct_head=True, H=h, D=D)
+        y = o.rope(y, 10000.0, 0) if rope else y
+        want = y.astype(np.float64)
+        # the projection's pass line, once more for the rotation of its rounded values
+        assert np.abs(got.cpu().numpy().astype(np.float64) - want).max() <= 2.0 ** -8 * max(1.0, np.sqrt(np.mean(want ** 2)) * 2)
+    assert bridge.device_error() == 0
