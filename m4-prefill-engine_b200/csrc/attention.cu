@@ -1046,7 +1046,12 @@ cudaError_t launch_attention(const Params& p, uint32_t D, cudaStream_t stream) {
         ws::Args a;
         a.Q = p.Q; a.K = p.K; a.V = p.V; a.O = p.O; a.Hq = p.Hq; a.Hkv = p.Hkv; a.M = p.M; a.Mkv = p.Mkv; a.D = D; a.pos0 = p.pos0;
         a.scale_log2e = p.scale_log2e; a.out_tokens_major = p.out_tokens_major; a.kv_fp16 = p.kv_fp16;
-        if (ws::usable(a)) return ws::launch(a, stream, &g_last_launches);
+        if (ws::usable(a)) {
+            const cudaError_t e = ws::launch(a, stream, &g_last_launches);
+            if (e != cudaErrorMemoryAllocation) return e;
+            cudaGetLastError();              // no scratch for the expanded cache: the kernels below unpack it themselves
+            g_last_launches = 1;
+        }
     }
     // the kernel that unpacks the Q8_0 tiles itself (hooks 2 and 3)
     if (tc_ok && !p.kv_fp16 && g_force_legacy != 1) {

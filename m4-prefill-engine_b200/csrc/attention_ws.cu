@@ -587,14 +587,20 @@ template <int D> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* l
         return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / BK + 1);
     };
     const uint32_t n_last = tiles(a.M - 1), n_first = tiles(2ull * p.BP - 1);
-    const uint32_t splits = choose_splits(a.Hkv, blocks, n_first, n_last);
-    p.tiles_per_split = (n_last + splits - 1) / splits;
+    uint32_t splits = choose_splits(a.Hkv, blocks, n_first, n_last);
     // scratch: the expanded cache, then the partial results
     const size_t kv_elems = (size_t)a.Hkv * a.Mkv * D;
     const size_t kv_bytes = a.kv_fp16 ? 0 : (2 * kv_elems * sizeof(__half) + 255) & ~(size_t)255;
     const size_t rows = (size_t)a.Hq * a.M;
-    const size_t o_bytes = splits > 1 ? splits * rows * D * sizeof(float) : 0, ml_bytes = splits > 1 ? splits * rows * sizeof(float2) : 0;
-    if (kv_bytes + o_bytes + ml_bytes > 0 && !bridge::g.kv_fp16.ensure(kv_bytes + o_bytes + ml_bytes)) return cudaErrorMemoryAllocation;
+    size_t o_bytes = splits > 1 ? splits * rows * D * sizeof(float) : 0, ml_bytes = splits > 1 ? splits * rows * sizeof(float2) : 0;
+    if (kv_bytes + o_bytes + ml_bytes > bridge::g.kv_fp16.cap) {
+        // under capture the block cannot grow: without a split, or (see launch_attention) on the kernels that need no scratch
+        if (bridge::capturing(stream)) {
+            splits = 1; o_bytes = ml_bytes = 0;
+            if (kv_bytes > bridge::g.kv_fp16.cap) return cudaErrorMemoryAllocation;
+        } else if (!bridge::g.kv_fp16.ensure(kv_bytes + o_bytes + ml_bytes)) return cudaErrorMemoryAllocation;
+    }
+    p.tiles_per_split = (n_last + splits - 1) / splits;
     uint8_t* scratch = static_cast<uint8_t*>(bridge::g.kv_fp16.p);
     p.split = splits > 1;
     // A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit

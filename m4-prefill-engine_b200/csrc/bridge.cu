@@ -108,10 +108,22 @@ const void* stage_in(const void* ptr, size_t bytes, StageSlot& sl, DevBuf& buf, 
 
 }  // namespace
 
-bool ensure_workspace(size_t floats) {
-    if (floats == 0) return true;
-    if (!g.ws_partial.ensure(floats * sizeof(float))) return false;
-    return true;
+bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) { cudaGetLastError(); return false; }
+    return cap != cudaStreamCaptureStatusNone;
+}
+
+// Scratch for a launch.  Under capture the block cannot grow: the launch then does with what is there, by the rules that need
+// the least.
+bool ensure_workspace(qg::GemmArgs& a) {
+    size_t floats = qg::workspace_floats(a);
+    if (floats * sizeof(float) <= g.ws_partial.cap) return true;
+    if (capturing(g.stream)) {
+        a.lean = 1;
+        return qg::workspace_floats(a) * sizeof(float) <= g.ws_partial.cap;
+    }
+    return g.ws_partial.ensure(floats * sizeof(float));
 }
 
 int validate_gemm(const void* X, size_t Xb, const void* W, size_t Wb, const void* Y, size_t Yb, int format, bool extended,
@@ -165,7 +177,7 @@ int run_gemm(void* X, size_t Xb, void* W0, void* W1, size_t Wb, void* Y, size_t 
     a.M = M; a.N = N; a.K = K; a.layout = layout; a.H = H; a.D = D;
     a.force_generic = g.force_generic;
     (void)Xb; (void)Wb; (void)Yb;
-    if (!ensure_workspace(qg::workspace_floats(a))) return -5;
+    if (!ensure_workspace(a)) return -5;
     if (staged_in) {
         cudaEventRecord(sl.ev_in, g.stream_in);
         cudaStreamWaitEvent(g.stream, sl.ev_in, 0);
@@ -318,7 +330,7 @@ int b200_bridge_dispatch_gemm_grouped(const void* X, const void* const* W, void*
     a.n_extra = count - 1;
     for (uint32_t i = 1; i < count; i++) { a.W_extra[i - 1] = W[i]; a.Y_extra[i - 1] = Y[i]; a.N_extra[i - 1] = N[i]; }
     a.force_generic = g.force_generic;
-    if (!ensure_workspace(qg::workspace_floats(a))) return -5;      // few-token grouped launches split K
+    if (!ensure_workspace(a)) return -5;      // few-token grouped launches split K
     qg::Workspace ws;
     ws.partial = (float*)g.ws_partial.p; ws.partial_floats = g.ws_partial.cap / sizeof(float);
     ws.counters = g.counters; ws.err = g.err_word;
@@ -361,7 +373,7 @@ int b200_bridge_dispatch_qkv_fused(const void* X, const void* Wq, const void* Wk
         a.rope_table = g.rope_table.p;
     }
     if (!a.post[0] && !a.post[1] && !a.post[2]) {}            // nothing to fuse: a plain grouped launch
-    if (!ensure_workspace(qg::workspace_floats(a))) return -5;
+    if (!ensure_workspace(a)) return -5;
     qg::Workspace ws;
     ws.partial = (float*)g.ws_partial.p; ws.partial_floats = g.ws_partial.cap / sizeof(float);
     ws.counters = g.counters; ws.err = g.err_word;

@@ -67,6 +67,8 @@ void set_error(const std::string& s);
 bool is_device_ptr(const void* ptr);
 const void* resolve_in(const void* ptr, size_t bytes, DevBuf& stage, bool weights, int* rc);
 void* resolve_out(void* ptr, size_t bytes, DevBuf& stage, void** host_dst, int* rc);
+// The stream is being captured: nothing may be allocated now (cudaMalloc would invalidate the capture).
+bool capturing(cudaStream_t stream);
 // Device -> host copy of a staged result on the main stream (entry points other than the projections).
 int copy_back(void* host_dst, const void* dev_src, size_t bytes);
 // Static split-K scratch of the allocation-free entry point (no_alloc.cu): made resident at init, forgotten at shutdown.

@@ -24,7 +24,8 @@ struct GemmArgs {
     int early_weights;        // the caller knows that no kernel still running when this one is placed writes the packed weights (a
                               // kernel that waited for everything before it, and only then let its successors be placed, runs
                               // somewhere in front): they are fetched before the wait for the preceding kernel
-    int lean;                 // little scratch: K split into equal parts only, no padded copy of the weights
+    int lean;                 // little scratch: K split into equal parts only, no padded copy of the weights, SwiGLU and grouped
+                              // launches on the persistent kernel
     // Grouped launch: up to two more projections of the same X (same K, format, layout and D) run in the same
     // grid, their weight tiles queued behind those of W0.  n_extra == 0: off.  Plain fp16 outputs only.
     uint32_t n_extra;

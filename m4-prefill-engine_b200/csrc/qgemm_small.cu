@@ -591,6 +591,7 @@ extern "C" int b200_debug_small_trace(unsigned long long* out) {
 bool small_path_ok(const GemmArgs& a) {
     if (small::g_mode == 0 || a.force_generic) return false;
     if (a.partial_out || a.scatter.world || a.wait_rows.flags || a.post[0] || a.post[1] || a.post[2]) return false;
+    if (a.lean && (a.W1 || a.n_extra || (a.N + 127u) / 128u >= (uint32_t)small::sms())) return false;
     if (a.W1 && (((uintptr_t)a.W1 & 15u) || a.residual || a.layout != 0 || a.n_extra)) return false;
     // (matrices of a grouped launch: plain block formats, as on the persistent kernel)
     if (a.n_extra && (a.n_extra > 2 || a.residual || a.format == QUANT_TERNARY_ROW || a.format == QUANT_MLX_4BIT_G64 || a.format == QUANT_MLX_4BIT_PLANAR)) return false;
