@@ -35,6 +35,7 @@
 
 #include "attention_ws.cuh"
 #include "bridge_state.cuh"
+#include "exp2_poly.cuh"
 #include "ptx.cuh"
 
 namespace attn {
@@ -60,7 +61,7 @@ struct Params {
     float* part_o;               // [split][Hq * M][D], unnormalised (split launches)
     float2* part_ml;             // [split][Hq * M]: reference maximum (log2 domain), sum
     uint32_t Hq, M, Mkv, pos0, G, BP, tiles_per_split;
-    float scale_log2e, lag;
+    float scale_log2e;
     int out_tokens_major, split;
     int* err;
 };
@@ -94,33 +95,30 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return r;
 }
 // 2^x of two values without the special-function unit: x = n + f with n the nearest integer (in the low mantissa bits of
-// x + 1.5 * 2^23) and |f| <= 1/2, 2^f as the degree-5 Taylor polynomial (relative error 3e-6, far below the fp16 rounding of
-// the probabilities), n added to the exponent field.  Inputs below -120 (masked scores are -inf) give 2^-120; a NaN stays
-// non-finite (the maximum propagates it).
+// x + 1.5 * 2^23) and |f| <= 1/2, 2^f as a polynomial (exp2_poly.cuh), n added to the exponent field.  Inputs below -120
+// (masked scores are -inf) give 2^-120; a NaN stays non-finite in fp16 (the maximum propagates it).
 __device__ __forceinline__ float max_nan(float a, float b) {
     float y;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
     return y;
 }
-__device__ __forceinline__ void ex2_poly2(float x0, float x1, float& e0, float& e1) {
+template <int DEG> __device__ __forceinline__ void ex2_poly2(float x0, float x1, float& e0, float& e1) {
     const uint64_t x = pack2(max_nan(x0, -120.0f), max_nan(x1, -120.0f));
     const uint64_t r = add2(x, pack2(12582912.0f, 12582912.0f));
     const uint64_t n = add2(r, pack2(-12582912.0f, -12582912.0f));
     const uint64_t f = fma2(n, pack2(-1.0f, -1.0f), x);
-    uint64_t p = pack2(1.3333558146e-3f, 1.3333558146e-3f);
-    p = fma2(p, f, pack2(9.6181291076e-3f, 9.6181291076e-3f));
-    p = fma2(p, f, pack2(5.5504108665e-2f, 5.5504108665e-2f));
-    p = fma2(p, f, pack2(2.4022650696e-1f, 2.4022650696e-1f));
-    p = fma2(p, f, pack2(6.9314718056e-1f, 6.9314718056e-1f));
-    p = fma2(p, f, pack2(1.0f, 1.0f));
+    uint64_t p = pack2(exp2poly::coef<DEG>(DEG), exp2poly::coef<DEG>(DEG));
+#pragma unroll
+    for (int i = DEG - 1; i >= 0; i--) p = fma2(p, f, pack2(exp2poly::coef<DEG>(i), exp2poly::coef<DEG>(i)));
     float p0, p1, r0, r1;
     unpack2(p, p0, p1);
     unpack2(r, r0, r1);
     e0 = __int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23));
     e1 = __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23));
 }
-// Two pairs of eight: what the special-function unit and the issue slots of the softmax warps can both take (32 heads of 64,
-// 2048 tokens: none 37.4 us, one 36.4, two 34.9, three 39.6; 128 wide behind 8000 cached tokens 162 / 157 / 150 / 161).
+// Two pairs of eight: what the special-function unit and the issue slots of the softmax warps can both take: whole calls from Q8_0
+// caches, 32 heads of 64 over 2048 tokens (degree 6) none 45.9 us, one 44.9, two 43.4, three 45.9; 8B prefill (degree 5) 44.2 /
+// 43.6 / 41.5 / 43.8.
 __device__ constexpr bool poly_pair(int j) { return (j & 3) == 1; }
 
 __device__ __forceinline__ void tmem_ld_x32(uint32_t taddr, float* r) {
@@ -161,7 +159,8 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-template <int D>
+// LAG: the reference maximum lags (see below) and the polynomial share of the exponentials is the short one
+template <int D, bool LAG>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                const Params p) {
@@ -342,7 +341,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             // With a lag of 8 the reference maximum moves only for jumps above 2^8: probabilities are then at most 256 instead of 1,
             // the division by the row sum removes the common factor, and O is rescaled hardly ever after the first step.
             float corr = 1.0f;
-            if (mx > m_run + p.lag) { corr = ex2(m_run - mx); m_run = mx; }
+            if (mx > m_run + (LAG ? 8.0f : 0.0f)) { corr = ex2(m_run - mx); m_run = mx; }
             if (it > 0u && __any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll
                 for (int c = 0; c < D; c += 16) {
@@ -364,7 +363,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     const int e = h * 64 + 2 * j;
                     float x0, x1, e0, e1;
                     unpack2(fma2(pack2(sc[e], sc[e + 1]), sc2, nm2), x0, x1);     // masked: -inf stays -inf, 2^-inf = 0
-                    if (poly_pair(j)) ex2_poly2(x0, x1, e0, e1);
+                    if (poly_pair(j)) ex2_poly2<LAG ? 5 : 6>(x0, x1, e0, e1);
                     else { e0 = ex2(x0); e1 = ex2(x1); }
                     if (j & 1) rs1 = add2(rs1, pack2(e0, e1)); else rs0 = add2(rs0, pack2(e0, e1));
                     pk[j] = pack_h2(e0, e1);
@@ -569,11 +568,11 @@ uint32_t choose_splits(uint32_t heads, uint32_t blocks, uint32_t n_first, uint32
     return best;
 }
 
-template <int D> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* launches) {
+template <int D, bool LAG> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* launches) {
     using C = Cfg<D>;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attn_ws_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(attn_ws_kernel<D, LAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
@@ -603,11 +602,6 @@ template <int D> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* l
     p.tiles_per_split = (n_last + splits - 1) / splits;
     uint8_t* scratch = static_cast<uint8_t*>(bridge::g.kv_fp16.p);
     p.split = splits > 1;
-    // A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
-    // arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O: 43.8 against 47.4 us at the 8B
-    // prefill, 42.0 against 43.6 for the heads of 64.  128-wide heads in groups of 1, 2, 4 and 8 have always run with it; the others
-    // have not, and follow the maximum exactly.
-    p.lag = D == 128 && (p.G == 1u || p.G == 2u || p.G == 4u || p.G == 8u) ? 8.0f : 0.0f;
     p.part_o = reinterpret_cast<float*>(scratch + kv_bytes);
     p.part_ml = reinterpret_cast<float2*>(scratch + kv_bytes + o_bytes);
 
@@ -631,7 +625,7 @@ template <int D> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* l
     if (!make_map(&tmK, Kf, D, a.Hkv, a.Mkv, BK, 1) || !make_map(&tmV, Vf, D, a.Hkv, a.Mkv, BK, 1) || !make_map(&tmQ, a.Q, D, a.Hq, a.M, p.BP, p.G))
         return cudaErrorInvalidValue;
     cfg.gridDim = dim3(a.Hkv, blocks, splits); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = C::SMEM;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attn_ws_kernel<D>, tmQ, tmK, tmV, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attn_ws_kernel<D, LAG>, tmQ, tmK, tmV, p);
     if (e != cudaSuccess) return e;
     ++*launches;
     if (splits > 1) {
@@ -656,7 +650,15 @@ bool usable(const Args& a) {
 }
 
 cudaError_t launch(const Args& a, cudaStream_t stream, int* launches) {
-    return a.D == 128 ? launch_d<128>(a, stream, launches) : launch_d<64>(a, stream, launches);
+    // A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
+    // arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O: 43.8 against 47.4 us at the 8B
+    // prefill, 42.0 against 43.6 for the heads of 64.  128-wide heads in groups of 1, 2, 4 and 8 have always run with it, and with
+    // the short polynomial; the others have not: they follow the maximum exactly, and a third of a unit in the last place is what
+    // their polynomial adds to fp32 rounding (3.8271e-4 with it, without it and with the short one; the 3.8204e-4 of the warp-level
+    // kernels come from their steps of 64 keys: every new maximum of a row is a probability of exactly 1, and they see more of them).
+    const uint32_t G = a.Hq / a.Hkv;
+    if (a.D == 128) return G == 1u || G == 2u || G == 4u || G == 8u ? launch_d<128, true>(a, stream, launches) : launch_d<128, false>(a, stream, launches);
+    return launch_d<64, false>(a, stream, launches);
 }
 
 }  // namespace ws
