@@ -1196,6 +1196,13 @@ __device__ float generic_weight(int fmt, const uint8_t* W, uint32_t n, uint32_t 
     }
 }
 
+__device__ __forceinline__ void generic_store(const Params& p, uint32_t tok, uint32_t n, float acc, float acc2, bool dual) {
+    if (dual) acc = acc / (1.0f + expf(-acc)) * acc2;
+    if (p.partial_out) { p.partial_out[(size_t)tok * p.N + n] = acc; return; }
+    const size_t o = out_index(p, tok, n);
+    if (p.residual) acc += __half2float(p.residual[o]);
+    p.Y[o] = __float2half_rn(acc);
+}
 __global__ void qgemm_generic_kernel(int fmt, const __half* X, const uint8_t* W0, const uint8_t* W1, Params p) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t tok = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1207,11 +1214,53 @@ __global__ void qgemm_generic_kernel(int fmt, const __half* X, const uint8_t* W0
         acc += a * generic_weight(fmt, W0, n, k, p.N, p.K);
         if (W1) acc2 += a * generic_weight(fmt, W1, n, k, p.N, p.K);
     }
-    if (W1) acc = acc / (1.0f + expf(-acc)) * acc2;
-    if (p.partial_out) { p.partial_out[(size_t)tok * p.N + n] = acc; return; }
-    const size_t o = out_index(p, tok, n);
-    if (p.residual) acc += __half2float(p.residual[o]);
-    p.Y[o] = __float2half_rn(acc);
+    generic_store(p, tok, n, acc, acc2, W1 != nullptr);
+}
+
+// Behind a launch on a padded copy (qgemm_pad.cu): every output that is not finite is computed again with the weights as they
+// are, in fp32.  The copy holds a weight as a sum of fp16 terms, which is exact for finite products only: an infinite activation
+// meets a term of zero, or terms of both signs, and q * s of a term may lie beyond fp16 where the sum over K does not; all of these leave
+// an infinity or a NaN behind.  A thread looks at eight outputs; the warp takes the marked ones together, K strided over its lanes.
+// With nothing to do (reading 284 KB: 129 tokens, N = 1100) the launch costs 1.5 us.
+__global__ void __launch_bounds__(256) repair_nonfinite_kernel(int fmt, const __half* __restrict__ X, const uint8_t* __restrict__ W0, const uint8_t* __restrict__ W1,
+                                                               const Params p) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+    const size_t outputs = (size_t)p.M * p.N, i0 = ((size_t)blockIdx.x * 256u + threadIdx.x) * 8u;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t bad = 0u;
+    if (p.partial_out) {
+        for (uint32_t e = 0; e < 8u; e++) if (i0 + e < outputs && !isfinite(p.partial_out[i0 + e])) bad |= 1u << e;
+    } else if (i0 + 8u <= outputs && (reinterpret_cast<uintptr_t>(p.Y) & 15u) == 0) {
+        const uint4 v = *reinterpret_cast<const uint4*>(p.Y + i0);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (uint32_t e = 0; e < 8u; e++) if (((w[e >> 1] >> (16u * (e & 1u))) & 0x7C00u) == 0x7C00u) bad |= 1u << e;
+    } else {
+        for (uint32_t e = 0; e < 8u; e++) if (i0 + e < outputs && (__half_as_ushort(p.Y[i0 + e]) & 0x7C00u) == 0x7C00u) bad |= 1u << e;
+    }
+    for (uint32_t who = __ballot_sync(0xffffffffu, bad != 0u); who; who &= who - 1u) {
+        const int src = __ffs((int)who) - 1;
+        const size_t base = i0 + ((size_t)src - lane) * 8u;
+        for (uint32_t b = __shfl_sync(0xffffffffu, bad, src); b; b &= b - 1u) {
+            const size_t o = base + (uint32_t)(__ffs((int)b) - 1);
+            uint32_t tok, n;
+            if (p.layout == 1u && !p.partial_out) {           // [head][token][D]
+                const size_t row = o / p.D;
+                tok = (uint32_t)(row % p.M); n = (uint32_t)(row / p.M) * p.D + (uint32_t)(o % p.D);
+            } else { tok = (uint32_t)(o / p.N); n = (uint32_t)(o % p.N); }
+            const __half* x = X + (size_t)tok * p.K;
+            float acc = 0.0f, acc2 = 0.0f;
+            for (uint32_t k = lane; k < p.K; k += 32u) {
+                const float a = __half2float(x[k]);
+                acc += a * generic_weight(fmt, W0, n, k, p.N, p.K);
+                if (W1) acc2 += a * generic_weight(fmt, W1, n, k, p.N, p.K);
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) { acc += __shfl_xor_sync(0xffffffffu, acc, d); acc2 += __shfl_xor_sync(0xffffffffu, acc2, d); }
+            if (lane == 0u) generic_store(p, tok, n, acc, acc2, W1 != nullptr);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1604,6 +1653,29 @@ bool fast_path_ok(const GemmArgs& a) {
 }
 
 namespace {
+// The repair behind a padded launch reads the residual a second time: one that Y overwrites is kept in the scratch.
+size_t kept_residual_bytes(const GemmArgs& a) {
+    const uintptr_t r = (uintptr_t)a.residual, y = (uintptr_t)a.Y, n = (size_t)a.M * a.N * 2;
+    return a.residual && r < y + n && y < r + n ? (n + 255) & ~(size_t)255 : 0;
+}
+Params generic_params(const GemmArgs& a) {
+    Params p;
+    memset(&p, 0, sizeof(p));
+    p.M = a.M; p.N = a.N; p.K = a.K;
+    p.Y = (__half*)a.Y; p.residual = (const __half*)a.residual; p.partial_out = a.partial_out;
+    p.layout = (uint32_t)a.layout; p.H = a.H; p.D = a.D ? a.D : 1;
+    return p;
+}
+cudaError_t launch_repair(const GemmArgs& a, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(((size_t)a.M * a.N + 2047) / 2048)); cfg.blockDim = dim3(256); cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, repair_nonfinite_kernel, a.format, (const __half*)a.X, (const uint8_t*)a.W0, (const uint8_t*)a.W1, generic_params(a));
+}
 // what a launch on a padded copy looks like to the planners (the copy itself is not there yet)
 GemmArgs padded_probe(const GemmArgs& a) {
     GemmArgs b = a;
@@ -1622,7 +1694,7 @@ bool persistent_splits_poorly(const GemmArgs& a) {
 }
 
 size_t workspace_floats(const GemmArgs& a) {
-    if (pad_path_ok(a)) return workspace_floats(padded_probe(a)) + (padded_bytes(a) + 512) / sizeof(float);
+    if (pad_path_ok(a)) return workspace_floats(padded_probe(a)) + (padded_bytes(a) + kept_residual_bytes(a) + 512) / sizeof(float);
     if (gemv_path_ok(a)) return 0;
     if (small_path_ok(a)) return small_scratch_floats(a);
     if (!fast_path_ok(a)) return 0;
@@ -1638,27 +1710,30 @@ cudaError_t launch(const GemmArgs& a, const Workspace& ws, cudaStream_t stream) 
     if (small_path_ok(a)) return launch_small(a, ws, stream);
     if (fast_path_ok(a)) return dispatch_fast(a, ws, stream);
     if (pad_path_ok(a) && ws.partial && ws.partial_floats >= workspace_floats(a)) {
-        // [padded copies][split-K scratch], both on 256-byte boundaries
-        const size_t bytes = padded_bytes(a);
+        // [padded copies][residual that Y overwrites][split-K scratch], each on a 256-byte boundary
+        const size_t bytes = padded_bytes(a), kept = kept_residual_bytes(a);
         uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws.partial) + 255) & ~(uintptr_t)255);
-        GemmArgs b;
-        cudaError_t e = launch_pad(a, base, b, stream);
+        GemmArgs src = a, b;
+        cudaError_t e = cudaSuccess;
+        if (kept) {
+            src.residual = base + bytes;
+            e = cudaMemcpyAsync(base + bytes, a.residual, (size_t)a.M * a.N * 2, cudaMemcpyDeviceToDevice, stream);
+            if (e != cudaSuccess) return e;
+        }
+        e = launch_pad(src, base, b, stream);
         if (e != cudaSuccess) return e;
         Workspace rest = ws;
-        rest.partial = reinterpret_cast<float*>(base + bytes);
+        rest.partial = reinterpret_cast<float*>(base + bytes + kept);
         rest.partial_floats = ws.partial_floats - (size_t)(rest.partial - ws.partial);
         e = launch(b, rest, stream);
-        g_last_launches = 2;
+        if (e != cudaSuccess) return e;
+        e = launch_repair(src, stream);
+        g_last_launches = 3;
         return e;
     }
     if (a.scatter.world || a.n_extra) return cudaErrorInvalidValue;   // fused reduce-scatter and grouped launches exist on the tensor-core path only
-    Params p;
-    memset(&p, 0, sizeof(p));
-    p.M = a.M; p.N = a.N; p.K = a.K;
-    p.Y = (__half*)a.Y; p.residual = (const __half*)a.residual; p.partial_out = a.partial_out;
-    p.layout = (uint32_t)a.layout; p.H = a.H; p.D = a.D ? a.D : 1;
     dim3 block(32, 8), grid((a.N + 31) / 32, (a.M + 7) / 8);
-    qgemm_generic_kernel<<<grid, block, 0, stream>>>(a.format, (const __half*)a.X, (const uint8_t*)a.W0, (const uint8_t*)a.W1, p);
+    qgemm_generic_kernel<<<grid, block, 0, stream>>>(a.format, (const __half*)a.X, (const uint8_t*)a.W0, (const uint8_t*)a.W1, generic_params(a));
     return cudaGetLastError();
 }
 

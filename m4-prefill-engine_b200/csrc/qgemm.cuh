@@ -99,7 +99,7 @@ bool persistent_splits_poorly(const GemmArgs& a);
 cudaError_t launch_small(const GemmArgs& a, const Workspace& ws, cudaStream_t stream);
 void set_small_kernel_enabled(int mode);     // testing hook: 0 routes those shapes to the persistent kernel again, 1 default,
                                              // 2 takes every shape the kernel can compute (any number of token tiles)
-// Number of kernels the last launch() enqueued (1, or 2 with the generic tail) -- for launch accounting.
+// Number of kernels the last launch() enqueued (1; 3 on a padded copy) -- for launch accounting.
 int last_launch_count();
 void set_pair_kernel_enabled(bool on);        // testing hook: off keeps every launch of the persistent kernel on one CTA per MMA
 int last_launch_pairs();                      // CTA pairs (cta_group::2) of the last persistent-kernel launch, 0 if it ran without
