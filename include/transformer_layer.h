@@ -91,6 +91,7 @@ public:
     uint32_t kernels_per_forward() const { return launches_; }
 
 private:
+    void size_attention_scratch();
     struct Impl;
     Impl* impl_;
     TransformerLayerConfig config_;

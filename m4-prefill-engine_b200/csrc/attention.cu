@@ -1027,7 +1027,7 @@ template <int G> cudaError_t launch_tc(const Params& p, cudaStream_t stream) {
 }
 
 
-int g_last_launches = 1;     // kernels the last launch_attention call enqueued
+thread_local int g_last_launches = 1;     // kernels this thread's last launch_attention call enqueued
 
 template <int D> size_t smem_bytes() {
     constexpr int LD = D + 8;
@@ -1035,7 +1035,14 @@ template <int D> size_t smem_bytes() {
     return (size_t)(BQ + 2 * BK) * LD * 2 + 4 * (size_t)RAW_TILE_PAD;
 }
 
-cudaError_t launch_attention(const Params& p, uint32_t D, cudaStream_t stream) {
+static ws::Args ws_args(const Params& p, uint32_t D) {
+    ws::Args a;
+    a.Q = p.Q; a.K = p.K; a.V = p.V; a.O = p.O; a.Hq = p.Hq; a.Hkv = p.Hkv; a.M = p.M; a.Mkv = p.Mkv; a.D = D; a.pos0 = p.pos0;
+    a.scale_log2e = p.scale_log2e; a.out_tokens_major = p.out_tokens_major; a.kv_fp16 = p.kv_fp16;
+    return a;
+}
+
+cudaError_t launch_attention(const Params& p, uint32_t D, const ws::Scratch& scratch, cudaStream_t stream) {
     // grouped-head kernel when the group size divides its 128-row tile into whole warps
     const uint32_t G = p.Hq / p.Hkv;
     g_last_launches = 1;
@@ -1043,11 +1050,9 @@ cudaError_t launch_attention(const Params& p, uint32_t D, cudaStream_t stream) {
     // What it cannot take -- O not 16-byte aligned, more than 128 query heads per kv head -- stays on the kernels below.
     const bool tc_ok = D == 128 && ((uintptr_t)p.Q & 15u) == 0 && ((uintptr_t)p.O & 15u) == 0;
     if (g_force_legacy == 0) {
-        ws::Args a;
-        a.Q = p.Q; a.K = p.K; a.V = p.V; a.O = p.O; a.Hq = p.Hq; a.Hkv = p.Hkv; a.M = p.M; a.Mkv = p.Mkv; a.D = D; a.pos0 = p.pos0;
-        a.scale_log2e = p.scale_log2e; a.out_tokens_major = p.out_tokens_major; a.kv_fp16 = p.kv_fp16;
+        const ws::Args a = ws_args(p, D);
         if (ws::usable(a)) {
-            const cudaError_t e = ws::launch(a, stream, &g_last_launches);
+            const cudaError_t e = ws::launch(a, scratch, stream, &g_last_launches);
             if (e != cudaErrorMemoryAllocation) return e;
             cudaGetLastError();              // no scratch for the expanded cache: the kernels below unpack it themselves
             g_last_launches = 1;
@@ -1102,15 +1107,26 @@ cudaError_t launch_dequantize(const void* src, void* dst, size_t n_elements, cud
 
 int last_attention_launches() { return g_last_launches; }
 
-cudaError_t launch_attention_simple(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv,
-                                    uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int out_tokens_major,
-                                    int kv_fp16, cudaStream_t stream) {
+static Params simple_params(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv,
+                            float scale, uint32_t pos0, int out_tokens_major, int kv_fp16) {
     Params p;
     p.Q = (const __half*)Q; p.K = (const uint8_t*)K; p.V = (const uint8_t*)V; p.O = (__half*)O;
     p.Hq = Hq; p.Hkv = Hkv; p.M = M; p.Mkv = Mkv; p.pos0 = pos0;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.out_tokens_major = out_tokens_major; p.kv_fp16 = kv_fp16;
-    return launch_attention(p, D, stream);
+    return p;
+}
+
+size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16) {
+    void* at16 = (void*)16;                                  // alignment probe only
+    const ws::Args a = ws_args(simple_params(at16, at16, at16, at16, Hq, Hkv, M, Mkv, scale, pos0, 1, kv_fp16), D);
+    return ws::usable(a) ? ws::scratch_bytes(a, true) : 0;
+}
+
+cudaError_t launch_attention_simple(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv,
+                                    uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int out_tokens_major,
+                                    int kv_fp16, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
+    return launch_attention(simple_params(Q, K, V, O, Hq, Hkv, M, Mkv, scale, pos0, out_tokens_major, kv_fp16), D, ws::Scratch{scratch, scratch_bytes}, stream);
 }
 
 }  // namespace attn
@@ -1191,7 +1207,11 @@ int b200_bridge_dispatch_attention_q8kv(void* Q, void* K, void* V, void* O, uint
     p.Hq = Hq; p.Hkv = Hkv; p.M = M; p.Mkv = Mkv; p.pos0 = pos0;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.out_tokens_major = out_tokens_major; p.kv_fp16 = kv_fp16;
-    if (attn::launch_attention(p, D, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
+    // scratch of the bridge's own stream; under capture it cannot grow, and the launch does with what is there
+    const attn::ws::Args wa = attn::ws_args(p, D);
+    const size_t need = attn::ws::usable(wa) ? attn::ws::scratch_bytes(wa, true) : 0;
+    if (need > g.attn_scratch.cap && !capturing(g.stream)) g.attn_scratch.ensure(need);
+    if (attn::launch_attention(p, D, attn::ws::Scratch{g.attn_scratch.p, g.attn_scratch.cap}, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
     g.launches += (uint64_t)attn::g_last_launches;
     if (host_dst && copy_back(host_dst, p.O, q_bytes) != 0) return -5;
     return 0;

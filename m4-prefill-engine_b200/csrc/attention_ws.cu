@@ -568,7 +568,25 @@ uint32_t choose_splits(uint32_t heads, uint32_t blocks, uint32_t n_first, uint32
     return best;
 }
 
-template <int D, bool LAG> cudaError_t launch_d(const Args& a, cudaStream_t stream, int* launches) {
+struct Plan { uint32_t BP, blocks, n_last, splits; size_t kv_elems, kv_bytes, o_bytes, ml_bytes; };
+Plan make_plan(const Args& a, bool split) {
+    Plan pl;
+    pl.BP = (uint32_t)ROWS / (a.Hq / a.Hkv);
+    pl.blocks = (a.M + 2 * pl.BP - 1) / (2 * pl.BP);
+    auto tiles = [&](uint64_t pos) {      // key tiles of a block whose last position is `pos`
+        const uint64_t last = (uint64_t)a.pos0 + (pos < a.M ? pos : a.M - 1);
+        return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / BK + 1);
+    };
+    pl.n_last = tiles(a.M - 1);
+    pl.splits = split ? choose_splits(a.Hkv, pl.blocks, tiles(2ull * pl.BP - 1), pl.n_last) : 1u;
+    pl.kv_elems = (size_t)a.Hkv * a.Mkv * a.D;
+    pl.kv_bytes = a.kv_fp16 ? 0 : (2 * pl.kv_elems * sizeof(__half) + 255) & ~(size_t)255;
+    const size_t rows = pl.splits > 1 ? pl.splits * (size_t)a.Hq * a.M : 0;
+    pl.o_bytes = rows * a.D * sizeof(float); pl.ml_bytes = rows * sizeof(float2);
+    return pl;
+}
+
+template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc, cudaStream_t stream, int* launches) {
     using C = Cfg<D>;
     static bool attr_set = false;
     if (!attr_set) {
@@ -576,31 +594,17 @@ template <int D, bool LAG> cudaError_t launch_d(const Args& a, cudaStream_t stre
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
+    Plan pl = make_plan(a, true);
+    if (pl.kv_bytes + pl.o_bytes + pl.ml_bytes > sc.bytes) pl = make_plan(a, false);
+    if (pl.kv_bytes > sc.bytes) return cudaErrorMemoryAllocation;
+    const uint32_t splits = pl.splits, blocks = pl.blocks;
+    const size_t kv_elems = pl.kv_elems, kv_bytes = pl.kv_bytes, o_bytes = pl.o_bytes, rows = (size_t)a.Hq * a.M;
     Params p;
-    p.G = a.Hq / a.Hkv; p.BP = (uint32_t)ROWS / p.G;
+    p.G = a.Hq / a.Hkv; p.BP = pl.BP;
     p.Hq = a.Hq; p.M = a.M; p.Mkv = a.Mkv; p.pos0 = a.pos0; p.scale_log2e = a.scale_log2e;
     p.out_tokens_major = a.out_tokens_major; p.O = (__half*)a.O; p.err = bridge::g.err_word;
-    const uint32_t blocks = (a.M + 2 * p.BP - 1) / (2 * p.BP);
-    auto tiles = [&](uint64_t pos) {      // key tiles of a block whose last position is `pos`
-        const uint64_t last = (uint64_t)a.pos0 + (pos < a.M ? pos : a.M - 1);
-        return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / BK + 1);
-    };
-    const uint32_t n_last = tiles(a.M - 1), n_first = tiles(2ull * p.BP - 1);
-    uint32_t splits = choose_splits(a.Hkv, blocks, n_first, n_last);
-    // scratch: the expanded cache, then the partial results
-    const size_t kv_elems = (size_t)a.Hkv * a.Mkv * D;
-    const size_t kv_bytes = a.kv_fp16 ? 0 : (2 * kv_elems * sizeof(__half) + 255) & ~(size_t)255;
-    const size_t rows = (size_t)a.Hq * a.M;
-    size_t o_bytes = splits > 1 ? splits * rows * D * sizeof(float) : 0, ml_bytes = splits > 1 ? splits * rows * sizeof(float2) : 0;
-    if (kv_bytes + o_bytes + ml_bytes > bridge::g.kv_fp16.cap) {
-        // under capture the block cannot grow: without a split, or (see launch_attention) on the kernels that need no scratch
-        if (bridge::capturing(stream)) {
-            splits = 1; o_bytes = ml_bytes = 0;
-            if (kv_bytes > bridge::g.kv_fp16.cap) return cudaErrorMemoryAllocation;
-        } else if (!bridge::g.kv_fp16.ensure(kv_bytes + o_bytes + ml_bytes)) return cudaErrorMemoryAllocation;
-    }
-    p.tiles_per_split = (n_last + splits - 1) / splits;
-    uint8_t* scratch = static_cast<uint8_t*>(bridge::g.kv_fp16.p);
+    p.tiles_per_split = (pl.n_last + splits - 1) / splits;
+    uint8_t* scratch = static_cast<uint8_t*>(sc.p);
     p.split = splits > 1;
     p.part_o = reinterpret_cast<float*>(scratch + kv_bytes);
     p.part_ml = reinterpret_cast<float2*>(scratch + kv_bytes + o_bytes);
@@ -649,7 +653,12 @@ bool usable(const Args& a) {
     return encode_fn() != nullptr;
 }
 
-cudaError_t launch(const Args& a, cudaStream_t stream, int* launches) {
+size_t scratch_bytes(const Args& a, bool split) {
+    const Plan pl = make_plan(a, split);
+    return pl.kv_bytes + pl.o_bytes + pl.ml_bytes;
+}
+
+cudaError_t launch(const Args& a, const Scratch& sc, cudaStream_t stream, int* launches) {
     // A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
     // arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O: 43.8 against 47.4 us at the 8B
     // prefill, 42.0 against 43.6 for the heads of 64.  128-wide heads in groups of 1, 2, 4 and 8 have always run with it, and with
@@ -657,8 +666,8 @@ cudaError_t launch(const Args& a, cudaStream_t stream, int* launches) {
     // their polynomial adds to fp32 rounding (3.8271e-4 with it, without it and with the short one; the 3.8204e-4 of the warp-level
     // kernels come from their steps of 64 keys: every new maximum of a row is a probability of exactly 1, and they see more of them).
     const uint32_t G = a.Hq / a.Hkv;
-    if (a.D == 128) return G == 1u || G == 2u || G == 4u || G == 8u ? launch_d<128, true>(a, stream, launches) : launch_d<128, false>(a, stream, launches);
-    return launch_d<64, false>(a, stream, launches);
+    if (a.D == 128) return G == 1u || G == 2u || G == 4u || G == 8u ? launch_d<128, true>(a, sc, stream, launches) : launch_d<128, false>(a, sc, stream, launches);
+    return launch_d<64, false>(a, sc, stream, launches);
 }
 
 }  // namespace ws

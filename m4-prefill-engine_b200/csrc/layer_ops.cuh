@@ -14,7 +14,7 @@ cudaError_t rmsnorm_add(const void* A, const void* B, const void* weight, void* 
 cudaError_t rope(void* X, uint32_t H, uint32_t M, uint32_t D, float theta, uint32_t pos0, cudaStream_t s);
 // table[m][j] = (cos, sin) of (pos0 + m) * theta^(-2j/D), float2 [M][D/2]: the rotation operand of the fused projection epilogue.
 cudaError_t build_rope_table(void* table, uint32_t M, uint32_t D, float theta, uint32_t pos0, cudaStream_t s);
-// One launch for everything between the Q/K/V projections and attention (head size 128): rotary embedding on Q [Hq][M][D] and
+// One launch for everything between the Q/K/V projections and attention (head sizes 64 and 128): rotary embedding on Q [Hq][M][D] and
 // K [Hkv][M][D] in place (rope), K and V compressed to Q8_0 records [Hkv][M][D/32] (q8).  Bit-identical to rope() on Q and K
 // followed by attn::launch_quantize on K and V.  With dequant_in_place (and q8) K and V are overwritten by what the records
 // give back, fp16(q * d): the operands of attention over this Q8_0 cache, ready for it as fp16 tiles.
@@ -31,9 +31,11 @@ namespace attn {
 struct Params;
 cudaError_t launch_quantize(const void* src, void* dst, size_t n_elements, cudaStream_t stream);
 cudaError_t launch_dequantize(const void* src, void* dst, size_t n_elements, cudaStream_t stream);
-// thin wrapper so other translation units need not see attn::Params
-int last_attention_launches();     // kernels the last launch_attention_simple call enqueued (2 when a Q8_0 cache was dequantised first)
+int last_attention_launches();     // kernels the calling thread's last launch_attention_simple call enqueued
+// Attention for other translation units, with the caller's scratch (attention_scratch_bytes of it; less is served too, by an unsplit
+// launch or, for a Q8_0 cache, by the kernels that unpack it themselves).
+size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16);
 cudaError_t launch_attention_simple(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv,
                                     uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int out_tokens_major,
-                                    int kv_fp16, cudaStream_t stream);
+                                    int kv_fp16, void* scratch, size_t scratch_bytes, cudaStream_t stream);
 }  // namespace attn

@@ -29,6 +29,8 @@ struct TransformerLayerCoordinator::Impl {
     size_t ws_floats = 0;
     uint32_t* counters = nullptr;
     int* err = nullptr;
+    void* attn_scratch = nullptr;    // of this layer's attention launches (its own: layers may run on several streams)
+    size_t attn_scratch_bytes = 0;
     const void *norm1 = nullptr, *norm2 = nullptr;
     AllReduceFn allreduce = nullptr;
     void* allreduce_ctx = nullptr;
@@ -61,7 +63,7 @@ TransformerLayerCoordinator::TransformerLayerCoordinator(int device, cudaStream_
 
 TransformerLayerCoordinator::~TransformerLayerCoordinator() {
     void* bufs[] = {impl_->xn, impl_->q, impl_->k, impl_->v, impl_->kq, impl_->vq, impl_->attn, impl_->x_mid, impl_->act,
-                    impl_->partial, impl_->ws, impl_->counters, impl_->own_px.done_counter, impl_->rope_table};
+                    impl_->partial, impl_->ws, impl_->counters, impl_->own_px.done_counter, impl_->rope_table, impl_->attn_scratch};
     for (void* b : bufs) if (b) cudaFree(b);
     for (cudaEvent_t e : impl_->events) cudaEventDestroy(e);
     delete impl_;
@@ -132,9 +134,20 @@ bool TransformerLayerCoordinator::initialize_pipelines(const void*) {
         }
     }
     if (!ok) { status_ = -5; return false; }
+    size_attention_scratch();
     impl_->bound = true;
     status_ = 0;
     return true;
+}
+
+// Attention reads fp16 tiles, or (behind the fused Q/K/V epilogue) the Q8_0 records.  Without the memory it runs unsplit.
+void TransformerLayerCoordinator::size_attention_scratch() {
+    const TransformerLayerConfig& c = config_;
+    const uint32_t hq = c.H / c.tp_size, hkv = c.num_kv_heads / c.tp_size;
+    const size_t need = attn::attention_scratch_bytes(hq, hkv, c.M, c.M, c.D, c.attn_scale, 0, impl_->fuse_kv && c.kv_q8_0 ? 0 : 1);
+    if (need <= impl_->attn_scratch_bytes) return;
+    if (impl_->attn_scratch) cudaFree(impl_->attn_scratch);      // (waits for launches that still use it)
+    impl_->attn_scratch_bytes = dev_alloc(&impl_->attn_scratch, need) ? need : 0;
 }
 
 void TransformerLayerCoordinator::set_norm_weights(const void* a, const void* m) { impl_->norm1 = a; impl_->norm2 = m; }
@@ -175,7 +188,10 @@ bool TransformerLayerCoordinator::attach_peer_exchange(peer::Exchange* shared) {
 }
 
 void TransformerLayerCoordinator::set_profiling(bool on) { impl_->profiling = on; }
-void TransformerLayerCoordinator::set_fused_kv_epilogue(bool on) { impl_->fuse_kv = on; }
+void TransformerLayerCoordinator::set_fused_kv_epilogue(bool on) {
+    impl_->fuse_kv = on;
+    if (impl_->bound) size_attention_scratch();
+}
 
 size_t TransformerLayerCoordinator::profile(const char** labels, float* us, size_t cap) const {
     const Impl& im = *impl_;
@@ -291,7 +307,8 @@ void TransformerLayerCoordinator::forward(cudaStream_t stream, const void* X_in,
             mark("quantize k, v to q8_0");
         }
     }
-    check(attn::launch_attention_simple(im.q, kk, vv, im.attn, hq, hkv, c.M, c.M, c.D, c.attn_scale, 0, 1, kv_as_fp16 ? 1 : 0, stream));
+    check(attn::launch_attention_simple(im.q, kk, vv, im.attn, hq, hkv, c.M, c.M, c.D, c.attn_scale, 0, 1, kv_as_fp16 ? 1 : 0,
+                                        im.attn_scratch, im.attn_scratch_bytes, stream));
     launches_ += (uint32_t)(attn::last_attention_launches() - 1);
     mark("attention");
     // 2. O projection + first residual
