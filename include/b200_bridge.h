@@ -131,6 +131,10 @@ int b200_bridge_device_error(void);
 /* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
  * holds now, without a wait on the host.  -6 if that is not possible (a stream under capture). */
 int b200_bridge_wait_stream(void* stream);
+/* Bytes of device memory that captured graphs hold as scratch.  A launch of the bridge under stream capture gets a block of its
+ * graph's own: it is shared with no other launch and given back once the graph and every instance of it are destroyed (at the
+ * next launch outside a capture, or by this call). */
+size_t b200_bridge_graph_scratch_bytes(void);
 const char* b200_bridge_last_error_string(void);
 
 /* Kernels enqueued by this library since init (launch accounting for benchmarks). */

@@ -80,6 +80,8 @@ def bind(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.b200_bridge_unregister_weights.restype = _i
     lib.b200_bridge_wait_stream.argtypes = [_vp]
     lib.b200_bridge_wait_stream.restype = _i
+    lib.b200_bridge_graph_scratch_bytes.argtypes = []
+    lib.b200_bridge_graph_scratch_bytes.restype = ctypes.c_size_t
     lib.b200_bridge_device_error.argtypes = []
     lib.b200_bridge_device_error.restype = _i
     lib.b200_bridge_last_error_string.argtypes = []

@@ -1207,11 +1207,10 @@ int b200_bridge_dispatch_attention_q8kv(void* Q, void* K, void* V, void* O, uint
     p.Hq = Hq; p.Hkv = Hkv; p.M = M; p.Mkv = Mkv; p.pos0 = pos0;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.out_tokens_major = out_tokens_major; p.kv_fp16 = kv_fp16;
-    // scratch of the bridge's own stream; under capture it cannot grow, and the launch does with what is there
     const attn::ws::Args wa = attn::ws_args(p, D);
-    const size_t need = attn::ws::usable(wa) ? attn::ws::scratch_bytes(wa, true) : 0;
-    if (need > g.attn_scratch.cap && !capturing(g.stream)) g.attn_scratch.ensure(need);
-    if (attn::launch_attention(p, D, attn::ws::Scratch{g.attn_scratch.p, g.attn_scratch.cap}, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
+    Block scratch;                          // (without one the kernels that need none take over)
+    if (attn::ws::usable(wa)) launch_block(g.attn_scratch, attn::ws::scratch_bytes(wa, true), &scratch);
+    if (attn::launch_attention(p, D, attn::ws::Scratch{scratch.p, scratch.bytes}, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
     g.launches += (uint64_t)attn::g_last_launches;
     if (host_dst && copy_back(host_dst, p.O, q_bytes) != 0) return -5;
     return 0;

@@ -7,6 +7,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <list>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -114,16 +115,91 @@ bool capturing(cudaStream_t stream) {
     return cap != cudaStreamCaptureStatusNone;
 }
 
-// Scratch for a launch.  Under capture the block cannot grow: the launch then does with what is there, by the rules that need
-// the least.
-bool ensure_workspace(qg::GemmArgs& a) {
-    size_t floats = qg::workspace_floats(a);
-    if (floats * sizeof(float) <= g.ws_partial.cap) return true;
-    if (capturing(g.stream)) {
-        a.lean = 1;
-        return qg::workspace_floats(a) * sizeof(float) <= g.ws_partial.cap;
+namespace {
+
+// Blocks of captured graphs.  A graph holds its block through a user object, whose destructor may not call into CUDA: it marks the
+// block, and the next launch outside a capture frees it (or the next capture takes it over).
+struct GraphBlock { unsigned long long capture; uint8_t* p; size_t bytes; std::atomic<bool> released; };
+std::list<GraphBlock> graph_blocks;                         // (under State::mu; entries do not move)
+constexpr size_t COUNTER_BYTES = 4096 * sizeof(uint32_t);    // in front of a block's scratch
+
+// cudaMalloc and cudaFree are not allowed to a thread while a capture in global mode is under way, unless the thread says that it
+// knows what it is doing; neither touches the capturing stream.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+void CUDART_CB graph_block_released(void* b) { static_cast<GraphBlock*>(b)->released.store(true); }
+
+void free_released_blocks() {
+    for (auto it = graph_blocks.begin(); it != graph_blocks.end();) {
+        if (!it->released.load()) { ++it; continue; }
+        RelaxedCapture relaxed;
+        cudaFree(it->p);
+        it = graph_blocks.erase(it);
     }
-    return g.ws_partial.ensure(floats * sizeof(float));
+}
+
+bool graph_block(unsigned long long capture, cudaGraph_t graph, size_t bytes, Block* out) {
+    GraphBlock* b = nullptr;
+    for (GraphBlock& o : graph_blocks) if (!o.released.load() && o.capture == capture && o.bytes >= bytes) b = &o;
+    if (!b) {
+        for (GraphBlock& o : graph_blocks) if (o.released.load() && o.bytes >= bytes && (!b || o.bytes < b->bytes)) b = &o;
+        if (!b) {
+            void* p = nullptr;
+            {
+                RelaxedCapture relaxed;
+                if (cudaMalloc(&p, COUNTER_BYTES + bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+            }
+            graph_blocks.emplace_back();
+            b = &graph_blocks.back();
+            b->p = static_cast<uint8_t*>(p); b->bytes = bytes;
+        }
+        b->capture = capture;
+        b->released.store(false);
+        cudaUserObject_t owner;
+        if (cudaUserObjectCreate(&owner, b, graph_block_released, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+            cudaGetLastError(); b->released.store(true); return false;
+        }
+        if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+            cudaGetLastError(); cudaUserObjectRelease(owner, 1); return false;          // (the release marks the block)
+        }
+        if (cudaMemsetAsync(b->p, 0, COUNTER_BYTES, g.stream) != cudaSuccess) { cudaGetLastError(); return false; }
+    }
+    out->p = b->p + COUNTER_BYTES; out->bytes = b->bytes; out->counters = reinterpret_cast<uint32_t*>(b->p);
+    return true;
+}
+
+}  // namespace
+
+bool launch_block(DevBuf& buf, size_t bytes, Block* out) {
+    *out = Block{};
+    out->counters = g.counters;
+    if (bytes == 0) return true;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(g.stream, &status, &capture, &graph) != cudaSuccess) cudaGetLastError();
+    if (status == cudaStreamCaptureStatusActive) return graph_block(capture, graph, bytes, out);
+    if (!graph_blocks.empty()) free_released_blocks();
+    if (!buf.ensure(bytes)) return false;
+    out->p = buf.p; out->bytes = buf.cap;
+    return true;
+}
+
+// Scratch for a projection; where a graph cannot have its block, by the rules that need the least.
+bool workspace_for(qg::GemmArgs& a, qg::Workspace& ws) {
+    Block b;
+    if (!launch_block(g.ws_partial, qg::workspace_floats(a) * sizeof(float), &b)) {
+        if (!capturing(g.stream)) return false;
+        a.lean = 1;
+        if (!launch_block(g.ws_partial, qg::workspace_floats(a) * sizeof(float), &b)) return false;
+    }
+    ws.partial = (float*)b.p; ws.partial_floats = b.bytes / sizeof(float);
+    ws.counters = b.counters; ws.err = g.err_word;
+    return true;
 }
 
 int validate_gemm(const void* X, size_t Xb, const void* W, size_t Wb, const void* Y, size_t Yb, int format, bool extended,
@@ -177,15 +253,13 @@ int run_gemm(void* X, size_t Xb, void* W0, void* W1, size_t Wb, void* Y, size_t 
     a.M = M; a.N = N; a.K = K; a.layout = layout; a.H = H; a.D = D;
     a.force_generic = g.force_generic;
     (void)Xb; (void)Wb; (void)Yb;
-    if (!ensure_workspace(a)) return -5;
+    qg::Workspace ws;
+    if (!workspace_for(a, ws)) return -5;
     if (staged_in) {
         cudaEventRecord(sl.ev_in, g.stream_in);
         cudaStreamWaitEvent(g.stream, sl.ev_in, 0);
     }
     if (host_dst && sl.out_pending) cudaStreamWaitEvent(g.stream, sl.ev_out, 0);
-    qg::Workspace ws;
-    ws.partial = (float*)g.ws_partial.p; ws.partial_floats = g.ws_partial.cap / sizeof(float);
-    ws.counters = g.counters; ws.err = g.err_word;
     cudaError_t e = qg::launch(a, ws, g.stream);
     if (e != cudaSuccess) { set_error(std::string("kernel launch failed: ") + cudaGetErrorString(e)); return -6; }
     g.launches += (uint64_t)qg::last_launch_count();
@@ -330,10 +404,8 @@ int b200_bridge_dispatch_gemm_grouped(const void* X, const void* const* W, void*
     a.n_extra = count - 1;
     for (uint32_t i = 1; i < count; i++) { a.W_extra[i - 1] = W[i]; a.Y_extra[i - 1] = Y[i]; a.N_extra[i - 1] = N[i]; }
     a.force_generic = g.force_generic;
-    if (!ensure_workspace(a)) return -5;      // few-token grouped launches split K
     qg::Workspace ws;
-    ws.partial = (float*)g.ws_partial.p; ws.partial_floats = g.ws_partial.cap / sizeof(float);
-    ws.counters = g.counters; ws.err = g.err_word;
+    if (!workspace_for(a, ws)) return -5;      // few-token grouped launches split K
     cudaError_t e = qg::launch(a, ws, g.stream);
     if (e == cudaErrorInvalidValue) { cudaGetLastError(); return -4; }
     if (e != cudaSuccess) { set_error(std::string("kernel launch failed: ") + cudaGetErrorString(e)); return -6; }
@@ -373,10 +445,8 @@ int b200_bridge_dispatch_qkv_fused(const void* X, const void* Wq, const void* Wk
         a.rope_table = g.rope_table.p;
     }
     if (!a.post[0] && !a.post[1] && !a.post[2]) {}            // nothing to fuse: a plain grouped launch
-    if (!ensure_workspace(a)) return -5;
     qg::Workspace ws;
-    ws.partial = (float*)g.ws_partial.p; ws.partial_floats = g.ws_partial.cap / sizeof(float);
-    ws.counters = g.counters; ws.err = g.err_word;
+    if (!workspace_for(a, ws)) return -5;
     cudaError_t e = qg::launch(a, ws, g.stream);
     if (e == cudaErrorInvalidValue) { cudaGetLastError(); return -4; }
     if (e != cudaSuccess) { set_error(std::string("kernel launch failed: ") + cudaGetErrorString(e)); return -6; }
@@ -473,6 +543,7 @@ void m4_bridge_shutdown(void) {
     g.ws_partial.release();
     g.rope_table.release(); g.rope_M = g.rope_D = 0;
     g.attn_scratch.release();
+    free_released_blocks();              // (graphs that are still there keep theirs)
     for (auto& kv : g.registered) cudaFree(kv.second.dev);
     g.registered.clear();
     cudaFree(g.counters); g.counters = nullptr; g.err_word = nullptr;
@@ -523,6 +594,15 @@ int b200_bridge_debug_set_tile_counter(uint32_t index, uint32_t value) {
     if (index >= 4096) return -2;
     cudaStreamSynchronize(g.stream);
     return cudaMemcpy(g.counters + index, &value, sizeof(uint32_t), cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -6;
+}
+
+/* Device memory that captured graphs hold as scratch (what graphs that are gone have left is given back first). */
+size_t b200_bridge_graph_scratch_bytes(void) {
+    std::lock_guard<std::mutex> lock(g.mu);
+    free_released_blocks();
+    size_t n = 0;
+    for (const GraphBlock& b : graph_blocks) n += COUNTER_BYTES + b.bytes;
+    return n;
 }
 
 const char* b200_bridge_last_error_string(void) { return g.last_error.c_str(); }

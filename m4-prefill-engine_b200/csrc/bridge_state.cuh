@@ -67,8 +67,12 @@ void set_error(const std::string& s);
 bool is_device_ptr(const void* ptr);
 const void* resolve_in(const void* ptr, size_t bytes, DevBuf& stage, bool weights, int* rc);
 void* resolve_out(void* ptr, size_t bytes, DevBuf& stage, void** host_dst, int* rc);
-// The stream is being captured: nothing may be allocated now (cudaMalloc would invalidate the capture).
 bool capturing(cudaStream_t stream);
+// Scratch for a launch on the bridge's stream, and the split-K counters that go with it.  Outside a capture: `buf`, grown as needed.
+// Under capture: a block of the graph that is being captured, which no other launch uses and which stays until the graph and
+// everything instantiated from it are destroyed; the counters are zeroed by a node of the graph.  False: no memory.
+struct Block { void* p = nullptr; size_t bytes = 0; uint32_t* counters = nullptr; };
+bool launch_block(DevBuf& buf, size_t bytes, Block* out);
 // Device -> host copy of a staged result on the main stream (entry points other than the projections).
 int copy_back(void* host_dst, const void* dev_src, size_t bytes);
 // Static split-K scratch of the allocation-free entry point (no_alloc.cu): made resident at init, forgotten at shutdown.
