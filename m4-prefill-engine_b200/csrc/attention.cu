@@ -1117,10 +1117,10 @@ static Params simple_params(const void* Q, const void* K, const void* V, void* O
     return p;
 }
 
-size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16) {
+size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16, bool split) {
     void* at16 = (void*)16;                                  // alignment probe only
     const ws::Args a = ws_args(simple_params(at16, at16, at16, at16, Hq, Hkv, M, Mkv, scale, pos0, 1, kv_fp16), D);
-    return ws::usable(a) ? ws::scratch_bytes(a, true) : 0;
+    return ws::usable(a) ? ws::scratch_bytes(a, split) : 0;
 }
 
 cudaError_t launch_attention_simple(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv,
@@ -1208,8 +1208,9 @@ int b200_bridge_dispatch_attention_q8kv(void* Q, void* K, void* V, void* O, uint
     p.scale_log2e = scale * 1.4426950408889634f;
     p.out_tokens_major = out_tokens_major; p.kv_fp16 = kv_fp16;
     const attn::ws::Args wa = attn::ws_args(p, D);
-    Block scratch;                          // (without one the kernels that need none take over)
-    if (attn::ws::usable(wa)) launch_block(g.attn_scratch, attn::ws::scratch_bytes(wa, true), &scratch);
+    Block scratch;                          // (without the memory: an unsplit launch, or the kernels that need none)
+    if (attn::ws::usable(wa) && !launch_block(g.attn_scratch, attn::ws::scratch_bytes(wa, true), &scratch))
+        launch_block(g.attn_scratch, attn::ws::scratch_bytes(wa, false), &scratch);
     if (attn::launch_attention(p, D, attn::ws::Scratch{scratch.p, scratch.bytes}, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
     g.launches += (uint64_t)attn::g_last_launches;
     if (host_dst && copy_back(host_dst, p.O, q_bytes) != 0) return -5;

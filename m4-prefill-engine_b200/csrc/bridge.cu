@@ -22,12 +22,20 @@ namespace bridge {
 
 State g;
 
+cudaError_t scratch_malloc(void** p, size_t bytes) {
+    const size_t limit = g.scratch_limit;
+    if (limit && bytes > limit) { *p = nullptr; return cudaErrorMemoryAllocation; }
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }
+    return e;
+}
+
 bool DevBuf::ensure(size_t n) {
     if (n <= cap) return true;
     if (p) cudaFree(p);        // implicit device sync: nothing in flight still uses the old block
     p = nullptr; cap = 0;
     size_t want = n + n / 4;
-    if (cudaMalloc(&p, want) != cudaSuccess) { cudaGetLastError(); p = nullptr; return false; }
+    if (scratch_malloc(&p, want) != cudaSuccess) return false;
     cap = want;
     return true;
 }
@@ -151,7 +159,7 @@ bool graph_block(unsigned long long capture, cudaGraph_t graph, size_t bytes, Bl
             void* p = nullptr;
             {
                 RelaxedCapture relaxed;
-                if (cudaMalloc(&p, COUNTER_BYTES + bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+                if (scratch_malloc(&p, COUNTER_BYTES + bytes) != cudaSuccess) return false;
             }
             graph_blocks.emplace_back();
             b = &graph_blocks.back();
@@ -189,11 +197,10 @@ bool launch_block(DevBuf& buf, size_t bytes, Block* out) {
     return true;
 }
 
-// Scratch for a projection; where a graph cannot have its block, by the rules that need the least.
+// Scratch for a projection; where the memory is not to be had, by the rules that need the least.
 bool workspace_for(qg::GemmArgs& a, qg::Workspace& ws) {
     Block b;
     if (!launch_block(g.ws_partial, qg::workspace_floats(a) * sizeof(float), &b)) {
-        if (!capturing(g.stream)) return false;
         a.lean = 1;
         if (!launch_block(g.ws_partial, qg::workspace_floats(a) * sizeof(float), &b)) return false;
     }
@@ -585,6 +592,12 @@ int b200_bridge_clear_device_error(void) {
     // A split-K launch that gave up on a bounded wait leaves its tile counters part-way: the counters and the error
     // word are one block and are cleared together, so the next split-K launch starts from zero again.
     return cudaMemset(g.counters, 0, 4096 * sizeof(uint32_t) + 64) == cudaSuccess ? 0 : -6;
+}
+
+/* Testing hook: allocations of scratch beyond `bytes` fail as if the GPU were full (0: no limit). */
+void b200_bridge_debug_limit_scratch(size_t bytes) {
+    std::lock_guard<std::mutex> lock(g.mu);
+    g.scratch_limit = bytes;
 }
 
 /* Testing hook: writes `value` into split-K tile counter `index` (what an aborted split-K launch leaves behind). */

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -59,10 +60,13 @@ struct State {
     std::string last_error;
     uint64_t launches = 0, h2d_bytes = 0, d2h_bytes = 0;
     int force_generic = 0;
+    std::atomic<size_t> scratch_limit{0};   // testing hook: larger allocations of scratch fail
 };
 
 extern State g;
 
+// cudaMalloc for scratch that a launch can do without, or with less of
+cudaError_t scratch_malloc(void** p, size_t bytes);
 void set_error(const std::string& s);
 bool is_device_ptr(const void* ptr);
 const void* resolve_in(const void* ptr, size_t bytes, DevBuf& stage, bool weights, int* rc);

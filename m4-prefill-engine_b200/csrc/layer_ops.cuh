@@ -32,9 +32,10 @@ struct Params;
 cudaError_t launch_quantize(const void* src, void* dst, size_t n_elements, cudaStream_t stream);
 cudaError_t launch_dequantize(const void* src, void* dst, size_t n_elements, cudaStream_t stream);
 int last_attention_launches();     // kernels the calling thread's last launch_attention_simple call enqueued
-// Attention for other translation units, with the caller's scratch (attention_scratch_bytes of it; less is served too, by an unsplit
-// launch or, for a Q8_0 cache, by the kernels that unpack it themselves).
-size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16);
+// Attention for other translation units, with the caller's scratch (attention_scratch_bytes of it, with or without a split key range;
+// less is served too: a Q8_0 cache by the kernels that unpack it themselves).
+size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16,
+                               bool split);
 cudaError_t launch_attention_simple(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv,
                                     uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int out_tokens_major,
                                     int kv_fp16, void* scratch, size_t scratch_bytes, cudaStream_t stream);

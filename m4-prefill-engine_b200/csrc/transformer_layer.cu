@@ -31,6 +31,7 @@ struct TransformerLayerCoordinator::Impl {
     int* err = nullptr;
     void* attn_scratch = nullptr;    // of this layer's attention launches (its own: layers may run on several streams)
     size_t attn_scratch_bytes = 0;
+    int lean = 0;                    // the projections' scratch is the least they can do with
     const void *norm1 = nullptr, *norm2 = nullptr;
     AllReduceFn allreduce = nullptr;
     void* allreduce_ctx = nullptr;
@@ -98,12 +99,12 @@ bool TransformerLayerCoordinator::initialize_pipelines(const void*) {
              lops::build_rope_table(impl_->rope_table, c.M, c.D, c.rope_theta, 0, impl_->stream) == cudaSuccess;
     }
     // scratch (split K, padded copies): sized for the largest projection of this layer, each probed with the outputs it has
-    if (ok) {
+    const void* at16 = (const void*)16;                     // alignment probes only
+    auto scratch_floats = [&](int lean) {
         size_t need = 0;
-        const void* at16 = (const void*)16;                 // alignment probes only
         auto probe = [&](uint32_t n, uint32_t k, bool dual, bool residual, bool partial) {
             qg::GemmArgs a; memset(&a, 0, sizeof(a));
-            a.format = c.weight_format; a.M = c.M; a.N = n; a.K = k; a.D = c.D;
+            a.format = c.weight_format; a.M = c.M; a.N = n; a.K = k; a.D = c.D; a.lean = lean;
             a.X = at16; a.W0 = at16; a.W1 = dual ? at16 : nullptr; a.Y = (void*)16;
             a.residual = residual ? at16 : nullptr; a.partial_out = partial ? (float*)16 : nullptr;
             const size_t w = qg::workspace_floats(a);
@@ -116,17 +117,23 @@ bool TransformerLayerCoordinator::initialize_pipelines(const void*) {
             probe(c.K, f, false, form == 1, form == 2);
         }
         probe(f, c.K, true, false, false);
-        {   // the grouped Q + K + V launch
-            qg::GemmArgs a; memset(&a, 0, sizeof(a));
-            a.format = c.weight_format; a.M = c.M; a.N = hq * c.D; a.K = c.K; a.layout = LAYOUT_DIRECT_HEAD; a.H = hq; a.D = c.D;
-            a.X = (const void*)16; a.W0 = (const void*)16; a.Y = (void*)16;
-            a.n_extra = 2; a.W_extra[0] = a.W_extra[1] = (const void*)16; a.Y_extra[0] = a.Y_extra[1] = (void*)16;
-            a.N_extra[0] = a.N_extra[1] = hkv * c.D;
-            const size_t w = qg::workspace_floats(a);
-            if (w > need) need = w;
+        // the grouped Q + K + V launch
+        qg::GemmArgs a; memset(&a, 0, sizeof(a));
+        a.format = c.weight_format; a.M = c.M; a.N = hq * c.D; a.K = c.K; a.layout = LAYOUT_DIRECT_HEAD; a.H = hq; a.D = c.D; a.lean = lean;
+        a.X = at16; a.W0 = at16; a.Y = (void*)16;
+        a.n_extra = 2; a.W_extra[0] = a.W_extra[1] = at16; a.Y_extra[0] = a.Y_extra[1] = (void*)16;
+        a.N_extra[0] = a.N_extra[1] = hkv * c.D;
+        const size_t w = qg::workspace_floats(a);
+        return w > need ? w : need;
+    };
+    if (ok) {
+        impl_->ws_floats = scratch_floats(0);
+        if (impl_->ws_floats && bridge::scratch_malloc((void**)&impl_->ws, impl_->ws_floats * 4) != cudaSuccess) {
+            // no room: every projection by the rules that need the least
+            impl_->lean = 1;
+            impl_->ws_floats = scratch_floats(1);
+            if (impl_->ws_floats) ok = dev_alloc((void**)&impl_->ws, impl_->ws_floats * 4);
         }
-        impl_->ws_floats = need;
-        if (need) ok = dev_alloc((void**)&impl_->ws, need * 4);
         if (ok) ok = dev_alloc((void**)&impl_->counters, 4096 * 4 + 64);
         if (ok) {
             cudaMemset(impl_->counters, 0, 4096 * 4 + 64);
@@ -144,10 +151,12 @@ bool TransformerLayerCoordinator::initialize_pipelines(const void*) {
 void TransformerLayerCoordinator::size_attention_scratch() {
     const TransformerLayerConfig& c = config_;
     const uint32_t hq = c.H / c.tp_size, hkv = c.num_kv_heads / c.tp_size;
-    const size_t need = attn::attention_scratch_bytes(hq, hkv, c.M, c.M, c.D, c.attn_scale, 0, impl_->fuse_kv && c.kv_q8_0 ? 0 : 1);
-    if (need <= impl_->attn_scratch_bytes) return;
-    if (impl_->attn_scratch) cudaFree(impl_->attn_scratch);      // (waits for launches that still use it)
-    impl_->attn_scratch_bytes = dev_alloc(&impl_->attn_scratch, need) ? need : 0;
+    for (bool split : {true, false}) {
+        const size_t need = attn::attention_scratch_bytes(hq, hkv, c.M, c.M, c.D, c.attn_scale, 0, impl_->fuse_kv && c.kv_q8_0 ? 0 : 1, split);
+        if (need <= impl_->attn_scratch_bytes) return;
+        if (impl_->attn_scratch) cudaFree(impl_->attn_scratch);      // (waits for launches that still use it)
+        impl_->attn_scratch_bytes = bridge::scratch_malloc(&impl_->attn_scratch, need) == cudaSuccess ? need : 0;
+    }
 }
 
 void TransformerLayerCoordinator::set_norm_weights(const void* a, const void* m) { impl_->norm1 = a; impl_->norm2 = m; }
@@ -228,7 +237,7 @@ void TransformerLayerCoordinator::forward(cudaStream_t stream, const void* X_in,
         if (status_) return;
         qg::GemmArgs a; memset(&a, 0, sizeof(a));
         a.format = kb.format; a.X = X; a.W0 = W0; a.W1 = W1; a.Y = Y; a.M = c.M; a.N = N; a.K = K;
-        a.layout = kb.layout; a.H = H; a.D = c.D; a.residual = residual; a.partial_out = partial_out; a.early_weights = early;
+        a.layout = kb.layout; a.H = H; a.D = c.D; a.residual = residual; a.partial_out = partial_out; a.early_weights = early; a.lean = im.lean;
         if (qg::launch(a, ws, stream) != cudaSuccess) { status_ = -6; return; }
         launches_ += (uint32_t)qg::last_launch_count();
     };
@@ -263,7 +272,7 @@ void TransformerLayerCoordinator::forward(cudaStream_t stream, const void* X_in,
         a.layout = im.head_binding.layout; a.H = hq; a.D = c.D;
         a.n_extra = 2; a.W_extra[0] = W_k; a.W_extra[1] = W_v; a.Y_extra[0] = im.k; a.Y_extra[1] = im.v;
         a.N_extra[0] = a.N_extra[1] = hkv * c.D;
-        a.early_weights = early;
+        a.early_weights = early; a.lean = im.lean;
         if (fuse) {
             const uint32_t rope = c.rope_theta > 0.0f ? 1u : 0u, q8 = c.kv_q8_0 ? 2u : 0u;
             a.post[0] = rope; a.post[1] = rope | q8; a.post[2] = q8;

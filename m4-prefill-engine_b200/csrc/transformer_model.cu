@@ -45,6 +45,7 @@ struct TransformerModel::Impl {
     peer::Exchange* px = nullptr;
     float* ws = nullptr;             // split-K scratch of the head projection
     size_t ws_floats = 0;
+    int lean = 0;                    // that scratch is the least the launch can do with
     uint32_t* counters = nullptr;
     int* err = nullptr;
     KernelBinding head_binding;
@@ -99,10 +100,15 @@ bool TransformerModel::set_head(const void* final_norm, const void* lm_head, uin
     qg::GemmArgs a; memset(&a, 0, sizeof(a));
     a.format = c.weight_format; a.M = c.M; a.N = vocab_rows; a.K = c.K;
     a.X = (const void*)16; a.W0 = (const void*)16; a.Y = (void*)16;     // alignment probes only
-    const size_t need = qg::workspace_floats(a);
+    size_t need = qg::workspace_floats(a);
+    impl_->lean = 0;
     if (need > impl_->ws_floats) {
         if (impl_->ws) { cudaStreamSynchronize(impl_->stream); cudaFree(impl_->ws); impl_->ws = nullptr; impl_->ws_floats = 0; }
-        if (cudaMalloc((void**)&impl_->ws, need * 4) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (bridge::scratch_malloc((void**)&impl_->ws, need * 4) != cudaSuccess) {
+            a.lean = impl_->lean = 1;                                   // no room: by the rules that need the least
+            need = qg::workspace_floats(a);
+            if (need && cudaMalloc((void**)&impl_->ws, need * 4) != cudaSuccess) { cudaGetLastError(); return false; }
+        }
         impl_->ws_floats = need;
     }
     impl_->final_norm = final_norm; impl_->lm_head = lm_head; impl_->vocab_rows = vocab_rows;
@@ -157,6 +163,7 @@ int TransformerModel::forward(cudaStream_t stream, const int32_t* tokens, void* 
         qg::GemmArgs a; memset(&a, 0, sizeof(a));
         a.format = im.head_binding.format; a.X = x; a.W0 = im.lm_head; a.Y = logits; a.M = c.M; a.N = im.vocab_rows; a.K = c.K;
         a.layout = im.head_binding.layout;
+        a.lean = im.lean;
         a.early_weights = c.rms_eps > 0.0f && c.tp_size == 1 ? 1 : 0;      // behind the final normalisation
         qg::Workspace ws;
         ws.partial = im.ws; ws.partial_floats = im.ws_floats; ws.counters = im.counters; ws.err = im.err;
