@@ -129,7 +129,7 @@ int b200_bridge_unregister_weights(const void* host_ptr);
  * embedding table. */
 int b200_bridge_device_error(void);
 /* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
- * holds now, without a wait on the host.  -6 if that is not possible (a stream under capture). */
+ * holds now, without a wait on the host.  -6 if that is not possible (it, or a stream of the bridge, is under capture). */
 int b200_bridge_wait_stream(void* stream);
 /* Bytes of device memory that captured graphs hold as scratch.  A launch of the bridge under stream capture gets a block of its
  * graph's own: it is shared with no other launch and given back once the graph and every instance of it are destroyed (at the

@@ -560,12 +560,14 @@ void m4_bridge_shutdown(void) {
 }
 
 /* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
- * holds now.  -6 if that is not possible (a stream that is being captured): wait on the host instead. */
+ * holds now.  -6 if that is not possible (`stream` or one of the bridge's own is being captured: an edge from work outside the
+ * capture would end it): wait on the host instead. */
 int b200_bridge_wait_stream(void* stream) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.initialized) return -1;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { cudaGetLastError(); return -6; }
+    if (capturing(g.stream) || capturing(g.stream_in)) return -6;
     if (cudaStreamQuery((cudaStream_t)stream) == cudaSuccess) return 0;         // nothing to wait for: one call instead of three
     cudaGetLastError();
     if (cudaEventRecord(g.ev_caller, (cudaStream_t)stream) != cudaSuccess || cudaStreamWaitEvent(g.stream, g.ev_caller, 0) != cudaSuccess ||

@@ -49,3 +49,25 @@ def test_stream_under_capture_is_refused(bridge):
     g.replay()
     torch.cuda.synchronize()
     assert float(t.sum()) == 8.0
+
+
+def test_bridge_stream_under_capture_is_left_alone(bridge):
+    """The bridge's own stream is being captured and the caller's stream is busy: no edge from uncaptured work may enter the capture."""
+    own = torch.cuda.ExternalStream(bridge.lib.b200_bridge_stream())
+    side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    t = torch.zeros(8, device="cuda")
+    with torch.cuda.stream(own):
+        t.add_(0)                                   # the kernel is loaded before the capture
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=own):
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000_000)          # about a tenth of a second
+        rc = bridge.lib.b200_bridge_wait_stream(side.cuda_stream)
+        t.add_(1)
+    assert rc == -6
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(t.sum()) == 8.0
