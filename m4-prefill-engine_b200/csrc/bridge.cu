@@ -333,7 +333,15 @@ bool m4_bridge_init(const char*) {
     g.slot_seq = 0; g.main_d2h_pending = false;
     if (cudaMalloc(&g.counters, 4096 * sizeof(uint32_t) + 64) != cudaSuccess) { cudaGetLastError(); return false; }
     cudaMemsetAsync(g.counters, 0, 4096 * sizeof(uint32_t) + 64, g.stream);
-    g.err_word = reinterpret_cast<int*>(g.counters + 4096);
+    // (the error word lies in host memory that the GPU sees: reading it costs no copy)
+    void *err_host = nullptr, *err_dev = nullptr;
+    if (cudaHostAlloc(&err_host, 64, cudaHostAllocMapped) != cudaSuccess || cudaHostGetDevicePointer(&err_dev, err_host, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    g.err_host = static_cast<int*>(err_host);
+    *g.err_host = 0;
+    g.err_word = static_cast<int*>(err_dev);
     cudaStreamSynchronize(g.stream);
     // everything that makes the driver load code or reserve memory happens here, not in a later dispatch: the kernels'
     // shared-memory attributes (which load the module image) and the static scratch array of the allocation-free entry point
@@ -553,7 +561,8 @@ void m4_bridge_shutdown(void) {
     free_released_blocks();              // (graphs that are still there keep theirs)
     for (auto& kv : g.registered) cudaFree(kv.second.dev);
     g.registered.clear();
-    cudaFree(g.counters); g.counters = nullptr; g.err_word = nullptr;
+    cudaFree(g.counters); g.counters = nullptr;
+    cudaFreeHost(const_cast<int*>(g.err_host)); g.err_host = nullptr; g.err_word = nullptr;
     cudaStreamDestroy(g.stream); g.stream = nullptr;
     static_scratch_forget();
     g.initialized = false;
@@ -581,18 +590,23 @@ int b200_bridge_wait_stream(void* stream) {
 int b200_bridge_device_error(void) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.initialized) return -1;
-    int v = 0;
     cudaStreamSynchronize(g.stream);
-    cudaMemcpy(&v, g.err_word, sizeof(int), cudaMemcpyDeviceToHost);
-    return v;
+    return *g.err_host;
+}
+
+/* The same without waiting and without the lock: what kernels that have finished reported (0 before init). */
+int b200_bridge_error_flag(void) {
+    volatile int* err = g.err_host;
+    return err ? *err : 0;
 }
 
 int b200_bridge_clear_device_error(void) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.initialized) return -1;
     sync_all_streams(g.stream, g.stream_in, g.stream_out);
-    // A split-K launch that gave up on a bounded wait leaves its tile counters part-way: the counters and the error
-    // word are one block and are cleared together, so the next split-K launch starts from zero again.
+    // A split-K launch that gave up on a bounded wait leaves its tile counters part-way: they are cleared with the error word,
+    // so the next split-K launch starts from zero again.
+    *g.err_host = 0;
     return cudaMemset(g.counters, 0, 4096 * sizeof(uint32_t) + 64) == cudaSuccess ? 0 : -6;
 }
 

@@ -55,7 +55,8 @@ struct State {
     uint32_t rope_M = 0, rope_D = 0, rope_pos0 = 0;
     float rope_theta = 0.0f;
     uint32_t* counters = nullptr;  // 4096 tile counters (kept zero between launches) + error word
-    int* err_word = nullptr;
+    int* err_word = nullptr;             // first error that a kernel reported: device address ...
+    volatile int* err_host = nullptr;    // ... and host address of the word
     std::unordered_map<const void*, Registered> registered;
     std::string last_error;
     uint64_t launches = 0, h2d_bytes = 0, d2h_bytes = 0;
