@@ -477,33 +477,38 @@ __global__ void __launch_bounds__(256) combine_kernel(const Params p) {
     else *reinterpret_cast<uint32_t*>(dst) = pack_h2(acc[0], acc[1]);
 }
 
-// Q8_0 records (34 bytes: fp16 d, 32 codes; 2-byte aligned) of K and then V -> fp16, value = fp16(q * d), one rounding.  A
-// thread takes half a record (16 codes, two 16-byte stores); the integer becomes fp16 through the mantissa: 0x6400 | (q + 128)
-// is 1152 + q.
+// Q8_0 records (34 bytes: fp16 d, 32 codes; 2-byte aligned) of K and then V -> fp16, value = fp16(q * d), one rounding.  Of the
+// `total` records that the cache holds per kv head only the first `used` are expanded: those of the keys that some row sees (one
+// token at position 4096 of a cache laid out for 32768, 8 heads of 128: 18 us instead of 58).  blockIdx.y walks over the heads
+// of K and then of V.  A thread takes half a record (16 codes, two 16-byte stores); the integer becomes fp16 through the
+// mantissa: 0x6400 | (q + 128) is 1152 + q.
 constexpr uint32_t DEQUANT_THREADS = 256;
 __global__ void __launch_bounds__(DEQUANT_THREADS) dequant_q8_0_kernel(const uint8_t* __restrict__ K, const uint8_t* __restrict__ V, __half* __restrict__ out,
-                                                                       size_t blocks) {
+                                                                       uint32_t heads, size_t total, size_t used) {
     ptx::grid_dependency_wait();
     ptx::launch_dependents();
     const size_t i = (size_t)blockIdx.x * DEQUANT_THREADS + threadIdx.x;
     const size_t b = i >> 1;
-    if (b >= 2 * blocks) return;
-    const uint16_t* blk = reinterpret_cast<const uint16_t*>(b < blocks ? K + b * 34 : V + (b - blocks) * 34);
-    const uint16_t* c = blk + 1 + ((uint32_t)i & 1u) * 8u;
-    uint16_t q[8];
+    if (b >= used) return;
+    const __half2 off = __half2half2(__ushort_as_half((unsigned short)0x6480));      // 1152
+    for (uint32_t h = blockIdx.y; h < 2u * heads; h += gridDim.y) {
+        const uint16_t* blk = reinterpret_cast<const uint16_t*>((h < heads ? K + h * total * 34 : V + (h - heads) * total * 34) + b * 34);
+        const uint16_t* c = blk + 1 + ((uint32_t)i & 1u) * 8u;
+        uint16_t q[8];
 #pragma unroll
-    for (int e = 0; e < 8; e++) q[e] = __ldg(c + e);
-    const __half2 d2 = __half2half2(__ushort_as_half(__ldg(blk))), off = __half2half2(__ushort_as_half((unsigned short)0x6480));      // 1152
-    uint32_t o[8];
+        for (int e = 0; e < 8; e++) q[e] = __ldg(c + e);
+        const __half2 d2 = __half2half2(__ushort_as_half(__ldg(blk)));
+        uint32_t o[8];
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const uint32_t x = (__byte_perm((uint32_t)q[e], 0u, 0x4140u) ^ 0x00800080u) | 0x64006400u;
-        const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&x), off), d2);
-        o[e] = *reinterpret_cast<const uint32_t*>(&v);
+        for (int e = 0; e < 8; e++) {
+            const uint32_t x = (__byte_perm((uint32_t)q[e], 0u, 0x4140u) ^ 0x00800080u) | 0x64006400u;
+            const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&x), off), d2);
+            o[e] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(out + (h * used + b) * 32 + ((uint32_t)i & 1u) * 16u);
+        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
-    uint4* dst = reinterpret_cast<uint4*>(out + b * 32 + ((uint32_t)i & 1u) * 16u);
-    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -568,7 +573,7 @@ uint32_t choose_splits(uint32_t heads, uint32_t blocks, uint32_t n_first, uint32
     return best;
 }
 
-struct Plan { uint32_t BP, blocks, n_last, splits; size_t kv_elems, kv_bytes, o_bytes, ml_bytes; };
+struct Plan { uint32_t BP, blocks, n_last, splits, kv_rows; size_t kv_bytes, o_bytes, ml_bytes; };      // kv_rows: keys that some row sees
 Plan make_plan(const Args& a, bool split) {
     Plan pl;
     pl.BP = (uint32_t)ROWS / (a.Hq / a.Hkv);
@@ -579,8 +584,8 @@ Plan make_plan(const Args& a, bool split) {
     };
     pl.n_last = tiles(a.M - 1);
     pl.splits = split ? choose_splits(a.Hkv, pl.blocks, tiles(2ull * pl.BP - 1), pl.n_last) : 1u;
-    pl.kv_elems = (size_t)a.Hkv * a.Mkv * a.D;
-    pl.kv_bytes = a.kv_fp16 ? 0 : (2 * pl.kv_elems * sizeof(__half) + 255) & ~(size_t)255;
+    pl.kv_rows = a.pos0 + a.M < a.Mkv ? a.pos0 + a.M : a.Mkv;
+    pl.kv_bytes = a.kv_fp16 ? 0 : (2 * (size_t)a.Hkv * pl.kv_rows * a.D * sizeof(__half) + 255) & ~(size_t)255;
     const size_t rows = pl.splits > 1 ? pl.splits * (size_t)a.Hq * a.M : 0;
     pl.o_bytes = rows * a.D * sizeof(float); pl.ml_bytes = rows * sizeof(float2);
     return pl;
@@ -598,7 +603,7 @@ template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc
     if (pl.kv_bytes + pl.o_bytes + pl.ml_bytes > sc.bytes) pl = make_plan(a, false);
     if (pl.kv_bytes > sc.bytes) return cudaErrorMemoryAllocation;
     const uint32_t splits = pl.splits, blocks = pl.blocks;
-    const size_t kv_elems = pl.kv_elems, kv_bytes = pl.kv_bytes, o_bytes = pl.o_bytes, rows = (size_t)a.Hq * a.M;
+    const size_t kv_bytes = pl.kv_bytes, o_bytes = pl.o_bytes, rows = (size_t)a.Hq * a.M;
     Params p;
     p.G = a.Hq / a.Hkv; p.BP = pl.BP;
     p.Hq = a.Hq; p.M = a.M; p.Mkv = a.Mkv; p.pos0 = a.pos0; p.scale_log2e = a.scale_log2e;
@@ -618,15 +623,17 @@ template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc
     *launches = 0;
     const void *Kf = a.K, *Vf = a.V;
     if (!a.kv_fp16) {
-        const size_t nb = kv_elems / 32;
-        cfg.gridDim = dim3((unsigned)((4 * nb + DEQUANT_THREADS - 1) / DEQUANT_THREADS)); cfg.blockDim = dim3(DEQUANT_THREADS);
-        cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_q8_0_kernel, (const uint8_t*)a.K, (const uint8_t*)a.V, (__half*)scratch, nb);
+        const size_t total = (size_t)a.Mkv * (D / 32), used = (size_t)pl.kv_rows * (D / 32);
+        cfg.gridDim = dim3((unsigned)((2 * used + DEQUANT_THREADS - 1) / DEQUANT_THREADS), 2 * a.Hkv < 65535u ? 2 * a.Hkv : 65535u);
+        cfg.blockDim = dim3(DEQUANT_THREADS);
+        cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_q8_0_kernel, (const uint8_t*)a.K, (const uint8_t*)a.V, (__half*)scratch, a.Hkv, total, used);
         if (e != cudaSuccess) return e;
-        Kf = scratch; Vf = scratch + kv_elems * sizeof(__half);
+        Kf = scratch; Vf = scratch + (size_t)a.Hkv * pl.kv_rows * D * sizeof(__half);
         ++*launches;
     }
     CUtensorMap tmQ, tmK, tmV;
-    if (!make_map(&tmK, Kf, D, a.Hkv, a.Mkv, BK, 1) || !make_map(&tmV, Vf, D, a.Hkv, a.Mkv, BK, 1) || !make_map(&tmQ, a.Q, D, a.Hq, a.M, p.BP, p.G))
+    const uint32_t map_rows = a.kv_fp16 ? a.Mkv : pl.kv_rows;
+    if (!make_map(&tmK, Kf, D, a.Hkv, map_rows, BK, 1) || !make_map(&tmV, Vf, D, a.Hkv, map_rows, BK, 1) || !make_map(&tmQ, a.Q, D, a.Hq, a.M, p.BP, p.G))
         return cudaErrorInvalidValue;
     cfg.gridDim = dim3(a.Hkv, blocks, splits); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = C::SMEM;
     cudaError_t e = cudaLaunchKernelEx(&cfg, attn_ws_kernel<D, LAG>, tmQ, tmK, tmV, p);

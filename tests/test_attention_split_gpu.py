@@ -1,6 +1,6 @@
 """The tensor-memory attention kernel at the edges of its query tiles (128 / G positions, two tiles per block), of its key
 steps (128) and of the split key range, for both head sizes, against the CPU oracle."""
-from ctypes import c_float
+from ctypes import c_float, c_size_t
 
 import numpy as np
 import pytest
@@ -29,6 +29,7 @@ CASES = [
     (6, 2, 64, 85, 43, 0, False, True),             # three heads per kv head: 42 positions and two unused rows per tile
     (10, 2, 128, 51, 0, 0, False, True), (16, 1, 64, 17, 111, 0, False, True), (128, 1, 64, 3, 254, 0, True, True),
     (8, 2, 128, 1, 1535, 0, False, True), (8, 2, 64, 1, 4096, 0, True, False), (24, 8, 128, 2, 2047, 0, False, False),   # split key range
+    (8, 2, 64, 3, 700, 5000, False, True), (6, 3, 128, 200, 0, 777, False, False),                                      # a long tail that no row sees
     (4, 2, 64, 130, 1500, 0, False, True), (8, 8, 128, 300, 900, 100, True, True), (8, 2, 128, 70, 3000, 5, False, True),
 ]
 
@@ -57,3 +58,29 @@ def test_attention_edges(bridge, case):
     got = O.cpu().numpy().astype(np.float64).reshape(gold.shape)
     assert np.all(np.isfinite(got))
     assert np.abs(got - gold).max() <= TOL
+
+
+def test_unseen_cache_is_not_expanded(bridge):
+    """A cache laid out for 60000 tokens, 4008 of them in use: the call needs scratch for those only."""
+    L, Hq, Hkv, D, M, pos0, Mkv = bridge.lib, 8, 2, 128, 8, 4000, 60000
+    rng = np.random.default_rng(5)
+    Q = rng.standard_normal((Hq, M, D), dtype=np.float32).astype(np.float16)
+    K, V = (rng.standard_normal((Hkv, pos0 + M, D), dtype=np.float32).astype(np.float16) for _ in range(2))
+    used = [o.quantize_q8_0(t).reshape(Hkv, -1) for t in (K, V)]
+    cache = [torch.full((Hkv, Mkv * D // 32 * 34), 0xFF, dtype=torch.uint8, device="cuda") for _ in used]       # NaN scales behind what is in use
+    for c, u in zip(cache, used):
+        c[:, :u.shape[1]] = torch.from_numpy(u).cuda()
+    gold = o.attention(Q, *(o.dequantize_q8_0(u.reshape(-1), K.shape) for u in used), D ** -0.5, pos0, False).astype(np.float64)
+    Qd, O = torch.from_numpy(Q).cuda(), torch.empty(Hq, M, D, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    L.b200_bridge_debug_limit_scratch.argtypes = [c_size_t]
+    L.b200_bridge_debug_limit_scratch(32 << 20)              # the whole cache would take 61 MB
+    try:
+        assert L.b200_bridge_dispatch_attention_q8kv(Qd.data_ptr(), cache[0].data_ptr(), cache[1].data_ptr(), O.data_ptr(), Hq, Hkv, M, Mkv, D,
+                                                     c_float(D ** -0.5), pos0, 0, 0) == 0
+        launches = L.b200_bridge_attention_launches()
+    finally:
+        L.b200_bridge_debug_limit_scratch(0)
+    bridge.synchronize()
+    assert launches == 3                                     # expansion, split attention, combination: not the kernels without scratch
+    assert np.abs(O.cpu().numpy().astype(np.float64) - gold).max() <= TOL
