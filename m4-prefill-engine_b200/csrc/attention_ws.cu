@@ -30,6 +30,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 
@@ -593,11 +594,14 @@ Plan make_plan(const Args& a, bool split) {
 
 template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc, cudaStream_t stream, int* launches) {
     using C = Cfg<D>;
-    static bool attr_set = false;
-    if (!attr_set) {
+    static std::atomic<uint64_t> attr_done{0};               // bit d: set on device d
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (!(attr_done.load() & bit)) {
         cudaError_t e = cudaFuncSetAttribute(attn_ws_kernel<D, LAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
         if (e != cudaSuccess) return e;
-        attr_set = true;
+        attr_done |= bit;
     }
     Plan pl = make_plan(a, true);
     if (pl.kv_bytes + pl.o_bytes + pl.ml_bytes > sc.bytes) pl = make_plan(a, false);
