@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 #include <mutex>
 
 #include "../../include/b200_bridge.h"
@@ -88,6 +89,8 @@ __global__ void __launch_bounds__(THREADS) attn_q8kv_kernel(const Params p) {
     const uint32_t q0 = qt * BQ;
     const uint32_t last_pos = min(p.pos0 + min(q0 + BQ, p.M) - 1, p.Mkv - 1);   // last key any row of the tile may see
     const uint32_t n_ktiles = last_pos / BK + 1;
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
 
     // ---- stage the Q tile (rows past M are zero) ----
     for (int i = tid; i < BQ * (D / 8); i += THREADS) {
@@ -310,6 +313,8 @@ __global__ void __launch_bounds__(GQ_THREADS) attn_gqa_kernel(const Params p) {
     const uint32_t p0 = pb * BP;
     const uint32_t last_pos = min(p.pos0 + min(p0 + BP, p.M) - 1, p.Mkv - 1);
     const uint32_t n_ktiles = last_pos / BK + 1;
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
 
     // ---- stage Q: row r = head (r / BP), position p0 + r % BP ----
     for (int i = tid; i < GQ_ROWS * (D / 8); i += GQ_THREADS) {
@@ -518,12 +523,24 @@ template <int D> size_t gqa_smem_bytes() {
     return (size_t)(GQ_ROWS + 4 * BK) * LD * 2 + 4 * (size_t)RAW_TILE_PAD;
 }
 
+// The warp-level kernels may be placed while the kernel in front of them drains.
+cudaError_t launch_pdl(void (*kernel)(Params), dim3 grid, unsigned threads, size_t smem, const Params& p, cudaStream_t stream) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 template <int D, int G> cudaError_t launch_gqa(const Params& p, cudaStream_t stream) {
     constexpr int BP = GQ_ROWS / G;
     dim3 grid((p.M + BP - 1) / BP, p.Hkv);
-    cudaFuncSetAttribute(attn_gqa_kernel<D, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gqa_smem_bytes<D>());
-    attn_gqa_kernel<D, G><<<grid, GQ_THREADS, gqa_smem_bytes<D>(), stream>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(attn_gqa_kernel<D, G>, grid, GQ_THREADS, gqa_smem_bytes<D>(), p, stream);
 }
 
 // Q8_0 compression, one thread per 32-value block.  Bit-exact with the reference: the scale is
@@ -1042,21 +1059,29 @@ static ws::Args ws_args(const Params& p, uint32_t D) {
     return a;
 }
 
-cudaError_t launch_attention(const Params& p, uint32_t D, const ws::Scratch& scratch, cudaStream_t stream) {
+// What the tensor-memory kernel of attention_ws.cu takes (K and V as fp16 through TMA, a Q8_0 cache expanded once per call): not
+// O off a 16-byte boundary, nor more than 128 query heads per kv head; and not what one step of the warp-level kernels covers, 64
+// keys, for the shapes that had always run on them: those take one launch and no set-up of tensor memory (heads of 64, Q8_0, 1 / 16 /
+// 64 tokens with nothing cached: 5.2 / 4.8 / 5.3 us at 32/8 heads against 6.4 / 6.5 / 7.3; fp16 4.0 / 4.3 / 4.8 against 4.9 / 5.0 /
+// 5.8; from 65 keys on they take a second step and lose).
+static bool use_ws(const Params& p, const ws::Args& a) {
+    if (g_force_legacy != 0 || !ws::usable(a)) return false;
+    const uint32_t G = p.Hq / p.Hkv;
+    if (a.D == 128 && (G == 1 || G == 2 || G == 4 || G == 8)) return true;
+    return (p.Mkv < (uint64_t)p.pos0 + p.M ? p.Mkv : (uint64_t)p.pos0 + p.M) > (uint64_t)BK;
+}
+
+// `wa` and `plan`: of this call, where use_ws says so (plan then not null)
+cudaError_t launch_attention(const Params& p, uint32_t D, const ws::Args& wa, const ws::Plan* plan, const ws::Scratch& scratch, cudaStream_t stream) {
     // grouped-head kernel when the group size divides its 128-row tile into whole warps
     const uint32_t G = p.Hq / p.Hkv;
     g_last_launches = 1;
-    // Default: the tensor-memory kernel of attention_ws.cu (K and V as fp16 through TMA, a Q8_0 cache expanded once per call).
-    // What it cannot take -- O not 16-byte aligned, more than 128 query heads per kv head -- stays on the kernels below.
     const bool tc_ok = D == 128 && ((uintptr_t)p.Q & 15u) == 0 && ((uintptr_t)p.O & 15u) == 0;
-    if (g_force_legacy == 0) {
-        const ws::Args a = ws_args(p, D);
-        if (ws::usable(a)) {
-            const cudaError_t e = ws::launch(a, scratch, stream, &g_last_launches);
-            if (e != cudaErrorMemoryAllocation) return e;
-            cudaGetLastError();              // no scratch for the expanded cache: the kernels below unpack it themselves
-            g_last_launches = 1;
-        }
+    if (plan) {
+        const cudaError_t e = ws::launch(wa, *plan, scratch, stream, &g_last_launches);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();              // no scratch for the expanded cache: the kernels below unpack it themselves
+        g_last_launches = 1;
     }
     // the kernel that unpacks the Q8_0 tiles itself (hooks 2 and 3)
     if (tc_ok && !p.kv_fp16 && g_force_legacy != 1) {
@@ -1079,16 +1104,9 @@ cudaError_t launch_attention(const Params& p, uint32_t D, const ws::Scratch& scr
         if (G == 8) return launch_gqa<64, 8>(p, stream);
     }
     dim3 grid((p.M + BQ - 1) / BQ, p.Hq);
-    if (D == 128) {
-        cudaFuncSetAttribute(attn_q8kv_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<128>());
-        attn_q8kv_kernel<128><<<grid, THREADS, smem_bytes<128>(), stream>>>(p);
-    } else if (D == 64) {
-        cudaFuncSetAttribute(attn_q8kv_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<64>());
-        attn_q8kv_kernel<64><<<grid, THREADS, smem_bytes<64>(), stream>>>(p);
-    } else {
-        return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    if (D == 128) return launch_pdl(attn_q8kv_kernel<128>, grid, THREADS, smem_bytes<128>(), p, stream);
+    if (D == 64) return launch_pdl(attn_q8kv_kernel<64>, grid, THREADS, smem_bytes<64>(), p, stream);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_quantize(const void* src, void* dst, size_t n_elements, cudaStream_t stream) {
@@ -1119,14 +1137,20 @@ static Params simple_params(const void* Q, const void* K, const void* V, void* O
 
 size_t attention_scratch_bytes(uint32_t Hq, uint32_t Hkv, uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int kv_fp16, bool split) {
     void* at16 = (void*)16;                                  // alignment probe only
-    const ws::Args a = ws_args(simple_params(at16, at16, at16, at16, Hq, Hkv, M, Mkv, scale, pos0, 1, kv_fp16), D);
-    return ws::usable(a) ? ws::scratch_bytes(a, split) : 0;
+    const Params p = simple_params(at16, at16, at16, at16, Hq, Hkv, M, Mkv, scale, pos0, 1, kv_fp16);
+    const ws::Args a = ws_args(p, D);
+    return use_ws(p, a) ? ws::make_plan(a, split).scratch_bytes() : 0;
 }
 
 cudaError_t launch_attention_simple(const void* Q, const void* K, const void* V, void* O, uint32_t Hq, uint32_t Hkv,
                                     uint32_t M, uint32_t Mkv, uint32_t D, float scale, uint32_t pos0, int out_tokens_major,
                                     int kv_fp16, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
-    return launch_attention(simple_params(Q, K, V, O, Hq, Hkv, M, Mkv, scale, pos0, out_tokens_major, kv_fp16), D, ws::Scratch{scratch, scratch_bytes}, stream);
+    const Params p = simple_params(Q, K, V, O, Hq, Hkv, M, Mkv, scale, pos0, out_tokens_major, kv_fp16);
+    const ws::Args a = ws_args(p, D);
+    ws::Plan plan;
+    const bool on_ws = use_ws(p, a);
+    if (on_ws) plan = ws::make_plan(a, true);
+    return launch_attention(p, D, a, on_ws ? &plan : nullptr, ws::Scratch{scratch, scratch_bytes}, stream);
 }
 
 }  // namespace attn
@@ -1208,10 +1232,17 @@ int b200_bridge_dispatch_attention_q8kv(void* Q, void* K, void* V, void* O, uint
     p.scale_log2e = scale * 1.4426950408889634f;
     p.out_tokens_major = out_tokens_major; p.kv_fp16 = kv_fp16;
     const attn::ws::Args wa = attn::ws_args(p, D);
+    attn::ws::Plan plan;
+    const bool on_ws = attn::use_ws(p, wa);
     Block scratch;                          // (without the memory: an unsplit launch, or the kernels that need none)
-    if (attn::ws::usable(wa) && !launch_block(g.attn_scratch, attn::ws::scratch_bytes(wa, true), &scratch))
-        launch_block(g.attn_scratch, attn::ws::scratch_bytes(wa, false), &scratch);
-    if (attn::launch_attention(p, D, attn::ws::Scratch{scratch.p, scratch.bytes}, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
+    if (on_ws) {
+        plan = attn::ws::make_plan(wa, true);
+        if (!launch_block(g.attn_scratch, plan.scratch_bytes(), &scratch)) {
+            plan = attn::ws::make_plan(wa, false);
+            launch_block(g.attn_scratch, plan.scratch_bytes(), &scratch);
+        }
+    }
+    if (attn::launch_attention(p, D, wa, on_ws ? &plan : nullptr, attn::ws::Scratch{scratch.p, scratch.bytes}, g.stream) != cudaSuccess) { set_error("attention launch failed"); return -6; }
     g.launches += (uint64_t)attn::g_last_launches;
     if (host_dst && copy_back(host_dst, p.O, q_bytes) != 0) return -5;
     return 0;

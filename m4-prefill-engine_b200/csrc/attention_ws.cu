@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -64,6 +65,7 @@ struct Params {
     uint32_t Hq, M, Mkv, pos0, G, BP, tiles_per_split;
     float scale_log2e;
     int out_tokens_major, split;
+    uint32_t tiles;              // query tiles of a CTA (1 or 2)
     int* err;
 };
 
@@ -181,10 +183,11 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // kv heads along x, position blocks along y, latest (longest) block first; splits of the key range along z
     const uint32_t hk = blockIdx.x;
-    const uint32_t p0 = (gridDim.y - 1u - blockIdx.y) * 2u * p.BP;
+    const uint32_t p0 = (gridDim.y - 1u - blockIdx.y) * p.tiles * p.BP;
     const uint32_t t0 = blockIdx.z * p.tiles_per_split;
     // steps of tile g inside this split
     auto steps_of = [&](uint32_t g) {
+        if (g >= p.tiles) return 0u;
         const uint32_t n = key_tiles(p0 + g * p.BP, p.BP, p.M, p.Mkv, p.pos0);
         return n > t0 ? min(n - t0, p.tiles_per_split) : 0u;
     };
@@ -546,45 +549,50 @@ uint32_t sm_count() {
     return (uint32_t)n;
 }
 
-// Splits of the key range.  A step (128 keys against 256 query rows) is the unit; a CTA costs about FIXED steps on top of its
-// own, the pass over the partial results about COMBINE.  One CTA runs per SM, so items beyond a whole number of waves cost a
-// wave where all items are equally long (a chunk behind a long cache); a causal triangle from position 0 packs better than
-// that, its sum is what counts there.
-uint32_t choose_splits(uint32_t heads, uint32_t blocks, uint32_t n_first, uint32_t n_last) {
-    constexpr float FIXED = 3.0f, COMBINE = 5.0f;
-    const float sms = (float)sm_count();
-    uint32_t best = 1;
-    float best_cost = 0.0f;
-    for (uint32_t s = 1; s <= (uint32_t)MAX_SPLITS && s <= n_last; s++) {
-        const uint32_t len = (n_last + s - 1) / s;
-        if ((n_last + len - 1) / len != s) continue;                   // the last split would be empty
-        float cost;
-        if (2u * n_first >= n_last) {
-            const uint32_t items = heads * blocks * s;
-            cost = (float)((items + sm_count() - 1) / sm_count()) * ((float)len + FIXED);
-        } else {
-            const float steps = (float)heads * blocks * 0.5f * (float)(n_first + n_last);
-            const float items = (float)heads * blocks * (0.5f * (float)(s + 1));
-            const float even = (steps + items * FIXED) / sms + 0.5f * (float)len;
-            cost = even > (float)len + FIXED ? even : (float)len + FIXED;
-        }
-        if (s > 1) cost += COMBINE;
-        if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
-    }
-    return best;
-}
+// Query tiles of a CTA and splits of the key range, by estimated time.  The unit is a step (128 keys) of a CTA with two tiles, 1.7 to
+// 2.1 us.  One tile is hardly cheaper a step and much cheaper a CTA (FIXED), so one is taken while that leaves no more CTAs waiting for
+// an SM (4 heads of 128, fp16: 200 tokens 8.6 -> 7.1 us, behind 500 others 15.9 -> 13.4; 700 alone 15.3 -> 13.1).  Partial results
+// cost a launch (COMBINE) and their way through memory (PER_BYTE).  One CTA runs per SM, so items beyond a whole number of waves
+// cost a wave where all items are equally long (a chunk behind a long cache); a causal triangle from position 0 packs better than
+// that, its sum is what counts there.  The constants: least regret over 320 shapes of both head sizes (1 to 1400 tokens behind 0 to
+// 3000, 1 to 32 kv heads), each timed with every choice: 0.6 % on average, 14 % at most.
+}  // namespace
 
-struct Plan { uint32_t BP, blocks, n_last, splits, kv_rows; size_t kv_bytes, o_bytes, ml_bytes; };      // kv_rows: keys that some row sees
 Plan make_plan(const Args& a, bool split) {
+    constexpr float STEP[2] = {0.975f, 1.0f}, FIXED[2] = {2.0f, 4.1f}, COMBINE = 2.7f, PER_BYTE = 0.091e-6f;
+    const float sms = (float)sm_count();
     Plan pl;
     pl.BP = (uint32_t)ROWS / (a.Hq / a.Hkv);
-    pl.blocks = (a.M + 2 * pl.BP - 1) / (2 * pl.BP);
-    auto tiles = [&](uint64_t pos) {      // key tiles of a block whose last position is `pos`
+    auto key_tiles_at = [&](uint64_t pos) {      // key tiles of a block whose last position is `pos`
         const uint64_t last = (uint64_t)a.pos0 + (pos < a.M ? pos : a.M - 1);
         return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / BK + 1);
     };
-    pl.n_last = tiles(a.M - 1);
-    pl.splits = split ? choose_splits(a.Hkv, pl.blocks, tiles(2ull * pl.BP - 1), pl.n_last) : 1u;
+    pl.n_last = key_tiles_at(a.M - 1);
+    float best = 0.0f;
+    pl.tiles = 0;
+    for (uint32_t t = 2; t >= 1; t--) {
+        const uint32_t blocks = (a.M + t * pl.BP - 1) / (t * pl.BP);
+        if (t == 1u && blocks > 65535u) continue;
+        const uint32_t n_first = key_tiles_at((uint64_t)t * pl.BP - 1);
+        const bool even_lengths = 2u * n_first >= pl.n_last;
+        for (uint32_t s = 1; s <= (split ? (uint32_t)MAX_SPLITS : 1u) && s <= pl.n_last; s++) {
+            if (s > 2u && (float)a.Hkv * blocks * (s - 1) >= 2.0f * sms) break;        // the SMs are full without any more of them
+            const uint32_t len = (pl.n_last + s - 1) / s;
+            if ((pl.n_last + len - 1) / len != s) continue;                // the last split would be empty
+            const float one = (float)len * STEP[t - 1] + FIXED[t - 1];
+            float cost;
+            if (even_lengths) {
+                cost = ceilf((float)a.Hkv * blocks * s / sms) * one;
+            } else {
+                const float steps = (float)a.Hkv * blocks * 0.5f * (float)(n_first + pl.n_last);
+                const float items = (float)a.Hkv * blocks * 0.5f * (float)((n_first + len - 1) / len + s);
+                const float even = (steps * STEP[t - 1] + items * FIXED[t - 1]) / sms + 0.5f * (float)len * STEP[t - 1];
+                cost = even > one ? even : one;
+            }
+            if (s > 1) cost += COMBINE + PER_BYTE * ((float)s * a.Hq * a.M * a.D * sizeof(float));
+            if (pl.tiles == 0 || cost < best) { best = cost; pl.tiles = t; pl.blocks = blocks; pl.splits = s; }
+        }
+    }
     pl.kv_rows = a.pos0 + a.M < a.Mkv ? a.pos0 + a.M : a.Mkv;
     pl.kv_bytes = a.kv_fp16 ? 0 : (2 * (size_t)a.Hkv * pl.kv_rows * a.D * sizeof(__half) + 255) & ~(size_t)255;
     const size_t rows = pl.splits > 1 ? pl.splits * (size_t)a.Hq * a.M : 0;
@@ -592,7 +600,9 @@ Plan make_plan(const Args& a, bool split) {
     return pl;
 }
 
-template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc, cudaStream_t stream, int* launches) {
+namespace {
+
+template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Plan& planned, const Scratch& sc, cudaStream_t stream, int* launches) {
     using C = Cfg<D>;
     static std::atomic<uint64_t> attr_done{0};               // bit d: set on device d
     int dev = 0;
@@ -603,8 +613,7 @@ template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc
         if (e != cudaSuccess) return e;
         attr_done |= bit;
     }
-    Plan pl = make_plan(a, true);
-    if (pl.kv_bytes + pl.o_bytes + pl.ml_bytes > sc.bytes) pl = make_plan(a, false);
+    const Plan pl = planned.scratch_bytes() <= sc.bytes ? planned : make_plan(a, false);
     if (pl.kv_bytes > sc.bytes) return cudaErrorMemoryAllocation;
     const uint32_t splits = pl.splits, blocks = pl.blocks;
     const size_t kv_bytes = pl.kv_bytes, o_bytes = pl.o_bytes, rows = (size_t)a.Hq * a.M;
@@ -614,7 +623,7 @@ template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Scratch& sc
     p.out_tokens_major = a.out_tokens_major; p.O = (__half*)a.O; p.err = bridge::g.err_word;
     p.tiles_per_split = (pl.n_last + splits - 1) / splits;
     uint8_t* scratch = static_cast<uint8_t*>(sc.p);
-    p.split = splits > 1;
+    p.split = splits > 1; p.tiles = pl.tiles;
     p.part_o = reinterpret_cast<float*>(scratch + kv_bytes);
     p.part_ml = reinterpret_cast<float2*>(scratch + kv_bytes + o_bytes);
 
@@ -664,12 +673,7 @@ bool usable(const Args& a) {
     return encode_fn() != nullptr;
 }
 
-size_t scratch_bytes(const Args& a, bool split) {
-    const Plan pl = make_plan(a, split);
-    return pl.kv_bytes + pl.o_bytes + pl.ml_bytes;
-}
-
-cudaError_t launch(const Args& a, const Scratch& sc, cudaStream_t stream, int* launches) {
+cudaError_t launch(const Args& a, const Plan& plan, const Scratch& sc, cudaStream_t stream, int* launches) {
     // A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
     // arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O: 43.8 against 47.4 us at the 8B
     // prefill, 42.0 against 43.6 for the heads of 64.  128-wide heads in groups of 1, 2, 4 and 8 have always run with it, and with
@@ -677,8 +681,8 @@ cudaError_t launch(const Args& a, const Scratch& sc, cudaStream_t stream, int* l
     // their polynomial adds to fp32 rounding (3.8271e-4 with it, without it and with the short one; the 3.8204e-4 of the warp-level
     // kernels come from their steps of 64 keys: every new maximum of a row is a probability of exactly 1, and they see more of them).
     const uint32_t G = a.Hq / a.Hkv;
-    if (a.D == 128) return G == 1u || G == 2u || G == 4u || G == 8u ? launch_d<128, true>(a, sc, stream, launches) : launch_d<128, false>(a, sc, stream, launches);
-    return launch_d<64, false>(a, sc, stream, launches);
+    if (a.D == 128) return G == 1u || G == 2u || G == 4u || G == 8u ? launch_d<128, true>(a, plan, sc, stream, launches) : launch_d<128, false>(a, plan, sc, stream, launches);
+    return launch_d<64, false>(a, plan, sc, stream, launches);
 }
 
 }  // namespace ws
