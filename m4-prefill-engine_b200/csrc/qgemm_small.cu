@@ -56,22 +56,27 @@ __device__ unsigned long long g_qs_trace[8][64];
 #define QST(role, slot) do { } while (0)
 #endif
 
+// (in the order in which a launch needs them, 64 bytes to a line of the constant cache, which is cold when a CTA starts)
 struct Params {
-    uint32_t M, N, K, T;
-    uint32_t x_wrap;             // K after which the activation columns start over
-    uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;       // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
-    uint32_t raw_stages, b_stages;
+    uint32_t n_w_tiles, k_splits, split_shift, chunks;       // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits); k_splits = 1 << split_shift
+    uint32_t raw_stages, b_stages, T;
     uint32_t early;              // packed weights may be fetched before the preceding kernel has finished
-    uint32_t swiglu;             // tiles of 64 gate rows (matrix 0) and their 64 up rows (matrix 1); output silu(g) * u
-    // grouped launch: weight tiles [0, tiles[0]) belong to matrix 0, the next tiles[1] to matrix 1, ...
-    uint32_t groups, tiles[3], grp_N[3];
-    __half* grp_Y[3];
-    const __half* residual;
-    uint32_t layout, D;
+    uint32_t x_wrap;             // K after which the activation columns start over
+    uint32_t M, N, K, layout, D;
     int* err;
+    __half* Y;
+    const __half* residual;
     float* scratch;              // [k_splits][tiles][T][128] partial tiles (k_splits > 1, or SwiGLU)
-    const uint8_t *meta0, *meta1;
-    const __half *row_scale0, *row_scale1;
+    const uint8_t* meta0;
+    const __half* row_scale0;
+    uint32_t n_tok_tiles;
+    // SwiGLU and grouped launches
+    uint32_t swiglu;             // tiles of 64 gate rows (matrix 0) and their 64 up rows (matrix 1); output silu(g) * u
+    uint32_t groups, tiles[2];   // grouped launch: weight tiles [0, tiles[0]) belong to matrix 0, the next tiles[1] to matrix 1, ...
+    uint32_t extra_N[2];         // features and results of the matrices behind the first
+    __half* extra_Y[2];
+    const uint8_t* meta1;
+    const __half* row_scale1;
 };
 __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
@@ -123,10 +128,14 @@ template <int S> struct IntC { static constexpr int value = S; };
 template <class F, int... S>
 __device__ __forceinline__ void for_each_sub(F& f, std::integer_sequence<int, S...>) { (f(IntC<S>{}), ...); }
 
-template <int FMT>
+// Maps of the activations and of the packed matrices: one, or (MULTI: SwiGLU and grouped launches) up to three.  A plain launch has
+// neither their maps among its parameters nor their branches.
+template <bool MULTI> struct Maps { CUtensorMap x, w[MULTI ? 3 : 1]; };
+
+template <int FMT, bool MULTI>
 __global__ void __launch_bounds__(THREADS, 2)
-qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW0,
-                   const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2, const Params p) {
+qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
+    const bool swiglu = MULTI && p.swiglu;
     using Cd = cdc::Codec<FMT>;
     constexpr int ROW_BYTES = Cd::ROW_BYTES;
     constexpr int RAW_TILE_BYTES = ROW_BYTES * W_TILE;
@@ -153,21 +162,23 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t ks = blockIdx.x % p.k_splits;                    // == rank inside the cluster
-    const uint32_t tile = blockIdx.x / p.k_splits;
+    const uint32_t ks = blockIdx.x & (p.k_splits - 1u);             // == rank inside the cluster
+    const uint32_t tile = blockIdx.x >> p.split_shift;
     const uint32_t wt = tile % p.n_w_tiles, tt = tile / p.n_w_tiles;
     // grouped launch: this tile's matrix, and the tile's place in it
     uint32_t gi = 0u, wl = wt;
-    if (p.groups > 1u && wl >= p.tiles[0]) { wl -= p.tiles[0]; gi = 1u; if (wl >= p.tiles[1]) { wl -= p.tiles[1]; gi = 2u; } }
-    const uint32_t N = p.grp_N[gi];
-    __half* const Y = p.grp_Y[gi];
-    const uint32_t kc0 = ks * p.chunks / p.k_splits, kcn = (ks + 1u) * p.chunks / p.k_splits - kc0;     // this split's packed chunks
+    if (MULTI && p.groups > 1u && wl >= p.tiles[0]) { wl -= p.tiles[0]; gi = 1u; if (wl >= p.tiles[1]) { wl -= p.tiles[1]; gi = 2u; } }
+    const uint32_t N = !MULTI || gi == 0u ? p.N : (gi == 1u ? p.extra_N[0] : p.extra_N[1]);
+    __half* const Y = !MULTI || gi == 0u ? p.Y : (gi == 1u ? p.extra_Y[0] : p.extra_Y[1]);
+    const uint32_t kc0 = (ks * p.chunks) >> p.split_shift, kcn = (((ks + 1u) * p.chunks) >> p.split_shift) - kc0;     // this split's packed chunks
     const uint32_t ksteps = kcn * (uint32_t)SUBS;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < MAX_RAW_STAGES; i++) { ptx::mbar_init(&raw_full[i], 1); ptx::mbar_init(&raw_empty[i], UNPACK_WARPS); }
+#pragma unroll
+        for (uint32_t i = 0; i < (uint32_t)MAX_RAW_STAGES; i++) if (i < p.raw_stages) { ptx::mbar_init(&raw_full[i], 1); ptx::mbar_init(&raw_empty[i], UNPACK_WARPS); }
         for (int i = 0; i < A_STAGES; i++) { ptx::mbar_init(&a_full[i], 4); ptx::mbar_init(&a_empty[i], 1); }
-        for (int i = 0; i < MAX_B_STAGES; i++) { ptx::mbar_init(&b_full[i], 1); ptx::mbar_init(&b_empty[i], 1); }
+#pragma unroll
+        for (uint32_t i = 0; i < (uint32_t)MAX_B_STAGES; i++) if (i < p.b_stages) { ptx::mbar_init(&b_full[i], 1); ptx::mbar_init(&b_empty[i], 1); }
         ptx::mbar_init(acc_full, 1);
         *abort_flag = 0u;
         ptx::fence_barrier_init();
@@ -189,8 +200,8 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         // ---------------- copies: packed weight chunks run ahead of the activation tiles ----------------
         // (the packed bytes are what the launch waits for: every chunk that has a free stage is requested before the
         // activation tiles of the chunk in front of it)
-        const CUtensorMap* tmW = gi == 0u ? &tmW0 : (gi == 1u ? &tmW1 : &tmW2);
-        if (lane == 0) { ptx::prefetch_tensormap(tmW); ptx::prefetch_tensormap(&tmX); }
+        const CUtensorMap* tmW = &maps.w[MULTI ? gi : 0u];
+        if (lane == 0) { ptx::prefetch_tensormap(tmW); ptx::prefetch_tensormap(&maps.x); }
         uint32_t rs = 0, rph = 0, bs = 0, bph = 0, raw_next = 0;
         bool ok = true;
         auto issue_raw = [&](bool block) {       // request chunk raw_next if its stage is free (block: wait for it)
@@ -205,9 +216,9 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 QST(1, raw_next);
                 ptx::mbar_arrive_expect_tx(&raw_full[rs], RAW_TILE_BYTES);
                 const int x = (int)((kc0 + raw_next) * (ROW_BYTES / Cd::TMA_ELEM_BYTES));
-                if (p.swiglu) {          // 64-row boxes: gate rows, then the same rows of up
-                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &tmW0, &raw_full[rs], x, (int)(wt * GATE_ROWS));
-                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES + GATE_ROWS * ROW_BYTES, &tmW1, &raw_full[rs], x, (int)(wt * GATE_ROWS));
+                if (swiglu) {          // 64-row boxes: gate rows, then the same rows of up
+                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &maps.w[0], &raw_full[rs], x, (int)(wt * GATE_ROWS));
+                    ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES + GATE_ROWS * ROW_BYTES, &maps.w[MULTI ? 1 : 0], &raw_full[rs], x, (int)(wt * GATE_ROWS));
                 } else {
                     ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, tmW, &raw_full[rs], x, (int)(wl * W_TILE));
                 }
@@ -218,6 +229,7 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         };
         for (uint32_t i = 0; i < p.raw_stages; i++) issue_raw(false);
         if (p.early) ptx::grid_dependency_wait();
+        uint32_t x = (kc0 * (uint32_t)Cd::CHUNK) % p.x_wrap;      // column of the next activation tile (x_wrap: whole chunks)
         for (uint32_t kc = 0; ok && kc < kcn; kc++) {
             if (raw_next <= kc) issue_raw(true);              // the chunk these activation tiles belong to must be on its way
             for (uint32_t s = 0; ok && s < (uint32_t)SUBS; s++) {
@@ -225,10 +237,11 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 if (!ok) break;
                 if (lane == 0) {
                     ptx::mbar_arrive_expect_tx(&b_full[bs], b_stage_bytes);
-                    ptx::tma_load_2d(sB + bs * b_stage_bytes, &tmX, &b_full[bs],
-                                     (int)(((kc0 + kc) * Cd::CHUNK + s * KSTEP) % p.x_wrap), (int)(tt * p.T));
+                    ptx::tma_load_2d(sB + bs * b_stage_bytes, &maps.x, &b_full[bs], (int)x, (int)(tt * p.T));
                 }
                 __syncwarp();
+                x += (uint32_t)KSTEP;
+                if (x == p.x_wrap) x = 0u;
                 if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
                 issue_raw(false);                             // a packed stage may have been released meanwhile
             }
@@ -273,10 +286,10 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             // before the wait for the packed bytes
             uint32_t meta[MW] = {};
             if (Cd::META_WORDS != 0) {
-                const uint32_t n = p.swiglu ? wt * GATE_ROWS + (row & 63u) : wt * W_TILE + row;
+                const uint32_t n = swiglu ? wt * GATE_ROWS + (row & 63u) : wt * W_TILE + row;
                 if (n < p.N) {
                     const uint32_t groups = (p.K / 256u) * MW;
-                    const uint8_t* mp = (p.swiglu && row >= 64u ? p.meta1 : p.meta0) + ((size_t)n * groups + (size_t)(kc0 + kc) * MW) * 2;
+                    const uint8_t* mp = (swiglu && row >= 64u ? p.meta1 : p.meta0) + ((size_t)n * groups + (size_t)(kc0 + kc) * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
                         const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
@@ -336,11 +349,11 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (warp < 4 && !bad) {
         ptx::tc_fence_after_sync();
         const uint32_t f = warp * 32u + lane;                       // feature row of the tile
-        const uint32_t n = p.swiglu ? wt * GATE_ROWS + (f & 63u) : wl * W_TILE + f;
+        const uint32_t n = swiglu ? wt * GATE_ROWS + (f & 63u) : wl * W_TILE + f;
         float rsc = 1.0f;
-        if (Cd::ROW_SCALE) rsc = n < N ? __half2float((p.swiglu && f >= 64u ? p.row_scale1 : p.row_scale0)[n]) : 0.0f;
+        if (Cd::ROW_SCALE) rsc = n < N ? __half2float((swiglu && f >= 64u ? p.row_scale1 : p.row_scale0)[n]) : 0.0f;
         const uint32_t taddr = tmem_base + ((warp * 32u) << 16) + ACC_COL;
-        if (p.k_splits > 1u || p.swiglu) {
+        if (p.k_splits > 1u || swiglu) {
             // [split][tile][token column][feature]: a warp's store covers 32 consecutive features of one column
             float* dst = p.scratch + ((size_t)ks * n_tiles + tile) * tile_floats + f;
             for (uint32_t c0 = 0; c0 < p.T; c0 += 16) {
@@ -375,9 +388,9 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // every partial tile of the cluster is written (release / acquire at cluster scope covers the global stores)
     cluster_sync_all();
     if (threadIdx.x == 0) QST(0, 6);
-    if (!bad && (p.k_splits > 1u || p.swiglu)) {
+    if (!bad && (p.k_splits > 1u || swiglu)) {
         // this CTA's token columns [ks * cols, (ks + 1) * cols): sum over the splits in split order, write fp16
-        const uint32_t cols = p.T / p.k_splits;
+        const uint32_t cols = p.T >> p.split_shift;
         const float* base = p.scratch + (size_t)tile * tile_floats + (size_t)(ks * cols) * W_TILE;
         const size_t split_stride = (size_t)n_tiles * tile_floats;
         const uint32_t tok0 = tt * p.T + ks * cols;
@@ -390,14 +403,15 @@ qgemm_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             return acc;
         };
         // four features per thread; a SwiGLU tile's features 64 .. 127 are the up projections of 0 .. 63
-        const uint32_t quads = p.swiglu ? GATE_ROWS / 4 : W_TILE / 4;
+        const uint32_t quads = swiglu ? GATE_ROWS / 4 : W_TILE / 4, quad_shift = swiglu ? 4u : 5u;
+        static_assert(GATE_ROWS == 64 && W_TILE == 128, "quads per column: 16 and 32");
         for (uint32_t i = threadIdx.x; i < cols * quads; i += THREADS) {
-            const uint32_t cl = i / quads, f = (i % quads) * 4u;
-            const uint32_t tok = tok0 + cl, n = p.swiglu ? wt * GATE_ROWS + f : wl * W_TILE + f;
+            const uint32_t cl = i >> quad_shift, f = (i & (quads - 1u)) * 4u;
+            const uint32_t tok = tok0 + cl, n = swiglu ? wt * GATE_ROWS + f : wl * W_TILE + f;
             if (tok >= p.M || n >= N) continue;
             const float4 acc = sum4(base + (size_t)cl * W_TILE + f);
             float a[4] = {acc.x, acc.y, acc.z, acc.w};
-            if (p.swiglu) {
+            if (swiglu) {
                 const float4 u = sum4(base + (size_t)cl * W_TILE + GATE_ROWS + f);
                 a[0] = silu_mul(a[0], u.x); a[1] = silu_mul(a[1], u.y); a[2] = silu_mul(a[2], u.z); a[3] = silu_mul(a[3], u.w);
             }
@@ -510,7 +524,7 @@ template <int FMT> size_t scratch_floats_fmt(const GemmArgs& a) {
     return (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE;
 }
 
-template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws, cudaStream_t stream) {
+template <int FMT, bool MULTI> cudaError_t launch_multi(const GemmArgs& a, const Workspace& ws, cudaStream_t stream) {
     using Cd = cdc::Codec<FMT>;
     Plan pl;
     if (!make_plan<FMT>(a, pl)) return cudaErrorInvalidValue;
@@ -518,8 +532,8 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
         return cudaErrorInvalidValue;
     const uint64_t w_row_bytes = (uint64_t)(a.K / Cd::CHUNK) * Cd::ROW_BYTES;
     const uint32_t x_cols = a.x_cols ? a.x_cols : a.K;          // columns past the end read as zero
-    CUtensorMap tmX, tmW0, tmW1, tmW2;
-    if (!make_map(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.X, x_cols, a.M, (uint64_t)x_cols * 2, KSTEP, pl.T, CU_TENSOR_MAP_SWIZZLE_128B))
+    Maps<MULTI> maps;
+    if (!make_map(&maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.X, x_cols, a.M, (uint64_t)x_cols * 2, KSTEP, pl.T, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     constexpr int EB = Cd::TMA_ELEM_BYTES;
     auto weight_map = [&](CUtensorMap* m, const void* w, uint32_t n) {
@@ -527,22 +541,23 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
                         Cd::ROW_BYTES / EB, a.W1 ? GATE_ROWS : W_TILE, Cd::RAW_SWIZZLE_128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
     };
     // second and third map: the up matrix of a SwiGLU launch, or the extra matrices of a grouped one
-    if (!weight_map(&tmW0, a.W0, a.N)) return cudaErrorInvalidValue;
-    tmW1 = tmW0; tmW2 = tmW0;
-    if (a.W1 && !weight_map(&tmW1, a.W1, a.N)) return cudaErrorInvalidValue;
-    if (a.n_extra > 0 && !weight_map(&tmW1, a.W_extra[0], a.N_extra[0])) return cudaErrorInvalidValue;
-    if (a.n_extra > 1 && !weight_map(&tmW2, a.W_extra[1], a.N_extra[1])) return cudaErrorInvalidValue;
+    if (!weight_map(&maps.w[0], a.W0, a.N)) return cudaErrorInvalidValue;
+    if constexpr (MULTI) {
+        maps.w[1] = maps.w[2] = maps.w[0];
+        if (a.W1 && !weight_map(&maps.w[1], a.W1, a.N)) return cudaErrorInvalidValue;
+        for (uint32_t e = 0; e < a.n_extra; e++)
+            if (!weight_map(&maps.w[1 + e], a.W_extra[e], a.N_extra[e])) return cudaErrorInvalidValue;
+    }
     Params p;
     p.M = a.M; p.N = a.N; p.K = a.K; p.T = pl.T; p.x_wrap = a.x_wrap ? a.x_wrap : a.K;
     p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
+    p.split_shift = 0u;
+    while ((1u << p.split_shift) < pl.k_splits) p.split_shift++;
     p.raw_stages = pl.raw_stages; p.b_stages = pl.b_stages; p.early = a.early_weights ? 1u : 0u; p.swiglu = a.W1 ? 1u : 0u;
     p.groups = 1u + a.n_extra;
-    p.tiles[0] = (a.N + W_TILE - 1) / W_TILE; p.grp_N[0] = a.N; p.grp_Y[0] = (__half*)a.Y;
-    for (uint32_t e = 0; e < 2u; e++) {
-        const bool on = e < a.n_extra;
-        p.tiles[1 + e] = on ? (a.N_extra[e] + W_TILE - 1) / W_TILE : 0u;
-        p.grp_N[1 + e] = on ? a.N_extra[e] : 0u; p.grp_Y[1 + e] = on ? (__half*)a.Y_extra[e] : nullptr;
-    }
+    p.Y = (__half*)a.Y;
+    p.tiles[0] = (a.N + W_TILE - 1) / W_TILE; p.tiles[1] = a.n_extra ? (a.N_extra[0] + W_TILE - 1) / W_TILE : 0u;
+    for (uint32_t e = 0; e < 2u; e++) { p.extra_N[e] = e < a.n_extra ? a.N_extra[e] : 0u; p.extra_Y[e] = e < a.n_extra ? (__half*)a.Y_extra[e] : nullptr; }
     p.residual = (const __half*)a.residual; p.layout = (uint32_t)a.layout; p.D = a.D ? a.D : 2;
     p.err = ws.err; p.scratch = ws.partial;
     p.meta0 = (const uint8_t*)a.W0 + (size_t)a.N * w_row_bytes;
@@ -555,7 +570,7 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
         cudaGetDevice(&dev);
         std::lock_guard<std::mutex> lock(mu);
         if (!(dev >= 0 && dev < 64 && ((attr_mask >> dev) & 1u))) {
-            cudaError_t e = cudaFuncSetAttribute(qgemm_small_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
+            cudaError_t e = cudaFuncSetAttribute(qgemm_small_kernel<FMT, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 64) attr_mask |= 1ull << dev;
         }
@@ -572,7 +587,11 @@ template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // prologue may overlap the previous kernel's tail
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, qgemm_small_kernel<FMT>, tmX, tmW0, tmW1, tmW2, p);
+    return cudaLaunchKernelEx(&cfg, qgemm_small_kernel<FMT, MULTI>, maps, p);
+}
+
+template <int FMT> cudaError_t launch_fmt(const GemmArgs& a, const Workspace& ws, cudaStream_t stream) {
+    return a.W1 || a.n_extra ? launch_multi<FMT, true>(a, ws, stream) : launch_multi<FMT, false>(a, ws, stream);
 }
 
 int g_mode = 1;
