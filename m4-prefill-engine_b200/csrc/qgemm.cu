@@ -108,18 +108,21 @@ template <int FMT> struct Cfg {
     static constexpr int THREADS = (EPI_WARP0 + 4) * 32;
 };
 
+// (what every role reads first stands in the first line of 64 bytes: the constant cache is cold when a CTA starts)
 struct Params {
-    uint32_t M, N, K;
-    uint32_t early;              // packed weights may be fetched before the preceding kernel has finished
-    uint32_t x_wrap;             // K after which the activation columns start over
+    uint32_t n_tok_tiles, n_w_tiles, k_splits, split_shift, chunks;    // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits); k_splits = 1 << split_shift
     uint32_t T;                  // tokens per tile (multiple of 16)
-    uint32_t n_tok_tiles, n_w_tiles, k_splits, chunks;    // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits)
     uint32_t raw_stages, b_stage_bytes, b_stages;         // ring depth of packed weights; bytes of one activation stage (T*128); activation ring depth
     uint32_t a_stages;                                    // ring depth of unpacked weight tiles (STAGES; more for CTA pairs)
+    uint32_t early;              // packed weights may be fetched before the preceding kernel has finished
+    uint32_t x_wrap;             // K after which the activation columns start over
+    uint32_t tt_shift;           // rotation of the token-tile order (fused reduce-scatter only, else 0)
+    uint32_t swiglu;             // 1: tiles are 64 gate rows (matrix 0) + their 64 up rows (matrix 1); output = silu(g) * u
+    uint32_t M, N, K;
+    uint32_t layout, H, D;
     __half* Y;
     const __half* residual;
     float* partial_out;
-    uint32_t layout, H, D;
     float* ws_partial;
     uint32_t split_cluster;      // the splits of a tile are one cluster and share out the sums
     uint32_t* ws_counters;
@@ -130,9 +133,7 @@ struct Params {
     __half* grp_Y[3];
     GemmArgs::Scatter scatter;   // fused reduce-scatter of fp32 partial sums to peer ranks (world == 0: off)
     GemmArgs::WaitRows wait_rows; // activations other ranks are still writing (flags == nullptr: off)
-    uint32_t tt_shift;           // rotation of the token-tile order (fused reduce-scatter only, else 0)
     uint32_t tiles_per_owner;    // output tiles whose token rows belong to one rank (fused reduce-scatter only)
-    uint32_t swiglu;             // 1: tiles are 64 gate rows (matrix 0) + their 64 up rows (matrix 1); output = silu(g) * u
     uint32_t row_epi;            // 1: outputs leave through the row-wise epilogue (16-byte stores of whole token rows)
     // per matrix of a (grouped) head-major launch: POST_ROPE rotates each head's pairs (i, i + D/2) with the table's
     // cosines and sines of the token's position; POST_Q8 writes block_q8_0 records [head][token][D/32] instead of fp16
@@ -193,8 +194,8 @@ __device__ __forceinline__ void for_each_sub(F& f, std::integer_sequence<int, S.
 struct Tile { uint32_t wt, tt, ks, id, kc0, kcn; };     // kc0, kcn: first packed chunk of K and how many
 __device__ __forceinline__ Tile decode_tile(uint32_t idx, const Params& p) {
     Tile t;
-    t.ks = idx % p.k_splits;
-    uint32_t rest = idx / p.k_splits;
+    t.ks = idx & (p.k_splits - 1u);
+    const uint32_t rest = idx >> p.split_shift;
     t.wt = rest % p.n_w_tiles;
     t.tt = rest / p.n_w_tiles;
     // fused reduce-scatter: rank r starts with the token rows of owner r + 1 and ends with its own, so that at any
@@ -202,8 +203,8 @@ __device__ __forceinline__ Tile decode_tile(uint32_t idx, const Params& p) {
     // owner's NVLink port at a time) and the last, local tiles overlap the tail of the remote transfers
     if (p.tt_shift) { t.tt += p.tt_shift; if (t.tt >= p.n_tok_tiles) t.tt -= p.n_tok_tiles; }
     t.id = t.tt * p.n_w_tiles + t.wt;
-    t.kc0 = t.ks * p.chunks / p.k_splits;
-    t.kcn = (t.ks + 1u) * p.chunks / p.k_splits - t.kc0;
+    t.kc0 = (t.ks * p.chunks) >> p.split_shift;
+    t.kcn = (((t.ks + 1u) * p.chunks) >> p.split_shift) - t.kc0;
     return t;
 }
 
@@ -599,7 +600,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         uint32_t rows_seen = 0;               // bit o: owner o's rows are known to be there
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
-            const uint32_t k0 = t.kc0 * (uint32_t)C::CHUNK, ksteps = t.kcn * (uint32_t)C::SUBS;
+            const uint32_t ksteps = t.kcn * (uint32_t)C::SUBS;
+            uint32_t x = (t.kc0 * (uint32_t)C::CHUNK) % p.x_wrap;         // column of the next activation tile (x_wrap: whole chunks)
             if (p.wait_rows.flags) {
                 // rows this CTA is about to load: wait until their owners have written them (system-scope acquire, then the
                 // proxy fence that orders the TMA reads behind it)
@@ -631,10 +633,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (lane == 0) {
                     QTR(1, xtr, 0);
                     ptx::mbar_arrive_expect_tx(&b_full[bs], b_rows * 128u);
-                    ptx::tma_load_2d(sB + bs * p.b_stage_bytes, &tmX, &b_full[bs], (int)((k0 + ks * KSTEP) % p.x_wrap), (int)(t.tt * p.T + pair_rank * b_rows));
+                    ptx::tma_load_2d(sB + bs * p.b_stage_bytes, &tmX, &b_full[bs], (int)x, (int)(t.tt * p.T + pair_rank * b_rows));
                     QTR(1, xtr, 1); xtr++;
                 }
                 __syncwarp();
+                x += (uint32_t)KSTEP;
+                if (x == p.x_wrap) x = 0u;
                 if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
             }
         }
@@ -1478,6 +1482,8 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
     p.early = a.early_weights ? 1u : 0u;
     p.split_cluster = 0u;
     p.T = pl.T; p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
+    p.split_shift = 0u;
+    while ((1u << p.split_shift) < pl.k_splits) p.split_shift++;
     p.swiglu = a.W1 ? 1u : 0u;
     // Row-wise epilogue: wherever every output row can take 16-byte stores (and, with a residual, 8-byte loads).  SwiGLU
     // tiles and split-K partial tiles have their own paths.
