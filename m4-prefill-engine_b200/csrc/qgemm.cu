@@ -1228,8 +1228,8 @@ __global__ void qgemm_generic_kernel(int fmt, const __half* X, const uint8_t* W0
 // With nothing to do (reading 284 KB: 129 tokens, N = 1100) the launch costs 1.5 us.
 __global__ void __launch_bounds__(256) repair_nonfinite_kernel(int fmt, const __half* __restrict__ X, const uint8_t* __restrict__ W0, const uint8_t* __restrict__ W1,
                                                                const Params p) {
-    ptx::grid_dependency_wait();
     ptx::launch_dependents();
+    ptx::grid_dependency_wait();
     const size_t outputs = (size_t)p.M * p.N, i0 = ((size_t)blockIdx.x * 256u + threadIdx.x) * 8u;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t bad = 0u;

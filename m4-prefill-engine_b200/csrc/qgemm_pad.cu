@@ -147,8 +147,8 @@ __device__ __forceinline__ void pad_plane(const Plane& p, const uint8_t* __restr
 }
 
 __global__ void __launch_bounds__(128) pad_rows_kernel(const uint8_t* __restrict__ w0, const uint8_t* __restrict__ w1, uint8_t* __restrict__ dst, const Planes pl) {
+    ptx::launch_dependents();              // (the projection touches nothing before its own wait)
     ptx::grid_dependency_wait();           // the scratch may still be read by the launch before
-    ptx::launch_dependents();
     const uint32_t which = blockIdx.z % pl.n, matrix = blockIdx.z / pl.n;
     const Plane p = pl.p[which];
     const uint8_t* src = (matrix ? w1 : w0) + p.src;
