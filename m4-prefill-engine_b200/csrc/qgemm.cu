@@ -1361,7 +1361,9 @@ Plan make_plan(const GemmArgs& a) {
     // Where even so at least half of the SMs would idle, shorter token tiles: a tile's epilogue and MMAs grow with its tokens,
     // its main loop (unpacking) does not, and every output is the same sum (K = 512: 301 tokens, N = 512 9.2 -> 8.7 us, SwiGLU
     // F = 1024 9.9 -> 8.6 us; K = 2080, N = 1100, 129 tokens 23.1 -> 19.7 us).
-    if (!a.lean && !a.scatter.world && !a.wait_rows.flags) {
+    // Not for SwiGLU in the variable-rate format: unpacking is all its time, and the taller tiles run as CTA pairs that unpack faster
+    // (K = 4096, F = 2048, 128 tokens: 35.3 us on pairs, 38.4 on short tiles).
+    if (!a.lean && !a.scatter.world && !a.wait_rows.flags && !(a.W1 && a.format == QUANT_VAR_RATE_AFFINE)) {
         const uint32_t sms = (uint32_t)sm_count(), fit = sms / (pl.n_w_tiles * pl.k_splits), most = (a.M + 31u) / 32u;
         const uint32_t want = fit < most ? fit : most;
         if (want >= 2u * pl.n_tok_tiles) {
@@ -1695,13 +1697,6 @@ GemmArgs padded_probe(const GemmArgs& a) {
     return b;
 }
 }  // namespace
-
-bool persistent_splits_poorly(const GemmArgs& a) {
-    if (row_bytes_256(a.format) == 0 || a.K % chunk_elems(a.format) != 0) return false;
-    const Plan pl = make_plan(a);
-    // (the cluster capacity is that of one CTA per SM: the same for every format)
-    return pl.k_splits == 8u || (pl.k_splits > 1u && pl.n_tok_tiles * pl.n_w_tiles > max_split_clusters<QUANT_Q4_0>(pl.k_splits));
-}
 
 size_t workspace_floats(const GemmArgs& a) {
     if (pad_path_ok(a)) return workspace_floats(padded_probe(a)) + (padded_bytes(a) + kept_residual_bytes(a) + 512) / sizeof(float);

@@ -86,16 +86,14 @@ bool fast_path_ok(const GemmArgs& a);
 // Floats of split-K scratch the launch will use (0 when it does not split).
 size_t workspace_floats(const GemmArgs& a);
 // Enqueue on `stream`.  Returns cudaSuccess or the launch error.
-// Single-token path on CUDA cores (qgemv.cu): M == 1, plain standard-layout output, K % 256 == 0.
+// Single-token path on warp-level MMAs (qgemv.cu): M == 1, plain standard-layout output, K % 256 == 0.
 bool gemv_path_ok(const GemmArgs& a);
 cudaError_t launch_gemv(const GemmArgs& a, cudaStream_t stream);
 cudaError_t launch(const GemmArgs& a, const Workspace& ws, cudaStream_t stream);
 // Few-token path (qgemm_small.cu): weights unpacked straight into tensor memory, K split across a thread-block cluster whose
-// CTAs share out the sum of the partial tiles.  Taken for M <= 128 where the persistent kernel would leave SMs idle.
+// CTAs share out the sum of the partial tiles.  Taken for M <= 128, and beyond where a long K and few tiles would leave SMs idle.
 bool small_path_ok(const GemmArgs& a);
 size_t small_scratch_floats(const GemmArgs& a);
-// The persistent kernel would split this launch's K eight ways, or into more clusters than the GPU holds at once.
-bool persistent_splits_poorly(const GemmArgs& a);
 cudaError_t launch_small(const GemmArgs& a, const Workspace& ws, cudaStream_t stream);
 void set_small_kernel_enabled(int mode);     // testing hook: 0 routes those shapes to the persistent kernel again, 1 default,
                                              // 2 takes every shape the kernel can compute (any number of token tiles)

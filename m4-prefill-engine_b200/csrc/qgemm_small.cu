@@ -629,11 +629,17 @@ bool small_path_ok(const GemmArgs& a) {
     }
     if (a.K % chunk != 0) return false;
     if (small::g_mode == 2) return true;
-    // More than one token tile unpacks every weight tile more than once, which costs nothing where most of the GPU would idle: a
-    // projection that the persistent kernel splits eight ways, or into more clusters than fit (its CTAs take an SM each), has
-    // its work in twice as many CTAs here (K = 4096: 160 tokens N = 2048 19.3 -> 12.3 us, 200 tokens N = 1100 16.3 -> 12.8, 300 tokens
-    // N = 1000 19.2 -> 13.7; 300 tokens K = N = 2304 17.1 -> 14.5; 140 tokens K = 5120 N = 640 10.7 -> 11.2).
-    if (a.M > (uint32_t)small::MAX_T) return !a.W1 && !a.n_extra && !a.lean && persistent_splits_poorly(a);
+    // More than one token tile unpacks every weight tile more than once, which costs nothing where most of the GPU would idle: where the
+    // persistent kernel (an SM per CTA) has so few tiles that it could split a long K eight ways, this one has its work in twice as
+    // many CTAs -- as long as its clusters of eight are all resident at once (two CTAs an SM, but up to an eighth of the SMs are left over
+    // where a GPC is not whole clusters: 32 of them are, 36 are not), and from 16 tiles on (below, the persistent kernel is as fast).  K = 4096: 160 tokens N = 2048 19.3 -> 12.3 us, 300 tokens N = 1000 19.2 -> 13.7; with 36 clusters, K = 14336, N = 2304,
+    // 129 tokens, it takes 33 us against 24.  Not in the variable-rate format, where unpacking twice does cost (N = 2048, K = 14336:
+    // 1.2 to 1.4 times).  324 of 2592 timed shapes of 129 to 768 tokens come here, none more than 17 % slower than there.
+    if (a.M > (uint32_t)small::MAX_T) {
+        if (a.W1 || a.n_extra || a.lean || a.format == QUANT_VAR_RATE_AFFINE || a.K / chunk < 16u) return false;
+        const uint32_t w_tiles = (a.N + 127u) / 128u, tiles = (a.M + 127u) / 128u * w_tiles, persistent = (a.M + 255u) / 256u * w_tiles;
+        return tiles >= 16u && persistent * 8u <= (uint32_t)small::sms() && tiles * 8u <= (uint32_t)small::sms() / 4u * 7u;
+    }
     // One token tile: at most two weight tiles per SM.  Beyond that the persistent kernel, which starts on the next tile while the
     // last one drains, is as fast.
     uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
@@ -644,6 +650,10 @@ bool small_path_ok(const GemmArgs& a) {
     // against 10.2 / 13.0 us there; 64 tokens, K = 512 / 1024: 9.6 / 11.0 against 9.1 / 11.5; F = 14336, K = 4096, 128 tokens: 44.5
     // against 47.5, the variable-rate codec 75.8 against 72.2).
     const uint32_t T = (a.M + 15u) & ~15u;
+    // Grouped launches with a short K for their tokens: the same (512 + 2 x 128 features, K = 512: 64 tokens 7.9 us against 7.0, 128 tokens 9.9
+    // against 8.4; 1024 + 2 x 256, K = 1024: 64 tokens 10.4 against 10.8, 128 tokens 14.3 against 12.5; K = 2048, 128 tokens 14.3 against
+    // 14.9), and earlier in the variable-rate format (K = 512, one token 9.3 against 7.6; K = 1024, 33 tokens 12.6 against 11.3).
+    if (a.n_extra && (a.format == QUANT_VAR_RATE_AFFINE ? a.K <= 512u || a.K < 22u * T : a.K < 12u * T)) return false;
     if (a.W1 && (a.K < T * T / 4u || (T == (uint32_t)small::MAX_T && a.format == QUANT_VAR_RATE_AFFINE))) return false;
     return true;
 }
