@@ -183,8 +183,9 @@ cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
 template <int FMT>
 cudaError_t launch_gemv_fmt(const GemmArgs& a, cudaStream_t stream) {
     // Two rows per lane fill the fragment; the variable-rate codec's two rows take 179 registers, one row 124 (K = 4096, N = 14336:
-    // 31.3 against 23.5 us), and the codebook's 177 cost more than they give once a warp loops over K (K = 14336: 25.8 against 24.9).
-    const bool one = FMT == QUANT_VAR_RATE_AFFINE || (FMT == QUANT_EXL3 && a.K > 256u * 4u * GV_MAX_WARPS);
+    // 31.3 against 23.5 us), and the codebook's 177 registers cost more than they give (K = 4096, N = 32000: 42.3 against 39.1; K = 5120,
+    // N = 5120 18.3 against 11.6; K = 14336, N = 4096 25.8 against 24.9; the other way round K = N = 4096, 7.4 against 8.9).
+    const bool one = FMT == QUANT_VAR_RATE_AFFINE || FMT == QUANT_EXL3;
     return one ? launch_gemv_rows<FMT, 1>(a, stream) : launch_gemv_rows<FMT, 2>(a, stream);
 }
 
@@ -194,7 +195,7 @@ bool gemv_path_ok(const GemmArgs& a) {
     if (a.force_generic || a.M != 1 || a.W1 || a.residual || a.partial_out || a.layout != 0 || a.scatter.world || a.n_extra) return false;
     if (a.K == 0 || a.K % 256 != 0 || a.N == 0) return false;
     if (((uintptr_t)a.W0 & 15u) || ((uintptr_t)a.X & 1u)) return false;
-    if ((size_t)(a.K / 256) * 257 * sizeof(float) > 200 * 1024) return false;      // (longer rows go to the few-token kernel)
+    if (a.K > 199u * 256u) return false;      // longer rows stay on the few-token kernel, as they always have (shared memory would hold twice that)
     switch (a.format) {
         case QUANT_Q4_0: case QUANT_MLX_4BIT: case QUANT_Q4_K: case QUANT_TERNARY_1_58: case QUANT_VAR_RATE_AFFINE: case QUANT_EXL3:
         case QUANT_MLX_4BIT_G64: case QUANT_TERNARY_ROW: case QUANT_MLX_4BIT_PLANAR: return true;
