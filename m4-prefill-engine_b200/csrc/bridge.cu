@@ -576,9 +576,12 @@ int b200_bridge_wait_stream(void* stream) {
     if (!g.initialized) return -1;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { cudaGetLastError(); return -6; }
+    {
+        RelaxedCapture relaxed;         // (a query would end a capture in global mode that is under way on any stream)
+        if (cudaStreamQuery((cudaStream_t)stream) == cudaSuccess) return 0;     // nothing to wait for: one call instead of three
+        cudaGetLastError();
+    }
     if (capturing(g.stream) || capturing(g.stream_in)) return -6;
-    if (cudaStreamQuery((cudaStream_t)stream) == cudaSuccess) return 0;         // nothing to wait for: one call instead of three
-    cudaGetLastError();
     if (cudaEventRecord(g.ev_caller, (cudaStream_t)stream) != cudaSuccess || cudaStreamWaitEvent(g.stream, g.ev_caller, 0) != cudaSuccess ||
         cudaStreamWaitEvent(g.stream_in, g.ev_caller, 0) != cudaSuccess) {
         cudaGetLastError();

@@ -71,3 +71,23 @@ def test_bridge_stream_under_capture_is_left_alone(bridge):
     g.replay()
     torch.cuda.synchronize()
     assert float(t.sum()) == 8.0
+
+
+def test_other_captures_are_left_alone(bridge):
+    """A capture on a stream that the bridge has nothing to do with goes on while the bridge waits for idle and busy streams."""
+    own, busy, idle, g = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    t = torch.zeros(8, device="cuda")
+    with torch.cuda.stream(own):
+        t.add_(0)
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=own):
+        with torch.cuda.stream(busy):
+            torch.cuda._sleep(200_000_000)
+        rc = [bridge.lib.b200_bridge_wait_stream(s.cuda_stream) for s in (idle, busy)]
+        t.add_(1)
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert rc == [0, 0] and float(t.sum()) == 8.0
