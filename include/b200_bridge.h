@@ -128,8 +128,8 @@ int b200_bridge_unregister_weights(const void* host_ptr);
  * kernel (111..117), an attention kernel (201..204, 220..227) or the peer exchange (301, 302); 401: a token id outside the
  * embedding table. */
 int b200_bridge_device_error(void);
-/* The same without waiting for the stream: what kernels that have finished reported. */
-int b200_bridge_error_flag(void);
+/* What the last m4_bridge_synchronize or b200_bridge_device_error found (read only; 0 after init and clear). */
+extern int b200_bridge_error_seen;
 /* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
  * holds now, without a wait on the host.  -6 if that is not possible (it, or a stream of the bridge, is under capture). */
 int b200_bridge_wait_stream(void* stream);

@@ -84,8 +84,6 @@ def bind(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.b200_bridge_graph_scratch_bytes.restype = ctypes.c_size_t
     lib.b200_bridge_device_error.argtypes = []
     lib.b200_bridge_device_error.restype = _i
-    lib.b200_bridge_error_flag.argtypes = []
-    lib.b200_bridge_error_flag.restype = _i
     lib.b200_bridge_last_error_string.argtypes = []
     lib.b200_bridge_last_error_string.restype = ctypes.c_char_p
     lib.b200_bridge_kernel_launches.argtypes = []
@@ -139,7 +137,7 @@ class B200Bridge:
         self._lib = bind(ctypes.CDLL(str(path)))
         self._in_flight: list[tuple[torch.Tensor, ...]] = []
         self._pending_finite: list[torch.Tensor] = []
-        self.error_flag = self._lib.b200_bridge_error_flag      # `device_error` of the kernels that have finished, without a wait
+        self.error_seen = ctypes.c_int.in_dll(self._lib, "b200_bridge_error_seen")     # `device_error` as the last synchronize found it
 
     @property
     def lib(self) -> ctypes.CDLL:

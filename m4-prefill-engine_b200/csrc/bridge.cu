@@ -301,6 +301,8 @@ using namespace bridge;
 
 extern "C" {
 
+int b200_bridge_error_seen = 0;
+
 bool m4_bridge_init(const char*) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (g.initialized) return true;
@@ -341,6 +343,7 @@ bool m4_bridge_init(const char*) {
     }
     g.err_host = static_cast<int*>(err_host);
     *g.err_host = 0;
+    b200_bridge_error_seen = 0;
     g.err_word = static_cast<int*>(err_dev);
     cudaStreamSynchronize(g.stream);
     // everything that makes the driver load code or reserve memory happens here, not in a later dispatch: the kernels'
@@ -514,6 +517,7 @@ void m4_bridge_synchronize(void) {
         std::lock_guard<std::mutex> lock(g.mu);
         if (g.initialized) {
             if (copies && g.copy_seq == copy_seq_before) g.copies = false;
+            b200_bridge_error_seen = *g.err_host;
             for (StageSlot& sl : g.slots)
                 if (sl.out_pending && (sl.out_seq <= seq_before || cudaEventQuery(sl.ev_out) == cudaSuccess)) {
                     sl.out_pending = false; sl.out_ptr = nullptr; sl.out_bytes = 0;
@@ -594,13 +598,7 @@ int b200_bridge_device_error(void) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.initialized) return -1;
     cudaStreamSynchronize(g.stream);
-    return *g.err_host;
-}
-
-/* The same without waiting and without the lock: what kernels that have finished reported (0 before init). */
-int b200_bridge_error_flag(void) {
-    volatile int* err = g.err_host;
-    return err ? *err : 0;
+    return b200_bridge_error_seen = *g.err_host;
 }
 
 int b200_bridge_clear_device_error(void) {
@@ -609,7 +607,7 @@ int b200_bridge_clear_device_error(void) {
     sync_all_streams(g.stream, g.stream_in, g.stream_out);
     // A split-K launch that gave up on a bounded wait leaves its tile counters part-way: they are cleared with the error word,
     // so the next split-K launch starts from zero again.
-    *g.err_host = 0;
+    *g.err_host = b200_bridge_error_seen = 0;
     return cudaMemset(g.counters, 0, 4096 * sizeof(uint32_t) + 64) == cudaSuccess ? 0 : -6;
 }
 

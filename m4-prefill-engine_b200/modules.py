@@ -143,20 +143,21 @@ class M4QuantizedLinear(torch.nn.Module):
         dev = self.weight.device
         if x.numel() == 0:
             return torch.zeros((*x.shape[:-1], N), dtype=torch.float16, device=dev)
-        out_shape = (*x.shape[:-1], N)
+        lead = x.shape[:-1]
         if x.dtype != torch.float16:
             x = x.to(torch.float16)
         x = x.to(dev)
         # The projection writes every element -- unless a kernel gives up on a bounded wait, which the error word tells: no
         # memory that nothing wrote is handed out.  (The word keeps the first error, so behind one the output starts as zeros.)
-        bridge = B200Bridge.get_instance()
-        clean = bridge.error_flag() == 0 and not check_finite
+        error = B200Bridge.get_instance().error_seen
+        clean = error.value == 0 and not check_finite
         new = torch.empty if clean else torch.zeros
-        if x.dim() == 1:
+        if len(lead) == 0:
             y = new((N,), dtype=torch.float16, device=dev)
             m4_bridge_dispatch_gemv(x, self.weight, y, self.format, K, N, check_finite=check_finite)
         else:
-            x = x.reshape(-1, K)
+            if len(lead) != 1:
+                x = x.reshape(-1, K)
             m = x.shape[0]
             y = new((m, N), dtype=torch.float16, device=dev)
             if m == 1:
@@ -165,6 +166,6 @@ class M4QuantizedLinear(torch.nn.Module):
                 m4_bridge_dispatch_gemm(x, self.weight, y, self.format, m, K, N, check_finite=check_finite)
         # the result is handed back to torch code that runs on another stream: wait here
         m4_bridge_synchronize()
-        if clean and bridge.error_flag() != 0:
+        if clean and error.value != 0:
             y.zero_()
-        return y.reshape(out_shape)
+        return y if len(lead) < 2 else y.reshape(*lead, N)

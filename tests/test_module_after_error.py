@@ -1,5 +1,7 @@
 """M4QuantizedLinear when a kernel reports that it gave up: zeros where nothing was written, never memory as it was found (on the
 CPU, with the library replaced by a stand-in)."""
+from ctypes import c_int
+
 import pytest
 import torch
 
@@ -10,17 +12,14 @@ class Bridge:
     """Stands in for the library: the projection of call `failing` writes nothing and reports code 106."""
 
     def __init__(self, failing):
-        self.calls, self.failing, self.err = 0, failing, 0
+        self.calls, self.failing, self.error_seen = 0, failing, c_int(0)
 
     def is_initialized(self):
         return True
 
-    def error_flag(self):
-        return self.err
-
     def dispatch(self, x, w, y, *args, **kwargs):
         if self.calls == self.failing:
-            self.err = 106
+            self.error_seen.value = 106
         else:
             y.fill_(3.0)
         self.calls += 1
