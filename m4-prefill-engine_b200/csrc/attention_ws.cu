@@ -98,13 +98,17 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return r;
 }
 // 2^x of two values without the special-function unit: x = n + f with n the nearest integer (in the low mantissa bits of
-// x + 1.5 * 2^23) and |f| <= 1/2, 2^f as a polynomial (exp2_poly.cuh), n added to the exponent field.  Inputs below -120
-// (masked scores are -inf) give 2^-120; a NaN stays non-finite in fp16 (the maximum propagates it).
+// x + 1.5 * 2^23) and |f| <= 1/2, 2^f as a polynomial (exp2_poly.cuh), n added to the exponent field.  Inputs below
+// -120 (masked scores are -inf) give 2^-120.  A NaN (the maximum propagates it) gives the largest fp32 number: infinite as a
+// probability, and a sum that no row reaches otherwise (SUM_OF_NAN), by which the row is told to be NaN.  (Multiplying by 2^n instead
+// keeps the NaN and costs 3 % of the 8B prefill.)
 __device__ __forceinline__ float max_nan(float a, float b) {
     float y;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
     return y;
 }
+// a row's sum is at most 2^8 (see the lag) times 2^31 keys
+constexpr float SUM_OF_NAN = 1e12f;
 template <int DEG> __device__ __forceinline__ void ex2_poly2(float x0, float x1, float& e0, float& e1) {
     const uint64_t x = pack2(max_nan(x0, -120.0f), max_nan(x1, -120.0f));
     const uint64_t r = add2(x, pack2(12582912.0f, 12582912.0f));
@@ -380,7 +384,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (lane == 0) ptx::mbar_arrive(&p_full[g]);
             float a0, a1;
             unpack2(add2(rs0, rs1), a0, a1);
-            l_run = l_run * corr + (a0 + a1);
+            l_run = (l_run > SUM_OF_NAN ? l_run : l_run * corr) + (a0 + a1);
         }
         // ---------------- result ----------------
         if (cnt > 0u && ok) ok = __all_sync(0xffffffffu, ptx::mbar_wait<64>(&o_full[g], 0u, abort_flag, p.err, 227));
@@ -398,7 +402,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                                    : reinterpret_cast<uint8_t*>(p.O + (p.out_tokens_major ? ((size_t)pos * p.Hq + head) * D : r * D));
             if (!row_ok) dst = nullptr;
             if (p.split && row_ok) p.part_ml[split_row] = make_float2(m_run, l_run);
-            const float inv = p.split ? 1.0f : (l_run > 0.0f ? 1.0f / l_run : 0.0f);
+            const float inv = p.split ? 1.0f : (l_run > 0.0f && l_run <= SUM_OF_NAN ? 1.0f / l_run : 0.0f);      // (0: infinite O becomes NaN)
             uint8_t* stage = sQ + g * C::TILE;
             const uint32_t row0 = (warp & 3u) * 32u;
             const uint32_t cols = p.split ? D / 2u : (uint32_t)D;    // accumulator columns per pass
@@ -459,7 +463,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const Params p) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     const float w = lane < n ? ex2(ml.x - m) : 0.0f;
-    float l = w * ml.y;
+    float l = ml.y > SUM_OF_NAN ? INFINITY : w * ml.y;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
     const float wn = l > 0.0f ? w / l : 0.0f;

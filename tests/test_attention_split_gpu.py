@@ -84,3 +84,33 @@ def test_unseen_cache_is_not_expanded(bridge):
     bridge.synchronize()
     assert launches == 3                                     # expansion, split attention, combination: not the kernels without scratch
     assert np.abs(O.cpu().numpy().astype(np.float64) - gold).max() <= TOL
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,M,pos0", [(4, 2, 64, 200, 0), (6, 2, 64, 90, 300), (3, 1, 128, 150, 100), (8, 2, 128, 200, 0), (4, 4, 128, 3, 1500)])
+@pytest.mark.parametrize("where", ["q", 0, 3])          # 0, 3: a key whose exponential comes from the special-function unit, from the polynomial
+def test_nonfinite_scores(bridge, Hq, Hkv, D, M, pos0, where):
+    """NaN and infinities in Q or K: the rows that the warp-level kernels answer with NaN, and no others."""
+    L, Mkv = bridge.lib, pos0 + M
+    rng = np.random.default_rng(M)
+    Q, K, V = (rng.standard_normal(s, dtype=np.float32).astype(np.float16) for s in ((Hq, M, D), (Hkv, Mkv, D), (Hkv, Mkv, D)))
+    if where == "q":
+        Q[1, M // 2, 5], Q[0, M - 1, 0] = np.nan, np.inf
+    else:
+        K[0, pos0 // 8 * 8 + where, 7] = np.nan
+        K[Hkv - 1, Mkv - 2, 3] = -np.inf
+    Qd, Kd, Vd = (torch.from_numpy(t).cuda() for t in (Q, K, V))
+    out = []
+    for hook in (0, 1):
+        O = torch.empty(Hq, M, D, dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        L.b200_bridge_force_legacy_attention(hook)
+        try:
+            assert L.b200_bridge_dispatch_attention_q8kv(Qd.data_ptr(), Kd.data_ptr(), Vd.data_ptr(), O.data_ptr(), Hq, Hkv, M, Mkv, D, c_float(D ** -0.5), pos0, 0, 1) == 0
+        finally:
+            L.b200_bridge_force_legacy_attention(0)
+        bridge.synchronize()
+        out.append(O.cpu().numpy().astype(np.float64))
+    assert np.isnan(out[1]).any()
+    assert np.array_equal(np.isnan(out[0]), np.isnan(out[1]))
+    ok = ~np.isnan(out[1])
+    assert np.all(np.isfinite(out[0][ok])) and np.abs(out[0][ok] - out[1][ok]).max(initial=0.0) <= TOL
