@@ -40,3 +40,42 @@ def test_layer_shapes(pkg, bridge, case):
     # the layer's two residual blocks each round once more than a projection does, and a Q8_0 code on the edge between two
     # integers may fall either way: the pass line of the 8B layer, 2/128 or 2^-7 of the row
     assert np.all(diff <= np.maximum(2.0 / 128, 2.0 ** -7 * np.sqrt(np.mean(gold ** 2, axis=1, keepdims=True))))
+
+
+@pytest.mark.parametrize("M", [1, 33, 300])
+def test_weights_rewritten_just_before(pkg, bridge, M):
+    """Packed weights written on the layer's stream right before a forward are the ones it multiplies with, although its projections
+    fetch theirs before they wait for the kernel in front."""
+    import torch
+    from m4_prefill_engine_b200.layer import TransformerLayerConfig, TransformerLayerCoordinator
+    K, H, Hkv, D, F = 512, 8, 2, 64, 1024
+    sets = [layer_weights(o.Q4_0, K, H, Hkv, D, F)[0]]
+    sets.append({k: np.ascontiguousarray(np.roll(v.reshape(-1, 18), 1, axis=0)).reshape(-1) for k, v in sets[0].items()})
+    rng = np.random.default_rng(M)
+    X = dev((rng.standard_normal((M, K)) * 0.5).astype(np.float16))
+    norms = [dev(rng.uniform(0.5, 1.5, K).astype(np.float16)) for _ in range(2)]
+    layer = TransformerLayerCoordinator(TransformerLayerConfig(M=M, K=K, H=H, D=D, N_mlp=F, attn_scale=D ** -0.5, weight_format=o.Q4_0,
+                                                               num_kv_heads=Hkv, rms_eps=1e-5, rope_theta=10000.0, kv_q8_0=True))
+    layer.set_norm_weights(*norms)
+    src = [{k: dev(v) for k, v in w.items()} for w in sets]
+    names = ("q", "k", "v", "o", "gate", "up", "down")
+
+    def forward(w, y):
+        layer.forward(X, *[w[n] for n in names], y)
+    want = [torch.empty(M, K, dtype=torch.float16, device="cuda") for _ in range(2)]
+    for w, y in zip(src, want):
+        forward(w, y)
+        bridge.synchronize()
+    assert not torch.equal(*want)
+    used = {k: v.clone() for k, v in src[0].items()}
+    stream = torch.cuda.ExternalStream(bridge.lib.b200_bridge_stream())
+    got = [torch.empty(M, K, dtype=torch.float16, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        with torch.cuda.stream(stream):
+            for n in names:
+                used[n].copy_(src[i & 1][n])
+            forward(used, y)
+    bridge.synchronize()
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i & 1]), i
