@@ -1361,9 +1361,12 @@ Plan make_plan(const GemmArgs& a) {
     // Where even so at least half of the SMs would idle, shorter token tiles: a tile's epilogue and MMAs grow with its tokens,
     // its main loop (unpacking) does not, and every output is the same sum (K = 512: 301 tokens, N = 512 9.2 -> 8.7 us, SwiGLU
     // F = 1024 9.9 -> 8.6 us; K = 2080, N = 1100, 129 tokens 23.1 -> 19.7 us).
-    // Not for SwiGLU in the variable-rate format: unpacking is all its time, and the taller tiles run as CTA pairs that unpack faster
-    // (K = 4096, F = 2048, 128 tokens: 35.3 us on pairs, 38.4 on short tiles).
-    if (!a.lean && !a.scatter.world && !a.wait_rows.flags && !(a.W1 && a.format == QUANT_VAR_RATE_AFFINE)) {
+    // The variable-rate and the 34-byte Prism codecs are another matter: unpacking is nearly all their time, shorter tiles repeat it, and
+    // the taller ones run as CTA pairs.  They keep theirs beyond four weight tiles with a long K, and beyond twelve (variable rate K = 4096,
+    // N = 1100, 256 tokens 0.71 of the time on short tiles, SwiGLU K = 4096, F = 2048, 128 tokens 35.3 against 38.4 us; N = 256, K = 512 1.38).
+    const bool slow_unpack = a.format == QUANT_VAR_RATE_AFFINE || a.format == QUANT_PRISM_Q2_0;
+    const bool keep_tall = slow_unpack && (pl.n_w_tiles > 12u || (pl.n_w_tiles > 4u && a.K > 1024u));
+    if (!a.lean && !a.scatter.world && !a.wait_rows.flags && !keep_tall) {
         const uint32_t sms = (uint32_t)sm_count(), fit = sms / (pl.n_w_tiles * pl.k_splits), most = (a.M + 31u) / 32u;
         const uint32_t want = fit < most ? fit : most;
         if (want >= 2u * pl.n_tok_tiles) {
