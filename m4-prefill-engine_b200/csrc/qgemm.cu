@@ -1587,7 +1587,8 @@ cudaError_t launch_fast(const GemmArgs& a, const Workspace& ws, cudaStream_t str
     const uint32_t grid = total < (uint32_t)sm_count() ? total : (uint32_t)sm_count();
     // Programmatic stream serialization: this grid's CTAs may be placed (and run their prologue up to
     // griddepcontrol.wait) while the previous kernel in the stream drains, which hides the launch latency between
-    // back-to-back projections.  Stream order is unchanged: nothing is read or written before that wait.
+    // back-to-back projections.  Stream order is unchanged: nothing is read or written before that wait, except
+    // packed weights where the caller vouches for them (early_weights).
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(C::THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;

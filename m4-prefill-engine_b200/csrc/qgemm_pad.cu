@@ -13,9 +13,9 @@
 // takes two terms, the affine formats three; ternary weights are exact as they are.  (Exact as long as every product is finite:
 // outputs that come out infinite or NaN are computed again from the weights as they are, repair_nonfinite_kernel in qgemm.cu.)
 //
-// One launch and the packed bytes once or a few times more; K = 2080, N = 1100, 129 tokens took 1361 us on the CUDA cores and takes 17 us
-// (one token 13 us).
-// That kernel remains for activations that are not 16-byte aligned.
+// One launch in front, the packed bytes once or a few times more, and the repair pass behind: K = 2112, N = 1100, 129 tokens took
+// 1707 us on the CUDA cores and takes 18 us, one token 336 and 13.  The CUDA-core kernel remains for activations that are not
+// 16-byte aligned, for launches whose scratch has no room for the copy, and where the copy would be most of the work (pad_path_ok).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 

@@ -1,6 +1,6 @@
 // Few-token projection: Y[m][n] = sum_k X[m][k] * dequant(W)[n][k] for up to 128 tokens (the decode-like shapes M = 33 /
 // 127 / 128 of the router sweep, bench_universal_router.mm:764-773, and every projection of a short prefill: up to three
-// matrices in one launch, and the dual gate / up projection with SwiGLU).  HBM-bound: the packed weights are
+// matrices in one launch, and the dual gate / up projection with SwiGLU), and for more where a long K has few tiles (small_path_ok).  HBM-bound: the packed weights are
 // read once, so what matters is how fast an SM turns packed bytes into MMA operands.
 //
 // Differences from the persistent kernel in qgemm.cu, all aimed at that:
@@ -8,7 +8,7 @@
 //     elements to 32 registers of fp16 pairs and writes them with one tcgen05.st into a ring of A-operand stages in
 //     tensor memory; the MMA takes A from tensor memory (tcgen05.mma [d], [a], b-desc) and only the activations from
 //     shared memory.  That removes the 16 KB store + 16 KB operand read per 64-element step that bound the other kernel;
-//   * small CTAs (4 unpack warps = the 4 lane quadrants, a copy warp, an MMA warp; <= 100 KB of shared memory, 256
+//   * small CTAs (4 unpack warps = the 4 lane quadrants, a copy warp, an MMA warp; <= 112 KB of shared memory, 256
 //     tensor-memory columns) so that two CTAs share an SM and one's copies and unpacking overlap the other's;
 //   * one work item per CTA: K is split up to eight ways and the splits of a tile form a thread-block cluster.  Every CTA
 //     writes its partial tile to a scratch buffer (which stays in L2), one cluster barrier later each CTA of the cluster
