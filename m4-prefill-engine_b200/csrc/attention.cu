@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attn_tc_kernel(const Params p, 
     auto wait_raw = [&](uint32_t kt) {
         if (bulk_ok(kt)) {
             const uint32_t st = kt & 1u;
-            ptx::mbar_wait<32>(&bar_raw[st], (raw_phase >> st) & 1u, abort_flag, err, 204);
+            ptx::mbar_wait(&bar_raw[st], (raw_phase >> st) & 1u, abort_flag, err, 204);
             raw_phase ^= 1u << st;
         } else {
             cp_async_wait<0>();
@@ -893,11 +893,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attn_tc_kernel(const Params p, 
         }
         // PV(kt-1) must be done before sVt, sP and O are touched again (a failed wait sets the abort flag, which
         // is tested after the next CTA barrier)
-        if (kt > 0) ptx::mbar_wait<32>(bar_o, ph ^ 1u, abort_flag, err, 202);
+        if (kt > 0) ptx::mbar_wait(bar_o, ph ^ 1u, abort_flag, err, 202);
         if (worker) unpack(kt, 1);
         ATR(1);
         if (worker) {
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(bar_s, ph, abort_flag, err, 201));
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait(bar_s, ph, abort_flag, err, 201));
             ATR(2);
             // (a failed wait has set the abort flag; the code below still runs so that the pair barrier and the
             // warp-collective tensor-memory accesses stay matched, its results are discarded after the CTA barrier)
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attn_tc_kernel(const Params p, 
         ATR(7);
     }
     // the last PV
-    ptx::mbar_wait<32>(bar_o, (n_ktiles - 1u) & 1u, abort_flag, err, 203);
+    ptx::mbar_wait(bar_o, (n_ktiles - 1u) & 1u, abort_flag, err, 203);
     __syncthreads();
     ATR_FLUSH();
     cp_async_wait<0>();

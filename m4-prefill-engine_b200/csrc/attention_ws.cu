@@ -232,7 +232,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         uint32_t slot = 0, ph = 0;
         bool ok = true;
         for (uint32_t i = 0; ok && i < 2u * n_steps; i++) {
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&kv_empty[slot], ph ^ 1u, abort_flag, p.err, 220));
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&kv_empty[slot], ph ^ 1u, abort_flag, p.err, 220));
             if (!ok) break;
             if (lane == 0) {
                 const CUtensorMap* map = (i & 1u) ? &tmV : &tmK;
@@ -327,7 +327,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         float m_run = -1e30f, l_run = 0.0f;
         bool ok = true;
         for (uint32_t it = 0; it < cnt; it++) {
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&s_full[g], it & 1u, abort_flag, p.err, 226));
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&s_full[g], it & 1u, abort_flag, p.err, 226));
             if (!ok) break;
             ptx::tc_fence_after_sync();
             const uint32_t k0 = (t0 + it) * BK;
@@ -387,7 +387,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             l_run = (l_run > SUM_OF_NAN ? l_run : l_run * corr) + (a0 + a1);
         }
         // ---------------- result ----------------
-        if (cnt > 0u && ok) ok = __all_sync(0xffffffffu, ptx::mbar_wait<64>(&o_full[g], 0u, abort_flag, p.err, 227));
+        if (cnt > 0u && ok) ok = __all_sync(0xffffffffu, ptx::mbar_wait(&o_full[g], 0u, abort_flag, p.err, 227));
         if (cnt > 0u && ok) {
             ptx::tc_fence_after_sync();
             // Rows leave through the tile's Q buffer, which nothing reads any more: a thread deposits the 16-byte chunks of its

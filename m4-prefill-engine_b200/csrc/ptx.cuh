@@ -57,21 +57,24 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Bounded wait.  `abort_flag` lives in shared memory: the first waiter that runs out of time
-// sets it (and the global error word) so every other waiter of the CTA leaves at once.
-// mbarrier.try_wait itself parks the thread for a hardware-defined interval, so the loop is
-// cheap; the clock and the abort flag are looked at only every 1024 failed tries so that waiting
-// warps do not take issue slots from the warps doing the unpacking.  SLEEP_NS > 0 adds a
-// nanosleep between tries for waits that are long by construction (a whole tile).
-template <int SLEEP_NS = 0>
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
-                                          int* err_word, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
+// Bounded wait.  `abort_flag` lives in shared memory: the first waiter that runs out of time sets it (and the global error
+// word) so every other waiter of the CTA leaves at once.  The first look is all that is inlined; what follows a miss is a
+// call.  With the retry loop, the clock and the abort flag inlined behind the first look, an MMA step (four 128 x 48 x 16 MMAs,
+// one commit) whose barrier was complete already took 294 cycles, like this 136, without any wait 97: the loop's second
+// way out makes the compiler guard every wait of a divergent thread with convergence barriers.
+// mbarrier.try_wait itself parks the thread for a hardware-defined interval (about 8000 cycles), so the loop is cheap; the clock
+// and the abort flag are looked at only every 256 failed tries.
+static __device__ __noinline__ bool mbar_wait_missed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
     long long t0 = 0;
     for (uint32_t spin = 1;; ++spin) {
-        if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 1023u) == 0u) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((spin & 255u) == 0u || spin == 1u) {
             if (*abort_flag) return false;
             const long long now = clock64();
             if (t0 == 0) t0 = now;
@@ -82,6 +85,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
             }
         }
     }
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                          int* err_word, int code) {
+    if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait_missed(smem_u32(bar), parity, abort_flag, err_word, code);
 }
 
 // ---- TMA ------------------------------------------------------------------------------
@@ -181,18 +189,21 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(bar)), "r"(rank));
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(ra) : "memory");
 }
-// bounded wait on a local barrier that the other CTA of the cluster arrives on too (acquire at cluster scope)
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+// bounded wait on a local barrier that the other CTA of the cluster arrives on too (acquire at cluster scope); as mbar_wait
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+static __device__ __noinline__ bool mbar_wait_cluster_missed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
     long long t0 = 0;
-    for (uint32_t spin = 0;; ++spin) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-        if (ok) return true;
-        if ((spin & 1023u) == 1023u) {
+    for (uint32_t spin = 1;; ++spin) {
+        if (mbar_try_wait_cluster(bar, parity)) return true;
+        if ((spin & 255u) == 0u || spin == 1u) {
             if (*abort_flag) return false;
             const long long now = clock64();
             if (t0 == 0) t0 = now;
@@ -203,6 +214,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
             }
         }
     }
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+    if (mbar_try_wait_cluster(smem_u32(bar), parity)) return true;
+    return mbar_wait_cluster_missed(smem_u32(bar), parity, abort_flag, err_word, code);
 }
 
 // 32 lanes x 16 consecutive fp32 columns -> 16 registers per thread (lane i of the warp reads

@@ -565,7 +565,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             for (uint32_t kc = 0; kc < t.kcn; kc++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<64>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(0, wtr, 0);
@@ -628,7 +628,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (!ok) break;
             }
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(1, xtr, 0);
@@ -762,7 +762,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     for (int i = 0; i < MW; i++) meta[i] = meta_next[i];
                     if (kc + 1 < t.kcn) load_meta(kc + 1, meta_next);
                 }
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&raw_full[rs], rph, abort_flag, p.err, 106));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_full[rs], rph, abort_flag, p.err, 106));
                 if (!ok) break;
                 if (row == 0) QTR(3, (kn >> 2) * 2 + grp, 0);
                 // Only the words a sub-tile needs are loaded, right before it is unpacked: a group handles one or
@@ -789,7 +789,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             if (own_st >= p.a_stages) { own_st -= p.a_stages; own_ph ^= 1u; }
                         }
                         else { const uint32_t step = kn + s; as = step % STAGES; aph = (step / STAGES) & 1u; }
-                        ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait<32>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107));
+                        ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107));
                         if (row == 0) QTR(4 + grp, kn + s, 1);
                         if (ok) {
                             uint8_t* dst = sA + as * A_TILE_BYTES + row_off;
@@ -861,7 +861,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (n0 + 64u < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + 128));
                 }
             }
-            if (!ptx::mbar_wait<256>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108)) { sc_ok = false; break; }
+            if (!ptx::mbar_wait(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108)) { sc_ok = false; break; }
             if (et == 0) QTRC(6, it, 0);
             ptx::tc_fence_after_sync();
             // grouped launch: the matrix this tile belongs to decides the output buffer and its width

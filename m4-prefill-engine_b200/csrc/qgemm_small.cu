@@ -8,8 +8,10 @@
 //     elements to 32 registers of fp16 pairs and writes them with one tcgen05.st into a ring of A-operand stages in
 //     tensor memory; the MMA takes A from tensor memory (tcgen05.mma [d], [a], b-desc) and only the activations from
 //     shared memory.  That removes the 16 KB store + 16 KB operand read per 64-element step that bound the other kernel;
-//   * small CTAs (4 unpack warps = the 4 lane quadrants, a copy warp, an MMA warp; <= 112 KB of shared memory, 256
+//   * small CTAs (4 unpack warps = the 4 lane quadrants, two copy warps, an MMA warp; <= 112 KB of shared memory, 256
 //     tensor-memory columns) so that two CTAs share an SM and one's copies and unpacking overlap the other's;
+//   * weights and activations of a step share a ring stage with one full and one empty barrier (128 elements of K; 64 for Prism): a wait costs
+//     the issuing thread more than the four MMAs of 48 tokens behind it (100 cycles);
 //   * one work item per CTA: K is split up to eight ways and the splits of a tile form a thread-block cluster.  Every CTA
 //     writes its partial tile to a scratch buffer (which stays in L2), one cluster barrier later each CTA of the cluster
 //     sums one slice of the token columns in split order -- deterministic -- and writes fp16 Y: no counters, no CTA that
@@ -18,6 +20,10 @@
 //
 // Every mbarrier wait is bounded (ptx::mbar_wait).  The cluster barrier is a hardware barrier: every thread of every
 // CTA reaches it on every path, including after a wait has given up.
+//
+// What bounds it: the unpack arithmetic.  Half-precision and logic instructions issue every other cycle, Q4_0 takes 64 and 48 of them for
+// 64 weights and a warp 255 cycles; a 128 x 64 step takes an SM 281 cycles (two CTAs; 325 with 64-element stages and two barriers each), where HBM
+// would need 196.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -34,15 +40,19 @@ namespace qg {
 namespace small {
 
 constexpr int W_TILE = 128;          // weight rows per tile = UMMA M = tensor-memory lanes
-constexpr int KSTEP = 64;            // K elements per MMA group (4 MMAs of K = 16) and per A stage
-constexpr int A_STAGES = 4;          // ring of unpacked-weight stages in tensor memory, 32 columns each
-constexpr int A_COLS = KSTEP / 2;    // fp16 pairs: 32 columns per stage
-constexpr int ACC_COL = A_STAGES * A_COLS;   // accumulator behind the A ring (columns 128 ..)
-constexpr int TMEM_COLS = 256;
-constexpr int MAX_RAW_STAGES = 6, MAX_B_STAGES = 4;   // ring depths are chosen per launch (stages_for)
-constexpr int UNPACK_WARPS = 4;      // one per lane quadrant (a second group of four measured slower: 2080 against 550 cycles per sub-tile)
-constexpr int THREADS = (UNPACK_WARPS + 2) * 32;    // warps 0-3 unpack + epilogue, warp 4 copies, warp 5 issues MMAs
-constexpr int COPY_WARP = UNPACK_WARPS, MMA_WARP = UNPACK_WARPS + 1;
+constexpr int KSTEP = 64;            // K elements per sub-tile (4 MMAs of K = 16)
+constexpr int SUB_COLS = KSTEP / 2;  // fp16 pairs: 32 tensor-memory columns per sub-tile
+// Sub-tiles per operand stage: one hand-over for two of them (33 tokens, K = 14336, N = 4096 17.3 -> 15.9 us, N = 14336, K = 4096 19.4 -> 17.7), except
+// where two stages of twice the activations do not fit beside two packed stages (the 272-byte rows)
+template <int FMT> struct Ring {
+    static constexpr int SPS = cdc::Codec<FMT>::CHUNK == 256 ? 2 : 1, A_COLS = SPS * SUB_COLS;
+};
+constexpr int TMEM_COLS = 256;       // accumulator (T columns), then the A ring
+constexpr int MAX_RAW_STAGES = 6, MAX_STAGES = 7;     // ring depths are chosen per launch (stages_for)
+constexpr int UNPACK_WARPS = 4;      // one per lane quadrant (a second group shares its schedulers, whose pipes one warp of each of the two CTAs
+                                     // keeps 90 % busy: 33 tokens K = 14336 16.2 -> 16.6 us; 128 tokens, N = 14336 24.2 -> 23.5)
+constexpr int THREADS = (UNPACK_WARPS + 3) * 32;    // warps 0-3 unpack + epilogue, then packed-weight copies, activation copies, MMAs
+constexpr int RAW_WARP = UNPACK_WARPS, ACT_WARP = UNPACK_WARPS + 1, MMA_WARP = UNPACK_WARPS + 2;
 constexpr int MAX_T = 128;
 constexpr int GATE_ROWS = W_TILE / 2;    // SwiGLU tile: 64 gate rows and the same 64 up rows
 constexpr size_t SMEM_LIMIT = 112 * 1024; // two CTAs per SM
@@ -59,7 +69,7 @@ __device__ unsigned long long g_qs_trace[8][64];
 // (in the order in which a launch needs them, 64 bytes to a line of the constant cache, which is cold when a CTA starts)
 struct Params {
     uint32_t n_w_tiles, k_splits, split_shift, chunks;       // chunks: packed chunks of K; split i works on [i * chunks / k_splits, (i + 1) * chunks / k_splits); k_splits = 1 << split_shift
-    uint32_t raw_stages, b_stages, T;
+    uint32_t raw_stages, stages, T;
     uint32_t early;              // packed weights may be fetched before the preceding kernel has finished
     uint32_t x_wrap;             // K after which the activation columns start over
     uint32_t M, N, K, layout, D;
@@ -147,19 +157,17 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
     ptx::launch_dependents();     // the next kernel in the stream may set itself up while this grid runs
     const uint32_t pad = (1024u - (ptx::smem_u32(smem_dyn) & 1023u)) & 1023u;
     uint8_t* sB = smem_dyn + pad;                                   // [B_STAGES][T rows of 128 bytes], 128-byte swizzle
-    const uint32_t b_stage_bytes = p.T * 128u;
-    uint8_t* sRaw = sB + p.b_stages * b_stage_bytes;                // [raw_stages][128 rows][ROW_BYTES]
+    constexpr int SPS = Ring<FMT>::SPS, A_COLS = Ring<FMT>::A_COLS;
+    const uint32_t b_sub_bytes = p.T * 128u, b_stage_bytes = SPS * b_sub_bytes;
+    uint8_t* sRaw = sB + p.stages * b_stage_bytes;                  // [raw_stages][128 rows][ROW_BYTES]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + p.raw_stages * RAW_TILE_BYTES);
     uint64_t* raw_full = bars;
     uint64_t* raw_empty = raw_full + MAX_RAW_STAGES;
-    uint64_t* a_full = raw_empty + MAX_RAW_STAGES;
-    uint64_t* a_empty = a_full + A_STAGES;
-    uint64_t* b_full = a_empty + A_STAGES;
-    uint64_t* b_empty = b_full + MAX_B_STAGES;
-    uint64_t* acc_full = b_empty + MAX_B_STAGES;
+    uint64_t* full = raw_empty + MAX_RAW_STAGES;                    // step's weights in tensor memory (4 warps) and activations in shared memory
+    uint64_t* empty = full + MAX_STAGES;                            // ... consumed: one tcgen05.commit
+    uint64_t* acc_full = empty + MAX_STAGES;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
     volatile uint32_t* abort_flag = tmem_holder + 1;
-
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t ks = blockIdx.x & (p.k_splits - 1u);             // == rank inside the cluster
@@ -171,14 +179,13 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
     const uint32_t N = !MULTI || gi == 0u ? p.N : (gi == 1u ? p.extra_N[0] : p.extra_N[1]);
     __half* const Y = !MULTI || gi == 0u ? p.Y : (gi == 1u ? p.extra_Y[0] : p.extra_Y[1]);
     const uint32_t kc0 = (ks * p.chunks) >> p.split_shift, kcn = (((ks + 1u) * p.chunks) >> p.split_shift) - kc0;     // this split's packed chunks
-    const uint32_t ksteps = kcn * (uint32_t)SUBS;
+    const uint32_t ksteps = kcn * (uint32_t)(SUBS / SPS);
 
     if (threadIdx.x == 0) {
 #pragma unroll
         for (uint32_t i = 0; i < (uint32_t)MAX_RAW_STAGES; i++) if (i < p.raw_stages) { ptx::mbar_init(&raw_full[i], 1); ptx::mbar_init(&raw_empty[i], UNPACK_WARPS); }
-        for (int i = 0; i < A_STAGES; i++) { ptx::mbar_init(&a_full[i], 4); ptx::mbar_init(&a_empty[i], 1); }
 #pragma unroll
-        for (uint32_t i = 0; i < (uint32_t)MAX_B_STAGES; i++) if (i < p.b_stages) { ptx::mbar_init(&b_full[i], 1); ptx::mbar_init(&b_empty[i], 1); }
+        for (uint32_t i = 0; i < (uint32_t)MAX_STAGES; i++) if (i < p.stages) { ptx::mbar_init(&full[i], UNPACK_WARPS + 1); ptx::mbar_init(&empty[i], 1); }
         ptx::mbar_init(acc_full, 1);
         *abort_flag = 0u;
         ptx::fence_barrier_init();
@@ -196,26 +203,20 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
     if (!p.early) ptx::grid_dependency_wait();
     if (threadIdx.x == 0) QST(0, 2);
 
-    if (warp == COPY_WARP) {
-        // ---------------- copies: packed weight chunks run ahead of the activation tiles ----------------
-        // (the packed bytes are what the launch waits for: every chunk that has a free stage is requested before the
-        // activation tiles of the chunk in front of it)
+    const uint32_t a_col = tmem_base + p.T;                         // A ring behind the accumulator
+    if (warp == RAW_WARP) {
+        // ---------------- packed weight chunks ----------------
         const CUtensorMap* tmW = &maps.w[MULTI ? gi : 0u];
-        if (lane == 0) { ptx::prefetch_tensormap(tmW); ptx::prefetch_tensormap(&maps.x); }
-        uint32_t rs = 0, rph = 0, bs = 0, bph = 0, raw_next = 0;
+        if (lane == 0) ptx::prefetch_tensormap(tmW);
+        uint32_t rs = 0, rph = 0;
         bool ok = true;
-        auto issue_raw = [&](bool block) {       // request chunk raw_next if its stage is free (block: wait for it)
-            if (raw_next >= kcn) return;
-            // (a look that never parks: with try_wait here every activation tile behind a full packed ring was held up by
-            // about 4 us -- K = 4096, N = 14336, 33 tokens 74.6 us instead of 19.5)
-            bool free_now = ptx::mbar_test_wait(&raw_empty[rs], rph ^ 1u);
-            if (!free_now && block) free_now = ptx::mbar_wait<32>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 111);
-            free_now = __all_sync(0xffffffffu, free_now);
-            if (!free_now) { if (block) ok = false; return; }
+        for (uint32_t kc = 0; kc < kcn; kc++) {
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 111));
+            if (!ok) break;
             if (lane == 0) {
-                QST(1, raw_next);
+                QST(1, kc);
                 ptx::mbar_arrive_expect_tx(&raw_full[rs], RAW_TILE_BYTES);
-                const int x = (int)((kc0 + raw_next) * (ROW_BYTES / Cd::TMA_ELEM_BYTES));
+                const int x = (int)((kc0 + kc) * (ROW_BYTES / Cd::TMA_ELEM_BYTES));
                 if (swiglu) {          // 64-row boxes: gate rows, then the same rows of up
                     ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES, &maps.w[0], &raw_full[rs], x, (int)(wt * GATE_ROWS));
                     ptx::tma_load_2d(sRaw + rs * RAW_TILE_BYTES + GATE_ROWS * ROW_BYTES, &maps.w[MULTI ? 1 : 0], &raw_full[rs], x, (int)(wt * GATE_ROWS));
@@ -224,62 +225,58 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
                 }
             }
             __syncwarp();
-            raw_next++;
             if (++rs == p.raw_stages) { rs = 0; rph ^= 1u; }
-        };
-        for (uint32_t i = 0; i < p.raw_stages; i++) issue_raw(false);
-        if (p.early) ptx::grid_dependency_wait();
-        uint32_t x = (kc0 * (uint32_t)Cd::CHUNK) % p.x_wrap;      // column of the next activation tile (x_wrap: whole chunks)
-        for (uint32_t kc = 0; ok && kc < kcn; kc++) {
-            if (raw_next <= kc) issue_raw(true);              // the chunk these activation tiles belong to must be on its way
-            for (uint32_t s = 0; ok && s < (uint32_t)SUBS; s++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 112));
-                if (!ok) break;
-                if (lane == 0) {
-                    ptx::mbar_arrive_expect_tx(&b_full[bs], b_stage_bytes);
-                    ptx::tma_load_2d(sB + bs * b_stage_bytes, &maps.x, &b_full[bs], (int)x, (int)(tt * p.T));
-                }
-                __syncwarp();
-                x += (uint32_t)KSTEP;
-                if (x == p.x_wrap) x = 0u;
-                if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
-                issue_raw(false);                             // a packed stage may have been released meanwhile
-            }
         }
-    } else if (warp == MMA_WARP) {
-        // ---------------- MMA issuer ----------------
-        const uint32_t idesc = ptx::umma_idesc_f16(W_TILE, p.T);
-        const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
-        const uint32_t b_lo0 = (ptx::smem_u32(sB) & 0x3FFFFu) >> 4;
-        uint32_t as = 0, aph = 0, bs = 0, bph = 0;
+    } else if (warp == ACT_WARP) {
+        // ---------------- activation tiles ----------------
+        if (lane == 0) ptx::prefetch_tensormap(&maps.x);
+        if (p.early) ptx::grid_dependency_wait();
+        uint32_t st = 0, ph = 0;
         bool ok = true;
-        for (uint32_t st = 0; st < ksteps; st++) {
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&a_full[as], aph, abort_flag, p.err, 113) &&
-                                             ptx::mbar_wait(&b_full[bs], bph, abort_flag, p.err, 114));
+        uint32_t x = (kc0 * (uint32_t)Cd::CHUNK) % p.x_wrap;      // column of the next activation tile (x_wrap: whole chunks)
+        for (uint32_t k = 0; k < ksteps; k++) {
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&empty[st], ph ^ 1u, abort_flag, p.err, 112));
             if (!ok) break;
-            ptx::tc_fence_after_sync();
-            if (lane == 0) QST(2, st);
-            if (ptx::elect_one()) {
-                const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + bs * (b_stage_bytes >> 4));
-                const uint32_t acol = tmem_base + as * A_COLS;
-#pragma unroll
-                for (int kk = 0; kk < KSTEP / 16; kk++)
-                    umma_f16_ts(tmem_base + ACC_COL, acol + kk * 8, bdesc + 2 * kk, idesc, (st | (uint32_t)kk) != 0u);
-                ptx::umma_commit(&a_empty[as]);
-                ptx::umma_commit(&b_empty[bs]);
+            if (lane == 0) {
+                ptx::mbar_arrive_expect_tx(&full[st], b_stage_bytes);
+                for (int j = 0; j < SPS; j++)
+                    ptx::tma_load_2d(sB + st * b_stage_bytes + j * b_sub_bytes, &maps.x, &full[st], (int)x + j * KSTEP, (int)(tt * p.T));
             }
             __syncwarp();
-            if (++as == A_STAGES) { as = 0; aph ^= 1u; }
-            if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
+            x += (uint32_t)(SPS * KSTEP);
+            if (x == p.x_wrap) x = 0u;
+            if (++st == p.stages) { st = 0; ph ^= 1u; }
         }
-        if (ok && ptx::elect_one()) ptx::umma_commit(acc_full);
+    } else if (warp == MMA_WARP) {
+        // ---------------- MMA issuer: one thread, chosen once ----------------
+        if (ptx::elect_one()) {
+            const uint32_t idesc = ptx::umma_idesc_f16(W_TILE, p.T);
+            const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
+            const uint32_t b_lo0 = (ptx::smem_u32(sB) & 0x3FFFFu) >> 4;
+            uint32_t st = 0, ph = 0;
+            for (uint32_t k = 0; k < ksteps; k++) {
+                ptx::mbar_wait(&full[st], ph, abort_flag, p.err, 113);
+                ptx::tc_fence_after_sync();
+                QST(2, k);
+                const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + st * (b_stage_bytes >> 4));
+                const uint32_t acol = a_col + st * A_COLS;
+#pragma unroll
+                for (int j = 0; j < SPS; j++)
+#pragma unroll
+                    for (int kk = 0; kk < KSTEP / 16; kk++)
+                        umma_f16_ts(tmem_base, acol + j * SUB_COLS + kk * 8, bdesc + (uint64_t)(j * (b_sub_bytes >> 4) + 2 * kk), idesc, (k | (uint32_t)(j | kk)) != 0u);
+                ptx::umma_commit(&empty[st]);
+                if (++st == p.stages) { st = 0; ph ^= 1u; }
+            }
+            ptx::umma_commit(acc_full);
+        }
         __syncwarp();
     } else {
         // ---------------- unpack: packed bytes -> registers -> tensor memory (A operand) ----------------
         const uint32_t quad = warp & 3u;                            // lane quadrant
         const uint32_t row = quad * 32u + lane;                     // weight row of the tile = tensor-memory lane
         const uint32_t lane_base = (quad * 32u) << 16;
-        uint32_t rs = 0, rph = 0;
+        uint32_t rs = 0, rph = 0, st = 0, ph = 0;
         bool ok = true;
         for (uint32_t kc = 0; ok && kc < kcn; kc++) {
             // planar layouts: this chunk's scales and biases come straight from their planes in global memory, requested
@@ -303,7 +300,7 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
                     }
                 }
             }
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait<32>(&raw_full[rs], rph, abort_flag, p.err, 115));
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_full[rs], rph, abort_flag, p.err, 115));
             if (!ok) break;
             if (threadIdx.x == 0) QST(3, kc);
             uint32_t r[ROW_BYTES / 4];
@@ -312,20 +309,24 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
             ld_words<0, Cd::HDR_WORDS, SW>(rowp, r, xr);
             auto sub_tile = [&](auto S) {
                 constexpr int s = decltype(S)::value;
-                // step of this CTA, its stage of the A ring and the parity of that stage's use
-                const uint32_t step = kc * (uint32_t)SUBS + (uint32_t)s, as = step % A_STAGES, aph = (step / A_STAGES) & 1u;
+                constexpr int j = s % SPS;                           // place inside the stage
                 uint32_t o[32];
                 ld_words<Cd::sub_lo(s), Cd::sub_hi(s), SW>(rowp, r, xr);
                 Cd::dequant64(r, s, o, meta);
-                ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait<32>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 116));
-                if (ok) {
+                if (j == 0) {
+                    ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait(&empty[st], ph ^ 1u, abort_flag, p.err, 116));
                     ptx::tc_fence_after_sync();                      // the MMAs that read this stage have completed
-                    tmem_st_x32(tmem_base + lane_base + as * A_COLS, o);
-                    ptx::tmem_st_wait();
-                    ptx::tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&a_full[as]);
-                    if (threadIdx.x == 0) QST(4, step);
+                }
+                if (ok) tmem_st_x32(a_col + lane_base + st * A_COLS + j * SUB_COLS, o);
+                if (j == SPS - 1) {
+                    if (ok) {
+                        ptx::tmem_st_wait();
+                        ptx::tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(&full[st]);
+                    }
+                    if (threadIdx.x == 0) QST(4, kc * SUBS + s);
+                    if (++st == p.stages) { st = 0; ph ^= 1u; }
                 }
             };
             for_each_sub(sub_tile, std::make_integer_sequence<int, SUBS>{});
@@ -339,7 +340,7 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
     if (p.early) ptx::grid_dependency_wait();      // (long over; orders this thread's stores behind it)
     if (warp < 4) {
         // the accumulator is complete once every MMA has; a failed wait sets the abort flag, the barrier is still reached
-        ptx::mbar_wait<64>(acc_full, 0u, abort_flag, p.err, 117);
+        ptx::mbar_wait(acc_full, 0u, abort_flag, p.err, 117);
     }
     __syncthreads();
     if (threadIdx.x == 0) QST(0, 3);
@@ -352,17 +353,18 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
         const uint32_t n = swiglu ? wt * GATE_ROWS + (f & 63u) : wl * W_TILE + f;
         float rsc = 1.0f;
         if (Cd::ROW_SCALE) rsc = n < N ? __half2float((swiglu && f >= 64u ? p.row_scale1 : p.row_scale0)[n]) : 0.0f;
-        const uint32_t taddr = tmem_base + ((warp * 32u) << 16) + ACC_COL;
+        const uint32_t taddr = tmem_base + ((warp * 32u) << 16);
         if (p.k_splits > 1u || swiglu) {
             // [split][tile][token column][feature]: a warp's store covers 32 consecutive features of one column
             float* dst = p.scratch + ((size_t)ks * n_tiles + tile) * tile_floats + f;
-            for (uint32_t c0 = 0; c0 < p.T; c0 += 16) {
+            const uint32_t valid = min(p.T, p.M - tt * p.T);
+            for (uint32_t c0 = 0; c0 < valid; c0 += 16) {
                 uint32_t v[16];
                 ptx::tmem_ld_x16(taddr + c0, v);
                 ptx::tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 16; j++)
-                    __stcg(dst + (size_t)(c0 + j) * W_TILE, Cd::ROW_SCALE ? __uint_as_float(v[j]) * rsc : __uint_as_float(v[j]));
+                    if (c0 + j < valid) __stcg(dst + (size_t)(c0 + j) * W_TILE, Cd::ROW_SCALE ? __uint_as_float(v[j]) * rsc : __uint_as_float(v[j]));
             }
         } else {
             // no split: this CTA's accumulator is the result
@@ -394,34 +396,48 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
         const float* base = p.scratch + (size_t)tile * tile_floats + (size_t)(ks * cols) * W_TILE;
         const size_t split_stride = (size_t)n_tiles * tile_floats;
         const uint32_t tok0 = tt * p.T + ks * cols;
-        auto sum4 = [&](const float* at) {
-            float4 acc = __ldcg(reinterpret_cast<const float4*>(at));
-            for (uint32_t s = 1; s < p.k_splits; s++) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(at + s * split_stride));
-                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        // two float4 of every split at a time -- items i and i + THREADS, or (SwiGLU) the gate and the up value of one item -- four
+        // splits' loads under way together
+        auto sum4x2 = [&](const float* a, const float* b, bool both, float4& x, float4& y) {
+            x = y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (uint32_t s0 = 0; s0 < p.k_splits; s0 += 4u) {
+                float4 v[4], w[4];
+#pragma unroll
+                for (uint32_t j = 0; j < 4u; j++) {
+                    const size_t o = (s0 + j) * split_stride;
+                    v[j] = w[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (s0 + j < p.k_splits) v[j] = __ldcg(reinterpret_cast<const float4*>(a + o));
+                    if (s0 + j < p.k_splits && both) w[j] = __ldcg(reinterpret_cast<const float4*>(b + o));
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < 4u; j++) {
+                    x.x += v[j].x; x.y += v[j].y; x.z += v[j].z; x.w += v[j].w;
+                    y.x += w[j].x; y.y += w[j].y; y.z += w[j].z; y.w += w[j].w;
+                }
             }
-            return acc;
         };
-        // four features per thread; a SwiGLU tile's features 64 .. 127 are the up projections of 0 .. 63
+        // four features per item; a SwiGLU tile's features 64 .. 127 are the up projections of 0 .. 63
         const uint32_t quads = swiglu ? GATE_ROWS / 4 : W_TILE / 4, quad_shift = swiglu ? 4u : 5u;
+        const uint32_t valid = tok0 < p.M ? min(cols, p.M - tok0) : 0u, items = valid << quad_shift;
         static_assert(GATE_ROWS == 64 && W_TILE == 128, "quads per column: 16 and 32");
-        for (uint32_t i = threadIdx.x; i < cols * quads; i += THREADS) {
-            const uint32_t cl = i >> quad_shift, f = (i & (quads - 1u)) * 4u;
-            const uint32_t tok = tok0 + cl, n = swiglu ? wt * GATE_ROWS + f : wl * W_TILE + f;
-            if (tok >= p.M || n >= N) continue;
-            const float4 acc = sum4(base + (size_t)cl * W_TILE + f);
-            float a[4] = {acc.x, acc.y, acc.z, acc.w};
-            if (swiglu) {
-                const float4 u = sum4(base + (size_t)cl * W_TILE + GATE_ROWS + f);
-                a[0] = silu_mul(a[0], u.x); a[1] = silu_mul(a[1], u.y); a[2] = silu_mul(a[2], u.z); a[3] = silu_mul(a[3], u.w);
-            }
+        auto write4 = [&](uint32_t i, float4 acc) {
+            const uint32_t f = (i & (quads - 1u)) * 4u, tok = tok0 + (i >> quad_shift), n = swiglu ? wt * GATE_ROWS + f : wl * W_TILE + f;
+            const float a[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 if (n + e >= N) break;
                 const size_t o = p.layout == 1 ? ((size_t)((n + e) / p.D) * p.M + tok) * p.D + ((n + e) % p.D) : (size_t)tok * N + n + e;
-                if (p.residual) a[e] += __half2float(p.residual[o]);
-                Y[o] = __float2half_rn(a[e]);
+                Y[o] = __float2half_rn(p.residual ? a[e] + __half2float(p.residual[o]) : a[e]);
             }
+        };
+        for (uint32_t i = threadIdx.x; i < items; i += swiglu ? THREADS : 2 * THREADS) {
+            const uint32_t i2 = i + THREADS;
+            const float* at = base + (size_t)(i >> quad_shift) * W_TILE + (i & (quads - 1u)) * 4u;
+            const float* at2 = swiglu ? at + GATE_ROWS : base + (size_t)(i2 >> quad_shift) * W_TILE + (i2 & (quads - 1u)) * 4u;
+            float4 x, y;
+            sum4x2(at, at2, swiglu || i2 < items, x, y);
+            if (swiglu) write4(i, make_float4(silu_mul(x.x, y.x), silu_mul(x.y, y.y), silu_mul(x.z, y.z), silu_mul(x.w, y.w)));
+            else { write4(i, x); if (i2 < items) write4(i2, y); }
         }
     }
     // ---------------- teardown ----------------
@@ -467,20 +483,19 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, uint64_t 
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, chunks, raw_stages, b_stages; size_t smem; };
+struct Plan { uint32_t T, n_tok_tiles, n_w_tiles, k_splits, chunks, raw_stages, stages; size_t smem; };
 
 // alignment slack + activation ring + packed ring + barrier block
-template <int FMT> size_t smem_bytes(uint32_t T, uint32_t raw_stages, uint32_t b_stages) {
-    return 1024 + (size_t)b_stages * T * 128 + (size_t)raw_stages * cdc::Codec<FMT>::ROW_BYTES * W_TILE + 256;
+template <int FMT> size_t smem_bytes(uint32_t T, uint32_t raw_stages, uint32_t stages) {
+    return 1024 + (size_t)stages * T * 128 * Ring<FMT>::SPS + (size_t)raw_stages * cdc::Codec<FMT>::ROW_BYTES * W_TILE + 256;
 }
-// Packed chunks in flight cover the latency of HBM: at least three of them where two CTAs still fit an SM, the fourth
-// activation stage giving way; what is left over goes to further chunks.
-template <int FMT> void stages_for(uint32_t T, uint32_t chunks, uint32_t& raw, uint32_t& b) {
-    b = MAX_B_STAGES;
-    while (b > 2u && smem_bytes<FMT>(T, 2, b) > SMEM_LIMIT) b--;          // (the 272-byte rows at 128 tokens: two)
-    if (b > 3u && smem_bytes<FMT>(T, 3, b) > SMEM_LIMIT && smem_bytes<FMT>(T, 3, b - 1) <= SMEM_LIMIT) b--;
+// Operand stages: as many as tensor memory holds behind the accumulator
+template <int FMT> void stages_for(uint32_t T, uint32_t chunks, uint32_t& raw, uint32_t& stages) {
+    stages = (TMEM_COLS - T) / Ring<FMT>::A_COLS;
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    while (stages > 2u && smem_bytes<FMT>(T, 2, stages) > SMEM_LIMIT) stages--;          // (the 272-byte rows at 128 tokens: two)
     raw = 2;
-    while (raw < (uint32_t)MAX_RAW_STAGES && raw < chunks && smem_bytes<FMT>(T, raw + 1, b) <= SMEM_LIMIT) raw++;
+    while (raw < (uint32_t)MAX_RAW_STAGES && raw < chunks && smem_bytes<FMT>(T, raw + 1, stages) <= SMEM_LIMIT) raw++;
 }
 
 int g_sms = 0;
@@ -491,7 +506,7 @@ int sms() {
 
 template <int FMT> bool make_plan(const GemmArgs& a, Plan& pl) {
     using Cd = cdc::Codec<FMT>;
-    static_assert(1024 + 2 * MAX_T * 128 + 2 * Cd::ROW_BYTES * W_TILE + 256 <= SMEM_LIMIT, "two stages of each ring fit half an SM");
+    static_assert(1024 + 2 * MAX_T * 128 * Ring<FMT>::SPS + 2 * Cd::ROW_BYTES * W_TILE + 256 <= SMEM_LIMIT, "two stages of each ring fit half an SM");
     pl.n_tok_tiles = (a.M + MAX_T - 1) / MAX_T;
     const uint32_t per = (a.M + pl.n_tok_tiles - 1) / pl.n_tok_tiles;
     pl.T = (per + 15u) & ~15u;
@@ -512,8 +527,8 @@ template <int FMT> bool make_plan(const GemmArgs& a, Plan& pl) {
     pl.chunks = chunks;
     // at least 80 KB, so that no more than two CTAs share an SM: each holds 256 of the SM's 512 tensor-memory columns, and a
     // third CTA would sit in tcgen05.alloc until one of the others leaves
-    stages_for<FMT>(pl.T, (chunks + pl.k_splits - 1) / pl.k_splits, pl.raw_stages, pl.b_stages);
-    pl.smem = smem_bytes<FMT>(pl.T, pl.raw_stages, pl.b_stages);
+    stages_for<FMT>(pl.T, (chunks + pl.k_splits - 1) / pl.k_splits, pl.raw_stages, pl.stages);
+    pl.smem = smem_bytes<FMT>(pl.T, pl.raw_stages, pl.stages);
     if (pl.smem < 80 * 1024) pl.smem = 80 * 1024;
     return tiles * pl.k_splits <= 65535u * 8u;
 }
@@ -553,7 +568,7 @@ template <int FMT, bool MULTI> cudaError_t launch_multi(const GemmArgs& a, const
     p.n_tok_tiles = pl.n_tok_tiles; p.n_w_tiles = pl.n_w_tiles; p.k_splits = pl.k_splits; p.chunks = pl.chunks;
     p.split_shift = 0u;
     while ((1u << p.split_shift) < pl.k_splits) p.split_shift++;
-    p.raw_stages = pl.raw_stages; p.b_stages = pl.b_stages; p.early = a.early_weights ? 1u : 0u; p.swiglu = a.W1 ? 1u : 0u;
+    p.raw_stages = pl.raw_stages; p.stages = pl.stages; p.early = a.early_weights ? 1u : 0u; p.swiglu = a.W1 ? 1u : 0u;
     p.groups = 1u + a.n_extra;
     p.Y = (__half*)a.Y;
     p.tiles[0] = (a.N + W_TILE - 1) / W_TILE; p.tiles[1] = a.n_extra ? (a.N_extra[0] + W_TILE - 1) / W_TILE : 0u;
