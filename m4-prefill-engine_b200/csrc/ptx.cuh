@@ -61,19 +61,31 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 // word) so every other waiter of the CTA leaves at once.  The first look is all that is inlined; what follows a miss is a
 // call.  With the retry loop, the clock and the abort flag inlined behind the first look, an MMA step (four 128 x 48 x 16 MMAs,
 // one commit) whose barrier was complete already took 294 cycles, like this 136, without any wait 97: the loop's second
-// way out makes the compiler guard every wait of a divergent thread with convergence barriers.
+// way out makes the compiler guard every wait of a divergent thread with convergence barriers.  CALL = false keeps it all inline, for
+// kernels that have no registers to spare around a call.
 // mbarrier.try_wait itself parks the thread for a hardware-defined interval (about 8000 cycles), so the loop is cheap; the clock
-// and the abort flag are looked at only every 256 failed tries.
-static __device__ __noinline__ bool mbar_wait_missed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    long long t0 = 0;
-    for (uint32_t spin = 1;; ++spin) {
-        uint32_t ok;
+// and the abort flag are looked at only after the first and every 256th failed try.
+template <bool CLUSTER> __device__ __forceinline__ bool mbar_look(uint32_t bar, uint32_t parity) {     // CLUSTER: acquire at cluster scope
+    uint32_t ok;
+    if (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    else
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
+    return ok != 0;
+}
+template <bool CLUSTER>
+__device__ __forceinline__ bool mbar_keep_looking(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+    long long t0 = 0;
+    for (uint32_t spin = 1;; ++spin) {
+        if (mbar_look<CLUSTER>(bar, parity)) return true;
         if ((spin & 255u) == 0u || spin == 1u) {
             if (*abort_flag) return false;
             const long long now = clock64();
@@ -86,10 +98,22 @@ static __device__ __noinline__ bool mbar_wait_missed(uint32_t bar, uint32_t pari
         }
     }
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
-                                          int* err_word, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
-    return mbar_wait_missed(smem_u32(bar), parity, abort_flag, err_word, code);
+static __device__ __noinline__ bool mbar_missed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+    return mbar_keep_looking<false>(bar, parity, abort_flag, err_word, code);
+}
+static __device__ __noinline__ bool mbar_missed_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+    return mbar_keep_looking<true>(bar, parity, abort_flag, err_word, code);
+}
+template <bool CALL = true>
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+    if (mbar_look<false>(smem_u32(bar), parity)) return true;
+    return CALL ? mbar_missed(smem_u32(bar), parity, abort_flag, err_word, code) : mbar_keep_looking<false>(smem_u32(bar), parity, abort_flag, err_word, code);
+}
+// on a local barrier that the other CTA of the cluster arrives on too
+template <bool CALL = true>
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
+    if (mbar_look<true>(smem_u32(bar), parity)) return true;
+    return CALL ? mbar_missed_cluster(smem_u32(bar), parity, abort_flag, err_word, code) : mbar_keep_looking<true>(smem_u32(bar), parity, abort_flag, err_word, code);
 }
 
 // ---- TMA ------------------------------------------------------------------------------
@@ -189,37 +213,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(bar)), "r"(rank));
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(ra) : "memory");
 }
-// bounded wait on a local barrier that the other CTA of the cluster arrives on too (acquire at cluster scope); as mbar_wait
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-static __device__ __noinline__ bool mbar_wait_cluster_missed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    long long t0 = 0;
-    for (uint32_t spin = 1;; ++spin) {
-        if (mbar_try_wait_cluster(bar, parity)) return true;
-        if ((spin & 255u) == 0u || spin == 1u) {
-            if (*abort_flag) return false;
-            const long long now = clock64();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > WAIT_LIMIT_CYCLES) {
-                *abort_flag = 1u;
-                if (err_word) atomicCAS(err_word, 0, code);
-                return false;
-            }
-        }
-    }
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    if (mbar_try_wait_cluster(smem_u32(bar), parity)) return true;
-    return mbar_wait_cluster_missed(smem_u32(bar), parity, abort_flag, err_word, code);
-}
-
 // 32 lanes x 16 consecutive fp32 columns -> 16 registers per thread (lane i of the warp reads
 // TMEM lane (taddr.lane + i)).  Warp w of a CTA may only touch lanes 32*(w%4) .. +31.
 __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {

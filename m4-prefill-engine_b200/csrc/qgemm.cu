@@ -89,6 +89,9 @@ template <int FMT> struct Cfg {
     // STAGES: the parity wait on a stage's "empty" barrier is only unambiguous if the waiting group is never
     // two phases ahead, which holds when its own previous wait already implied the phase before.
     static constexpr int DQ_GROUPS = cdc::Codec<FMT>::GROUPS;
+    // Waits that miss go on in a function, except in the format whose unpacking has no registers to save around a call (variable rate, 2048 tokens,
+    // K = N = 4096 92 us with calls, 82 without).
+    static constexpr bool WAIT_CALL = FMT != QUANT_VAR_RATE_AFFINE;
     static_assert(DQ_GROUPS >= 1 && DQ_GROUPS <= STAGES, "unpack groups are bounded by the operand ring depth");
     static constexpr int CHUNK = cdc::Codec<FMT>::CHUNK;          // K elements per packed stage
     static constexpr int SUBS = CHUNK / KSTEP;                    // 64-element sub-tiles (MMA steps) per packed stage
@@ -565,7 +568,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             for (uint32_t kc = 0; kc < t.kcn; kc++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(0, wtr, 0);
@@ -628,7 +631,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (!ok) break;
             }
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(1, xtr, 0);
@@ -649,7 +652,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const uint32_t ksteps = p.chunks * (uint32_t)C::SUBS;       // (pair launches do not split K)
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&b_full[bs], bph, abort_flag, p.err, 109));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL>(&b_full[bs], bph, abort_flag, p.err, 109));
                 if (!ok) break;
                 if (lane == 0) ptx::mbar_arrive_cluster(&b_full[bs], 0u);
                 __syncwarp();
@@ -662,57 +665,49 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // operand descriptors differ between stages only in the 14-bit start-address field
         const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
         const uint32_t a_lo0 = (ptx::smem_u32(sA) & 0x3FFFFu) >> 4, b_lo0 = (ptx::smem_u32(sB) & 0x3FFFFu) >> 4;
-        uint32_t st = 0, sph = 0, bst = 0, bsph = 0, it = 0, mtr = 0;
-        (void)mtr;
-        bool ok = true;
-        for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride, it++) {
-            const uint32_t buf = it & 1u;
-            ok = __all_sync(0xffffffffu, PAIR ? ptx::mbar_wait_cluster(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103)
-                                                   : ptx::mbar_wait(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103));
-            if (!ok) break;
-            ptx::tc_fence_after_sync();
-            if (lane == 0) QTRC(2, 200u + it, 0);
-            const uint32_t ksteps = tile_of(idx).kcn * (uint32_t)C::SUBS;
-            for (uint32_t ks = 0; ks < ksteps; ks++) {
-                if (lane == 0) QTR(2, mtr, 0);
-                // (no tcgen05 fence here: the stage was written by TMA and by generic stores that were
-                // followed by fence.proxy.async; the mbarrier acquire orders them before the MMA's reads)
-                // (the vote keeps the warp converged for elect.sync even if a wait gives up)
-                if (PAIR) ok = __all_sync(0xffffffffu, ptx::mbar_wait_cluster(&a_full[st], sph, abort_flag, p.err, 104) &&
-                                                           ptx::mbar_wait_cluster(&b_full[bst], bsph, abort_flag, p.err, 105));
-                else ok = __all_sync(0xffffffffu, ptx::mbar_wait(&a_full[st], sph, abort_flag, p.err, 104) &&
-                                                      ptx::mbar_wait(&b_full[bst], bsph, abort_flag, p.err, 105));
-                if (!ok) break;
-                if (ptx::elect_one()) {
+        // One thread, chosen once, walks the loop: chosen anew for every step and with the wait's outcome voted on, a step of four 128 x 128 x 16
+        // MMAs took 328 cycles instead of 257.  After a wait that gave up the rest runs out quickly, and nothing is written.
+        if (ptx::elect_one()) {
+            uint32_t st = 0, sph = 0, bst = 0, bsph = 0, it = 0, mtr = 0;
+            (void)mtr;
+            for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride, it++) {
+                const uint32_t buf = it & 1u;
+                if (PAIR) ptx::mbar_wait_cluster<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                else ptx::mbar_wait<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                ptx::tc_fence_after_sync();
+                QTRC(2, 200u + it, 0);
+                const uint32_t ksteps = tile_of(idx).kcn * (uint32_t)C::SUBS;
+                const uint32_t dcol = tmem_base + buf * ACC_STRIDE;
+                for (uint32_t ks = 0; ks < ksteps; ks++) {
+                    QTR(2, mtr, 0);
+                    // (no tcgen05 fence here: the stage was written by TMA and by generic stores that were
+                    // followed by fence.proxy.async; the mbarrier acquire orders them before the MMA's reads)
+                    if (PAIR) {
+                        ptx::mbar_wait_cluster<C::WAIT_CALL>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait_cluster<C::WAIT_CALL>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                    } else {
+                        ptx::mbar_wait<C::WAIT_CALL>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait<C::WAIT_CALL>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                    }
                     QTR(2, mtr, 2);
                     const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + bst * (p.b_stage_bytes >> 4));
                     const uint64_t adesc = desc_hi | (uint64_t)(a_lo0 + st * (A_TILE_BYTES >> 4));
-                    const uint32_t dcol = tmem_base + buf * ACC_STRIDE;
-                    if (PAIR) {
 #pragma unroll
-                        for (int kk = 0; kk < KSTEP / 16; kk++)
-                            ptx::umma_pair_f16_ss(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, (ks | (uint32_t)kk) != 0u);
-                        ptx::umma_pair_commit(&a_empty[st]);
-                        ptx::umma_pair_commit(&b_empty[bst]);
-                    } else {
-#pragma unroll
-                        for (int kk = 0; kk < KSTEP / 16; kk++)
-                            ptx::umma_f16_ss(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, (ks | (uint32_t)kk) != 0u);
-                        ptx::umma_commit(&a_empty[st]);
-                        ptx::umma_commit(&b_empty[bst]);
+                    for (int kk = 0; kk < KSTEP / 16; kk++) {
+                        if (PAIR) ptx::umma_pair_f16_ss(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, (ks | (uint32_t)kk) != 0u);
+                        else ptx::umma_f16_ss(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, (ks | (uint32_t)kk) != 0u);
                     }
+                    if (PAIR) { ptx::umma_pair_commit(&a_empty[st]); ptx::umma_pair_commit(&b_empty[bst]); }
+                    else { ptx::umma_commit(&a_empty[st]); ptx::umma_commit(&b_empty[bst]); }
                     QTR(2, mtr, 3); mtr++;
+                    if (++st == p.a_stages) { st = 0; sph ^= 1u; }
+                    if (++bst == p.b_stages) { bst = 0; bsph ^= 1u; }
                 }
-                __syncwarp();
-                if (++st == p.a_stages) { st = 0; sph ^= 1u; }
-                if (++bst == p.b_stages) { bst = 0; bsph ^= 1u; }
-            }
-            if (ok && ptx::elect_one()) {      // same lane as the MMAs
                 if (PAIR) ptx::umma_pair_commit(&tm_full[buf]); else ptx::umma_commit(&tm_full[buf]);
                 QTRC(2, 200u + it, 1);
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else if (pre_epi && wq != 2u && uw < (uint32_t)C::DQ_WARPS) {
         // ---------------- unpack warps: packed bytes -> swizzled fp16 K-major tile ----------------
         constexpr int G = C::DQ_GROUPS;
@@ -726,8 +721,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         uint32_t rs = 0, rph = 0, kn = 0;                     // kn: running 64-element step of this CTA
         uint32_t km = 0, own_ph = 0;                          // (kn / 4) % STAGES; phase of the group's next operand stage
         uint32_t own_st = grp;                                // ... and that stage: the group's steps g, g + 3, ... use stages (g + 3 j) % a_stages
-        bool ok = true;
-        for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
+        // (after a wait that gave up the rest runs out quickly, and nothing is written)
+        for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             // META_WORDS / 2 words of scales and as many of biases per chunk: one group per 64 elements (4 words)
             // or per 32 elements (8 words); the bias plane follows the scale plane
@@ -752,7 +747,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 }
             };
             (void)load_meta; (void)meta_next;
-            for (uint32_t kc = 0; ok && kc < t.kcn; kc++) {
+            for (uint32_t kc = 0; kc < t.kcn; kc++) {
                 // scales and biases kept outside the packed rows come straight from global memory, one chunk
                 // ahead of their use so the latency hides behind the unpacking of the current chunk
                 uint32_t meta[MW] = {};
@@ -762,8 +757,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     for (int i = 0; i < MW; i++) meta[i] = meta_next[i];
                     if (kc + 1 < t.kcn) load_meta(kc + 1, meta_next);
                 }
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_full[rs], rph, abort_flag, p.err, 106));
-                if (!ok) break;
+                ptx::mbar_wait<C::WAIT_CALL>(&raw_full[rs], rph, abort_flag, p.err, 106);
                 if (row == 0) QTR(3, (kn >> 2) * 2 + grp, 0);
                 // Only the words a sub-tile needs are loaded, right before it is unpacked: a group handles one or
                 // two of a chunk's four sub-tiles, and short-lived inputs leave the registers to the 32 outputs.
@@ -789,18 +783,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             if (own_st >= p.a_stages) { own_st -= p.a_stages; own_ph ^= 1u; }
                         }
                         else { const uint32_t step = kn + s; as = step % STAGES; aph = (step / STAGES) & 1u; }
-                        ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107));
+                        ptx::mbar_wait<C::WAIT_CALL>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107);
                         if (row == 0) QTR(4 + grp, kn + s, 1);
-                        if (ok) {
-                            uint8_t* dst = sA + as * A_TILE_BYTES + row_off;
+                        uint8_t* dst = sA + as * A_TILE_BYTES + row_off;
 #pragma unroll
-                            for (int c = 0; c < 8; c++)
-                                *reinterpret_cast<uint4*>(dst + ((c ^ xr) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-                            ptx::fence_proxy_async_smem();
-                            __syncwarp();                      // every lane's stores are fenced; one arrival per warp
-                            if (lane == 0) { if (PAIR && pair_rank == 1u) ptx::mbar_arrive_cluster(&a_full[as], 0u); else ptx::mbar_arrive(&a_full[as]); }
-                            if (row == 0) QTR(4 + grp, kn + s, 2);
-                        }
+                        for (int c = 0; c < 8; c++)
+                            *reinterpret_cast<uint4*>(dst + ((c ^ xr) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+                        ptx::fence_proxy_async_smem();
+                        __syncwarp();                      // every lane's stores are fenced; one arrival per warp
+                        if (lane == 0) { if (PAIR && pair_rank == 1u) ptx::mbar_arrive_cluster(&a_full[as], 0u); else ptx::mbar_arrive(&a_full[as]); }
+                        if (row == 0) QTR(4 + grp, kn + s, 2);
                     }
                 };
                 for_each_sub(sub_tile, std::make_integer_sequence<int, C::SUBS>{});
@@ -861,7 +853,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (n0 + 64u < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + 128));
                 }
             }
-            if (!ptx::mbar_wait(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108)) { sc_ok = false; break; }
+            if (!ptx::mbar_wait<C::WAIT_CALL>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108)) { sc_ok = false; break; }
             if (et == 0) QTRC(6, it, 0);
             ptx::tc_fence_after_sync();
             // grouped launch: the matrix this tile belongs to decides the output buffer and its width

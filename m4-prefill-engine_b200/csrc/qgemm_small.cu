@@ -277,8 +277,8 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
         const uint32_t row = quad * 32u + lane;                     // weight row of the tile = tensor-memory lane
         const uint32_t lane_base = (quad * 32u) << 16;
         uint32_t rs = 0, rph = 0, st = 0, ph = 0;
-        bool ok = true;
-        for (uint32_t kc = 0; ok && kc < kcn; kc++) {
+        // (after a wait that gave up the rest runs out quickly, and nothing is written)
+        for (uint32_t kc = 0; kc < kcn; kc++) {
             // planar layouts: this chunk's scales and biases come straight from their planes in global memory, requested
             // before the wait for the packed bytes
             uint32_t meta[MW] = {};
@@ -300,8 +300,7 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
                     }
                 }
             }
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&raw_full[rs], rph, abort_flag, p.err, 115));
-            if (!ok) break;
+            ptx::mbar_wait(&raw_full[rs], rph, abort_flag, p.err, 115);
             if (threadIdx.x == 0) QST(3, kc);
             uint32_t r[ROW_BYTES / 4];
             const uint8_t* rowp = sRaw + rs * RAW_TILE_BYTES + row * ROW_BYTES;
@@ -314,17 +313,16 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
                 ld_words<Cd::sub_lo(s), Cd::sub_hi(s), SW>(rowp, r, xr);
                 Cd::dequant64(r, s, o, meta);
                 if (j == 0) {
-                    ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait(&empty[st], ph ^ 1u, abort_flag, p.err, 116));
+                    ptx::mbar_wait(&empty[st], ph ^ 1u, abort_flag, p.err, 116);
+                    __syncwarp();
                     ptx::tc_fence_after_sync();                      // the MMAs that read this stage have completed
                 }
-                if (ok) tmem_st_x32(a_col + lane_base + st * A_COLS + j * SUB_COLS, o);
+                tmem_st_x32(a_col + lane_base + st * A_COLS + j * SUB_COLS, o);
                 if (j == SPS - 1) {
-                    if (ok) {
-                        ptx::tmem_st_wait();
-                        ptx::tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(&full[st]);
-                    }
+                    ptx::tmem_st_wait();
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(&full[st]);
                     if (threadIdx.x == 0) QST(4, kc * SUBS + s);
                     if (++st == p.stages) { st = 0; ph ^= 1u; }
                 }
