@@ -114,6 +114,23 @@ CDC_HD void nib_pairs(uint32_t sp, uint32_t& lo, uint32_t& hi) {
     hi = (sp & 0x00F000F0u) | H2_64;
 }
 
+// Sixteen 2-bit codes (code t at bits 2t) -> eight fp16 pairs, each 2^k + code: a multiplication by 1 + 2^14 puts the second code of
+// every other nibble 16 bits above the first, so a pair is one mask-and-or away (magic numbers 1024, 64 and 4 by where it ends
+// up).  Per 8 codes 7.5 logic instructions and two multiplications, on pipes of their own, where shifting out every pair took 16.
+// biased[i] is that 2^k, plus one: code - 1 = out - biased.
+CDC_HD void spread_2bit(uint32_t q, uint32_t* out) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint32_t q16 = h ? q >> 16 : q;
+        const uint32_t even = (q16 & 0x0F0Fu) * 0x4001u, odd = (q16 & 0xF0F0u) * 0x4001u;
+        out[4 * h] = (even & 0x00030003u) | 0x64006400u;                // 1024 + code
+        out[4 * h + 1] = (odd & 0x00300030u) | 0x54005400u;             // 64 + code
+        out[4 * h + 2] = (even & 0x03000300u) | 0x44004400u;            // 4 + code
+        out[4 * h + 3] = ((odd >> 4) & 0x03000300u) | 0x44004400u;      // 4 + code
+    }
+}
+CDC_HD constexpr uint32_t biased_2bit(int i) { return (i & 3) == 0 ? 0x64016401u : (i & 3) == 1 ? 0x54105410u : 0x45004500u; }   // 1025, 65, 5
+
 // Traits every codec may override: META_WORDS 32-bit words of per-chunk metadata that live outside the packed
 // row (fetched from global memory by the unpack thread), ROW_SCALE when the weights are unpacked to exact small
 // integers and one fp16 scale per output row is applied to the fp32 accumulator instead.
@@ -224,13 +241,10 @@ template <> struct Codec<QUANT_TERNARY_1_58> : CodecDefaults {
             const uint32_t d2 = prmt(r[w], 0u, 0x1010u);
 #pragma unroll
             for (int u = 0; u < 2; u++) {
-                const uint32_t q = r[w + 1 + u];
+                uint32_t x[8];
+                spread_2bit(r[w + 1 + u], x);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    uint32_t t = q >> (4 * i);
-                    uint32_t x = (t & 3u) | ((t << 14) & 0x30000u) | H2_1024;
-                    out[16 * bi + 8 * u + i] = h2mul(h2sub(x, H2_1025), d2);
-                }
+                for (int i = 0; i < 8; i++) out[16 * bi + 8 * u + i] = h2mul(h2sub(x[i], biased_2bit(i)), d2);
             }
         }
     }
@@ -305,30 +319,23 @@ template <> struct Codec<QUANT_VAR_RATE_AFFINE> : CodecDefaults {
             const uint32_t bits = mode & 7u, perm = (mode >> 3) & 3u;
             uint32_t pk[16];   // source-order pairs (2i, 2i+1)
             if (bits == 3u) {
-                const uint32_t w0 = r[w], w1 = r[w + 1], w2 = r[w + 2];
-                const uint32_t v[4] = {w0 & 0xFFFFFFu, ((w0 >> 24) | (w1 << 8)) & 0xFFFFFFu,
-                                       ((w1 >> 16) | (w2 << 16)) & 0xFFFFFFu, w2 >> 8};
+                // twelve bits = four codes at a time; times 1 + 2^13 the second code of a pair lies 16 bits above the first
 #pragma unroll
-                for (int g = 0; g < 4; g++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        uint32_t t = v[g] >> (6 * i);
-                        uint32_t x = (t & 7u) | ((t << 13) & 0x70000u) | H2_1024;
-                        pk[4 * g + i] = h2fma(h2sub(x, 0x64046404u), sc2, bs2);      // q - 4
-                    }
+                for (int g = 0; g < 8; g++) {
+                    const int bit = 12 * g, at = w + bit / 32, sh = bit % 32;
+                    const uint32_t t = sh <= 20 ? r[at] >> sh : (r[at] >> sh) | (r[at + 1] << ((32 - sh) & 31));
+                    const uint32_t x = (t & 0xFFFu) * 0x2001u;
+                    pk[2 * g] = h2fma(h2sub((x & 0x00070007u) | H2_1024, 0x64046404u), sc2, bs2);                  // 1024 + q; q - 4
+                    pk[2 * g + 1] = h2fma(h2sub((x & 0x01C001C0u) | 0x4C004C00u, 0x4D004D00u), sc2, bs2);          // 16 + q
+                }
             } else if (bits == 5u) {
+                // ten bits = two codes at a time; times 1 + 2^11 the second lies 16 bits above the first
 #pragma unroll
-                for (int g = 0; g < 4; g++) {
-                    // 40-bit group g starts at bit 40g of the 20-byte run = bit 8g of word g
-                    const uint32_t a = r[w + g], b = r[w + g + 1];
-                    const uint64_t v = (g == 0) ? ((uint64_t)a | ((uint64_t)(b & 0xFFu) << 32))
-                                                : (((((uint64_t)b << 32) | a) >> (8 * g)) & 0xFFFFFFFFFFull);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        uint32_t t = (uint32_t)(v >> (10 * i));
-                        uint32_t x = (t & 31u) | ((t << 11) & 0x1F0000u) | H2_1024;
-                        pk[4 * g + i] = h2fma(h2sub(x, 0x64106410u), sc2, bs2);      // q - 16
-                    }
+                for (int g = 0; g < 16; g++) {
+                    const int bit = 10 * g, at = w + bit / 32, sh = bit % 32;
+                    const uint32_t t = sh <= 22 ? r[at] >> sh : (r[at] >> sh) | (r[at + 1] << ((32 - sh) & 31));
+                    const uint32_t x = (t & 0x3FFu) * 0x801u;
+                    pk[g] = h2fma(h2sub((x & 0x001F001Fu) | H2_1024, 0x64106410u), sc2, bs2);                      // q - 16
                 }
             } else {
 #pragma unroll
@@ -429,13 +436,10 @@ template <> struct Codec<QUANT_TERNARY_ROW> : CodecDefaults {
     CDC_HD static void dequant64(const uint32_t* r, int s, uint32_t* out, const uint32_t* = nullptr) {
 #pragma unroll
         for (int wi = 0; wi < 4; wi++) {
-            const uint32_t q = r[4 * s + wi];
+            uint32_t x[8];
+            spread_2bit(r[4 * s + wi], x);
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t t = q >> (4 * i);
-                const uint32_t x = (t & 3u) | ((t << 14) & 0x30000u) | H2_1024;
-                out[8 * wi + i] = h2sub(x, H2_1025);
-            }
+            for (int i = 0; i < 8; i++) out[8 * wi + i] = h2sub(x[i], biased_2bit(i));
         }
     }
 };
@@ -461,13 +465,10 @@ template <> struct Codec<QUANT_PRISM_Q2_0> : CodecDefaults {
 #pragma unroll
         for (int wi = 0; wi < 4; wi++) {
             // 16 codes of elements 16wi .. 16wi+15 of the sub-tile
-            const uint32_t q = (c0 & 2) ? prmt(r[w0 + wi], r[w0 + wi + 1], 0x5432u) : r[w0 + wi];
+            uint32_t x[8];
+            spread_2bit((c0 & 2) ? prmt(r[w0 + wi], r[w0 + wi + 1], 0x5432u) : r[w0 + wi], x);
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t t = q >> (4 * i);
-                const uint32_t x = (t & 3u) | ((t << 14) & 0x30000u) | H2_1024;
-                out[8 * wi + i] = h2mul(h2sub(x, H2_1025), d2);
-            }
+            for (int i = 0; i < 8; i++) out[8 * wi + i] = h2mul(h2sub(x[i], biased_2bit(i)), d2);
         }
     }
 };
