@@ -10,21 +10,24 @@
 // K or V tile is fetched twice for the same positions.
 //
 //   warps 0-3, 4-7   softmax of tile 0 / tile 1: thread = query row = tensor-memory lane.  Scores come out of tensor
-//                    memory, P = 2^(s - m) goes back as fp16 over the front half of the same columns, from where
+//                    memory, P = 2^(s - m) goes back as fp16 into columns of its own, from where
 //                    tcgen05.mma takes it as its A operand: P never passes through shared memory, a row's maximum and sum
 //                    need no shuffle, no exchange and no CTA barrier.
-//   warp 8           issues every MMA: O0 += P0.V(kt), S0 = Q0.K(kt+1)^T, O1 += P1.V(kt), S1 = Q1.K(kt+1)^T.  While one
-//                    tile's MMAs run the other tile's softmax has the exponential unit to itself.
-//   warp 9           TMA: the Q tiles, then K(kt), V(kt), K(kt+1), ... through one ring of slots.
+//   warp 8           S(it) = Q.K(it)^T of both tiles; for 64-wide heads also O += P(it).V(it)
+//   warp 10          O += P(it).V(it) for 128-wide heads
+//   warp 9           TMA: the Q tiles, then K(0), K(1), V(0), K(2), V(1), ... through one ring of slots.
 //
-//   tensor memory    S0 / P0 columns 0..127, S1 / P1 128..255, O0 and O1 behind them (2 D columns).  S(kt+1) may overwrite
-//                    P(kt) because MMAs of one thread run in the order they are issued; the completion of S(kt+1) that a
-//                    softmax warp waits for therefore also covers PV(kt), so O is stable whenever that warp rescales it.
+//   tensor memory    S0, S1, then P0, P1, O0 and O1 in the last 2 D columns.  A softmax warp frees its scores as soon as they are in
+//                    registers (s_free), and the next step's are computed while it is at the exponentials; P is written, and O rescaled, once the
+//                    PV of the step before has completed (pv_done).  Both fit beside each other with steps of 64 keys for 128-wide heads, of 128 for
+//                    64-wide.  (With P over the front half of its scores, S(it + 1) waits for PV(it): a step of 128 keys then is softmax plus MMAs of one tile,
+//                    1520 + 1600 cycles, while the other tile has its turn.  32 / 8 heads of 128 over 2048 tokens, fp16, 37.7 -> 34.1 us; 32 heads of 64
+//                    37.0 -> 32.1; one token behind 8192 25.2 -> 23.1.)
 //
-// What bounds it: 2048 query tokens behind 8000 cached ones run at 1.0 PFLOP/s, the tensor pipe about 80 % busy (the score MMAs
-// read both operands from shared memory, 128 bytes per clock, which is all there is); short causal prompts at 0.8, where a
-// CTA's set-up and its first and last step overlap with nothing.  Sixteen softmax warps, two threads per row, measured no
-// faster (the two of a row exchange their maximum): 41.3 against 40.0 us at the 8B prefill shape.
+// What bounds it: 64-wide heads the softmax, two warps a scheduler at 2850 cycles per step of 128 keys and two tiles, of which the exponential
+// unit needs 1536; 128-wide heads the MMAs of 64 keys (1280 cycles, score MMAs of 64 columns read their Q operand from shared memory for 48 cycles each) and
+// the hand-overs between them, 1500.  A thread per MMA chain of one tile (41.9 -> 47.8 us), two threads per row (32.1 -> 33.4), P handed over in halves over
+// its scores (37.9 -> 37.5) were no better.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, stops issuing work, lets its copies land and leaves.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -43,19 +46,31 @@
 namespace attn {
 namespace ws {
 
-constexpr int ROWS = 128, BK = 128;                      // query rows of a tile, keys of a step
-constexpr int SOFTMAX_THREADS = 256, THREADS = SOFTMAX_THREADS + 64;
-constexpr int ATOM = 128 * 128;                          // bytes of [128 rows][64 fp16] in the 128-byte-swizzled layout
+constexpr int ROWS = 128;                                // query rows of a tile
+constexpr int SOFTMAX_THREADS = 256;
+constexpr int ATOM = 128 * 128;                          // bytes of [128 query rows][64 fp16] in the 128-byte-swizzled layout
 constexpr int MAX_SPLITS = 32;
 
+// keys of a step: as many as tensor memory has columns for beside the two accumulators
+__host__ __device__ constexpr uint32_t step_keys(uint32_t d) { return d == 128u ? 64u : 128u; }
 template <int D> struct Cfg {
+    static constexpr int BK = (int)step_keys(D);
+    // Score and value MMAs from a thread each, so that neither's waits leave the tensor pipe idle (128-wide heads, 32 / 8 over 2048 tokens, fp16 36.4 -> 35.1 us,
+    // 2048 behind 8192 274 -> 265), or from one in an order that keeps the tiles half a step apart where the softmax takes longer than the MMAs
+    // (64-wide, 32 heads, 2048 tokens 31.3 against 33.9).
+    static constexpr bool TWO = D == 128;
+    static constexpr int THREADS = SOFTMAX_THREADS + (TWO ? 96 : 64);
     static constexpr int ATOMS = D / 64;
-    static constexpr int TILE = ATOMS * ATOM;
-    static constexpr int SLOTS = D == 128 ? 5 : 6;       // K and V tiles in flight
-    static constexpr size_t USED = 1024 + (size_t)(2 + SLOTS) * TILE + 256;
+    static constexpr int TILE = ATOMS * ATOM;            // a query tile
+    static constexpr int KV_ATOM = BK * 128, KV_TILE = ATOMS * KV_ATOM;      // a K or V tile: [BK keys][64 fp16] twice or once
+    static constexpr int SLOTS = D == 128 ? 9 : 6;       // K and V tiles in flight
+    static constexpr size_t USED = 1024 + (size_t)2 * TILE + (size_t)SLOTS * KV_TILE + 512;
     // At least 160 KB: the CTA holds all 512 tensor-memory columns, so no CTA of a neighbouring kernel that also holds some
     // (the projection kernels, 80 KB and more) may share its SM.
     static constexpr size_t SMEM = USED < 160 * 1024 ? 160 * 1024 : USED;
+    // tensor-memory columns: scores of both tiles, probabilities (fp16 pairs) of both, accumulators of both
+    static constexpr uint32_t COL_S = 0, COL_P = 2 * BK, COL_O = 512 - 2 * D;
+    static_assert(3 * BK <= 512 - 2 * D, "scores, probabilities and accumulators fit tensor memory");
 };
 
 struct Params {
@@ -70,9 +85,9 @@ struct Params {
 };
 
 // key tiles that the rows at positions [p, p + BP) of this call attend
-__device__ __forceinline__ uint32_t key_tiles(uint32_t p, uint32_t BP, uint32_t M, uint32_t Mkv, uint32_t pos0) {
+template <int D> __device__ __forceinline__ uint32_t key_tiles(uint32_t p, uint32_t BP, uint32_t M, uint32_t Mkv, uint32_t pos0) {
     if (p >= M) return 0u;
-    return min(pos0 + min(p + BP, M) - 1u, Mkv - 1u) / (uint32_t)BK + 1u;
+    return min(pos0 + min(p + BP, M) - 1u, Mkv - 1u) / step_keys(D) + 1u;
 }
 
 __device__ __forceinline__ float ex2(float x) {           // 2^x, one instruction on the special-function unit; ex2(-inf) = 0
@@ -123,10 +138,12 @@ template <int DEG> __device__ __forceinline__ void ex2_poly2(float x0, float x1,
     e0 = __int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23));
     e1 = __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23));
 }
-// Two pairs of eight: what the special-function unit and the issue slots of the softmax warps can both take: whole calls from Q8_0
-// caches, 32 heads of 64 over 2048 tokens (degree 6) none 45.9 us, one 44.9, two 43.4, three 45.9; 8B prefill (degree 5) 44.2 /
-// 43.6 / 41.5 / 43.8.
-__device__ constexpr bool poly_pair(int j) { return (j & 3) == 1; }
+// How many pairs of eight, by what bounds the step.  64-wide heads, whose softmax follows the maximum exactly (32 heads, 2048 tokens, fp16): none 32.7 us, one
+// 32.2, two 31.3, three 33.4.  128-wide heads with the lag (32 / 8 heads, 2048 tokens): none 35.5, one 35.5, two 35.1, three 33.3; without it (24 / 8
+// heads, 1024 tokens): none 22.0, one 22.5, two 22.7.
+template <int D, bool LAG> __device__ constexpr bool poly_pair(int j) {
+    return D == 64 ? (j & 3) == 1 : LAG && ((j & 7) == 1 || (j & 7) == 4 || (j & 7) == 6);
+}
 
 __device__ __forceinline__ void tmem_ld_x32(uint32_t taddr, float* r) {
     uint32_t v[32];
@@ -168,18 +185,20 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 
 // LAG: the reference maximum lags (see below) and the polynomial share of the exponentials is the short one
 template <int D, bool LAG>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
 attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                const Params p) {
     using C = Cfg<D>;
+    constexpr int BK = C::BK;
     extern __shared__ uint8_t smem_raw_[];
     uint8_t* sQ = smem_raw_ + ((1024u - (ptx::smem_u32(smem_raw_) & 1023u)) & 1023u);    // [2 tiles]
     uint8_t* sKV = sQ + 2 * C::TILE;                                                      // [SLOTS]
-    uint64_t* q_full = reinterpret_cast<uint64_t*>(sKV + C::SLOTS * C::TILE);             // [2] query tile landed
-    uint64_t* s_full = q_full + 2;                        // [2] scores of the step complete (and with them the PV before it)
-    uint64_t* p_full = s_full + 2;                        // [2] probabilities written, O rescaled: one arrival per softmax warp
-    uint64_t* o_full = p_full + 2;                        // [2] last PV of the tile complete
-    uint64_t* kv_full = o_full + 2;                       // [SLOTS]
+    uint64_t* q_full = reinterpret_cast<uint64_t*>(sKV + C::SLOTS * C::KV_TILE);          // [2] query tile landed
+    uint64_t* s_full = q_full + 2;                        // [2] scores of the step complete
+    uint64_t* s_free = s_full + 2;                        // [2] ... and in registers: one arrival per softmax warp
+    uint64_t* p_full = s_free + 2;                        // [2] probabilities written, O rescaled: one arrival per softmax warp
+    uint64_t* pv_done = p_full + 2;                       // [2] O holds the step, the probabilities have been read
+    uint64_t* kv_full = pv_done + 2;                      // [SLOTS]
     uint64_t* kv_empty = kv_full + C::SLOTS;              // [SLOTS]
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(kv_empty + C::SLOTS);
     volatile uint32_t* abort_flag = tmem_holder + 1;
@@ -192,7 +211,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // steps of tile g inside this split
     auto steps_of = [&](uint32_t g) {
         if (g >= p.tiles) return 0u;
-        const uint32_t n = key_tiles(p0 + g * p.BP, p.BP, p.M, p.Mkv, p.pos0);
+        const uint32_t n = key_tiles<D>(p0 + g * p.BP, p.BP, p.M, p.Mkv, p.pos0);
         return n > t0 ? min(n - t0, p.tiles_per_split) : 0u;
     };
     const uint32_t cnt0 = steps_of(0u), cnt1 = steps_of(1u);
@@ -200,7 +219,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     if (n_steps == 0u) return;                            // this split lies behind the block's last key tile
 
     if (tid == SOFTMAX_THREADS + 32) {
-        for (int i = 0; i < 2; i++) { ptx::mbar_init(&q_full[i], 1); ptx::mbar_init(&s_full[i], 1); ptx::mbar_init(&p_full[i], 4); ptx::mbar_init(&o_full[i], 1); }
+        for (int i = 0; i < 2; i++) { ptx::mbar_init(&q_full[i], 1); ptx::mbar_init(&s_full[i], 1); ptx::mbar_init(&s_free[i], 4); ptx::mbar_init(&p_full[i], 4); ptx::mbar_init(&pv_done[i], 1); }
         for (int i = 0; i < C::SLOTS; i++) { ptx::mbar_init(&kv_full[i], 1); ptx::mbar_init(&kv_empty[i], 1); }
         *abort_flag = 0u;
         ptx::fence_barrier_init();
@@ -212,108 +231,168 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     __syncthreads();
     ptx::tc_fence_after_sync();
     const uint32_t tmem = *tmem_holder;
-    const uint32_t tO = tmem + 256u;
     // everything above touched only this CTA's shared and tensor memory; global memory is first touched below
     ptx::grid_dependency_wait();
     ptx::launch_dependents();
 
     if (warp == 9) {
-        // ---------------- copies ----------------
-        if (lane == 0) {
-            const uint32_t q_bytes = p.BP * p.G * 128u * (uint32_t)C::ATOMS;     // rows BP * G .. 127 of a tile stay unwritten: no output reads them
-            for (uint32_t g = 0; g < 2u; g++) {
-                if ((g ? cnt1 : cnt0) == 0u) continue;
-                ptx::mbar_arrive_expect_tx(&q_full[g], q_bytes);
-                for (int a = 0; a < C::ATOMS; a++)
-                    ptx::tma_load_3d(sQ + g * C::TILE + a * ATOM, &tmQ, &q_full[g], a * 64, (int)(p0 + g * p.BP), (int)(hk * p.G));
-            }
-        }
-        __syncwarp();
+        // ---------------- copies: Q0, K(0), Q1, K(1), V(0), K(2), V(1), ... ----------------
+        const uint32_t q_bytes = p.BP * p.G * 128u * (uint32_t)C::ATOMS;     // rows BP * G .. 127 of a tile stay unwritten: no output reads them
+        auto load_q = [&](uint32_t g) {
+            if (lane != 0u || (g ? cnt1 : cnt0) == 0u) return;
+            ptx::mbar_arrive_expect_tx(&q_full[g], q_bytes);
+            for (int a = 0; a < C::ATOMS; a++)
+                ptx::tma_load_3d(sQ + g * C::TILE + a * ATOM, &tmQ, &q_full[g], a * 64, (int)(p0 + g * p.BP), (int)(hk * p.G));
+        };
+        load_q(0u);
         uint32_t slot = 0, ph = 0;
         bool ok = true;
         for (uint32_t i = 0; ok && i < 2u * n_steps; i++) {
             ok = __all_sync(0xffffffffu, ptx::mbar_wait(&kv_empty[slot], ph ^ 1u, abort_flag, p.err, 220));
             if (!ok) break;
+            // i = 0: K(0); odd: the next K, or the last V; even: the V two steps behind it
+            const bool is_k = i == 0u || ((i & 1u) && i + 1u < 2u * n_steps);
+            const uint32_t step = i == 0u ? 0u : is_k ? (i + 1u) >> 1 : (i - 1u) >> 1;
             if (lane == 0) {
-                const CUtensorMap* map = (i & 1u) ? &tmV : &tmK;
-                ptx::mbar_arrive_expect_tx(&kv_full[slot], C::TILE);
+                ptx::mbar_arrive_expect_tx(&kv_full[slot], C::KV_TILE);
                 for (int a = 0; a < C::ATOMS; a++)
-                    ptx::tma_load_3d(sKV + slot * C::TILE + a * ATOM, map, &kv_full[slot], a * 64, (int)((t0 + (i >> 1)) * BK), (int)hk);
+                    ptx::tma_load_3d(sKV + slot * C::KV_TILE + a * C::KV_ATOM, is_k ? &tmK : &tmV, &kv_full[slot], a * 64, (int)((t0 + step) * BK), (int)hk);
             }
+            if (i == 0u) load_q(1u);
             __syncwarp();
             if (++slot == (uint32_t)C::SLOTS) { slot = 0; ph ^= 1u; }
         }
-    } else if (warp == 8) {
-        // ---------------- MMAs ----------------
-        const uint32_t idesc_s = ptx::umma_idesc_f16(128, 128);
-        const uint32_t idesc_pv = ptx::umma_idesc_f16(128, D) | (1u << 16);       // B (= V) MN-major
-        const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
-        // V [key][d]: the 64 d of an atom row are the contiguous run, the second atom lies ATOM bytes further (leading byte
-        // offset), groups of eight keys are 1024 bytes apart (stride byte offset); 16 keys further = 2048 bytes
-        const uint64_t vdesc_hi = ((uint64_t)(ATOM >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-        const uint32_t q_lo = (ptx::smem_u32(sQ) & 0x3FFFFu) >> 4, kv_lo = (ptx::smem_u32(sKV) & 0x3FFFFu) >> 4;
-        auto issue_s = [&](uint32_t g, uint32_t slot) {
-            const uint64_t qd = desc_hi | (uint64_t)(q_lo + g * (C::TILE >> 4)), kd = desc_hi | (uint64_t)(kv_lo + slot * (C::TILE >> 4));
+    } else if (C::TWO && warp == 8) {
+        // ---------------- scores: one thread, chosen once ----------------
+        // The scores of a step are computed while the softmax of the step before is under way (it has moved its scores to registers), so they
+        // are there when it ends.
+        if (ptx::elect_one()) {
+            const uint32_t idesc = ptx::umma_idesc_f16(128, BK);
+            const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
+            const uint32_t q_lo = (ptx::smem_u32(sQ) & 0x3FFFFu) >> 4, kv_lo = (ptx::smem_u32(sKV) & 0x3FFFFu) >> 4;
+            uint32_t slot = 0, ph = 0;                        // K(0), K(1), K(2), ... are copies 0, 1, 3, 5, ...
+            for (uint32_t it = 0; it < n_steps; it++) {
+                // (after a wait that gave up the rest runs out quickly, and nothing is written)
+                ptx::mbar_wait(&kv_full[slot], ph, abort_flag, p.err, 221);
 #pragma unroll
-            for (int a = 0; a < C::ATOMS; a++)
+                for (uint32_t g = 0; g < 2u; g++) {
+                    if (it >= (g ? cnt1 : cnt0)) continue;
+                    if (it == 0u) ptx::mbar_wait(&q_full[g], 0u, abort_flag, p.err, 222);
+                    else ptx::mbar_wait(&s_free[g], (it - 1u) & 1u, abort_flag, p.err, 225);
+                    ptx::tc_fence_after_sync();
+                    const uint64_t qd = desc_hi | (uint64_t)(q_lo + g * (C::TILE >> 4)), kd = desc_hi | (uint64_t)(kv_lo + slot * (C::KV_TILE >> 4));
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++)
-                    ptx::umma_f16_ss(tmem + g * 128u, qd + a * (ATOM >> 4) + 2 * kk, kd + a * (ATOM >> 4) + 2 * kk, idesc_s, (uint32_t)(a | kk) != 0u);
-            ptx::umma_commit(&s_full[g]);
-        };
-        auto issue_pv = [&](uint32_t g, uint32_t slot, bool first) {
-            const uint64_t vd = vdesc_hi | (uint64_t)(kv_lo + slot * (C::TILE >> 4));
+                    for (int a = 0; a < C::ATOMS; a++)
 #pragma unroll
-            for (int s = 0; s < BK / 16; s++)
-                umma_f16_ts(tO + g * (uint32_t)D, tmem + g * 128u + s * 8u, vd + s * (2048 >> 4), idesc_pv, (first ? 0u : 1u) | (uint32_t)(s != 0));
-        };
-        uint32_t slot = 0, ph = 0;                        // next slot of the ring to be consumed, and its parity
-        auto next_slot = [&]() { if (++slot == (uint32_t)C::SLOTS) { slot = 0; ph ^= 1u; } };
-        auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
-            const bool r = __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag, p.err, code));
-            ptx::tc_fence_after_sync();
-            return r;
-        };
-        bool ok = wait(&kv_full[0], 0u, 221);
-        for (uint32_t g = 0; g < 2u && ok; g++) {
-            if ((g ? cnt1 : cnt0) == 0u) continue;
-            ok = wait(&q_full[g], 0u, 222);
-            if (ok && ptx::elect_one()) issue_s(g, 0u);
-            __syncwarp();
+                        for (int kk = 0; kk < 4; kk++)
+                            ptx::umma_f16_ss(tmem + C::COL_S + g * BK, qd + a * (ATOM >> 4) + 2 * kk, kd + a * (C::KV_ATOM >> 4) + 2 * kk, idesc, (uint32_t)(a | kk) != 0u);
+                    ptx::umma_commit(&s_full[g]);
+                }
+                ptx::umma_commit(&kv_empty[slot]);
+                slot += it == 0u ? 1u : 2u;
+                if (slot >= (uint32_t)C::SLOTS) { slot -= C::SLOTS; ph ^= 1u; }
+            }
         }
-        if (ok && ptx::elect_one()) ptx::umma_commit(&kv_empty[0]);
         __syncwarp();
-        next_slot();
-        for (uint32_t it = 0; ok && it < n_steps; it++) {
-            const uint32_t v_slot = slot, v_ph = ph;
-            next_slot();
-            const uint32_t k_slot = slot, k_ph = ph;      // K of the next step
-            const bool more = it + 1u < n_steps;
-            if (more) next_slot();
-            ok = wait(&kv_full[v_slot], v_ph, 223);
+    } else if (C::TWO && warp == 10) {
+        // ---------------- values: another thread, so that neither's waits leave the tensor pipe idle ----------------
+        if (ptx::elect_one()) {
+            const uint32_t idesc = ptx::umma_idesc_f16(128, D) | (1u << 16);          // B (= V) MN-major
+            // V [key][d]: the 64 d of an atom row are the contiguous run, the second atom lies KV_ATOM bytes further (leading byte
+            // offset), groups of eight keys are 1024 bytes apart (stride byte offset); 16 keys further = 2048 bytes
+            const uint64_t vdesc_hi = ((uint64_t)(C::KV_ATOM >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+            const uint32_t kv_lo = (ptx::smem_u32(sKV) & 0x3FFFFu) >> 4;
+            uint32_t slot = n_steps > 1u ? 2u : 1u, ph = 0;   // V(0), V(1), ... are copies 2, 4, ..., and the last one the copy behind its predecessor
+            for (uint32_t it = 0; it < n_steps; it++) {
+                ptx::mbar_wait(&kv_full[slot], ph, abort_flag, p.err, 223);
+                const uint64_t vd = vdesc_hi | (uint64_t)(kv_lo + slot * (C::KV_TILE >> 4));
+#pragma unroll
+                for (uint32_t g = 0; g < 2u; g++) {
+                    if (it >= (g ? cnt1 : cnt0)) continue;
+                    ptx::mbar_wait(&p_full[g], it & 1u, abort_flag, p.err, 224);
+                    ptx::tc_fence_after_sync();
+#pragma unroll
+                    for (int s = 0; s < BK / 16; s++)
+                        umma_f16_ts(tmem + C::COL_O + g * D, tmem + C::COL_P + g * (BK / 2) + s * 8, vd + s * (2048 >> 4), idesc, (it | (uint32_t)s) != 0u);
+                    ptx::umma_commit(&pv_done[g]);
+                }
+                ptx::umma_commit(&kv_empty[slot]);
+                slot += it + 2u < n_steps ? 2u : 1u;
+                if (slot >= (uint32_t)C::SLOTS) { slot -= C::SLOTS; ph ^= 1u; }
+            }
+        }
+        __syncwarp();
+    } else if (!C::TWO && warp == 8) {
+        // ---------------- MMAs: one thread, chosen once ----------------
+        // Tile 0 is half a step ahead of tile 1: S0(it + 1), P1(it - 1).V, S1(it + 1), P0(it).V.  The scores of a step are computed while the softmax
+        // of the step before is under way (it has moved its scores to registers), so they are there when it ends.
+        if (ptx::elect_one()) {
+            const uint32_t idesc_s = ptx::umma_idesc_f16(128, BK);
+            const uint32_t idesc_pv = ptx::umma_idesc_f16(128, D) | (1u << 16);       // B (= V) MN-major
+            const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
+            // V [key][d]: the 64 d of an atom row are the contiguous run, the second atom lies KV_ATOM bytes further (leading byte
+            // offset), groups of eight keys are 1024 bytes apart (stride byte offset); 16 keys further = 2048 bytes
+            const uint64_t vdesc_hi = ((uint64_t)(C::KV_ATOM >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+            const uint32_t q_lo = (ptx::smem_u32(sQ) & 0x3FFFFu) >> 4, kv_lo = (ptx::smem_u32(sKV) & 0x3FFFFu) >> 4;
+            // (after a wait that gave up the rest runs out quickly, and nothing is written)
+            auto scores = [&](uint32_t g, uint32_t slot) {
+                const uint64_t qd = desc_hi | (uint64_t)(q_lo + g * (C::TILE >> 4)), kd = desc_hi | (uint64_t)(kv_lo + slot * (C::KV_TILE >> 4));
+#pragma unroll
+                for (int a = 0; a < C::ATOMS; a++)
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)
+                        ptx::umma_f16_ss(tmem + C::COL_S + g * BK, qd + a * (ATOM >> 4) + 2 * kk, kd + a * (C::KV_ATOM >> 4) + 2 * kk, idesc_s, (uint32_t)(a | kk) != 0u);
+                ptx::umma_commit(&s_full[g]);
+            };
+            auto values = [&](uint32_t g, uint32_t slot, uint32_t it) {
+                ptx::mbar_wait(&p_full[g], it & 1u, abort_flag, p.err, 224);
+                ptx::tc_fence_after_sync();
+                const uint64_t vd = vdesc_hi | (uint64_t)(kv_lo + slot * (C::KV_TILE >> 4));
+#pragma unroll
+                for (int s = 0; s < BK / 16; s++)
+                    umma_f16_ts(tmem + C::COL_O + g * D, tmem + C::COL_P + g * (BK / 2) + s * 8, vd + s * (2048 >> 4), idesc_pv, (it | (uint32_t)s) != 0u);
+                ptx::umma_commit(&pv_done[g]);
+            };
+            uint32_t slot = 0, ph = 0;                        // next slot of the ring, and its parity
+            auto take_slot = [&](int code) {
+                ptx::mbar_wait(&kv_full[slot], ph, abort_flag, p.err, code);
+                const uint32_t r = slot;
+                if (++slot == (uint32_t)C::SLOTS) { slot = 0; ph ^= 1u; }
+                return r;
+            };
+            uint32_t k_slot = take_slot(221), v_slot = 0u, v_before = 0u;
 #pragma unroll
             for (uint32_t g = 0; g < 2u; g++) {
-                const uint32_t cnt = g ? cnt1 : cnt0;
-                if (ok && it < cnt) {
-                    ok = wait(&p_full[g], it & 1u, 224);
-                    if (ok && ptx::elect_one()) {
-                        issue_pv(g, v_slot, it == 0u);
-                        if (it + 1u == cnt) ptx::umma_commit(&o_full[g]);
-                    }
-                    __syncwarp();
-                }
-                if (g == 1u && ok && ptx::elect_one()) ptx::umma_commit(&kv_empty[v_slot]);
-                __syncwarp();
-                if (ok && it + 1u < cnt) {
-                    ok = wait(&kv_full[k_slot], k_ph, 225);
-                    if (ok && ptx::elect_one()) issue_s(g, k_slot);
-                    __syncwarp();
-                }
+                if ((g ? cnt1 : cnt0) == 0u) continue;
+                ptx::mbar_wait(&q_full[g], 0u, abort_flag, p.err, 222);
+                scores(g, k_slot);
             }
-            if (more && ok && ptx::elect_one()) ptx::umma_commit(&kv_empty[k_slot]);
-            __syncwarp();
+            ptx::umma_commit(&kv_empty[k_slot]);
+            for (uint32_t it = 0; it <= n_steps; it++) {
+                const bool more = it + 1u < n_steps;
+                if (more) k_slot = take_slot(225);
+                if (it + 1u < cnt0) {
+                    ptx::mbar_wait(&s_free[0], it & 1u, abort_flag, p.err, 228);
+                    ptx::tc_fence_after_sync();
+                    scores(0u, k_slot);
+                }
+                if (it > 0u) {
+                    if (it - 1u < cnt1) values(1u, v_before, it - 1u);
+                    ptx::umma_commit(&kv_empty[v_before]);
+                }
+                if (it + 1u < cnt1) {
+                    ptx::mbar_wait(&s_free[1], it & 1u, abort_flag, p.err, 229);
+                    ptx::tc_fence_after_sync();
+                    scores(1u, k_slot);
+                }
+                if (more) ptx::umma_commit(&kv_empty[k_slot]);
+                if (it < n_steps) v_slot = take_slot(223);
+                if (it < cnt0) values(0u, v_slot, it);
+                v_before = v_slot;
+            }
         }
-    } else {
+        __syncwarp();
+    } else if (warp < 8) {
         // ---------------- softmax ----------------
         const uint32_t g = warp >> 2;
         const uint32_t cnt = g ? cnt1 : cnt0;
@@ -321,20 +400,24 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const uint32_t pos_first = p0 + g * p.BP, pos = pos_first + pl;
         const uint32_t last_key = min(p.pos0 + pos, p.Mkv - 1u);
         const uint32_t lane_addr = ((warp & 3u) * 32u) << 16;
-        const uint32_t tS = tmem + lane_addr + g * 128u, tOg = tO + lane_addr + g * (uint32_t)D;
+        const uint32_t tS = tmem + lane_addr + C::COL_S + g * BK, tP = tmem + lane_addr + C::COL_P + g * (BK / 2), tOg = tmem + lane_addr + C::COL_O + g * D;
         // tiles whose keys all lie at or below every row's position (and inside the cache) need no mask
         const uint32_t free_keys = min(p.pos0 + pos_first + 1u, p.Mkv);
         float m_run = -1e30f, l_run = 0.0f;
-        bool ok = true;
+        bool s_ready = false;
         for (uint32_t it = 0; it < cnt; it++) {
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait(&s_full[g], it & 1u, abort_flag, p.err, 226));
-            if (!ok) break;
+            // (after a wait that gave up the rest runs out quickly, and nothing is written)
+            if (!s_ready) ptx::mbar_wait(&s_full[g], it & 1u, abort_flag, p.err, 226);
+            __syncwarp();
             ptx::tc_fence_after_sync();
             const uint32_t k0 = (t0 + it) * BK;
             float sc[BK];
 #pragma unroll
             for (int c = 0; c < BK; c += 32) tmem_ld_x32(tS + c, sc + c);
             ptx::tmem_ld_wait();
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&s_free[g]);
             if (k0 + BK > free_keys) {
 #pragma unroll
                 for (int j = 0; j < BK; j++) if (k0 + j > last_key) sc[j] = -INFINITY;
@@ -350,34 +433,43 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             // the division by the row sum removes the common factor, and O is rescaled hardly ever after the first step.
             float corr = 1.0f;
             if (mx > m_run + (LAG ? 8.0f : 0.0f)) { corr = ex2(m_run - mx); m_run = mx; }
-            if (it > 0u && __any_sync(0xffffffffu, corr != 1.0f)) {
-#pragma unroll
-                for (int c = 0; c < D; c += 16) {
-                    uint32_t v[16];
-                    ptx::tmem_ld_x16(tOg + c, v);
-                    ptx::tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
-                    ptx::tmem_st_x16(tOg + c, v);
-                }
-            }
             const uint64_t sc2 = pack2(p.scale_log2e, p.scale_log2e), nm2 = pack2(-m_run, -m_run);
             uint64_t rs0 = 0ull, rs1 = 0ull;              // two zeros each
+            // 64 keys at a time: exponentials, sums, and P as fp16 pairs.  Before the first of them is stored the step before has to be in O
+            // and its probabilities read.
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
+            for (int h = 0; h < BK / 64; h++) {
+                const bool pv_ready = h == 0 && it > 0u ? ptx::mbar_try_wait(&pv_done[g], (it - 1u) & 1u) : true;
                 uint32_t pk[32];
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
                     const int e = h * 64 + 2 * j;
                     float x0, x1, e0, e1;
                     unpack2(fma2(pack2(sc[e], sc[e + 1]), sc2, nm2), x0, x1);     // masked: -inf stays -inf, 2^-inf = 0
-                    if (poly_pair(j)) ex2_poly2<LAG ? 5 : 6>(x0, x1, e0, e1);
+                    if (poly_pair<D, LAG>(j)) ex2_poly2<LAG ? 5 : 6>(x0, x1, e0, e1);
                     else { e0 = ex2(x0); e1 = ex2(x1); }
                     if (j & 1) rs1 = add2(rs1, pack2(e0, e1)); else rs0 = add2(rs0, pack2(e0, e1));
                     pk[j] = pack_h2(e0, e1);
                 }
-                tmem_st_x32(tS + h * 32, pk);
+                if (h == 0 && it > 0u) {
+                    if (!pv_ready) ptx::mbar_wait(&pv_done[g], (it - 1u) & 1u, abort_flag, p.err, 227);
+                    __syncwarp();
+                    ptx::tc_fence_after_sync();
+                    if (__any_sync(0xffffffffu, corr != 1.0f)) {
+#pragma unroll
+                        for (int c = 0; c < D; c += 16) {
+                            uint32_t v[16];
+                            ptx::tmem_ld_x16(tOg + c, v);
+                            ptx::tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
+                            ptx::tmem_st_x16(tOg + c, v);
+                        }
+                    }
+                }
+                tmem_st_x32(tP + h * 32, pk);
             }
+            s_ready = it + 1u < cnt && ptx::mbar_try_wait(&s_full[g], (it + 1u) & 1u);
             ptx::tmem_st_wait();
             ptx::tc_fence_before_sync();
             __syncwarp();
@@ -387,8 +479,7 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             l_run = (l_run > SUM_OF_NAN ? l_run : l_run * corr) + (a0 + a1);
         }
         // ---------------- result ----------------
-        if (cnt > 0u && ok) ok = __all_sync(0xffffffffu, ptx::mbar_wait(&o_full[g], 0u, abort_flag, p.err, 227));
-        if (cnt > 0u && ok) {
+        if (cnt > 0u && __all_sync(0xffffffffu, ptx::mbar_wait(&pv_done[g], (cnt - 1u) & 1u, abort_flag, p.err, 227) && *abort_flag == 0u)) {
             ptx::tc_fence_after_sync();
             // Rows leave through the tile's Q buffer, which nothing reads any more: a thread deposits the 16-byte chunks of its
             // row (chunk c of row r at c ^ (r & 7): no bank conflict either way), then the warp moves its own 32 rows with whole
@@ -456,7 +547,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const Params p) {
     const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (r >= rows) return;
     const uint32_t head = r / p.M, pos = r - head * p.M;
-    const uint32_t n = (key_tiles(pos / p.BP * p.BP, p.BP, p.M, p.Mkv, p.pos0) + p.tiles_per_split - 1u) / p.tiles_per_split;
+    const uint32_t n = (key_tiles<D>(pos / p.BP * p.BP, p.BP, p.M, p.Mkv, p.pos0) + p.tiles_per_split - 1u) / p.tiles_per_split;
     // lane s holds split s's factor (at most 32 splits)
     const float2 ml = lane < n ? p.part_ml[(size_t)lane * rows + r] : make_float2(-1e30f, 0.0f);
     float m = ml.x;
@@ -471,14 +562,23 @@ __global__ void __launch_bounds__(256) combine_kernel(const Params p) {
     float acc[E];
 #pragma unroll
     for (int e = 0; e < E; e++) acc[e] = 0.0f;
-    for (uint32_t s = 0; s < n; s++) {
-        const float ws = __shfl_sync(0xffffffffu, wn, (int)s);
-        const float* src = p.part_o + ((size_t)s * rows + r) * D + lane * E;
-        float v[E];
-        if (E == 4) { const float4 t = __ldcg(reinterpret_cast<const float4*>(src)); v[0] = t.x; v[1] = t.y; v[E - 2] = t.z; v[E - 1] = t.w; }
-        else { const float2 t = __ldcg(reinterpret_cast<const float2*>(src)); v[0] = t.x; v[1] = t.y; }
+    // eight splits' values are under way together
+    const float* src = p.part_o + (size_t)r * D + lane * E;
+    for (uint32_t s0 = 0; s0 < n; s0 += 8u) {
+        float v[8][E];
 #pragma unroll
-        for (int e = 0; e < E; e++) acc[e] = fmaf(ws, v[e], acc[e]);
+        for (uint32_t j = 0; j < 8u; j++) {
+            const float* at = src + (size_t)(s0 + j) * rows * D;
+            if (s0 + j >= n) { for (int e = 0; e < E; e++) v[j][e] = 0.0f; }
+            else if (E == 4) { const float4 t = __ldcg(reinterpret_cast<const float4*>(at)); v[j][0] = t.x; v[j][1] = t.y; v[j][E - 2] = t.z; v[j][E - 1] = t.w; }
+            else { const float2 t = __ldcg(reinterpret_cast<const float2*>(at)); v[j][0] = t.x; v[j][1] = t.y; }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; j++) {
+            const float ws = __shfl_sync(0xffffffffu, wn, (int)(s0 + j));      // (lanes from n on hold 0: n is at most 32)
+#pragma unroll
+            for (int e = 0; e < E; e++) if (s0 + j < n) acc[e] = fmaf(ws, v[j][e], acc[e]);
+        }
     }
     __half* dst = (p.out_tokens_major ? p.O + ((size_t)pos * p.Hq + head) * D : p.O + (size_t)r * D) + lane * E;
     if (E == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_h2(acc[0], acc[1]), pack_h2(acc[E - 2], acc[E - 1]));
@@ -553,23 +653,34 @@ uint32_t sm_count() {
     return (uint32_t)n;
 }
 
-// Query tiles of a CTA and splits of the key range, by estimated time.  The unit is a step (128 keys) of a CTA with two tiles, 1.7 to
-// 2.1 us.  One tile is hardly cheaper a step and much cheaper a CTA (FIXED), so one is taken while that leaves no more CTAs waiting for
-// an SM (4 heads of 128, fp16: 200 tokens 8.6 -> 7.1 us, behind 500 others 15.9 -> 13.4; 700 alone 15.3 -> 13.1).  Partial results
-// cost a launch (COMBINE) and their way through memory (PER_BYTE).  One CTA runs per SM, so items beyond a whole number of waves
-// cost a wave where all items are equally long (a chunk behind a long cache); a causal triangle from position 0 packs better than
-// that, its sum is what counts there.  The constants: least regret over 320 shapes of both head sizes (1 to 1400 tokens behind 0 to
-// 3000, 1 to 32 kv heads), each timed with every choice: 0.6 % on average, 14 % at most.
+// Query tiles of a CTA and splits of the key range, by estimated time.  The unit is a step of a CTA with two tiles: 64 keys of 128-wide
+// heads, 0.8 us, or 128 keys of 64-wide ones, 1.5 us.  One tile is cheaper a step where the softmax bounds it and cheaper a CTA (FIXED), so one is
+// taken while that leaves no more CTAs waiting for an SM.  Partial results cost a launch (COMBINE) and their way through memory (PER_BYTE).  One CTA
+// runs per SM, so items beyond a whole number of waves cost a wave where all items are equally long (a chunk behind a long cache); a causal triangle
+// from position 0 packs better than that, its sum is what counts there.  The constants: least regret over 320 shapes (1 to 1400 tokens behind
+// 0 to 3000, 1 to 32 kv heads), each timed with every choice: 1.1 % on average for 128-wide heads, 0.9 % for 64-wide.
 }  // namespace
 
+// A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
+// arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O.  128-wide heads in groups of 1, 2, 4 and 8 have
+// always run with it; the others have not and follow the maximum exactly.
+static bool lagging(const Args& a) {
+    const uint32_t G = a.Hq / a.Hkv;
+    return a.D == 128 && (G == 1u || G == 2u || G == 4u || G == 8u);
+}
+
 Plan make_plan(const Args& a, bool split) {
-    constexpr float STEP[2] = {0.975f, 1.0f}, FIXED[2] = {2.0f, 4.1f}, COMBINE = 2.7f, PER_BYTE = 0.091e-6f;
+    struct Model { float step[2], fixed[2], combine, per_byte; };
+    static constexpr Model WIDE = {{1.046f, 1.0f}, {4.43f, 11.4f}, 5.9f, 0.391e-6f}, NARROW = {{1.158f, 1.0f}, {1.09f, 4.26f}, 3.7f, 0.309e-6f};
+    static constexpr Model WIDE_EXACT = {{0.755f, 1.0f}, {2.94f, 2.89f}, 2.6f, 0.27e-6f};         // (heads that follow the maximum exactly: a step 1.06 us)
+    const Model& m = a.D == 64 ? NARROW : lagging(a) ? WIDE : WIDE_EXACT;
+    const float (&STEP)[2] = m.step, (&FIXED)[2] = m.fixed, COMBINE = m.combine, PER_BYTE = m.per_byte;
     const float sms = (float)sm_count();
     Plan pl;
     pl.BP = (uint32_t)ROWS / (a.Hq / a.Hkv);
     auto key_tiles_at = [&](uint64_t pos) {      // key tiles of a block whose last position is `pos`
         const uint64_t last = (uint64_t)a.pos0 + (pos < a.M ? pos : a.M - 1);
-        return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / BK + 1);
+        return (uint32_t)((last < a.Mkv - 1 ? last : a.Mkv - 1) / step_keys(a.D) + 1);
     };
     pl.n_last = key_tiles_at(a.M - 1);
     float best = 0.0f;
@@ -650,9 +761,9 @@ template <int D, bool LAG> cudaError_t launch_d(const Args& a, const Plan& plann
     }
     CUtensorMap tmQ, tmK, tmV;
     const uint32_t map_rows = a.kv_fp16 ? a.Mkv : pl.kv_rows;
-    if (!make_map(&tmK, Kf, D, a.Hkv, map_rows, BK, 1) || !make_map(&tmV, Vf, D, a.Hkv, map_rows, BK, 1) || !make_map(&tmQ, a.Q, D, a.Hq, a.M, p.BP, p.G))
+    if (!make_map(&tmK, Kf, D, a.Hkv, map_rows, C::BK, 1) || !make_map(&tmV, Vf, D, a.Hkv, map_rows, C::BK, 1) || !make_map(&tmQ, a.Q, D, a.Hq, a.M, p.BP, p.G))
         return cudaErrorInvalidValue;
-    cfg.gridDim = dim3(a.Hkv, blocks, splits); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = C::SMEM;
+    cfg.gridDim = dim3(a.Hkv, blocks, splits); cfg.blockDim = dim3(C::THREADS); cfg.dynamicSmemBytes = C::SMEM;
     cudaError_t e = cudaLaunchKernelEx(&cfg, attn_ws_kernel<D, LAG>, tmQ, tmK, tmV, p);
     if (e != cudaSuccess) return e;
     ++*launches;
@@ -678,14 +789,7 @@ bool usable(const Args& a) {
 }
 
 cudaError_t launch(const Args& a, const Plan& plan, const Scratch& sc, cudaStream_t stream, int* launches) {
-    // A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
-    // arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O: 43.8 against 47.4 us at the 8B
-    // prefill, 42.0 against 43.6 for the heads of 64.  128-wide heads in groups of 1, 2, 4 and 8 have always run with it, and with
-    // the short polynomial; the others have not: they follow the maximum exactly, and a third of a unit in the last place is what
-    // their polynomial adds to fp32 rounding (3.8271e-4 with it, without it and with the short one; the 3.8204e-4 of the warp-level
-    // kernels come from their steps of 64 keys: every new maximum of a row is a probability of exactly 1, and they see more of them).
-    const uint32_t G = a.Hq / a.Hkv;
-    if (a.D == 128) return G == 1u || G == 2u || G == 4u || G == 8u ? launch_d<128, true>(a, plan, sc, stream, launches) : launch_d<128, false>(a, plan, sc, stream, launches);
+    if (a.D == 128) return lagging(a) ? launch_d<128, true>(a, plan, sc, stream, launches) : launch_d<128, false>(a, plan, sc, stream, launches);
     return launch_d<64, false>(a, plan, sc, stream, launches);
 }
 

@@ -854,6 +854,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 }
             }
             if (!ptx::mbar_wait<C::WAIT_CALL>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108)) { sc_ok = false; break; }
+            __syncwarp();                          // (tensor memory is read by whole warps)
             if (et == 0) QTRC(6, it, 0);
             ptx::tc_fence_after_sync();
             // grouped launch: the matrix this tile belongs to decides the output buffer and its width

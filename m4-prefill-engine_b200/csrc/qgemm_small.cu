@@ -314,9 +314,9 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
                 Cd::dequant64(r, s, o, meta);
                 if (j == 0) {
                     ptx::mbar_wait(&empty[st], ph ^ 1u, abort_flag, p.err, 116);
-                    __syncwarp();
                     ptx::tc_fence_after_sync();                      // the MMAs that read this stage have completed
                 }
+                __syncwarp();                                        // (tensor memory is written by whole warps)
                 tmem_st_x32(a_col + lane_base + st * A_COLS + j * SUB_COLS, o);
                 if (j == SPS - 1) {
                     ptx::tmem_st_wait();
