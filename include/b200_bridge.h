@@ -133,6 +133,10 @@ extern int b200_bridge_error_seen;
 /* What the bridge enqueues from here on waits on the GPU for everything `stream` (a cudaStream_t; NULL: the default stream)
  * holds now, without a wait on the host.  -6 if that is not possible (it, or a stream of the bridge, is under capture). */
 int b200_bridge_wait_stream(void* stream);
+/* b200_bridge_wait_stream, m4_bridge_dispatch_gemm and m4_bridge_synchronize in one call.  1: the GPU cannot wait for `stream` (see
+ * above) and nothing was enqueued; else the dispatch's code, without a wait for the result if that is an error. */
+int b200_bridge_project(void* stream, void* X, size_t X_bytes, void* W, size_t W_bytes, void* Y, size_t Y_bytes, int format,
+                        uint32_t M, uint32_t K, uint32_t N);
 /* Bytes of device memory that captured graphs hold as scratch.  A launch of the bridge under stream capture gets a block of its
  * graph's own: it is shared with no other launch and given back once the graph and every instance of it are destroyed (at the
  * next launch outside a capture, or by this call). */

@@ -80,6 +80,8 @@ def bind(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.b200_bridge_unregister_weights.restype = _i
     lib.b200_bridge_wait_stream.argtypes = [_vp]
     lib.b200_bridge_wait_stream.restype = _i
+    lib.b200_bridge_project.argtypes = [_vp, _vp, _sz, _vp, _sz, _vp, _sz, _i, _u32, _u32, _u32]
+    lib.b200_bridge_project.restype = _i
     lib.b200_bridge_graph_scratch_bytes.argtypes = []
     lib.b200_bridge_graph_scratch_bytes.restype = ctypes.c_size_t
     lib.b200_bridge_device_error.argtypes = []
@@ -121,10 +123,12 @@ def _addr(t: torch.Tensor) -> tuple[int, int]:
     return t.data_ptr(), t.numel() * t.element_size()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _current_stream() -> int:
     """cudaStream_t of torch's current stream (the raw accessor where this torch has it: a tenth of the cost of the object)."""
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device()) if _raw_stream is not None else torch.cuda.current_stream().cuda_stream
 
 
 class B200Bridge:
@@ -237,12 +241,29 @@ class B200Bridge:
         self._in_flight.append((Xc, Gc, Uc, Out))
         return ret
 
+    def project(self, X, W, Y, format, M, K, N) -> bool:
+        """``dispatch_gemm`` of contiguous GPU tensors and ``synchronize`` in one call of the library.  False, with nothing enqueued, where
+        the GPU cannot wait for torch's current stream (it is being captured)."""
+        xp, xb = _addr(X)
+        wp, wb = _addr(W)
+        yp, yb = _addr(Y)
+        ret = self._lib.b200_bridge_project(_current_stream(), xp, xb, wp, wb, yp, yb, int(format), M, K, N)
+        if ret == 1:
+            return False
+        if ret != 0:
+            raise RuntimeError(f"m4_bridge_dispatch_{'gemv' if M == 1 else 'gemm'} failed with status code {ret}")
+        self._completed()
+        return True
+
     def register_weights(self, W: torch.Tensor) -> int:
         p, n = _addr(W)
         return int(self._lib.b200_bridge_register_weights(p, n))
 
     def synchronize(self) -> None:
         self._lib.m4_bridge_synchronize()
+        self._completed()
+
+    def _completed(self) -> None:
         self._in_flight.clear()
         if self._pending_finite:
             checks, self._pending_finite = self._pending_finite, []

@@ -594,6 +594,14 @@ int b200_bridge_wait_stream(void* stream) {
     return 0;
 }
 
+int b200_bridge_project(void* stream, void* X, size_t Xb, void* W, size_t Wb, void* Y, size_t Yb, int format, uint32_t M, uint32_t K,
+                        uint32_t N) {
+    if (b200_bridge_wait_stream(stream) == -6) return 1;
+    const int rc = m4_bridge_dispatch_gemm(X, Xb, W, Wb, Y, Yb, format, M, K, N);
+    if (rc == 0) m4_bridge_synchronize();
+    return rc;
+}
+
 int b200_bridge_device_error(void) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.initialized) return -1;

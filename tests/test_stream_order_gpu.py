@@ -91,3 +91,28 @@ def test_other_captures_are_left_alone(bridge):
     g.replay()
     torch.cuda.synchronize()
     assert rc == [0, 0] and float(t.sum()) == 8.0
+
+
+def test_module_under_capture_takes_the_calls_one_by_one(bridge):
+    """M4QuantizedLinear.forward in one call of the library: behind a busy torch stream, and refused (nothing enqueued) for a captured one."""
+    from m4_prefill_engine_b200.modules import M4QuantizedLinear
+    import oracle as o
+    X, W = o.baseline_inputs(o.Q4_0, 1, 512, 256, 5)
+    lin = M4QuantizedLinear(512, 256, format=o.Q4_0, weight=torch.from_numpy(W.reshape(-1).view("uint8").copy()))
+    want = lin(torch.from_numpy(X).cuda()).clone()
+    x, s, g, t = torch.zeros(1, 512, dtype=torch.float16, device="cuda"), torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros(8, device="cuda")
+    src = torch.from_numpy(X).cuda()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(20_000_000)               # about ten milliseconds: the input is written behind it
+        x.copy_(src)
+        got = lin(x)
+    assert torch.equal(got, want)
+    y = torch.zeros(1, 256, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=torch.cuda.Stream()):
+        served = bridge.project(x, lin.weight, y, 0, 1, 512, 256)
+        t.add_(1)
+    g.replay()
+    torch.cuda.synchronize()
+    assert served is False and float(y.abs().max()) == 0.0 and float(t.sum()) == 8.0
