@@ -76,7 +76,7 @@ struct Params {
     int* err;
     __half* Y;
     const __half* residual;
-    float* scratch;              // [k_splits][tiles][T][128] partial tiles (k_splits > 1, or SwiGLU)
+    float* scratch;              // [k_splits][tiles][T][128] partial tiles (k_splits > 1)
     const uint8_t* meta0;
     const __half* row_scale0;
     uint32_t n_tok_tiles;
@@ -352,7 +352,39 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
         float rsc = 1.0f;
         if (Cd::ROW_SCALE) rsc = n < N ? __half2float((swiglu && f >= 64u ? p.row_scale1 : p.row_scale0)[n]) : 0.0f;
         const uint32_t taddr = tmem_base + ((warp * 32u) << 16);
-        if (p.k_splits > 1u || swiglu) {
+        if (swiglu && p.k_splits == 1u) {
+            // A whole SwiGLU tile: lanes 0 .. 63 hold the gate projections of 64 features, lanes 64 .. 127 the up projections of the same.  16 token
+            // columns at a time change hands through the operand rings, which nothing reads any more, and leave as whole rows of the tile (through the scratch
+            // buffer and back, like split sums: F = 14336, K = 4096, 33 tokens 29.0 us against 27.4, 128 tokens 39.0 against 32.1).
+            float* stage = reinterpret_cast<float*>(sB);                 // [2][16 columns][128 features]
+            const uint32_t tok0 = tt * p.T, valid = min(p.T, p.M - tok0), col = threadIdx.x >> 3, f0 = (threadIdx.x & 7u) * 8u, n0 = wt * GATE_ROWS + f0;
+            const bool wide = N % 8u == 0u && (reinterpret_cast<uintptr_t>(Y) & 15u) == 0;
+            for (uint32_t c0 = 0, b = 0; c0 < valid; c0 += 16u, b ^= 1u) {
+                uint32_t v[16];
+                __syncwarp();                                            // (tensor memory is read by whole warps)
+                ptx::tmem_ld_x16(taddr + c0, v);
+                ptx::tmem_ld_wait();
+                float* buf = stage + b * (16 * W_TILE);
+#pragma unroll
+                for (int j = 0; j < 16; j++) buf[j * W_TILE + f] = Cd::ROW_SCALE ? __uint_as_float(v[j]) * rsc : __uint_as_float(v[j]);
+                ptx::bar_sync(1, 128);                                   // (the buffer after next is written behind the next barrier)
+                if (c0 + col >= valid) continue;
+                const float4* g = reinterpret_cast<const float4*>(buf + col * W_TILE + f0);
+                const float4 g0 = g[0], g1 = g[1], u0 = g[GATE_ROWS / 4], u1 = g[GATE_ROWS / 4 + 1];
+                const float a[8] = {silu_mul(g0.x, u0.x), silu_mul(g0.y, u0.y), silu_mul(g0.z, u0.z), silu_mul(g0.w, u0.w),
+                                    silu_mul(g1.x, u1.x), silu_mul(g1.y, u1.y), silu_mul(g1.z, u1.z), silu_mul(g1.w, u1.w)};
+                __half* dst = Y + (size_t)(tok0 + c0 + col) * N + n0;
+                if (wide && n0 < N) {
+                    __half2 h[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) h[e] = __floats2half2_rn(a[2 * e], a[2 * e + 1]);
+                    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; e++) if (n0 + e < N) dst[e] = __float2half_rn(a[e]);
+                }
+            }
+        } else if (p.k_splits > 1u) {
             // [split][tile][token column][feature]: a warp's store covers 32 consecutive features of one column
             float* dst = p.scratch + ((size_t)ks * n_tiles + tile) * tile_floats + f;
             const uint32_t valid = min(p.T, p.M - tt * p.T);
@@ -388,7 +420,7 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
     // every partial tile of the cluster is written (release / acquire at cluster scope covers the global stores)
     cluster_sync_all();
     if (threadIdx.x == 0) QST(0, 6);
-    if (!bad && (p.k_splits > 1u || swiglu)) {
+    if (!bad && p.k_splits > 1u) {
         // this CTA's token columns [ks * cols, (ks + 1) * cols): sum over the splits in split order, write fp16
         const uint32_t cols = p.T >> p.split_shift;
         const float* base = p.scratch + (size_t)tile * tile_floats + (size_t)(ks * cols) * W_TILE;
@@ -533,7 +565,7 @@ template <int FMT> bool make_plan(const GemmArgs& a, Plan& pl) {
 
 template <int FMT> size_t scratch_floats_fmt(const GemmArgs& a) {
     Plan pl;
-    if (!make_plan<FMT>(a, pl) || (pl.k_splits <= 1 && !a.W1)) return 0;
+    if (!make_plan<FMT>(a, pl) || pl.k_splits <= 1) return 0;
     return (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE;
 }
 
@@ -541,7 +573,7 @@ template <int FMT, bool MULTI> cudaError_t launch_multi(const GemmArgs& a, const
     using Cd = cdc::Codec<FMT>;
     Plan pl;
     if (!make_plan<FMT>(a, pl)) return cudaErrorInvalidValue;
-    if ((pl.k_splits > 1 || a.W1) && (!ws.partial || ws.partial_floats < (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE))
+    if (pl.k_splits > 1 && (!ws.partial || ws.partial_floats < (size_t)pl.k_splits * pl.n_tok_tiles * pl.n_w_tiles * pl.T * W_TILE))
         return cudaErrorInvalidValue;
     const uint64_t w_row_bytes = (uint64_t)(a.K / Cd::CHUNK) * Cd::ROW_BYTES;
     const uint32_t x_cols = a.x_cols ? a.x_cols : a.K;          // columns past the end read as zero
@@ -658,16 +690,17 @@ bool small_path_ok(const GemmArgs& a) {
     uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
     for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) tiles += (a.N_extra[e] + 127u) / 128u;
     if (tiles > 2u * (uint32_t)small::sms()) return false;
-    // SwiGLU tiles pass through the scratch buffer even unsplit, which grows with the tokens, and from 113 tokens on the
-    // persistent kernel pairs its CTAs: a short K does not make up for it (F = 8192, 128 tokens, K = 512 / 1024: 13.2 / 14.9
-    // against 10.2 / 13.0 us there; 64 tokens, K = 512 / 1024: 9.6 / 11.0 against 9.1 / 11.5; F = 14336, K = 4096, 128 tokens: 44.5
-    // against 47.5, the variable-rate codec 75.8 against 72.2).
+    // SwiGLU tiles that are not split leave straight from the accumulator and are always better here (F = 14336, K = 512: 33 tokens 7.3 us against
+    // 9.6 on the persistent kernel, 128 tokens 9.9 against 13.4; K = 4096: 27.0 against 41.1, 31.8 against 44.5).  Split ones pass through the scratch
+    // buffer, which grows with the tokens: a short K does not make up for it (F = 5632: K = 512, 64 tokens 8.3 against 7.3; K = 1024, 64 tokens 9.4 against
+    // 9.8, 128 tokens 12.6 against 12.2; K = 2048, 128 tokens 16.0 against 17.2), a shorter one does for the variable rate (K = 512, 64 tokens 10.0 against
+    // 10.5, K = 1024, 128 tokens 10.3 against 13.4 with F = 1024, 16.3 against 16.2 with F = 5632).
     const uint32_t T = (a.M + 15u) & ~15u;
     // Grouped launches with a short K for their tokens: the same (512 + 2 x 128 features, K = 512: 64 tokens 7.9 us against 7.0, 128 tokens 9.9
     // against 8.4; 1024 + 2 x 256, K = 1024: 64 tokens 10.4 against 10.8, 128 tokens 14.3 against 12.5; K = 2048, 128 tokens 14.3 against
     // 14.9), and earlier in the variable-rate format (K = 512, one token 9.3 against 7.6; K = 1024, 33 tokens 12.6 against 11.3).
     if (a.n_extra && (a.format == QUANT_VAR_RATE_AFFINE ? a.K <= 512u || a.K < 22u * T : a.K < 12u * T)) return false;
-    if (a.W1 && (a.K < T * T / 4u || (T == (uint32_t)small::MAX_T && a.format == QUANT_VAR_RATE_AFFINE))) return false;
+    if (a.W1 && 2u * tiles <= 2u * (uint32_t)small::sms() && a.K < (a.format == QUANT_VAR_RATE_AFFINE ? 8u : 10u) * T) return false;
     return true;
 }
 
