@@ -125,7 +125,7 @@ int b200_bridge_unregister_weights(const void* host_ptr);
 
 /* 0 if no kernel has reported a fault since init; otherwise the first code reported: a bounded wait ran out inside a
  * projection kernel (101..110; 109 the CTA-pair relay, 110 rows another rank had not written), the few-token projection
- * kernel (111..117), an attention kernel (201..204, 220..227) or the peer exchange (301, 302); 401: a token id outside the
+ * kernel (111..117), an attention kernel (201..204, 220..229) or the peer exchange (301, 302); 401: a token id outside the
  * embedding table. */
 int b200_bridge_device_error(void);
 /* What the last m4_bridge_synchronize or b200_bridge_device_error found (read only; 0 after init and clear). */

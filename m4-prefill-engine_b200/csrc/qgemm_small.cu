@@ -690,7 +690,7 @@ bool small_path_ok(const GemmArgs& a) {
     uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
     for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) tiles += (a.N_extra[e] + 127u) / 128u;
     if (tiles > 2u * (uint32_t)small::sms()) return false;
-    // SwiGLU tiles that are not split leave straight from the accumulator and are always better here (F = 14336, K = 512: 33 tokens 7.3 us against
+    // SwiGLU tiles that are not split (more of them than SMs) leave straight from the accumulator and are always better here (F = 14336, K = 512: 33 tokens 7.3 us against
     // 9.6 on the persistent kernel, 128 tokens 9.9 against 13.4; K = 4096: 27.0 against 41.1, 31.8 against 44.5).  Split ones pass through the scratch
     // buffer, which grows with the tokens: a short K does not make up for it (F = 5632: K = 512, 64 tokens 8.3 against 7.3; K = 1024, 64 tokens 9.4 against
     // 9.8, 128 tokens 12.6 against 12.2; K = 2048, 128 tokens 16.0 against 17.2), a shorter one does for the variable rate (K = 512, 64 tokens 10.0 against
@@ -700,7 +700,7 @@ bool small_path_ok(const GemmArgs& a) {
     // against 8.4; 1024 + 2 x 256, K = 1024: 64 tokens 10.4 against 10.8, 128 tokens 14.3 against 12.5; K = 2048, 128 tokens 14.3 against
     // 14.9), and earlier in the variable-rate format (K = 512, one token 9.3 against 7.6; K = 1024, 33 tokens 12.6 against 11.3).
     if (a.n_extra && (a.format == QUANT_VAR_RATE_AFFINE ? a.K <= 512u || a.K < 22u * T : a.K < 12u * T)) return false;
-    if (a.W1 && 2u * tiles <= 2u * (uint32_t)small::sms() && a.K < (a.format == QUANT_VAR_RATE_AFFINE ? 8u : 10u) * T) return false;
+    if (a.W1 && tiles <= (uint32_t)small::sms() && a.K < (a.format == QUANT_VAR_RATE_AFFINE ? 8u : 10u) * T) return false;
     return true;
 }
 
