@@ -9,6 +9,8 @@
 // (all eight columns alike); the MMA adds up the four lanes of a row.  The eight fragments' worth of K that one row's four lanes
 // do not cover are other warps' chunks; they meet in shared memory.  (128-row tiles of tcgen05 would spend their time on
 // latency here: K = N = 4096 takes 9.5 us on the few-token kernel.)
+// What bounds it: one dependent chain per warp (packed bytes, 2 x 4 x 130 instructions of unpacking at half rate, 64 MMAs) where the GPU has few warps, the
+// unpack arithmetic where it has many (4096 -> 14336 13.8 us, 33 MB).
 // Weights are those of the tensor-core kernels bit for bit (the same register-level codecs).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -41,8 +43,14 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// R: rows per lane, 8 R rows per warp and CTA (R == 1 leaves the fragment's rows 8 .. 15 zero)
-template <int FMT, int R>
+// bytes from one chunk to the next in a warp's buffer: an odd number of 16-byte pieces
+__host__ __device__ constexpr uint32_t gv_stride(uint32_t rb) { return rb / 16u % 2u ? rb : rb + 16u; }
+
+// R: rows per lane, 8 R rows per warp and CTA (R == 1 leaves the fragment's rows 8 .. 15 zero).
+// STAGED: a warp's packed bytes pass through shared memory in the order in which they lie.  For chunks of 128 bytes: read by a lane each they lie at the same
+// offset of 32 cache lines, on the same banks (group-64 layout, K = N = 4096 10.4 -> 8.2 us, N = 8192 11.4 -> 9.9, K = 14336, N = 4096 19.1 -> 16.8, K = 2048, N = 5120
+// 9.5 -> 8.2).  Elsewhere it costs what the copy takes (Q4_0 4096 x 4096 6.1 -> 7.1).
+template <int FMT, int R, bool STAGED>
 __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams p) {
     using Cd = cdc::Codec<FMT>;
     constexpr uint32_t ROWS = 8u * R;
@@ -63,11 +71,13 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
         for (int h = 0; h < R; h++) {
             const uint32_t n = min(n0 + g + 8u * h, p.N - 1u);
             if (c < p.chunks) {
-                const uint4* src = reinterpret_cast<const uint4*>(p.W + (size_t)n * row_bytes + (size_t)c * RB);
+                if constexpr (!STAGED) {
+                    const uint4* src = reinterpret_cast<const uint4*>(p.W + (size_t)n * row_bytes + (size_t)c * RB);
 #pragma unroll
-                for (int i = 0; i < RB / 16; i++) {
-                    const uint4 v = __ldg(src + i);
-                    r[h][4 * i] = v.x; r[h][4 * i + 1] = v.y; r[h][4 * i + 2] = v.z; r[h][4 * i + 3] = v.w;
+                    for (int i = 0; i < RB / 16; i++) {
+                        const uint4 v = __ldg(src + i);
+                        r[h][4 * i] = v.x; r[h][4 * i + 1] = v.y; r[h][4 * i + 2] = v.z; r[h][4 * i + 3] = v.w;
+                    }
                 }
                 if (Cd::META_WORDS != 0) {       // one scale and one bias per 64 (4 words) or 32 (8 words) elements, two planes
                     const uint32_t groups = (p.K / 256) * MW;
@@ -83,13 +93,31 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
                     }
                 }
             } else {
+                if constexpr (!STAGED) {
 #pragma unroll
-                for (int i = 0; i < RB / 4; i++) r[h][i] = 0u;
+                    for (int i = 0; i < RB / 4; i++) r[h][i] = 0u;
+                }
 #pragma unroll
                 for (int i = 0; i < MW; i++) meta[h][i] = 0u;
             }
         }
     };
+    // STAGED: four chunks of the warp's rows, rows past N and chunks past the end as above, in its buffer
+    constexpr uint32_t PIECES = RB / 16, STRIDE = gv_stride(RB);
+    uint8_t* buf = sx + (size_t)p.chunks * X_CHUNK + (size_t)warp * (ROWS * 4u * STRIDE);
+    auto fetch = [&](uint32_t c0) {
+        const uint32_t dst = ptx::smem_u32(buf);
+        static_assert(!STAGED || ROWS * 4u * PIECES % 32u == 0u, "whole turns of the warp");
+#pragma unroll 3                                       // (all at once: 156 registers for 114, K = 14336 18.9 us for 16.9)
+        for (uint32_t i = 0; i < ROWS * 4u * PIECES / 32u; i++) {
+            const uint32_t j = i * 32u + lane, row = j / (4u * PIECES), k = j % (4u * PIECES), c = k / PIECES;
+            const bool in = c0 + c < p.chunks;
+            const uint8_t* src = in ? p.W + (size_t)min(n0 + row, p.N - 1u) * row_bytes + (size_t)c0 * RB + k * 16u : p.W;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (row * 4u + c) * STRIDE + (k - c * PIECES) * 16u), "l"(src), "r"(in ? 16 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if constexpr (STAGED) fetch(warp * 4u);
     load(warp * 4u + t, r, meta);                     // under way while the activations are staged
     if (p.early) ptx::grid_dependency_wait();
 
@@ -119,6 +147,19 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
         const bool more = c0 + warps * 4u < p.chunks;
         uint32_t rn[AHEAD ? R : 1][AHEAD ? RB / 4 : 1], mn[AHEAD ? R : 1][AHEAD ? MW : 1];
         if constexpr (AHEAD) { if (more) load(c + warps * 4u, rn, mn); }
+        if constexpr (STAGED) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();                             // every lane's copies are there
+#pragma unroll
+            for (int h = 0; h < R; h++)
+#pragma unroll
+                for (int i = 0; i < RB / 16; i++) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(buf + ((g + 8u * h) * 4u + t) * STRIDE + i * 16);
+                    r[h][4 * i] = v.x; r[h][4 * i + 1] = v.y; r[h][4 * i + 2] = v.z; r[h][4 * i + 3] = v.w;
+                }
+            __syncwarp();                             // every lane has read: the next round may come while this one is multiplied
+            if (more) fetch(c0 + warps * 4u);
+        }
 #pragma unroll
         for (int s = 0; s < 4; s++) {
             uint32_t a[R][32];
@@ -150,7 +191,7 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
     }
 }
 
-template <int FMT, int R>
+template <int FMT, int R, bool STAGED = false>
 cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
     using Cd = cdc::Codec<FMT>;
     GvParams p;
@@ -161,7 +202,7 @@ cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
     p.early = a.early_weights ? 1u : 0u;
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, R, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
         attr = true;
     }
@@ -171,13 +212,20 @@ cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
     cfg.gridDim = dim3((a.N + 8 * R - 1) / (8 * R));
     const uint32_t rounds = (groups + GV_MAX_WARPS - 1) / GV_MAX_WARPS;
     cfg.blockDim = dim3(32u * ((groups + rounds - 1) / rounds));      // every warp the same number of rounds, as far as that goes
-    cfg.dynamicSmemBytes = (size_t)p.chunks * X_CHUNK;
+    static_assert(!STAGED || 199u * X_CHUNK + GV_MAX_WARPS * 8u * R * 4u * gv_stride(Cd::ROW_BYTES) <= 200u * 1024u, "activations and buffers of the longest rows");
+    cfg.dynamicSmemBytes = (size_t)p.chunks * X_CHUNK + (STAGED ? (cfg.blockDim.x / 32u) * (8u * R * 4u * gv_stride(Cd::ROW_BYTES)) : 0u);
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, R>, p);
+    return cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, R, STAGED>, p);
+}
+
+int gv_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    return n;
 }
 
 template <int FMT>
@@ -185,8 +233,17 @@ cudaError_t launch_gemv_fmt(const GemmArgs& a, cudaStream_t stream) {
     // Two rows per lane fill the fragment; the variable-rate codec's two rows take 179 registers, one row 124 (K = 4096, N = 14336:
     // 31.3 against 23.5 us), and the codebook's 177 registers cost more than they give (K = 4096, N = 32000: 42.3 against 39.1; K = 5120,
     // N = 5120 18.3 against 11.6; K = 14336, N = 4096 25.8 against 24.9; the other way round K = N = 4096, 7.4 against 8.9).
-    const bool one = FMT == QUANT_VAR_RATE_AFFINE || FMT == QUANT_EXL3;
-    return one ? launch_gemv_rows<FMT, 1>(a, stream) : launch_gemv_rows<FMT, 2>(a, stream);
+    constexpr bool ONE = FMT == QUANT_VAR_RATE_AFFINE || FMT == QUANT_EXL3, PLANAR = cdc::Codec<FMT>::META_WORDS != 0;
+    if constexpr (ONE) return launch_gemv_rows<FMT, 1>(a, stream);
+    else {
+        // Where one row per lane makes less than a warp for each scheduler, the chain of one warp is the time, and half as long (K = 512, N = 512: Q4_0 3.3 -> 3.1 us,
+        // Q4_K 3.9 -> 3.2, ternary 4.0 -> 3.3, group-64 4.1 -> 3.3; K = 4096, N = 512 3.6 -> 3.2, 4.2 -> 3.3, 4.3 -> 3.4, 4.9 -> 3.7).  With 3.5 of them on an SM the
+        // formats that unpack fast lose 3 to 10 % (Q4_0 K = 512, N = 4096 3.4 -> 3.7), the planar ones still gain (2 to 5 %; K = 8192, N = 512 7.1 -> 5.5).
+        const uint32_t warps = (a.N + 7u) / 8u * ((a.K / 256u + 3u) / 4u);
+        if (a.K / 256u <= 4u * GV_MAX_WARPS && warps <= (PLANAR ? 4u : 3u) * (uint32_t)gv_sms()) return launch_gemv_rows<FMT, 1>(a, stream);
+        if constexpr (PLANAR) { if (a.K >= 1024u) return launch_gemv_rows<FMT, 2, true>(a, stream); }      // (K = 512, N = 5120 4.7 us staged 5.1; K = 1024 5.6 and 5.3)
+        return launch_gemv_rows<FMT, 2>(a, stream);
+    }
 }
 
 }  // namespace
