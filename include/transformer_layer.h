@@ -161,6 +161,10 @@ int b200_layer_profile(void* layer, char* labels, size_t label_bytes, float* us,
  * buffers; the owner's reduction + residual + broadcast into out[]; the wait for every rank's rows. */
 int b200_peer_gemm_scatter(const void* X, const void* W, int format, uint32_t M, uint32_t K, uint32_t N, uint32_t rank,
                            uint32_t world, void* const* recv, void* const* flags, uint32_t epoch);
+/* A projection of rows that other ranks are still writing (each token tile waits for its owners' rows; device error 110 when a
+ * wait runs out): SwiGLU of W and W_up if that is given; to Y, or (recv given) its partial sums to the owners as above. */
+int b200_peer_gemm_wait_rows(const void* X, const void* W, const void* W_up, void* Y, int format, uint32_t M, uint32_t K, uint32_t N,
+                             uint32_t rank, uint32_t world, void* const* recv, void* const* flags, uint32_t epoch);
 int b200_peer_reduce_broadcast(uint32_t rank, uint32_t world, void* const* recv, void* const* out, void* const* flags,
                                uint32_t epoch, const void* residual, uint32_t M, uint32_t K);
 int b200_peer_wait_rows(uint32_t rank, uint32_t world, void* const* flags, uint32_t epoch);

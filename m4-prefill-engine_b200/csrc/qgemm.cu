@@ -665,8 +665,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // operand descriptors differ between stages only in the 14-bit start-address field
         const uint64_t desc_hi = ptx::umma_desc_k_sw128(0u);
         const uint32_t a_lo0 = (ptx::smem_u32(sA) & 0x3FFFFu) >> 4, b_lo0 = (ptx::smem_u32(sB) & 0x3FFFFu) >> 4;
-        // One thread, chosen once, walks the loop: chosen anew for every step and with the wait's outcome voted on, a step of four 128 x 128 x 16
-        // MMAs took 328 cycles instead of 257.  After a wait that gave up the rest runs out quickly, and nothing is written.
+        // One thread, chosen once, walks the loop: chosen anew for every step and with the wait's outcome voted on, a step of four
+        // 128 x 128 x 16 MMAs took 328 cycles instead of 257.  Waits that gave up are looked for twice a tile, in the abort flag:
+        // an accumulator that may still be read is not written, and a tile is announced only if every wait of this CTA for its
+        // operands succeeded (a thread whose wait failed has seen or set the flag before its warp arrives anywhere).
         if (ptx::elect_one()) {
             uint32_t st = 0, sph = 0, bst = 0, bsph = 0, it = 0, mtr = 0;
             (void)mtr;
@@ -674,6 +676,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 const uint32_t buf = it & 1u;
                 if (PAIR) ptx::mbar_wait_cluster<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
                 else ptx::mbar_wait<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                if (*abort_flag) break;
                 ptx::tc_fence_after_sync();
                 QTRC(2, 200u + it, 0);
                 const uint32_t ksteps = tile_of(idx).kcn * (uint32_t)C::SUBS;
@@ -703,6 +706,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (++st == p.a_stages) { st = 0; sph ^= 1u; }
                     if (++bst == p.b_stages) { bst = 0; bsph ^= 1u; }
                 }
+                if (*abort_flag) break;
                 if (PAIR) ptx::umma_pair_commit(&tm_full[buf]); else ptx::umma_commit(&tm_full[buf]);
                 QTRC(2, 200u + it, 1);
             }
@@ -721,7 +725,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         uint32_t rs = 0, rph = 0, kn = 0;                     // kn: running 64-element step of this CTA
         uint32_t km = 0, own_ph = 0;                          // (kn / 4) % STAGES; phase of the group's next operand stage
         uint32_t own_st = grp;                                // ... and that stage: the group's steps g, g + 3, ... use stages (g + 3 j) % a_stages
-        // (after a wait that gave up the rest runs out quickly, and nothing is written)
+        // After a wait that gave up the warp runs out its tile on whatever the stages hold and leaves.  Its arrivals do no harm in
+        // this CTA, whose issuing thread looks at the abort flag; on the other CTA of a pair, which has a flag of its own, it makes none.
         for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             // META_WORDS / 2 words of scales and as many of biases per chunk: one group per 64 elements (4 words)
@@ -791,7 +796,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             *reinterpret_cast<uint4*>(dst + ((c ^ xr) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
                         ptx::fence_proxy_async_smem();
                         __syncwarp();                      // every lane's stores are fenced; one arrival per warp
-                        if (lane == 0) { if (PAIR && pair_rank == 1u) ptx::mbar_arrive_cluster(&a_full[as], 0u); else ptx::mbar_arrive(&a_full[as]); }
+                        if (lane == 0) {
+                            if (!(PAIR && pair_rank == 1u)) ptx::mbar_arrive(&a_full[as]);
+                            else if (*abort_flag == 0u) ptx::mbar_arrive_cluster(&a_full[as], 0u);
+                        }
                         if (row == 0) QTR(4 + grp, kn + s, 2);
                     }
                 };
@@ -806,6 +814,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (row == 0) QTR(3, ((kn >> 2) - 1) * 2 + grp, 3);
                 if (++rs == p.raw_stages) { rs = 0; rph ^= 1u; }
             }
+            if (__any_sync(0xffffffffu, *abort_flag != 0u)) break;
         }
     } else if (warp >= (uint32_t)C::EPI_WARP0) {
         // ---------------- epilogue: tensor memory -> fp16 (or fp32 partials) ----------------
@@ -817,8 +826,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // in shared memory).  After its last tile the warp fences its peer stores at system scope once -- a system-scope
         // fence under full store traffic costs several microseconds, so there is one per warp and launch, not one per
         // owner -- and adds its counts to the rank-wide counters; the warp that completes an owner's count (tiles x 4
-        // epilogue warps) raises this rank's arrival flag on that owner.  Counting per warp needs no barrier among the
-        // epilogue warps, so a warp that gave up on a wait cannot strand the others.
+        // epilogue warps) raises this rank's arrival flag on that owner.
         uint32_t* sc_cnt = reinterpret_cast<uint32_t*>(bars) + 96 + q * 8;      // bytes 384..511 of the barrier block
         if (p.scatter.world && lane < 8u) sc_cnt[lane] = 0u;
         __syncwarp();
@@ -853,8 +861,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (n0 + 64u < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + 128));
                 }
             }
-            if (!ptx::mbar_wait<C::WAIT_CALL>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108)) { sc_ok = false; break; }
-            __syncwarp();                          // (tensor memory is read by whole warps)
+            // The epilogues below meet at barriers of all 128 threads, so the threads decide together whether the tile is there:
+            // one whose wait gave up, or that sees the abort flag, takes the others with it.
+            const bool got = ptx::mbar_wait<C::WAIT_CALL>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108) && *abort_flag == 0u;
+            __syncwarp();                          // (a barrier and tensor memory are taken by whole warps)
+            if (!ptx::bar_all(3, 128, got)) { sc_ok = false; break; }
             if (et == 0) QTRC(6, it, 0);
             ptx::tc_fence_after_sync();
             // grouped launch: the matrix this tile belongs to decides the output buffer and its width

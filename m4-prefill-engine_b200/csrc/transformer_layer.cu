@@ -635,24 +635,45 @@ bool peer_counter_ready() {
 }
 }  // namespace
 
-int b200_peer_gemm_scatter(const void* X, const void* W, int format, uint32_t M, uint32_t K, uint32_t N, uint32_t rank,
-                           uint32_t world, void* const* recv, void* const* flags, uint32_t epoch) {
+namespace {
+// recv != nullptr: partial rows to their owners; wait_flags != nullptr: rows of X appear while the projection runs
+int peer_gemm(const void* X, const void* W, const void* W_up, void* Y, int format, uint32_t M, uint32_t K, uint32_t N, uint32_t rank,
+              uint32_t world, void* const* recv, void* const* flags, const uint32_t* wait_flags, uint32_t epoch) {
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.initialized) return -1;
-    if (!X || !W || !recv || !flags || world < 1 || world > 8 || rank >= world) return -2;
+    if (!X || !W || (!Y && !recv) || !flags || world < 1 || world > 8 || rank >= world) return -2;
     if (M == 0 || K == 0 || N == 0 || M % world != 0) return -4;
     if (!peer_counter_ready()) return -5;
     qg::GemmArgs a; memset(&a, 0, sizeof(a));
-    a.format = format; a.X = X; a.W0 = W; a.M = M; a.N = N; a.K = K; a.layout = LAYOUT_STANDARD;
-    a.scatter.world = world; a.scatter.rank = rank; a.scatter.rows = M / world; a.scatter.epoch = epoch;
-    a.scatter.done_counter = g_peer_counter; a.scatter.fp16 = g_peer_partial_fp16 ? 1u : 0u;
-    for (uint32_t o = 0; o < world; o++) { a.scatter.recv[o] = (float*)recv[o]; a.scatter.flags[o] = (uint32_t*)flags[o]; }
+    a.format = format; a.X = X; a.W0 = W; a.W1 = W_up; a.Y = Y; a.M = M; a.N = N; a.K = K; a.layout = LAYOUT_STANDARD;
+    if (recv) {
+        a.scatter.world = world; a.scatter.rank = rank; a.scatter.rows = M / world; a.scatter.epoch = epoch;
+        a.scatter.done_counter = g_peer_counter; a.scatter.fp16 = g_peer_partial_fp16 ? 1u : 0u;
+        for (uint32_t o = 0; o < world; o++) { a.scatter.recv[o] = (float*)recv[o]; a.scatter.flags[o] = (uint32_t*)flags[o]; }
+    }
+    if (wait_flags) {
+        a.wait_rows.flags = wait_flags; a.wait_rows.rows = M / world; a.wait_rows.epoch = epoch;
+        a.wait_rows.limit_cycles = peer::wait_limit_cycles();
+    }
     qg::Workspace ws;
     ws.partial = (float*)g.ws_partial.p; ws.partial_floats = g.ws_partial.cap / sizeof(float); ws.counters = g.counters; ws.err = g.err_word;
     cudaError_t e = qg::launch(a, ws, g.stream);
-    if (e != cudaSuccess) { set_error(std::string("gemm_scatter launch failed: ") + cudaGetErrorString(e)); return e == cudaErrorInvalidValue ? -4 : -6; }
+    if (e != cudaSuccess) { set_error(std::string("peer projection launch failed: ") + cudaGetErrorString(e)); return e == cudaErrorInvalidValue ? -4 : -6; }
     g.launches += (uint64_t)qg::last_launch_count();
     return 0;
+}
+}  // namespace
+
+int b200_peer_gemm_scatter(const void* X, const void* W, int format, uint32_t M, uint32_t K, uint32_t N, uint32_t rank,
+                           uint32_t world, void* const* recv, void* const* flags, uint32_t epoch) {
+    if (!recv) return g.initialized ? -2 : -1;
+    return peer_gemm(X, W, nullptr, nullptr, format, M, K, N, rank, world, recv, flags, nullptr, epoch);
+}
+
+int b200_peer_gemm_wait_rows(const void* X, const void* W, const void* W_up, void* Y, int format, uint32_t M, uint32_t K, uint32_t N,
+                             uint32_t rank, uint32_t world, void* const* recv, void* const* flags, uint32_t epoch) {
+    if (!flags || world > 8 || rank >= world || !flags[rank]) return g.initialized ? -2 : -1;
+    return peer_gemm(X, W, W_up, Y, format, M, K, N, rank, world, recv, flags, (const uint32_t*)flags[rank] + 8, epoch);
 }
 
 int b200_peer_reduce_broadcast(uint32_t rank, uint32_t world, void* const* recv, void* const* out, void* const* flags,

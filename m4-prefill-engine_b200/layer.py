@@ -68,6 +68,7 @@ def _bind_layer(lib) -> None:
     lib.b200_peer_free.argtypes = [vp]
     lib.b200_layer_set_peer_exchange.argtypes = [vp, u32, u32, pp, pp, pp, pp]
     lib.b200_peer_gemm_scatter.argtypes = [vp, vp, ctypes.c_int, u32, u32, u32, u32, u32, pp, pp, u32]
+    lib.b200_peer_gemm_wait_rows.argtypes = [vp, vp, vp, vp, ctypes.c_int, u32, u32, u32, u32, u32, pp, pp, u32]
     lib.b200_peer_reduce_broadcast.argtypes = [u32, u32, pp, pp, pp, u32, vp, u32, u32]
     lib.b200_peer_wait_rows.argtypes = [u32, u32, pp, u32]
     lib.b200_peer_reduce_norm_broadcast.argtypes = [u32, u32, pp, pp, pp, u32, vp, u32, u32, vp, ctypes.c_float, vp]
@@ -82,7 +83,7 @@ def _bind_layer(lib) -> None:
     lib.b200_layer_set_fused_kv_epilogue.restype = ctypes.c_int
     lib.b200_layer_profile.argtypes = [vp, ctypes.c_char_p, ctypes.c_size_t, ctypes.POINTER(ctypes.c_float), ctypes.c_size_t]
     for f in ("b200_peer_alloc", "b200_peer_open", "b200_peer_close", "b200_peer_free", "b200_layer_set_peer_exchange",
-              "b200_peer_gemm_scatter", "b200_peer_reduce_broadcast", "b200_peer_wait_rows", "b200_layer_attach_peer_exchange",
+              "b200_peer_gemm_scatter", "b200_peer_gemm_wait_rows", "b200_peer_reduce_broadcast", "b200_peer_wait_rows", "b200_layer_attach_peer_exchange",
               "b200_layer_set_profiling", "b200_layer_profile"):
         getattr(lib, f).restype = ctypes.c_int
     lib._layer_bound = True
