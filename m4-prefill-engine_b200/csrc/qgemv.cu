@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 
@@ -200,11 +201,14 @@ cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
     p.meta = (const uint8_t*)a.W0 + (size_t)a.N * p.chunks * Cd::ROW_BYTES;
     p.row_scale = (const __half*)p.meta;
     p.early = a.early_weights ? 1u : 0u;
-    static bool attr = false;
-    if (!attr) {
+    static std::atomic<uint64_t> attr_done{0};               // bit d: set on device d
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (!(attr_done.load() & bit)) {
         cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, R, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
-        attr = true;
+        attr_done |= bit;
     }
     const uint32_t groups = (p.chunks + 3u) / 4u;            // a warp takes four chunks at a time
     cudaLaunchConfig_t cfg;
