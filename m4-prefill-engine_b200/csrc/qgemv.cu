@@ -226,9 +226,15 @@ cudaError_t launch_gemv_rows(const GemmArgs& a, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, R, STAGED>, p);
 }
 
+// SMs of the current device, asked of the runtime once for each
 int gv_sms() {
+    static std::atomic<int> known[64];
     int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    const bool keep = dev >= 0 && dev < 64;
+    if (keep && (n = known[dev].load()) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    if (keep) known[dev] = n;
     return n;
 }
 

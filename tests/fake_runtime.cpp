@@ -7,7 +7,7 @@
 
 #include "qgemm.cuh"
 
-static int g_dev = 0, g_queries = 0;
+static int g_dev = 0, g_queries = 0, g_blocks = 0;
 static size_t g_smem = 0;
 static std::map<std::pair<int, const void*>, int> g_attr;      // (device, kernel) -> dynamic shared memory allowed there
 
@@ -25,12 +25,14 @@ cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
     auto it = g_attr.find({g_dev, f});
     g_smem = c->dynamicSmemBytes;
+    g_blocks = (int)c->gridDim.x;
     return c->dynamicSmemBytes <= (it == g_attr.end() ? 48u * 1024u : (size_t)it->second) ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 void fake_device(int d) { g_dev = d; }
 int fake_queries() { return g_queries; }
 size_t fake_smem() { return g_smem; }
+int fake_blocks() { return g_blocks; }
 int fake_gemv(int format, unsigned K, unsigned N) {
     qg::GemmArgs a;
     memset(&a, 0, sizeof(a));

@@ -34,3 +34,18 @@ def test_second_device_gets_its_shared_memory(fake, fmt):
         fake.fake_device(d)
         assert fake.fake_gemv(fmt, 8192, 8192) == 0, f"device {d}"
         assert fake.fake_smem() > 48 * 1024
+
+
+def test_sm_count_is_asked_once_per_device(fake):
+    """The rows per lane follow the SMs of the device that launches, without a query per call."""
+    for d in (0, 1):
+        fake.fake_device(d)
+        assert fake.fake_gemv(o.Q4_0, 512, 512) == 0
+    before = fake.fake_queries()
+    rows = []
+    for d in (0, 1, 0, 1):
+        fake.fake_device(d)
+        assert fake.fake_gemv(o.Q4_0, 512, 512) == 0
+        rows.append(512 // fake.fake_blocks())
+    assert rows == [8, 16, 8, 16]                  # 64 warps: fewer than three for each of 148 SMs, more than for each of 2
+    assert fake.fake_queries() == before
