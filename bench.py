@@ -150,6 +150,15 @@ def cpu_baseline(fmt: int, budget_s: float = 12.0) -> dict:
             "sample": f"{rows} of {M} token rows x all {N} outputs, K={K}, double-precision verifier, {t:.2f} s, {cores} OpenMP threads"}
 
 
+def headline(line: dict) -> dict:
+    """The line of standard output: the record without what is measured beside the headline, which is 24 KB long (readers keep the last
+    few).  Of those parts the times stay."""
+    out = {k: v for k, v in line.items() if k not in ("sweep", "c4", "layer", "model", "ms_per_step_blocks")}
+    out["parity"] = {k: v for k, v in (line["parity"] or {}).items() if not isinstance(v, (list, dict))}
+    out["beside"] = {k: round(line[k]["ms"], 4) for k in ("layer", "model") if line[k] and "ms" in line[k]} | {"record": "standard error"}
+    return out
+
+
 def run_reference(args) -> None:
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -738,7 +747,8 @@ def run_ours(args) -> None:
         }
         if world == 1 and not args.no_cpu:
             line["cpu_baseline"] = cpu_baseline(fmt)
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)          # everything that was measured
+        print(json.dumps(headline(line)), flush=True)
     if dist:
         dist.barrier()
         dist.destroy_process_group()
