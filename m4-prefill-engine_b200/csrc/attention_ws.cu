@@ -53,6 +53,11 @@ constexpr int MAX_SPLITS = 32;
 
 // keys of a step: as many as tensor memory has columns for beside the two accumulators
 __host__ __device__ constexpr uint32_t step_keys(uint32_t d) { return d == 128u ? 64u : 128u; }
+// Steps after which the reference maximum of a row may lag.  Distance from 64 bits, 32 / 8 heads over 2048 tokens (queries of twice the size; 8 / 2,
+// 256 tokens behind 7936): 2.60e-4 (2.70e-4; 2.92e-4) with a lag from the first step on, 2.56e-4 (2.58e-4; 2.89e-4) after three exact ones, 2.55e-4 (2.54e-4;
+// 2.87e-4) after four; a lag with steps of 128 keys 2.58e-4 (2.64e-4; 2.88e-4), always exact 2.53e-4 (2.31e-4; 2.86e-4).  32 / 8 heads
+// over 2048 tokens, fp16: 35.0 us with none, 36.8 with four, 38.5 with eight.
+constexpr uint32_t EXACT_STEPS = 4;
 template <int D> struct Cfg {
     static constexpr int BK = (int)step_keys(D);
     // Score and value MMAs from a thread each, so that neither's waits leave the tensor pipe idle (128-wide heads, 32 / 8 over 2048 tokens, fp16 36.4 -> 35.1 us,
@@ -430,9 +435,10 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             }
             mx = fmaxf(mx, mx1) * p.scale_log2e;          // the scale is positive: max and scaling commute
             // With a lag of 8 the reference maximum moves only for jumps above 2^8: probabilities are then at most 256 instead of 1,
-            // the division by the row sum removes the common factor, and O is rescaled hardly ever after the first step.
+            // the division by the row sum removes the common factor, and O is rescaled hardly ever.  The first steps follow the maximum
+            // exactly: the key that sets it has a probability of exactly 1, every other one is rounded, and the largest weigh most.
             float corr = 1.0f;
-            if (mx > m_run + (LAG ? 8.0f : 0.0f)) { corr = ex2(m_run - mx); m_run = mx; }
+            if (mx > m_run + (LAG && it >= EXACT_STEPS ? 8.0f : 0.0f)) { corr = ex2(m_run - mx); m_run = mx; }
             const uint64_t sc2 = pack2(p.scale_log2e, p.scale_log2e), nm2 = pack2(-m_run, -m_run);
             uint64_t rs0 = 0ull, rs1 = 0ull;              // two zeros each
             // 64 keys at a time: exponentials, sums, and P as fp16 pairs.  Before the first of them is stored the step before has to be in O
@@ -661,9 +667,8 @@ uint32_t sm_count() {
 // 0 to 3000, 1 to 32 kv heads), each timed with every choice: 1.1 % on average for 128-wide heads, 0.9 % for 64-wide.
 }  // namespace
 
-// A lagging reference makes the row's largest probability inexact in fp16, which puts the result 0.8 % further from 64-bit
-// arithmetic (3.86e-4 against 3.83e-4, 32 heads of 64, 2048 tokens), and saves the rescaling of O.  128-wide heads in groups of 1, 2, 4 and 8 have
-// always run with it; the others have not and follow the maximum exactly.
+// A lagging reference saves the rescaling of O and puts the result further from 64-bit arithmetic
+// (EXACT_STEPS).  Results may not get less exact, so only the shapes whose results always had it have it.
 static bool lagging(const Args& a) {
     const uint32_t G = a.Hq / a.Hkv;
     return a.D == 128 && (G == 1u || G == 2u || G == 4u || G == 8u);
