@@ -44,7 +44,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Non-blocking look at a phase.  (try_wait may park the thread for a hardware-defined time, about 4 us on B200, before it
-// says no: a loop that only wants to know whether it may do something early must not use it.)
+// says no: code with something else to do meanwhile must not use it.)
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -81,39 +81,54 @@ template <bool CLUSTER> __device__ __forceinline__ bool mbar_look(uint32_t bar, 
             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-template <bool CLUSTER>
+// PAIR: whoever gives up sets the abort flag of both CTAs of the cluster (each lies at the same offset) before it returns, so what its
+// warp arrives on in the other CTA afterwards cannot pass for a success there.
+template <bool PAIR>
+__device__ __forceinline__ bool mbar_give_up(volatile uint32_t* abort_flag) {
+    if (PAIR) {
+        const uint32_t at = smem_u32(const_cast<const uint32_t*>(abort_flag));
+        asm volatile(
+            "{\n\t.reg .u32 r, a;\n\t"
+            "mov.u32 r, %%cluster_ctarank;\n\t"
+            "xor.b32 r, r, 1;\n\t"
+            "mapa.shared::cluster.u32 a, %0, r;\n\t"
+            "st.volatile.shared::cluster.u32 [a], 1;\n\t"
+            "fence.acq_rel.cluster;\n\t}"
+            ::"r"(at) : "memory");
+    }
+    return false;
+}
+template <bool CLUSTER, bool PAIR>
 __device__ __forceinline__ bool mbar_keep_looking(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
     long long t0 = 0;
     for (uint32_t spin = 1;; ++spin) {
         if (mbar_look<CLUSTER>(bar, parity)) return true;
         if ((spin & 255u) == 0u || spin == 1u) {
-            if (*abort_flag) return false;
+            if (*abort_flag) return mbar_give_up<PAIR>(abort_flag);
             const long long now = clock64();
             if (t0 == 0) t0 = now;
             else if (now - t0 > WAIT_LIMIT_CYCLES) {
                 *abort_flag = 1u;
                 if (err_word) atomicCAS(err_word, 0, code);
-                return false;
+                return mbar_give_up<PAIR>(abort_flag);
             }
         }
     }
 }
+template <bool CLUSTER, bool PAIR>
 static __device__ __noinline__ bool mbar_missed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    return mbar_keep_looking<false>(bar, parity, abort_flag, err_word, code);
+    return mbar_keep_looking<CLUSTER, PAIR>(bar, parity, abort_flag, err_word, code);
 }
-static __device__ __noinline__ bool mbar_missed_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    return mbar_keep_looking<true>(bar, parity, abort_flag, err_word, code);
-}
-template <bool CALL = true>
+template <bool CALL = true, bool PAIR = false, bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    if (mbar_look<false>(smem_u32(bar), parity)) return true;
-    return CALL ? mbar_missed(smem_u32(bar), parity, abort_flag, err_word, code) : mbar_keep_looking<false>(smem_u32(bar), parity, abort_flag, err_word, code);
+    if (mbar_look<CLUSTER>(smem_u32(bar), parity)) return true;
+    return CALL ? mbar_missed<CLUSTER, PAIR>(smem_u32(bar), parity, abort_flag, err_word, code)
+                : mbar_keep_looking<CLUSTER, PAIR>(smem_u32(bar), parity, abort_flag, err_word, code);
 }
-// on a local barrier that the other CTA of the cluster arrives on too
+// on a local barrier that the other CTA of a pair arrives on too
 template <bool CALL = true>
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    if (mbar_look<true>(smem_u32(bar), parity)) return true;
-    return CALL ? mbar_missed_cluster(smem_u32(bar), parity, abort_flag, err_word, code) : mbar_keep_looking<true>(smem_u32(bar), parity, abort_flag, err_word, code);
+    return mbar_wait<CALL, true, true>(bar, parity, abort_flag, err_word, code);
 }
 
 // ---- TMA ------------------------------------------------------------------------------

@@ -568,7 +568,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             for (uint32_t kc = 0; kc < t.kcn; kc++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, PAIR>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(0, wtr, 0);
@@ -618,6 +618,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                         if ((int32_t)(v - p.wait_rows.epoch) >= 0) break;
                         if (*abort_flag || clock64() - t0 > p.wait_rows.limit_cycles) {
                             *abort_flag = 1u;
+                            ptx::mbar_give_up<PAIR>(abort_flag);
                             if (p.err) atomicCAS(p.err, 0, 110);
                             ok = false;
                             break;
@@ -631,7 +632,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (!ok) break;
             }
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, PAIR>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(1, xtr, 0);
@@ -652,7 +653,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const uint32_t ksteps = p.chunks * (uint32_t)C::SUBS;       // (pair launches do not split K)
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL>(&b_full[bs], bph, abort_flag, p.err, 109));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, PAIR>(&b_full[bs], bph, abort_flag, p.err, 109));
                 if (!ok) break;
                 if (lane == 0) ptx::mbar_arrive_cluster(&b_full[bs], 0u);
                 __syncwarp();
@@ -667,19 +668,19 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         const uint32_t a_lo0 = (ptx::smem_u32(sA) & 0x3FFFFu) >> 4, b_lo0 = (ptx::smem_u32(sB) & 0x3FFFFu) >> 4;
         // One thread, chosen once, walks the loop: chosen anew for every step and with the wait's outcome voted on, a step of four
         // 128 x 128 x 16 MMAs took 328 cycles instead of 257.  Waits that gave up are looked for twice a tile, in the abort flag:
-        // an accumulator that may still be read is not written, and a tile is announced only if every wait of this CTA for its
-        // operands succeeded (a thread whose wait failed has seen or set the flag before its warp arrives anywhere).
+        // an accumulator that may still be read is not written, and a tile is announced only if every wait for its operands succeeded
+        // (a thread whose wait failed has seen or set the flag, in a pair that of both CTAs, before its warp arrives anywhere).
+        // (No way out of the loops for it: a second one costs every launch 0.2 to 1 %.)
         if (ptx::elect_one()) {
             uint32_t st = 0, sph = 0, bst = 0, bsph = 0, it = 0, mtr = 0;
             (void)mtr;
             for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride, it++) {
                 const uint32_t buf = it & 1u;
                 if (PAIR) ptx::mbar_wait_cluster<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
-                else ptx::mbar_wait<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
-                if (*abort_flag) break;
+                else ptx::mbar_wait<C::WAIT_CALL, PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
                 ptx::tc_fence_after_sync();
                 QTRC(2, 200u + it, 0);
-                const uint32_t ksteps = tile_of(idx).kcn * (uint32_t)C::SUBS;
+                const uint32_t ksteps = *abort_flag ? 0u : tile_of(idx).kcn * (uint32_t)C::SUBS;
                 const uint32_t dcol = tmem_base + buf * ACC_STRIDE;
                 for (uint32_t ks = 0; ks < ksteps; ks++) {
                     QTR(2, mtr, 0);
@@ -689,8 +690,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                         ptx::mbar_wait_cluster<C::WAIT_CALL>(&a_full[st], sph, abort_flag, p.err, 104);
                         ptx::mbar_wait_cluster<C::WAIT_CALL>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     } else {
-                        ptx::mbar_wait<C::WAIT_CALL>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait<C::WAIT_CALL>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait<C::WAIT_CALL, PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait<C::WAIT_CALL, PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     }
                     QTR(2, mtr, 2);
                     const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + bst * (p.b_stage_bytes >> 4));
@@ -706,8 +707,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (++st == p.a_stages) { st = 0; sph ^= 1u; }
                     if (++bst == p.b_stages) { bst = 0; bsph ^= 1u; }
                 }
-                if (*abort_flag) break;
-                if (PAIR) ptx::umma_pair_commit(&tm_full[buf]); else ptx::umma_commit(&tm_full[buf]);
+                if (*abort_flag == 0u) { if (PAIR) ptx::umma_pair_commit(&tm_full[buf]); else ptx::umma_commit(&tm_full[buf]); }
                 QTRC(2, 200u + it, 1);
             }
         }
@@ -725,8 +725,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         uint32_t rs = 0, rph = 0, kn = 0;                     // kn: running 64-element step of this CTA
         uint32_t km = 0, own_ph = 0;                          // (kn / 4) % STAGES; phase of the group's next operand stage
         uint32_t own_st = grp;                                // ... and that stage: the group's steps g, g + 3, ... use stages (g + 3 j) % a_stages
-        // After a wait that gave up the warp runs out its tile on whatever the stages hold and leaves.  Its arrivals do no harm in
-        // this CTA, whose issuing thread looks at the abort flag; on the other CTA of a pair, which has a flag of its own, it makes none.
+        // After a wait that gave up the warp runs out its tile on whatever the stages hold and leaves: the issuing thread looks at the
+        // abort flag before it announces a tile.
         for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             // META_WORDS / 2 words of scales and as many of biases per chunk: one group per 64 elements (4 words)
@@ -762,7 +762,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     for (int i = 0; i < MW; i++) meta[i] = meta_next[i];
                     if (kc + 1 < t.kcn) load_meta(kc + 1, meta_next);
                 }
-                ptx::mbar_wait<C::WAIT_CALL>(&raw_full[rs], rph, abort_flag, p.err, 106);
+                ptx::mbar_wait<C::WAIT_CALL, PAIR>(&raw_full[rs], rph, abort_flag, p.err, 106);
                 if (row == 0) QTR(3, (kn >> 2) * 2 + grp, 0);
                 // Only the words a sub-tile needs are loaded, right before it is unpacked: a group handles one or
                 // two of a chunk's four sub-tiles, and short-lived inputs leave the registers to the 32 outputs.
@@ -788,7 +788,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             if (own_st >= p.a_stages) { own_st -= p.a_stages; own_ph ^= 1u; }
                         }
                         else { const uint32_t step = kn + s; as = step % STAGES; aph = (step / STAGES) & 1u; }
-                        ptx::mbar_wait<C::WAIT_CALL>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107);
+                        ptx::mbar_wait<C::WAIT_CALL, PAIR>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107);
                         if (row == 0) QTR(4 + grp, kn + s, 1);
                         uint8_t* dst = sA + as * A_TILE_BYTES + row_off;
 #pragma unroll
@@ -796,10 +796,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             *reinterpret_cast<uint4*>(dst + ((c ^ xr) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
                         ptx::fence_proxy_async_smem();
                         __syncwarp();                      // every lane's stores are fenced; one arrival per warp
-                        if (lane == 0) {
-                            if (!(PAIR && pair_rank == 1u)) ptx::mbar_arrive(&a_full[as]);
-                            else if (*abort_flag == 0u) ptx::mbar_arrive_cluster(&a_full[as], 0u);
-                        }
+                        if (lane == 0) { if (PAIR && pair_rank == 1u) ptx::mbar_arrive_cluster(&a_full[as], 0u); else ptx::mbar_arrive(&a_full[as]); }
                         if (row == 0) QTR(4 + grp, kn + s, 2);
                     }
                 };
@@ -861,9 +858,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (n0 + 64u < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + 128));
                 }
             }
-            // The epilogues below meet at barriers of all 128 threads, so the threads decide together whether the tile is there:
-            // one whose wait gave up, or that sees the abort flag, takes the others with it.
-            const bool got = ptx::mbar_wait<C::WAIT_CALL>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108) && *abort_flag == 0u;
+            // The epilogues below meet at barriers of all 128 threads, so the threads decide together whether the tile is there: one
+            // whose wait gave up takes the others with it.
+            const bool got = ptx::mbar_wait<C::WAIT_CALL, PAIR>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108);
             __syncwarp();                          // (a barrier and tensor memory are taken by whole warps)
             if (!ptx::bar_all(3, 128, got)) { sc_ok = false; break; }
             if (et == 0) QTRC(6, it, 0);
@@ -1050,10 +1047,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     // ---------------- teardown ----------------
     if (p.early) ptx::grid_dependency_wait();      // (long over; the fix-up below is every warp's work)
     ptx::tc_fence_before_sync();
-    __syncthreads();
+    // (all threads decide alike: the other CTA of a pair may be setting the flag just now)
+    const bool gave_up = __syncthreads_or(*abort_flag != 0u) != 0;
     if (threadIdx.x == 0) QTRC(7, 0u, 1);
     QCTA(2);
-    if (*abort_flag) {
+    if (gave_up) {
         // let copies that are still in flight land before the CTA gives its shared memory back
         const long long t0 = clock64();
         while (clock64() - t0 < 4000000LL) { }
@@ -1070,7 +1068,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // Split-K fix-up by every CTA of the tile, each a share of the rows (the barrier orders every CTA's partial tile before it;
         // every thread of every CTA gets here on every path).  One CTA adding alone took 2 to 4.5 us.
         ptx::cluster_sync_all();
-        if (!*abort_flag) {
+        if (!gave_up) {
             const Tile t = decode_tile(blockIdx.x, p);
             const uint32_t i = t.ks * (uint32_t)C::THREADS + threadIdx.x, n = p.k_splits * (uint32_t)C::THREADS;
             switch (p.k_splits) {
@@ -1079,7 +1077,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 default: splitk_fixup<8>(p, t, i, n); break;
             }
         }
-    } else if (p.k_splits > 1 && *last_flag && !*abort_flag) {
+    } else if (p.k_splits > 1 && *last_flag && !gave_up) {
         // Split-K fix-up by the whole CTA: the partial tiles of this output tile are complete (this CTA's arrival
         // completed the count), every warp is idle by now, and 16 float4 loads per thread keep enough bytes in
         // flight to cover the L2 latency in one or two rounds.  The sum runs in split order, so the result does not
