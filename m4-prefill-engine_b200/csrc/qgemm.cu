@@ -89,8 +89,14 @@ template <int FMT> struct Cfg {
     // STAGES: the parity wait on a stage's "empty" barrier is only unambiguous if the waiting group is never
     // two phases ahead, which holds when its own previous wait already implied the phase before.
     static constexpr int DQ_GROUPS = cdc::Codec<FMT>::GROUPS;
-    // Waits that miss go on in a function, except in the format whose unpacking has no registers to save around a call (variable rate, 2048 tokens,
-    // K = N = 4096 92 us with calls, 82 without).
+    // Waits that miss go on in a function, except
+    //   * in the variable-rate format, whose unpacking has no registers to save around a call (2048 tokens, K = N = 4096 92 us with
+    //     calls, 82 without);
+    //   * in the epilogue of launches with a residual, whose ring of loads has none either (Q4_0, 2048 tokens, K = 512, N = 4096
+    //     25.5, 24.5);
+    //   * in the issuing thread of launches without CTA pairs, which unpacking bounds, so that its waits do miss (Q4_K SwiGLU, 129
+    //     tokens, K = 4096, F = 14336 52.9, 49.1; K = N = 512 loses 0.1 us).
+    // (Without calls anywhere: 2048 tokens, K = N = 512 7.8 us instead of 7.0, codebook SwiGLU 500 instead of 445.)
     static constexpr bool WAIT_CALL = FMT != QUANT_VAR_RATE_AFFINE;
     static_assert(DQ_GROUPS >= 1 && DQ_GROUPS <= STAGES, "unpack groups are bounded by the operand ring depth");
     static constexpr int CHUNK = cdc::Codec<FMT>::CHUNK;          // K elements per packed stage
@@ -676,8 +682,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             (void)mtr;
             for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride, it++) {
                 const uint32_t buf = it & 1u;
-                if (PAIR) ptx::mbar_wait_cluster<C::WAIT_CALL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
-                else ptx::mbar_wait<C::WAIT_CALL, PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                if (PAIR) ptx::mbar_wait_cluster<C::WAIT_CALL && PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                else ptx::mbar_wait<C::WAIT_CALL && PAIR, PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
                 ptx::tc_fence_after_sync();
                 QTRC(2, 200u + it, 0);
                 const uint32_t ksteps = *abort_flag ? 0u : tile_of(idx).kcn * (uint32_t)C::SUBS;
@@ -687,11 +693,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     // (no tcgen05 fence here: the stage was written by TMA and by generic stores that were
                     // followed by fence.proxy.async; the mbarrier acquire orders them before the MMA's reads)
                     if (PAIR) {
-                        ptx::mbar_wait_cluster<C::WAIT_CALL>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait_cluster<C::WAIT_CALL>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait_cluster<C::WAIT_CALL && PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait_cluster<C::WAIT_CALL && PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     } else {
-                        ptx::mbar_wait<C::WAIT_CALL, PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait<C::WAIT_CALL, PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait<C::WAIT_CALL && PAIR, PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait<C::WAIT_CALL && PAIR, PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     }
                     QTR(2, mtr, 2);
                     const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + bst * (p.b_stage_bytes >> 4));
@@ -860,7 +866,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             }
             // The epilogues below meet at barriers of all 128 threads, so the threads decide together whether the tile is there: one
             // whose wait gave up takes the others with it.
-            const bool got = ptx::mbar_wait<C::WAIT_CALL, PAIR>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108);
+            const bool got = ptx::mbar_wait<C::WAIT_CALL && !RESID, PAIR>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108);
             __syncwarp();                          // (a barrier and tensor memory are taken by whole warps)
             if (!ptx::bar_all(3, 128, got)) { sc_ok = false; break; }
             if (et == 0) QTRC(6, it, 0);
