@@ -66,6 +66,11 @@ template <int D> struct Cfg {
     // (64-wide, 32 heads, 2048 tokens 31.3 against 33.9).
     static constexpr bool TWO = D == 128;
     static constexpr int THREADS = SOFTMAX_THREADS + (TWO ? 96 : 64);
+    // Batches of 16 accumulator columns that a rescaling has under way together.  128-wide heads that follow the maximum rescale in most
+    // of their 64-key steps: 24 / 8 heads, 2048 tokens behind 8192, 267 us with one, 260 with two.  Four take 162 registers instead of
+    // 130, and no block of the next kernel fits beside this one (32 / 8 heads, 33 tokens behind 500, 9.9 -> 10.7).  64-wide heads have
+    // no registers for a second.
+    static constexpr int RESCALE = D == 128 ? 2 : 1;
     static constexpr int ATOMS = D / 64;
     static constexpr int TILE = ATOMS * ATOM;            // a query tile
     static constexpr int KV_ATOM = BK * 128, KV_TILE = ATOMS * KV_ATOM;      // a K or V tile: [BK keys][64 fp16] twice or once
@@ -464,13 +469,17 @@ attn_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     ptx::tc_fence_after_sync();
                     if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll
-                        for (int c = 0; c < D; c += 16) {
-                            uint32_t v[16];
-                            ptx::tmem_ld_x16(tOg + c, v);
+                        for (int c = 0; c < D; c += 16 * C::RESCALE) {
+                            uint32_t v[C::RESCALE][16];
+#pragma unroll
+                            for (int b = 0; b < C::RESCALE; b++) ptx::tmem_ld_x16(tOg + c + 16 * b, v[b]);
                             ptx::tmem_ld_wait();
 #pragma unroll
-                            for (int j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
-                            ptx::tmem_st_x16(tOg + c, v);
+                            for (int b = 0; b < C::RESCALE; b++) {
+#pragma unroll
+                                for (int j = 0; j < 16; j++) v[b][j] = __float_as_uint(__uint_as_float(v[b][j]) * corr);
+                                ptx::tmem_st_x16(tOg + c + 16 * b, v[b]);
+                            }
                         }
                     }
                 }
@@ -663,11 +672,12 @@ uint32_t sm_count() {
 }
 
 // Query tiles of a CTA and splits of the key range, by estimated time.  The unit is a step of a CTA with two tiles: 64 keys of 128-wide
-// heads, 0.8 us, or 128 keys of 64-wide ones, 1.5 us.  One tile is cheaper a step where the softmax bounds it and cheaper a CTA (FIXED), so one is
-// taken while that leaves no more CTAs waiting for an SM.  Partial results cost a launch (COMBINE) and their way through memory (PER_BYTE).  One CTA
-// runs per SM, so items beyond a whole number of waves cost a wave where all items are equally long (a chunk behind a long cache); a causal triangle
-// from position 0 packs better than that, its sum is what counts there.  The constants: least regret over 320 shapes (1 to 1400 tokens behind
-// 0 to 3000, 1 to 32 kv heads), each timed with every choice: 1.1 % on average for 128-wide heads, 0.9 % for 64-wide.
+// heads or 128 keys of 64-wide ones.  One tile is cheaper a step and a CTA (FIXED), so one is taken while that leaves no more CTAs waiting
+// for an SM.  Partial results cost a launch (COMBINE) and their way through memory (PER_BYTE).  One CTA runs per SM, so items beyond a whole
+// number of waves cost a wave where all items are equally long (a chunk behind a long cache); a causal triangle from position 0 packs
+// better than that, its sum is what counts there.
+// The constants: least regret over 956 shapes (1 to 1500 tokens behind 0 to 8192, 1 to 32 kv heads), each timed with every choice: 1.0 % on
+// average for 64-wide heads, 1.3 for 128-wide ones (0.7 where they follow the maximum exactly).
 }  // namespace
 
 // A lagging reference saves the rescaling of O and puts the result further from 64-bit arithmetic
@@ -679,8 +689,8 @@ static bool lagging(const Args& a) {
 
 Plan make_plan(const Args& a, bool split) {
     struct Model { float step[2], fixed[2], combine, per_byte; };
-    static constexpr Model WIDE = {{1.046f, 1.0f}, {4.43f, 11.4f}, 5.9f, 0.391e-6f}, NARROW = {{1.158f, 1.0f}, {1.09f, 4.26f}, 3.7f, 0.309e-6f};
-    static constexpr Model WIDE_EXACT = {{0.755f, 1.0f}, {2.94f, 2.89f}, 2.6f, 0.27e-6f};         // (heads that follow the maximum exactly: a step 1.06 us)
+    static constexpr Model WIDE = {{0.807f, 1.0f}, {8.42f, 9.28f}, 4.45f, 0.44e-6f}, NARROW = {{0.615f, 1.0f}, {2.08f, 1.93f}, 1.74f, 0.137e-6f};
+    static constexpr Model WIDE_EXACT = {{0.691f, 1.0f}, {2.87f, 2.86f}, 2.77f, 0.215e-6f};       // (heads that follow the maximum exactly)
     const Model& m = a.D == 64 ? NARROW : lagging(a) ? WIDE : WIDE_EXACT;
     const float (&STEP)[2] = m.step, (&FIXED)[2] = m.fixed, COMBINE = m.combine, PER_BYTE = m.per_byte;
     const float sms = (float)sm_count();
