@@ -18,16 +18,14 @@
 //   warp 9           TMA: the Q tiles, then K(0), K(1), V(0), K(2), V(1), ... through one ring of slots.
 //
 //   tensor memory    S0, S1, then P0, P1, O0 and O1 in the last 2 D columns.  A softmax warp frees its scores as soon as they are in
-//                    registers (s_free), and the next step's are computed while it is at the exponentials; P is written, and O rescaled, once the
-//                    PV of the step before has completed (pv_done).  Both fit beside each other with steps of 64 keys for 128-wide heads, of 128 for
-//                    64-wide.  (With P over the front half of its scores, S(it + 1) waits for PV(it): a step of 128 keys then is softmax plus MMAs of one tile,
-//                    1520 + 1600 cycles, while the other tile has its turn.  32 / 8 heads of 128 over 2048 tokens, fp16, 37.7 -> 34.1 us; 32 heads of 64
-//                    37.0 -> 32.1; one token behind 8192 25.2 -> 23.1.)
+//                    registers (s_free), and the next step's are computed while it is at the exponentials; P is written, and O
+//                    rescaled, once the PV of the step before has completed (pv_done).  Both fit beside each other with steps of 64
+//                    keys for 128-wide heads, of 128 for 64-wide.  (With P over the front half of its scores, S(it + 1) waits for
+//                    PV(it): 32 heads of 64 over 2048 tokens 37.0 us instead of 32.1.)
 //
-// What bounds it: 64-wide heads the softmax, two warps a scheduler at 2850 cycles per step of 128 keys and two tiles, of which the exponential
-// unit needs 1536; 128-wide heads the MMAs of 64 keys (1280 cycles, score MMAs of 64 columns read their Q operand from shared memory for 48 cycles each) and
-// the hand-overs between them, 1500.  A thread per MMA chain of one tile (41.9 -> 47.8 us), two threads per row (32.1 -> 33.4), P handed over in halves over
-// its scores (37.9 -> 37.5) were no better.
+// What bounds it: 64-wide heads the softmax, two warps a scheduler at 2850 cycles per step of 128 keys and two tiles, of which the
+// exponential unit needs 1536; 128-wide heads the MMAs of 64 keys (1280 cycles: score MMAs of 64 columns read their Q operand from
+// shared memory for 48 cycles each) and the hand-overs between them, 1500.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, its roles run out on whatever is there, the result is not stored, and it
 // leaves once its copies have landed.
 #include <cuda.h>
@@ -54,16 +52,19 @@ constexpr int MAX_SPLITS = 32;
 
 // keys of a step: as many as tensor memory has columns for beside the two accumulators
 __host__ __device__ constexpr uint32_t step_keys(uint32_t d) { return d == 128u ? 64u : 128u; }
-// Steps after which the reference maximum of a row may lag.  Distance from 64 bits, 32 / 8 heads over 2048 tokens (queries of twice the size; 8 / 2,
-// 256 tokens behind 7936): 2.60e-4 (2.70e-4; 2.92e-4) with a lag from the first step on, 2.56e-4 (2.58e-4; 2.89e-4) after three exact ones, 2.55e-4 (2.54e-4;
-// 2.87e-4) after four; a lag with steps of 128 keys 2.58e-4 (2.64e-4; 2.88e-4), always exact 2.53e-4 (2.31e-4; 2.86e-4).  32 / 8 heads
-// over 2048 tokens, fp16: 35.0 us with none, 36.8 with four, 38.5 with eight.
+// Steps after which the reference maximum of a row may lag.  Distance from 64 bits for 32 / 8 heads over 2048 tokens; the same with queries of
+// twice the size; 8 / 2 heads, 256 tokens behind 7936:
+//   lag from the first step on    2.60e-4  2.70e-4  2.92e-4      35.0 us for the first
+//   after three exact steps       2.56e-4  2.58e-4  2.89e-4
+//   after four                    2.55e-4  2.54e-4  2.87e-4      36.8 us
+//   never                         2.53e-4  2.31e-4  2.86e-4
+// A lag with steps of 128 keys, which results may not be further than: 2.58e-4, 2.64e-4, 2.88e-4.
 constexpr uint32_t EXACT_STEPS = 4;
 template <int D> struct Cfg {
     static constexpr int BK = (int)step_keys(D);
-    // Score and value MMAs from a thread each, so that neither's waits leave the tensor pipe idle (128-wide heads, 32 / 8 over 2048 tokens, fp16 36.4 -> 35.1 us,
-    // 2048 behind 8192 274 -> 265), or from one in an order that keeps the tiles half a step apart where the softmax takes longer than the MMAs
-    // (64-wide, 32 heads, 2048 tokens 31.3 against 33.9).
+    // Score and value MMAs from a thread each, so that neither's waits leave the tensor pipe idle (128-wide heads, 32 / 8 over 2048 tokens
+    // behind 8192, 274 -> 265 us), or from one in an order that keeps the tiles half a step apart where the softmax takes longer than
+    // the MMAs (64-wide, 32 heads, 2048 tokens 31.3 against 33.9).
     static constexpr bool TWO = D == 128;
     static constexpr int THREADS = SOFTMAX_THREADS + (TWO ? 96 : 64);
     // Batches of 16 accumulator columns that a rescaling has under way together.  128-wide heads that follow the maximum rescale in most
@@ -149,9 +150,9 @@ template <int DEG> __device__ __forceinline__ void ex2_poly2(float x0, float x1,
     e0 = __int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23));
     e1 = __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23));
 }
-// How many pairs of eight, by what bounds the step.  64-wide heads, whose softmax follows the maximum exactly (32 heads, 2048 tokens, fp16): none 32.7 us, one
-// 32.2, two 31.3, three 33.4.  128-wide heads with the lag (32 / 8 heads, 2048 tokens): none 35.5, one 35.5, two 35.1, three 33.3; without it (24 / 8
-// heads, 1024 tokens): none 22.0, one 22.5, two 22.7.
+// How many pairs of eight, by what bounds the step: two for 64-wide heads, whose softmax follows the maximum exactly (32 heads, 2048 tokens:
+// none 32.7 us, two 31.3, three 33.4), three for 128-wide heads with the lag (32 / 8 heads: none 35.5, two 35.1, three 33.3), none
+// without it (24 / 8 heads, 1024 tokens: none 22.0, one 22.5).
 template <int D, bool LAG> __device__ constexpr bool poly_pair(int j) {
     return D == 64 ? (j & 3) == 1 : LAG && ((j & 7) == 1 || (j & 7) == 4 || (j & 7) == 6);
 }

@@ -21,9 +21,8 @@
 // Every mbarrier wait is bounded (ptx::mbar_wait).  The cluster barrier is a hardware barrier: every thread of every
 // CTA reaches it on every path, including after a wait has given up.
 //
-// What bounds it: the unpack arithmetic.  Half-precision and logic instructions issue every other cycle, Q4_0 takes 64 and 48 of them for
-// 64 weights and a warp 255 cycles; a 128 x 64 step takes an SM 281 cycles (two CTAs; 325 with 64-element stages and two barriers each), where HBM
-// would need 196.
+// What bounds it: the unpack arithmetic.  Half-precision and logic instructions issue every other cycle, Q4_0 takes 64 and 48 of them
+// for 64 weights and a warp 255 cycles; a 128 x 64 step takes an SM 281 cycles (two CTAs), where HBM would need 196.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -42,15 +41,15 @@ namespace small {
 constexpr int W_TILE = 128;          // weight rows per tile = UMMA M = tensor-memory lanes
 constexpr int KSTEP = 64;            // K elements per sub-tile (4 MMAs of K = 16)
 constexpr int SUB_COLS = KSTEP / 2;  // fp16 pairs: 32 tensor-memory columns per sub-tile
-// Sub-tiles per operand stage: one hand-over for two of them (33 tokens, K = 14336, N = 4096 17.3 -> 15.9 us, N = 14336, K = 4096 19.4 -> 17.7), except
-// where two stages of twice the activations do not fit beside two packed stages (the 272-byte rows)
+// Sub-tiles per operand stage: one hand-over for two of them (33 tokens, K = 14336, N = 4096 17.3 -> 15.9 us), except where two stages
+// of twice the activations do not fit beside two packed stages (the 272-byte rows)
 template <int FMT> struct Ring {
     static constexpr int SPS = cdc::Codec<FMT>::CHUNK == 256 ? 2 : 1, A_COLS = SPS * SUB_COLS;
 };
 constexpr int TMEM_COLS = 256;       // accumulator (T columns), then the A ring
 constexpr int MAX_RAW_STAGES = 6, MAX_STAGES = 7;     // ring depths are chosen per launch (stages_for)
-constexpr int UNPACK_WARPS = 4;      // one per lane quadrant (a second group shares its schedulers, whose pipes one warp of each of the two CTAs
-                                     // keeps 90 % busy: 33 tokens K = 14336 16.2 -> 16.6 us; 128 tokens, N = 14336 24.2 -> 23.5)
+constexpr int UNPACK_WARPS = 4;      // one per lane quadrant (one warp of each of the two CTAs keeps a scheduler's pipes 90 % busy: a second
+                                     // group, 33 tokens, K = 14336 16.2 -> 16.6 us)
 constexpr int THREADS = (UNPACK_WARPS + 3) * 32;    // warps 0-3 unpack + epilogue, then packed-weight copies, activation copies, MMAs
 constexpr int RAW_WARP = UNPACK_WARPS, ACT_WARP = UNPACK_WARPS + 1, MMA_WARP = UNPACK_WARPS + 2;
 constexpr int MAX_T = 128;
@@ -353,9 +352,9 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
         if (Cd::ROW_SCALE) rsc = n < N ? __half2float((swiglu && f >= 64u ? p.row_scale1 : p.row_scale0)[n]) : 0.0f;
         const uint32_t taddr = tmem_base + ((warp * 32u) << 16);
         if (swiglu && p.k_splits == 1u) {
-            // A whole SwiGLU tile: lanes 0 .. 63 hold the gate projections of 64 features, lanes 64 .. 127 the up projections of the same.  16 token
-            // columns at a time change hands through the operand rings, which nothing reads any more, and leave as whole rows of the tile (through the scratch
-            // buffer and back, like split sums: F = 14336, K = 4096, 33 tokens 29.0 us against 27.4, 128 tokens 39.0 against 32.1).
+            // A whole SwiGLU tile: lanes 0 .. 63 hold the gate projections of 64 features, lanes 64 .. 127 the up projections of the same.
+            // 16 token columns at a time change hands through the operand rings, which nothing reads any more, and leave as whole rows
+            // of the tile (F = 14336, K = 4096, 128 tokens 32.1 us; through the scratch buffer and back, like split sums, 39.0).
             float* stage = reinterpret_cast<float*>(sB);                 // [2][16 columns][128 features]
             const uint32_t tok0 = tt * p.T, valid = min(p.T, p.M - tok0), col = threadIdx.x >> 3, f0 = (threadIdx.x & 7u) * 8u, n0 = wt * GATE_ROWS + f0;
             const bool wide = N % 8u == 0u && (reinterpret_cast<uintptr_t>(Y) & 15u) == 0;
@@ -674,12 +673,11 @@ bool small_path_ok(const GemmArgs& a) {
     }
     if (a.K % chunk != 0) return false;
     if (small::g_mode == 2) return true;
-    // More than one token tile unpacks every weight tile more than once, which costs nothing where most of the GPU would idle: where the
-    // persistent kernel (an SM per CTA) has so few tiles that it could split a long K eight ways, this one has its work in twice as
-    // many CTAs -- as long as its clusters of eight are all resident at once (two CTAs an SM, but up to an eighth of the SMs are left over
-    // where a GPC is not whole clusters: 32 of them are, 36 are not), and from 16 tiles on (below, the persistent kernel is as fast).  K = 4096: 160 tokens N = 2048 19.3 -> 12.3 us, 300 tokens N = 1000 19.2 -> 13.7; with 36 clusters, K = 14336, N = 2304,
-    // 129 tokens, it takes 33 us against 24.  Not in the variable-rate format, where unpacking twice does cost (N = 2048, K = 14336:
-    // 1.2 to 1.4 times).  324 of 2592 timed shapes of 129 to 768 tokens come here, none more than 17 % slower than there.
+    // More than one token tile unpacks every weight tile more than once, which costs nothing where most of the GPU would idle: where
+    // the persistent kernel (an SM per CTA) has so few tiles that it could split a long K eight ways, this one has its work in twice
+    // as many CTAs (160 tokens, K = 4096, N = 2048 19.3 -> 12.3 us).  Its clusters of eight have to be resident at once: 32 of them
+    // are, 36 are not (an eighth of the SMs is left over where a GPC is not whole clusters).  Below 16 tiles the persistent kernel
+    // is as fast; in the variable-rate format unpacking twice does cost (1.2 to 1.4 times).
     if (a.M > (uint32_t)small::MAX_T) {
         if (a.W1 || a.n_extra || a.lean || a.format == QUANT_VAR_RATE_AFFINE || a.K / chunk < 16u) return false;
         const uint32_t w_tiles = (a.N + 127u) / 128u, tiles = (a.M + 127u) / 128u * w_tiles, persistent = (a.M + 255u) / 256u * w_tiles;
@@ -690,15 +688,13 @@ bool small_path_ok(const GemmArgs& a) {
     uint32_t tiles = a.W1 ? (a.N + small::GATE_ROWS - 1) / small::GATE_ROWS : (a.N + 127u) / 128u;
     for (uint32_t e = 0; e < a.n_extra && e < 2u; e++) tiles += (a.N_extra[e] + 127u) / 128u;
     if (tiles > 2u * (uint32_t)small::sms()) return false;
-    // SwiGLU tiles that are not split (more of them than SMs) leave straight from the accumulator and are always better here (F = 14336, K = 512: 33 tokens 7.3 us against
-    // 9.6 on the persistent kernel, 128 tokens 9.9 against 13.4; K = 4096: 27.0 against 41.1, 31.8 against 44.5).  Split ones pass through the scratch
-    // buffer, which grows with the tokens: a short K does not make up for it (F = 5632: K = 512, 64 tokens 8.3 against 7.3; K = 1024, 64 tokens 9.4 against
-    // 9.8, 128 tokens 12.6 against 12.2; K = 2048, 128 tokens 16.0 against 17.2), a shorter one does for the variable rate (K = 512, 64 tokens 10.0 against
-    // 10.5, K = 1024, 128 tokens 10.3 against 13.4 with F = 1024, 16.3 against 16.2 with F = 5632).
+    // With more SwiGLU tiles than SMs K is not split, and the tiles leave straight from the accumulator: always better here (F = 14336,
+    // K = 4096: 33 tokens 27.0 us, 41.1 on the persistent kernel; 128 tokens 31.8, 44.5).  Fewer tiles are split (K of one chunk
+    // apart) and pass through the scratch buffer, which grows with the tokens: a short K does not make up for it (F = 5632: K = 512,
+    // 64 tokens 8.3 against 7.3 us; K = 1024, 64 tokens 9.4 against 9.8), in the variable-rate format a shorter one does.
     const uint32_t T = (a.M + 15u) & ~15u;
-    // Grouped launches with a short K for their tokens: the same (512 + 2 x 128 features, K = 512: 64 tokens 7.9 us against 7.0, 128 tokens 9.9
-    // against 8.4; 1024 + 2 x 256, K = 1024: 64 tokens 10.4 against 10.8, 128 tokens 14.3 against 12.5; K = 2048, 128 tokens 14.3 against
-    // 14.9), and earlier in the variable-rate format (K = 512, one token 9.3 against 7.6; K = 1024, 33 tokens 12.6 against 11.3).
+    // Grouped launches with a short K for their tokens: the same (1024 + 2 x 256 features, K = 1024: 64 tokens 10.4 against 10.8 us,
+    // 128 tokens 14.3 against 12.5), and earlier in the variable-rate format (K = 512, one token 9.3 against 7.6).
     if (a.n_extra && (a.format == QUANT_VAR_RATE_AFFINE ? a.K <= 512u || a.K < 22u * T : a.K < 12u * T)) return false;
     if (a.W1 && tiles <= (uint32_t)small::sms() && a.K < (a.format == QUANT_VAR_RATE_AFFINE ? 8u : 10u) * T) return false;
     return true;

@@ -9,8 +9,8 @@
 // (all eight columns alike); the MMA adds up the four lanes of a row.  The eight fragments' worth of K that one row's four lanes
 // do not cover are other warps' chunks; they meet in shared memory.  (128-row tiles of tcgen05 would spend their time on
 // latency here: K = N = 4096 takes 6.1 us here, 7.3 on the few-token kernel.)
-// What bounds it: one dependent chain per warp (packed bytes, 2 x 4 x 130 instructions of unpacking at half rate, 64 MMAs) where the GPU has few warps, the
-// unpack arithmetic where it has many (4096 -> 14336 13.8 us, 33 MB).
+// What bounds it: one dependent chain per warp (packed bytes, 2 x 4 x 130 instructions of unpacking at half rate, 64 MMAs) where the GPU
+// has few warps, the unpack arithmetic where it has many (4096 -> 14336 13.8 us, 33 MB).
 // Weights are those of the tensor-core kernels bit for bit (the same register-level codecs).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -48,9 +48,9 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 __host__ __device__ constexpr uint32_t gv_stride(uint32_t rb) { return rb / 16u % 2u ? rb : rb + 16u; }
 
 // R: rows per lane, 8 R rows per warp and CTA (R == 1 leaves the fragment's rows 8 .. 15 zero).
-// STAGED: a warp's packed bytes pass through shared memory in the order in which they lie.  For chunks of 128 bytes: read by a lane each they lie at the same
-// offset of 32 cache lines, on the same banks (group-64 layout, K = N = 4096 10.4 -> 8.2 us, N = 8192 11.4 -> 9.9, K = 14336, N = 4096 19.1 -> 16.8, K = 2048, N = 5120
-// 9.5 -> 8.2).  Elsewhere it costs what the copy takes (Q4_0 4096 x 4096 6.1 -> 7.1).
+// STAGED: a warp's packed bytes pass through shared memory in the order in which they lie.  For chunks of 128 bytes: read by a lane each
+// they lie at the same offset of 32 cache lines, on the same banks (group-64 layout, K = N = 4096 10.4 -> 8.2 us).  Elsewhere it
+// costs what the copy takes (Q4_0 6.1 -> 7.1).
 template <int FMT, int R, bool STAGED>
 __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams p) {
     using Cd = cdc::Codec<FMT>;
@@ -240,18 +240,18 @@ int gv_sms() {
 
 template <int FMT>
 cudaError_t launch_gemv_fmt(const GemmArgs& a, cudaStream_t stream) {
-    // Two rows per lane fill the fragment; the variable-rate codec's two rows take 179 registers, one row 124 (K = 4096, N = 14336:
-    // 31.3 against 23.5 us), and the codebook's 177 registers cost more than they give (K = 4096, N = 32000: 42.3 against 39.1; K = 5120,
-    // N = 5120 18.3 against 11.6; K = 14336, N = 4096 25.8 against 24.9; the other way round K = N = 4096, 7.4 against 8.9).
+    // Two rows per lane fill the fragment.  The variable-rate codec's two rows take 179 registers, one row 124 (K = 4096, N = 14336:
+    // 31.3 against 23.5 us), and the codebook's 177 cost more than they give (K = N = 5120 18.3 against 11.6).
     constexpr bool ONE = FMT == QUANT_VAR_RATE_AFFINE || FMT == QUANT_EXL3, PLANAR = cdc::Codec<FMT>::META_WORDS != 0;
     if constexpr (ONE) return launch_gemv_rows<FMT, 1>(a, stream);
     else {
-        // Where one row per lane makes less than a warp for each scheduler, the chain of one warp is the time, and half as long (K = 512, N = 512: Q4_0 3.3 -> 3.1 us,
-        // Q4_K 3.9 -> 3.2, ternary 4.0 -> 3.3, group-64 4.1 -> 3.3; K = 4096, N = 512 3.6 -> 3.2, 4.2 -> 3.3, 4.3 -> 3.4, 4.9 -> 3.7).  With 3.5 of them on an SM the
-        // formats that unpack fast lose 3 to 10 % (Q4_0 K = 512, N = 4096 3.4 -> 3.7), the planar ones still gain (2 to 5 %; K = 8192, N = 512 7.1 -> 5.5).
+        // Where one row per lane makes less than a warp for each scheduler, the chain of one warp is the time, and half as long (K = N = 512:
+        // Q4_K 3.9 -> 3.2 us, group-64 4.1 -> 3.3).  With 3.5 of them on an SM the formats that unpack fast lose 3 to 10 % (Q4_0 K = 512,
+        // N = 4096 3.4 -> 3.7), the planar ones still gain 2 to 5 %.
         const uint32_t warps = (a.N + 7u) / 8u * ((a.K / 256u + 3u) / 4u);
         if (a.K / 256u <= 4u * GV_MAX_WARPS && warps <= (PLANAR ? 4u : 3u) * (uint32_t)gv_sms()) return launch_gemv_rows<FMT, 1>(a, stream);
-        if constexpr (PLANAR) { if (a.K >= 1024u) return launch_gemv_rows<FMT, 2, true>(a, stream); }      // (K = 512, N = 5120 4.7 us staged 5.1; K = 1024 5.6 and 5.3)
+        // (N = 5120: K = 512 4.7 us, staged 5.1; K = 1024 5.6 and 5.3)
+        if constexpr (PLANAR) { if (a.K >= 1024u) return launch_gemv_rows<FMT, 2, true>(a, stream); }
         return launch_gemv_rows<FMT, 2>(a, stream);
     }
 }
