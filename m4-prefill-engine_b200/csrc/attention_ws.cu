@@ -677,8 +677,9 @@ uint32_t sm_count() {
 // for an SM.  Partial results cost a launch (COMBINE) and their way through memory (PER_BYTE).  One CTA runs per SM, so items beyond a whole
 // number of waves cost a wave where all items are equally long (a chunk behind a long cache); a causal triangle from position 0 packs
 // better than that, its sum is what counts there.
-// The constants: least regret over 956 shapes (1 to 1500 tokens behind 0 to 8192, 1 to 32 kv heads), each timed with every choice: 1.0 % on
-// average for 64-wide heads, 1.3 for 128-wide ones (0.7 where they follow the maximum exactly).
+// The constants: least regret over 1050 shapes (1 to 1500 tokens behind 0 to 8192, 1 to 32 kv heads), each timed with every choice, with a
+// penalty on choices worse than those of earlier constants: 1.4 % on average for 64-wide heads, 1.3 for 128-wide ones (0.7 where they follow
+// the maximum exactly).
 }  // namespace
 
 // A lagging reference saves the rescaling of O and puts the result further from 64-bit arithmetic
@@ -690,8 +691,8 @@ static bool lagging(const Args& a) {
 
 Plan make_plan(const Args& a, bool split) {
     struct Model { float step[2], fixed[2], combine, per_byte; };
-    static constexpr Model WIDE = {{0.807f, 1.0f}, {8.42f, 9.28f}, 4.45f, 0.44e-6f}, NARROW = {{0.615f, 1.0f}, {2.08f, 1.93f}, 1.74f, 0.137e-6f};
-    static constexpr Model WIDE_EXACT = {{0.691f, 1.0f}, {2.87f, 2.86f}, 2.77f, 0.215e-6f};       // (heads that follow the maximum exactly)
+    static constexpr Model WIDE = {{0.829f, 1.0f}, {5.62f, 6.66f}, 3.86f, 0.387e-6f}, NARROW = {{0.921f, 1.0f}, {1.35f, 3.21f}, 2.63f, 0.349e-6f};
+    static constexpr Model WIDE_EXACT = {{0.686f, 1.0f}, {0.97f, 0.9f}, 2.7f, 0.214e-6f};         // (heads that follow the maximum exactly)
     const Model& m = a.D == 64 ? NARROW : lagging(a) ? WIDE : WIDE_EXACT;
     const float (&STEP)[2] = m.step, (&FIXED)[2] = m.fixed, COMBINE = m.combine, PER_BYTE = m.per_byte;
     const float sms = (float)sm_count();
