@@ -94,10 +94,12 @@ template <int FMT> struct Cfg {
     //     calls, 82 without);
     //   * in the epilogue of launches with a residual, whose ring of loads has none either (Q4_0, 2048 tokens, K = 512, N = 4096
     //     25.5, 24.5);
-    //   * in the issuing thread of launches without CTA pairs, which unpacking bounds, so that its waits do miss (Q4_K SwiGLU, 129
-    //     tokens, K = 4096, F = 14336 52.9, 49.1; K = N = 512 loses 0.1 us).
+    //   * in the issuing thread of Q4_K launches without CTA pairs, which unpacking bounds, so that its waits do miss (SwiGLU, 129
+    //     tokens, K = 4096, F = 14336 52.9, 49.1 us; K = N = 512 loses 0.1; in line for every format, four layers of hidden size 512 over
+    //     301 tokens take 191.8 instead of 189.1).
     // (Without calls anywhere: 2048 tokens, K = N = 512 7.8 us instead of 7.0, codebook SwiGLU 500 instead of 445.)
     static constexpr bool WAIT_CALL = FMT != QUANT_VAR_RATE_AFFINE;
+    template <bool PAIR> static constexpr bool MMA_WAIT_CALL = WAIT_CALL && (PAIR || FMT != QUANT_Q4_K);
     static_assert(DQ_GROUPS >= 1 && DQ_GROUPS <= STAGES, "unpack groups are bounded by the operand ring depth");
     static constexpr int CHUNK = cdc::Codec<FMT>::CHUNK;          // K elements per packed stage
     static constexpr int SUBS = CHUNK / KSTEP;                    // 64-element sub-tiles (MMA steps) per packed stage
@@ -682,8 +684,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             (void)mtr;
             for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride, it++) {
                 const uint32_t buf = it & 1u;
-                if (PAIR) ptx::mbar_wait_cluster<C::WAIT_CALL && PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
-                else ptx::mbar_wait<C::WAIT_CALL && PAIR, PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                if (PAIR) ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                else ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
                 ptx::tc_fence_after_sync();
                 QTRC(2, 200u + it, 0);
                 const uint32_t ksteps = *abort_flag ? 0u : tile_of(idx).kcn * (uint32_t)C::SUBS;
@@ -693,11 +695,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     // (no tcgen05 fence here: the stage was written by TMA and by generic stores that were
                     // followed by fence.proxy.async; the mbarrier acquire orders them before the MMA's reads)
                     if (PAIR) {
-                        ptx::mbar_wait_cluster<C::WAIT_CALL && PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait_cluster<C::WAIT_CALL && PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     } else {
-                        ptx::mbar_wait<C::WAIT_CALL && PAIR, PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait<C::WAIT_CALL && PAIR, PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     }
                     QTR(2, mtr, 2);
                     const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + bst * (p.b_stage_bytes >> 4));
