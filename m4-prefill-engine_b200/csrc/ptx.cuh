@@ -126,9 +126,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
                 : mbar_keep_looking<CLUSTER, PAIR>(smem_u32(bar), parity, abort_flag, err_word, code);
 }
 // on a local barrier that the other CTA of a pair arrives on too
-template <bool CALL = true>
+template <bool CALL = true, bool PAIR = true>
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, int* err_word, int code) {
-    return mbar_wait<CALL, true, true>(bar, parity, abort_flag, err_word, code);
+    return mbar_wait<CALL, PAIR, true>(bar, parity, abort_flag, err_word, code);
 }
 
 // ---- TMA ------------------------------------------------------------------------------

@@ -484,6 +484,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
              const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2, const Params p) {
     using C = Cfg<FMT>;
     using Cd = cdc::Codec<FMT>;
+    // A wait that gives up sets the abort flags of both CTAs of a pair; not in the variable-rate format, where code for that beside every wait costs
+    // 1 to 6 % (512 tokens, K = 2048, N = 5632 27.8 -> 29.7 us): there the odd CTA's unpack warps look at their own flag before they
+    // arrive on the even one, and each CTA runs out by itself.
+    constexpr bool TELL = PAIR && C::WAIT_CALL;
     static_assert(!PAIR || (C::EPI_WARP0 > 14 && C::DQ_WARPS == 12), "the pair kernel uses the idle warp 14 as its relay");
     constexpr int ROW_BYTES = Cd::ROW_BYTES;
     constexpr int RAW_TILE_BYTES = ROW_BYTES * W_TILE;
@@ -576,7 +580,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const Tile t = tile_of(idx);
             for (uint32_t kc = 0; kc < t.kcn; kc++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, PAIR>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, TELL>(&raw_empty[rs], rph ^ 1u, abort_flag, p.err, 101));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(0, wtr, 0);
@@ -626,7 +630,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                         if ((int32_t)(v - p.wait_rows.epoch) >= 0) break;
                         if (*abort_flag || clock64() - t0 > p.wait_rows.limit_cycles) {
                             *abort_flag = 1u;
-                            ptx::mbar_give_up<PAIR>(abort_flag);
+                            ptx::mbar_give_up<TELL>(abort_flag);
                             if (p.err) atomicCAS(p.err, 0, 110);
                             ok = false;
                             break;
@@ -640,7 +644,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 if (!ok) break;
             }
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, PAIR>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, TELL>(&b_empty[bs], bph ^ 1u, abort_flag, p.err, 102));
                 if (!ok) break;
                 if (lane == 0) {
                     QTR(1, xtr, 0);
@@ -661,7 +665,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         for (uint32_t idx = first_tile; ok && idx < total_tiles; idx += tile_stride) {
             const uint32_t ksteps = p.chunks * (uint32_t)C::SUBS;       // (pair launches do not split K)
             for (uint32_t ks = 0; ks < ksteps; ks++) {
-                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, PAIR>(&b_full[bs], bph, abort_flag, p.err, 109));
+                ok = __all_sync(0xffffffffu, ptx::mbar_wait<C::WAIT_CALL, TELL>(&b_full[bs], bph, abort_flag, p.err, 109));
                 if (!ok) break;
                 if (lane == 0) ptx::mbar_arrive_cluster(&b_full[bs], 0u);
                 __syncwarp();
@@ -677,15 +681,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // One thread, chosen once, walks the loop: chosen anew for every step and with the wait's outcome voted on, a step of four
         // 128 x 128 x 16 MMAs took 328 cycles instead of 257.  Waits that gave up are looked for twice a tile, in the abort flag:
         // an accumulator that may still be read is not written, and a tile is announced only if every wait for its operands succeeded
-        // (a thread whose wait failed has seen or set the flag, in a pair that of both CTAs, before its warp arrives anywhere).
+        // (a thread whose wait failed has seen or set the flag, in a pair that of both CTAs, before its warp arrives anywhere; or, in the
+        // odd CTA, see TELL, its warp does not arrive).
         // (No way out of the loops for it: a second one costs every launch 0.2 to 1 %.)
         if (ptx::elect_one()) {
             uint32_t st = 0, sph = 0, bst = 0, bsph = 0, it = 0, mtr = 0;
             (void)mtr;
             for (uint32_t idx = first_tile; idx < total_tiles; idx += tile_stride, it++) {
                 const uint32_t buf = it & 1u;
-                if (PAIR) ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
-                else ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, PAIR>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                if (PAIR) ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>, TELL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
+                else ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, TELL>(&tm_empty[buf], ((it >> 1) & 1u) ^ 1u, abort_flag, p.err, 103);
                 ptx::tc_fence_after_sync();
                 QTRC(2, 200u + it, 0);
                 const uint32_t ksteps = *abort_flag ? 0u : tile_of(idx).kcn * (uint32_t)C::SUBS;
@@ -695,11 +700,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     // (no tcgen05 fence here: the stage was written by TMA and by generic stores that were
                     // followed by fence.proxy.async; the mbarrier acquire orders them before the MMA's reads)
                     if (PAIR) {
-                        ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>, TELL>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait_cluster<C::MMA_WAIT_CALL<PAIR>, TELL>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     } else {
-                        ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, PAIR>(&a_full[st], sph, abort_flag, p.err, 104);
-                        ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, PAIR>(&b_full[bst], bsph, abort_flag, p.err, 105);
+                        ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, TELL>(&a_full[st], sph, abort_flag, p.err, 104);
+                        ptx::mbar_wait<C::MMA_WAIT_CALL<PAIR>, TELL>(&b_full[bst], bsph, abort_flag, p.err, 105);
                     }
                     QTR(2, mtr, 2);
                     const uint64_t bdesc = desc_hi | (uint64_t)(b_lo0 + bst * (p.b_stage_bytes >> 4));
@@ -770,7 +775,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     for (int i = 0; i < MW; i++) meta[i] = meta_next[i];
                     if (kc + 1 < t.kcn) load_meta(kc + 1, meta_next);
                 }
-                ptx::mbar_wait<C::WAIT_CALL, PAIR>(&raw_full[rs], rph, abort_flag, p.err, 106);
+                ptx::mbar_wait<C::WAIT_CALL, TELL>(&raw_full[rs], rph, abort_flag, p.err, 106);
                 if (row == 0) QTR(3, (kn >> 2) * 2 + grp, 0);
                 // Only the words a sub-tile needs are loaded, right before it is unpacked: a group handles one or
                 // two of a chunk's four sub-tiles, and short-lived inputs leave the registers to the 32 outputs.
@@ -796,7 +801,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             if (own_st >= p.a_stages) { own_st -= p.a_stages; own_ph ^= 1u; }
                         }
                         else { const uint32_t step = kn + s; as = step % STAGES; aph = (step / STAGES) & 1u; }
-                        ptx::mbar_wait<C::WAIT_CALL, PAIR>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107);
+                        ptx::mbar_wait<C::WAIT_CALL, TELL>(&a_empty[as], aph ^ 1u, abort_flag, p.err, 107);
                         if (row == 0) QTR(4 + grp, kn + s, 1);
                         uint8_t* dst = sA + as * A_TILE_BYTES + row_off;
 #pragma unroll
@@ -804,7 +809,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             *reinterpret_cast<uint4*>(dst + ((c ^ xr) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
                         ptx::fence_proxy_async_smem();
                         __syncwarp();                      // every lane's stores are fenced; one arrival per warp
-                        if (lane == 0) { if (PAIR && pair_rank == 1u) ptx::mbar_arrive_cluster(&a_full[as], 0u); else ptx::mbar_arrive(&a_full[as]); }
+                        if (lane == 0) {
+                            if (!(PAIR && pair_rank == 1u)) ptx::mbar_arrive(&a_full[as]);
+                            else if (TELL || *abort_flag == 0u) ptx::mbar_arrive_cluster(&a_full[as], 0u);
+                        }
                         if (row == 0) QTR(4 + grp, kn + s, 2);
                     }
                 };
@@ -868,7 +876,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             }
             // The epilogues below meet at barriers of all 128 threads, so the threads decide together whether the tile is there: one
             // whose wait gave up takes the others with it.
-            const bool got = ptx::mbar_wait<C::WAIT_CALL && !RESID, PAIR>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108);
+            const bool got = ptx::mbar_wait<C::WAIT_CALL && !RESID, TELL>(&tm_full[buf], (it >> 1) & 1u, abort_flag, p.err, 108);
             __syncwarp();                          // (a barrier and tensor memory are taken by whole warps)
             if (!ptx::bar_all(3, 128, got)) { sc_ok = false; break; }
             if (et == 0) QTRC(6, it, 0);
