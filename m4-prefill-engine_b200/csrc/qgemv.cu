@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
                     const uint4* src = reinterpret_cast<const uint4*>(p.W + (size_t)n * row_bytes + (size_t)c * RB);
 #pragma unroll
                     for (int i = 0; i < RB / 16; i++) {
-                        const uint4 v = __ldg(src + i);
+                        const uint4 v = ptx::ld(src + i);
                         r[h][4 * i] = v.x; r[h][4 * i + 1] = v.y; r[h][4 * i + 2] = v.z; r[h][4 * i + 3] = v.w;
                     }
                 }
@@ -85,10 +85,10 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
                     const uint8_t* mp = p.meta + ((size_t)n * groups + (size_t)c * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
-                        const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp)), bi = __ldg(reinterpret_cast<const uint2*>(bp));
+                        const uint2 sc = ptx::ld(reinterpret_cast<const uint2*>(mp)), bi = ptx::ld(reinterpret_cast<const uint2*>(bp));
                         meta[h][0] = sc.x; meta[h][1] = sc.y; meta[h][2] = bi.x; meta[h][3] = bi.y;
                     } else {
-                        const uint4 sc = __ldg(reinterpret_cast<const uint4*>(mp)), bi = __ldg(reinterpret_cast<const uint4*>(bp));
+                        const uint4 sc = ptx::ld(reinterpret_cast<const uint4*>(mp)), bi = ptx::ld(reinterpret_cast<const uint4*>(bp));
                         meta[h][0] = sc.x; meta[h][1] = sc.y; meta[h][2] = sc.z; meta[h][3] = sc.w;
                         meta[h][MW - 4] = bi.x; meta[h][MW - 3] = bi.y; meta[h][MW - 2] = bi.z; meta[h][MW - 1] = bi.w;
                     }
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
     if ((reinterpret_cast<uintptr_t>(p.X) & 15u) == 0 && p.x_cols % 8u == 0u) {
         for (uint32_t i = tid; i < p.K / 8u; i += blockDim.x) {
             const uint32_t k = i * 8u, col = p.x_wrap == p.K ? k : k % p.x_wrap;
-            const uint4 v = col < p.x_cols ? __ldg(reinterpret_cast<const uint4*>(p.X + col)) : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 v = col < p.x_cols ? ptx::ld(reinterpret_cast<const uint4*>(p.X + col)) : make_uint4(0u, 0u, 0u, 0u);
             *reinterpret_cast<uint4*>(sx + (k >> 8) * X_CHUNK + (k & 255u) * 2u) = v;
         }
     } else {
