@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const Params p) {
 // of K and then of V.  A thread takes half a record (16 codes, two 16-byte stores); the integer becomes fp16 through the
 // mantissa: 0x6400 | (q + 128) is 1152 + q.
 constexpr uint32_t DEQUANT_THREADS = 256;
-__global__ void __launch_bounds__(DEQUANT_THREADS) dequant_q8_0_kernel(const uint8_t* __restrict__ K, const uint8_t* __restrict__ V, __half* __restrict__ out,
+__global__ void __launch_bounds__(DEQUANT_THREADS) dequant_q8_0_kernel(const uint8_t* K, const uint8_t* V, __half* __restrict__ out,
                                                                        uint32_t heads, size_t total, size_t used) {
     ptx::grid_dependency_wait();
     ptx::launch_dependents();
@@ -623,8 +623,8 @@ __global__ void __launch_bounds__(DEQUANT_THREADS) dequant_q8_0_kernel(const uin
         const uint16_t* c = blk + 1 + ((uint32_t)i & 1u) * 8u;
         uint16_t q[8];
 #pragma unroll
-        for (int e = 0; e < 8; e++) q[e] = __ldg(c + e);
-        const __half2 d2 = __half2half2(__ushort_as_half(__ldg(blk)));
+        for (int e = 0; e < 8; e++) q[e] = ptx::ld(c + e);
+        const __half2 d2 = __half2half2(__ushort_as_half(ptx::ld(blk)));
         uint32_t o[8];
 #pragma unroll
         for (int e = 0; e < 8; e++) {

@@ -55,7 +55,7 @@ __device__ __forceinline__ uint4 scale_row(const uint4& v, const uint4& w, float
     return o;
 }
 
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* __restrict__ X, const __half* __restrict__ W,
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const __half* X, const __half* __restrict__ W,
                                                       __half* __restrict__ Y, uint32_t K, float eps) {
     ptx::grid_dependency_wait();
     ptx::launch_dependents();
@@ -209,7 +209,7 @@ __global__ void add_residual_f16_kernel(const __half* __restrict__ A, const __ha
 // residual), Y = rmsnorm(S) * W.  One CTA of 256 threads per row; a thread reads back only the vectors it wrote itself,
 // and the barrier of the row reduction separates every read of A from the first write of Y, so Y may alias A.
 // Rows must be 16-byte aligned with K a multiple of 8 (checked by the launcher).
-__global__ void __launch_bounds__(256) rmsnorm_add_kernel(const __half* A, const __half* __restrict__ B,
+__global__ void __launch_bounds__(256) rmsnorm_add_kernel(const __half* A, const __half* B,
                                                           const __half* __restrict__ W, __half* __restrict__ S, __half* Y,
                                                           uint32_t K, float eps) {
     ptx::launch_dependents();

@@ -358,7 +358,7 @@ __device__ __forceinline__ void row_epilogue(const Params& p, uint8_t* stage, ui
 #pragma unroll
             for (int h = 0; h < 16 / ROWS; h++) {
                 const uint32_t tok = c0 + jrow + h * ROWS;
-                res[h] = (n_ok && tok < valid) ? __ldg(reinterpret_cast<const uint2*>(p.residual + col_base + (size_t)tok * tok_stride))
+                res[h] = (n_ok && tok < valid) ? ptx::ld(reinterpret_cast<const uint2*>(p.residual + col_base + (size_t)tok * tok_stride))
                                                : make_uint2(0u, 0u);
             }
         }
@@ -753,12 +753,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     const uint8_t* mp = (mat == 0 ? p.meta0 : p.meta1) + ((size_t)n * groups + (size_t)(t.kc0 + kc) * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
-                        const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
-                        const uint2 bi = __ldg(reinterpret_cast<const uint2*>(bp));
+                        const uint2 sc = ptx::ld(reinterpret_cast<const uint2*>(mp));
+                        const uint2 bi = ptx::ld(reinterpret_cast<const uint2*>(bp));
                         m[0] = sc.x; m[1] = sc.y; m[2] = bi.x; m[3] = bi.y;
                     } else {
-                        const uint4 sc = __ldg(reinterpret_cast<const uint4*>(mp));
-                        const uint4 bi = __ldg(reinterpret_cast<const uint4*>(bp));
+                        const uint4 sc = ptx::ld(reinterpret_cast<const uint4*>(mp));
+                        const uint4 bi = ptx::ld(reinterpret_cast<const uint4*>(bp));
                         m[0] = sc.x; m[1] = sc.y; m[2] = sc.z; m[3] = sc.w;
                         m[MW - 4] = bi.x; m[MW - 3] = bi.y; m[MW - 2] = bi.z; m[MW - 1] = bi.w;
                     }
@@ -982,7 +982,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     const uint32_t lim = valid - c0;
                     const __half* src = p.residual + out_base + (size_t)(tok0 + c0) * out_stride;
 #pragma unroll
-                    for (int j = 0; j < 16; j++) dst[j] = (uint32_t)j < lim ? __ldg(src + j * out_stride) : __half(0.0f);
+                    for (int j = 0; j < 16; j++) dst[j] = (uint32_t)j < lim ? __ushort_as_half(ptx::ld(reinterpret_cast<const uint16_t*>(src + j * out_stride))) : __half(0.0f);
                 }
             };
 #pragma unroll
@@ -1244,7 +1244,7 @@ __global__ void qgemm_generic_kernel(int fmt, const __half* X, const uint8_t* W0
 // meets a term of zero, or terms of both signs, and q * s of a term may lie beyond fp16 where the sum over K does not; all of these leave
 // an infinity or a NaN behind.  A thread looks at eight outputs; the warp takes the marked ones together, K strided over its lanes.
 // With nothing to do (reading 284 KB: 129 tokens, N = 1100) the launch costs 1.5 us.
-__global__ void __launch_bounds__(256) repair_nonfinite_kernel(int fmt, const __half* __restrict__ X, const uint8_t* __restrict__ W0, const uint8_t* __restrict__ W1,
+__global__ void __launch_bounds__(256) repair_nonfinite_kernel(int fmt, const __half* X, const uint8_t* W0, const uint8_t* W1,
                                                                const Params p) {
     ptx::launch_dependents();
     ptx::grid_dependency_wait();

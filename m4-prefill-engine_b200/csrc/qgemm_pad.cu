@@ -95,7 +95,7 @@ __device__ __forceinline__ uint16_t scale_term(uint16_t bits, uint32_t t) {
 // where it stands in a term, in a record and in its source row is worked out once.  Source rows are only 2-byte aligned in
 // general; whole units come in with 4-byte loads, shifted by a half word where the row asks for it.
 template <int UNIT>
-__device__ __forceinline__ void pad_plane(const Plane& p, const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, uint32_t terms) {
+__device__ __forceinline__ void pad_plane(const Plane& p, const uint8_t* src, uint8_t* dst, uint32_t terms) {
     constexpr int H = UNIT / 2;                                  // 16-bit fields per unit
     const uint32_t dst_row = p.dst_term * terms;
     const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) * UNIT;
@@ -109,12 +109,12 @@ __device__ __forceinline__ void pad_plane(const Plane& p, const uint8_t* __restr
         const bool odd = (reinterpret_cast<uintptr_t>(s) & 2u) != 0;
         if (whole && !odd) {
 #pragma unroll
-            for (int i = 0; i < H / 2; i++) v[i] = __ldg(reinterpret_cast<const uint32_t*>(s) + i);
+            for (int i = 0; i < H / 2; i++) v[i] = ptx::ld(reinterpret_cast<const uint32_t*>(s) + i);
         } else if (whole && odd && (row > 0u || off > 0u) && (row + 1u < p.rows || off + UNIT + 2u <= p.src_row)) {
             // the words around it also hold the field before and the field behind, both inside the matrix
             uint32_t w[H / 2 + 1];
 #pragma unroll
-            for (int i = 0; i <= H / 2; i++) w[i] = __ldg(reinterpret_cast<const uint32_t*>(s - 2) + i);
+            for (int i = 0; i <= H / 2; i++) w[i] = ptx::ld(reinterpret_cast<const uint32_t*>(s - 2) + i);
 #pragma unroll
             for (int i = 0; i < H / 2; i++) v[i] = __funnelshift_r(w[i], w[i + 1], 16);
         } else {
@@ -146,7 +146,7 @@ __device__ __forceinline__ void pad_plane(const Plane& p, const uint8_t* __restr
     }
 }
 
-__global__ void __launch_bounds__(128) pad_rows_kernel(const uint8_t* __restrict__ w0, const uint8_t* __restrict__ w1, uint8_t* __restrict__ dst, const Planes pl) {
+__global__ void __launch_bounds__(128) pad_rows_kernel(const uint8_t* w0, const uint8_t* w1, uint8_t* dst, const Planes pl) {
     ptx::launch_dependents();              // (the projection touches nothing before its own wait)
     ptx::grid_dependency_wait();           // the scratch may still be read by the launch before
     const uint32_t which = blockIdx.z % pl.n, matrix = blockIdx.z / pl.n;

@@ -288,12 +288,12 @@ qgemm_small_kernel(const __grid_constant__ Maps<MULTI> maps, const Params p) {
                     const uint8_t* mp = (swiglu && row >= 64u ? p.meta1 : p.meta0) + ((size_t)n * groups + (size_t)(kc0 + kc) * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
-                        const uint2 sc = __ldg(reinterpret_cast<const uint2*>(mp));
-                        const uint2 bi = __ldg(reinterpret_cast<const uint2*>(bp));
+                        const uint2 sc = ptx::ld(reinterpret_cast<const uint2*>(mp));
+                        const uint2 bi = ptx::ld(reinterpret_cast<const uint2*>(bp));
                         meta[0] = sc.x; meta[1] = sc.y; meta[2] = bi.x; meta[3] = bi.y;
                     } else {
-                        const uint4 sc = __ldg(reinterpret_cast<const uint4*>(mp));
-                        const uint4 bi = __ldg(reinterpret_cast<const uint4*>(bp));
+                        const uint4 sc = ptx::ld(reinterpret_cast<const uint4*>(mp));
+                        const uint4 bi = ptx::ld(reinterpret_cast<const uint4*>(bp));
                         meta[0] = sc.x; meta[1] = sc.y; meta[2] = sc.z; meta[3] = sc.w;
                         meta[MW - 4] = bi.x; meta[MW - 3] = bi.y; meta[MW - 2] = bi.z; meta[MW - 1] = bi.w;
                     }
