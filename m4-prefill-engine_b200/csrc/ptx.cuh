@@ -294,7 +294,8 @@ __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontr
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Loads of what a kernel in front may have written.  __ldg and const __restrict__ promise that the data does not change while the kernel is
-// there, which began before the one in front had finished: such loads were moved in front of grid_dependency_wait.  These stay behind it.
+// there, which began before the one in front had finished: such loads were moved in front of grid_dependency_wait.  These stay behind it, as
+// ordinary loads do (the wait is a barrier to them).
 __device__ __forceinline__ uint4 ld(const uint4* p) {
     uint4 v;
     asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));

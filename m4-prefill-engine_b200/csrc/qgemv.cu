@@ -8,7 +8,8 @@
 // own pairs are the A fragment as they come out of the codec, and the B fragment is the activation pairs of the same elements
 // (all eight columns alike); the MMA adds up the four lanes of a row.  The eight fragments' worth of K that one row's four lanes
 // do not cover are other warps' chunks; they meet in shared memory.  (128-row tiles of tcgen05 would spend their time on
-// latency here: K = N = 4096 takes 6.1 us here, 7.3 on the few-token kernel.)
+// latency here.  Q4_0 K = N = 4096, launches back to back: 8.1 us.  It was 6.1 while the weights were read in front of the wait for the launch before,
+// which only callers that know who writes them may allow: early.)
 // What bounds it: one dependent chain per warp (packed bytes, 2 x 4 x 130 instructions of unpacking at half rate, 64 MMAs) where the GPU
 // has few warps, the unpack arithmetic where it has many (4096 -> 14336 13.8 us, 33 MB).
 // Weights are those of the tensor-core kernels bit for bit (the same register-level codecs).
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
     ptx::launch_dependents();
     if (!p.early) ptx::grid_dependency_wait();
 
+    // (Ordinary loads, no __ldg: the launch in front may be writing what they read, a padded copy, and __ldg may be moved in front of the wait.)
     // packed bytes (and planar scales) of rows g, g + 8 and chunk c; rows past N repeat the last one, chunks past the end are zero
     uint32_t r[R][RB / 4], meta[R][MW];
     auto load = [&](uint32_t c, uint32_t (&r)[R][RB / 4], uint32_t (&meta)[R][MW]) {
@@ -76,7 +78,7 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
                     const uint4* src = reinterpret_cast<const uint4*>(p.W + (size_t)n * row_bytes + (size_t)c * RB);
 #pragma unroll
                     for (int i = 0; i < RB / 16; i++) {
-                        const uint4 v = ptx::ld(src + i);
+                        const uint4 v = *(src + i);
                         r[h][4 * i] = v.x; r[h][4 * i + 1] = v.y; r[h][4 * i + 2] = v.z; r[h][4 * i + 3] = v.w;
                     }
                 }
@@ -85,10 +87,10 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
                     const uint8_t* mp = p.meta + ((size_t)n * groups + (size_t)c * MW) * 2;
                     const uint8_t* bp = mp + (size_t)p.N * groups * 2;
                     if (MW == 4) {
-                        const uint2 sc = ptx::ld(reinterpret_cast<const uint2*>(mp)), bi = ptx::ld(reinterpret_cast<const uint2*>(bp));
+                        const uint2 sc = *reinterpret_cast<const uint2*>(mp), bi = *reinterpret_cast<const uint2*>(bp);
                         meta[h][0] = sc.x; meta[h][1] = sc.y; meta[h][2] = bi.x; meta[h][3] = bi.y;
                     } else {
-                        const uint4 sc = ptx::ld(reinterpret_cast<const uint4*>(mp)), bi = ptx::ld(reinterpret_cast<const uint4*>(bp));
+                        const uint4 sc = *reinterpret_cast<const uint4*>(mp), bi = *reinterpret_cast<const uint4*>(bp);
                         meta[h][0] = sc.x; meta[h][1] = sc.y; meta[h][2] = sc.z; meta[h][3] = sc.w;
                         meta[h][MW - 4] = bi.x; meta[h][MW - 3] = bi.y; meta[h][MW - 2] = bi.z; meta[h][MW - 1] = bi.w;
                     }
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(GV_MAX_WARPS * 32) qgemv_kernel(const GvParams
     if ((reinterpret_cast<uintptr_t>(p.X) & 15u) == 0 && p.x_cols % 8u == 0u) {
         for (uint32_t i = tid; i < p.K / 8u; i += blockDim.x) {
             const uint32_t k = i * 8u, col = p.x_wrap == p.K ? k : k % p.x_wrap;
-            const uint4 v = col < p.x_cols ? ptx::ld(reinterpret_cast<const uint4*>(p.X + col)) : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 v = col < p.x_cols ? *reinterpret_cast<const uint4*>(p.X + col) : make_uint4(0u, 0u, 0u, 0u);
             *reinterpret_cast<uint4*>(sx + (k >> 8) * X_CHUNK + (k & 255u) * 2u) = v;
         }
     } else {
